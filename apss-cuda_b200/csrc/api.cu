@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "ctx.cuh"
+#include "fold.cuh"
 #include "index.cuh"
 #include "prep.cuh"
 #include "prims.cuh"
@@ -80,6 +81,9 @@ struct TileCostModel {
 constexpr TileCostModel kProbedTail{388.0, 1.6, 0.06};
 constexpr TileCostModel kRarePaired{340.0, 1.84, 0.3};
 constexpr int kMaxModelHead = 8192;
+// Lowest threshold of the folded join: its margins (about 0.01) stay small
+// against t, and empty rows stay below it.
+constexpr float kFoldMinT = 0.05f;
 constexpr double kUnitCostCap = 512.0;  // unit cost cap (tile weights, 1 + tail / mean)
 
 namespace {
@@ -154,7 +158,11 @@ TilePlan plan_tiles(int precision, int64_t n, int64_t d, int64_t nnz,
                     bool forced) {
   TilePlan plan;
   plan.p = fixed_p > 0 ? fixed_p : choose_head_width(precision, n, d, nnz, prefix);
-  if (cands.empty() || n <= 0 || prefix.size() < 2) return plan;
+  if (n <= 0 || prefix.size() < 2) return plan;
+  if (cands.empty()) {
+    plan.tile_ns = tile_ns(precision, plan.p, n, probed_postings(plan.p, nnz, prefix, 0, 0), false);
+    return plan;
+  }
   const double nbk = std::ceil((double)n / kBlockRows);
   const double tiles = nbk * (nbk + 1.0) / 2.0;
   auto cost_at = [&](const RareCandidate* c, int* p_out) {
@@ -184,6 +192,7 @@ TilePlan plan_tiles(int precision, int64_t n, int64_t d, int64_t nnz,
       plan.rare = c;
     }
   }
+  plan.tile_ns = best / tiles;
   return plan;
 }
 
@@ -280,7 +289,46 @@ float elapsed(cudaEvent_t a, cudaEvent_t b) {
   return ms;
 }
 
+// The plan's split of the features, as the probing path counts it: postings
+// left to probe, and the rare features' pairs (without the head's features).
+void plan_split_stats(const TilePlan& plan, int p, int64_t nnz, const std::vector<int64_t>& prefix,
+                      cuapss_stats* stats) {
+  const bool paired = plan.rare.max_count > 0;
+  stats->rare_max_count = plan.rare.max_count;
+  stats->tail_entries = probed_postings(p, nnz, prefix, paired ? plan.rare.rank : 0,
+                                        paired ? plan.rare.postings : 0);
+  if (!paired) return;
+  int64_t pairs = plan.rare.pairs;
+  for (int64_t r = plan.rare.rank; r < std::min<int64_t>(p, (int64_t)prefix.size() - 1); ++r) {
+    const int64_t c = prefix[(size_t)r + 1] - prefix[(size_t)r];
+    pairs -= c * (c - 1) / 2;
+  }
+  stats->explicit_pairs = pairs;
+}
+
 }  // namespace
+
+cuapss_status emit_pairs(cuapss_ctx* ctx, uint64_t* key, uint32_t* idx, const float* sim,
+                         int64_t npairs, int keybits, int rbitsJ, cuapss_pairs* out) {
+  cudaStream_t st = ctx->stream;
+  Workspace& ws = ctx->ws;
+  ST_TRY(radix_sort_pairs(key, idx, npairs, keybits, ws, "out", st));
+  out->count = npairs;
+  if (npairs > out->capacity) return CUAPSS_EOVERFLOW;
+  if (npairs == 0) return CUAPSS_OK;
+  if (out->on_device)
+    return launch_split_pairs(key, idx, sim, npairs, rbitsJ, out->i, out->j, out->sim, st);
+  int32_t *di = nullptr, *dj = nullptr;
+  float* ds = nullptr;
+  ST_TRY(ws.get("out:i", (size_t)npairs, &di));
+  ST_TRY(ws.get("out:j", (size_t)npairs, &dj));
+  ST_TRY(ws.get("out:s", (size_t)npairs, &ds));
+  ST_TRY(launch_split_pairs(key, idx, sim, npairs, rbitsJ, di, dj, ds, st));
+  CU_TRY(cudaMemcpyAsync(out->i, di, sizeof(int32_t) * npairs, cudaMemcpyDeviceToHost, st));
+  CU_TRY(cudaMemcpyAsync(out->j, dj, sizeof(int32_t) * npairs, cudaMemcpyDeviceToHost, st));
+  CU_TRY(cudaMemcpyAsync(out->sim, ds, sizeof(float) * npairs, cudaMemcpyDeviceToHost, st));
+  return CUAPSS_OK;
+}
 
 cuapss_status join_device(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float t,
                           cuapss_pairs* out, cuapss_stats* stats, int shard, int nshards) {
@@ -372,6 +420,46 @@ cuapss_status join_device(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, flo
     po.rare_shard = shard;
     po.rare_nshards = nshards;
   }
+  const double nrm2 = nrm_a * nrm_b;
+  if (nrm2 >= 1.9) return CUAPSS_EINVAL;  // fixed-point tail needs ~unit norms
+  if (d - p > (int64_t)(1u << 20) - 2) return CUAPSS_EINVAL;  // 20-bit tail feature keys
+  if (a.nnz >= (int64_t)UINT32_MAX - 1 || bb.nnz >= (int64_t)UINT32_MAX - 1) return CUAPSS_EINVAL;
+  // The folded join, unless the options fix how the probing path works (a
+  // head width, a rare-feature threshold, no remap) or a shard owns rows by
+  // their place.
+  if (mixed && ctx->opts.head_width == 0 && forced_rare == 0 && ctx->opts.remap && nshards == 1 &&
+      a.n > 0 && bb.n > 0 && t >= kFoldMinT) {
+    nvtx.next("cuapss_run:tiles");
+    cudaEventRecord(ctx->ev[1], st);
+    FoldResult fr;
+    bool done = false;
+    ST_TRY(join_fold(ctx, a, b, t, perm, nrm2, plan.tile_ns, &fr, &done));
+    if (done) {
+      cudaEventRecord(ctx->ev[2], st);
+      nvtx.next("cuapss_run:finalize");
+      const cuapss_status result = emit_pairs(ctx, fr.okey, fr.oidx, fr.osim, fr.npairs,
+                                              fr.rbitsI + fr.rbitsJ, fr.rbitsJ, out);
+      if (result != CUAPSS_OK && result != CUAPSS_EOVERFLOW) return result;
+      cudaEventRecord(ctx->ev[3], st);
+      CU_TRY(cudaStreamSynchronize(st));
+      if (stats) {
+        memset(stats, 0, sizeof(*stats));
+        stats->pairs = fr.npairs;
+        stats->candidates = stats->rescored = fr.ncand;
+        stats->tiles = fr.tiles;
+        stats->head_width = p;
+        plan_split_stats(plan, p, nnz_all, prefix, stats);
+        stats->max_band = fr.max_band;
+        stats->ms_preprocess = elapsed(ctx->ev[0], ctx->ev[1]);
+        stats->ms_tiles = elapsed(ctx->ev[1], ctx->ev[2]);
+        stats->ms_finalize = elapsed(ctx->ev[2], ctx->ev[3]);
+        stats->ms_total = elapsed(ctx->ev[0], ctx->ev[3]);
+        stats->launches = g_launches.load() - launches0;
+      }
+      return result;
+    }
+    nvtx.next("cuapss_run:prepare");
+  }
   const bool head_bound = mixed && head_bound_plan(p, n_all, nnz_all, prefix, plan.rare);
   Side SA, SB;
   SA.rp0 = a.rp;
@@ -397,7 +485,6 @@ cuapss_status join_device(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, flo
   cudaEventRecord(ctx->ev[1], st);
   nvtx.next("cuapss_run:tiles");
   // ---- pair tiles ----
-  const double nrm2 = nrm_a * nrm_b;
   TileArgs ta{};
   ta.headI32 = SA.head32;
   ta.nI = SA.n;
@@ -423,8 +510,6 @@ cuapss_status join_device(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, flo
   ta.p = SA.p;
   ta.self = self ? 1 : 0;
   ta.t = t;
-  if (nrm2 >= 1.9) return CUAPSS_EINVAL;  // fixed-point tail needs ~unit norms
-  if (d - SA.p > (int64_t)(1u << 20) - 2) return CUAPSS_EINVAL;  // 20-bit tail feature keys
   set_tile_margins(ta, nrm2, mixed);
   // ---- units: I block x J range; an I block's J range is cut into chunks
   // of about equal cost, heavier blocks get shorter ranges. CTAs take units
@@ -549,26 +634,9 @@ cuapss_status join_device(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, flo
   CU_TRY(cudaMemcpyAsync(hcnt, ocount, sizeof(hcnt), cudaMemcpyDeviceToHost, st));
   CU_TRY(cudaStreamSynchronize(st));
   const int64_t npairs = (int64_t)hcnt[0];
-  ST_TRY(radix_sort_pairs(okey, oidx, npairs, rbitsI + rbitsJ, ws, "out", st));
-  out->count = npairs;
-  cuapss_status result = CUAPSS_OK;
-  if (npairs > out->capacity) {
-    result = CUAPSS_EOVERFLOW;
-  } else if (npairs > 0) {
-    if (out->on_device) {
-      ST_TRY(launch_split_pairs(okey, oidx, osim, npairs, rbitsJ, out->i, out->j, out->sim, st));
-    } else {
-      int32_t *di = nullptr, *dj = nullptr;
-      float* ds = nullptr;
-      ST_TRY(ws.get("out:i", (size_t)npairs, &di));
-      ST_TRY(ws.get("out:j", (size_t)npairs, &dj));
-      ST_TRY(ws.get("out:s", (size_t)npairs, &ds));
-      ST_TRY(launch_split_pairs(okey, oidx, osim, npairs, rbitsJ, di, dj, ds, st));
-      CU_TRY(cudaMemcpyAsync(out->i, di, sizeof(int32_t) * npairs, cudaMemcpyDeviceToHost, st));
-      CU_TRY(cudaMemcpyAsync(out->j, dj, sizeof(int32_t) * npairs, cudaMemcpyDeviceToHost, st));
-      CU_TRY(cudaMemcpyAsync(out->sim, ds, sizeof(float) * npairs, cudaMemcpyDeviceToHost, st));
-    }
-  }
+  const cuapss_status result =
+      emit_pairs(ctx, okey, oidx, osim, npairs, rbitsI + rbitsJ, rbitsJ, out);
+  if (result != CUAPSS_OK && result != CUAPSS_EOVERFLOW) return result;
   cudaEventRecord(ctx->ev[3], st);
   CU_TRY(cudaStreamSynchronize(st));
   if (stats) {

@@ -47,6 +47,12 @@ cuapss_status join_device(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, flo
                           cuapss_pairs* out, cuapss_stats* stats, int shard = 0,
                           int nshards = 1);
 
+// Sorts npairs unsorted output pairs (keys (i << rbitsJ) | j of keybits bits,
+// payload indexes into sim) and writes them to out: CUAPSS_EOVERFLOW, with
+// the count set, when its capacity is too small.
+cuapss_status emit_pairs(cuapss_ctx* ctx, uint64_t* key, uint32_t* idx, const float* sim,
+                         int64_t npairs, int keybits, int rbitsJ, cuapss_pairs* out);
+
 // Head width used when the options leave it to the library: n rows, nnz
 // non-zeros over d features; prefix[k] = postings of the k most frequent
 // features (rank_count_prefix; may be empty for FP32). Self-joins whose rare
@@ -69,6 +75,7 @@ bool head_bound_plan(int64_t p, int64_t n, int64_t nnz, const std::vector<int64_
 struct TilePlan {
   int p = 0;
   RareCandidate rare;  // max_count 0: no explicit pairs
+  double tile_ns = 0.0;  // modelled SM-nanoseconds of one tile, explicit pairs included
 };
 TilePlan plan_tiles(int precision, int64_t n, int64_t d, int64_t nnz,
                     const std::vector<int64_t>& prefix,

@@ -1,0 +1,547 @@
+// Folded-bound join: row order, folded operands, the choice of widths from
+// sampled rows, and the host side of the join (see fold.cuh).
+#include <cuda_runtime.h>
+#include <cuda_bf16.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+#include <string>
+#include <vector>
+
+#include "fold.cuh"
+#include "prims.cuh"
+
+namespace cuapss {
+
+namespace {
+
+constexpr int kThreads = 256;
+constexpr int kClasses = 16;  // length classes of a side
+// Upper edges of the classes as shares of the sorted rows: finer towards the
+// long rows, whose folded products spread the most.
+constexpr double kClassEdge[kClasses] = {0.125, 0.25, 0.375, 0.5,  0.625, 0.75,  0.8125, 0.875,
+                                         0.92,  0.95, 0.97,  0.98, 0.988, 0.994, 0.998,  1.0};
+// Sides of fewer blocks keep the caller's order and one width, whose
+// candidates are few or, past kSmallMaxCand, make the join fall back.
+constexpr int kSampleMinBlocks = 64;
+constexpr int kSmallLevel = 3;  // K = 256
+constexpr int64_t kSmallMaxCand = 1 << 21;
+
+// Cost model, SM-nanoseconds. A 256 x 128 tile takes kTileChunkNs per 64
+// columns (512 tensor-core cycles) and at least kTileMinNs (its epilogue);
+// a candidate kCandNs + kCandEntryNs per entry of its longer row in verify.
+constexpr double kTileChunkNs = 300.0, kTileMinNs = 330.0;
+constexpr double kCandNs = 60.0, kCandEntryNs = 0.6;
+
+inline unsigned grid_for(int64_t work, int per_block) {
+  const int64_t g = ceil_div(std::max<int64_t>(work, 1), per_block);
+  return (unsigned)std::min<int64_t>(g, 148 * 32);
+}
+
+// ---- row order: by length, in 256 classes of about 1/16 octave -----------
+__global__ void k_len_keys(const int64_t* __restrict__ rp, int64_t n, uint64_t* __restrict__ keys,
+                           uint32_t* __restrict__ vals) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const float len = (float)(rp[i + 1] - rp[i]);
+    keys[i] = (uint64_t)min(255, (int)(16.0f * __log2f(fmaxf(len, 1.0f))));
+    vals[i] = (uint32_t)i;
+  }
+}
+
+__global__ void k_order(const uint32_t* __restrict__ sorted, int64_t n, int64_t slots,
+                        int32_t* __restrict__ rowmap) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < slots;
+       i += (int64_t)gridDim.x * blockDim.x)
+    rowmap[i] = i < n ? (sorted ? (int32_t)sorted[i] : (int32_t)i) : -1;
+}
+
+// ---- sampled rows: up to 128 of each class, evenly spaced ----------------
+struct ClassRows {
+  int64_t row[kClasses + 1];  // first row of each class, n at the end
+};
+
+__global__ void k_sample_rows(const int32_t* __restrict__ rowmap, const int64_t* __restrict__ rp,
+                              ClassRows C, int32_t* __restrict__ sample,
+                              unsigned long long* __restrict__ len_sum) {
+  const int c = blockIdx.x, k = threadIdx.x;
+  const int64_t lo = C.row[c], m = C.row[c + 1] - lo;
+  int32_t r = -1;
+  if (m >= kBlockRows) r = rowmap[lo + (int64_t)k * m / kBlockRows];
+  else if (k < m) r = rowmap[lo + k];
+  sample[c * kBlockRows + k] = r;
+  if (r >= 0) atomicAdd(&len_sum[c], (unsigned long long)(rp[r + 1] - rp[r]));
+}
+
+// ---- folded rows ---------------------------------------------------------
+// One warp per place: the row's entries are summed per column in the warp's
+// shared-memory row (squares in the shared columns) and written as BF16, in
+// the 128-byte-swizzled chunk layout of the tensor cores (prep.cu). Head
+// values are rounded to nearest, which the margin covers; shared columns are
+// rounded up after widening by the largest error their FP32 sums can have
+// (2^-24 per addition), so their products bound the exact ones.
+struct FoldOut {
+  __nv_bfloat16* base[kFoldLevels];  // null: not built
+  int first[kFoldLevels];            // block at offset 0
+};
+
+template <int K>
+__device__ __forceinline__ void fold_row(float* __restrict__ acc, const int32_t* __restrict__ col,
+                                         const float* __restrict__ val,
+                                         const int32_t* __restrict__ perm, int64_t lo, int len,
+                                         __nv_bfloat16* __restrict__ out, int rr, int lane) {
+  constexpr int P = K / 4, M = K - P;
+  for (int k = lane; k < K; k += 32) acc[k] = 0.0f;
+  __syncwarp();
+  for (int e = lane; e < len; e += 32) {
+    const uint32_t r = (uint32_t)perm[col[lo + e]];
+    const float v = val[lo + e];
+    if (r < (uint32_t)P) acc[r] = v;
+    else atomicAdd(&acc[P + (r - P) % (uint32_t)M], v * v);
+  }
+  __syncwarp();
+  const float widen = 1.0f + (float)(len + 16) * 5.9604645e-8f * 1.01f;
+  for (int c8 = lane; c8 < K / 8; c8 += 32) {
+    __nv_bfloat162 w[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float x = acc[c8 * 8 + 2 * q], y = acc[c8 * 8 + 2 * q + 1];
+      if (c8 * 8 < P) {  // P is a multiple of 8
+        w[q].x = __float2bfloat16_rn(x);
+        w[q].y = __float2bfloat16_rn(y);
+      } else {
+        w[q].x = __float2bfloat16_ru(__fsqrt_ru(x) * widen);
+        w[q].y = __float2bfloat16_ru(__fsqrt_ru(y) * widen);
+      }
+    }
+    const int kc = c8 >> 3, c = c8 & 7;
+    uint4 u;
+    memcpy(&u, w, 16);
+    reinterpret_cast<uint4*>(out)[((size_t)kc * kBlockRows + rr) * 8 + (c ^ (rr & 7))] = u;
+  }
+  __syncwarp();
+}
+
+template <int LEV>
+__device__ __forceinline__ void fold_level(uint32_t mask, const FoldOut& O, float* acc,
+                                           const int32_t* col, const float* val,
+                                           const int32_t* perm, int64_t lo, int len, int b, int rr,
+                                           int lane) {
+  if (!((mask >> LEV) & 1u)) return;  // warp-uniform
+  constexpr int K = kFoldK[LEV];
+  fold_row<K>(acc, col, val, perm, lo, len,
+              O.base[LEV] + (size_t)(b - O.first[LEV]) * K * kBlockRows, rr, lane);
+}
+
+// Places [slot0, slot0 + slots) of rowmap; blk_mask[b]: levels of block b
+// (null: mask0 for all). stride: floats of shared memory per warp, the widest
+// level's columns.
+__global__ void __launch_bounds__(kThreads)
+    k_fold_rows(const int32_t* __restrict__ rowmap, int64_t slot0, int64_t slots,
+                const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
+                const float* __restrict__ val, const int32_t* __restrict__ perm,
+                const uint8_t* __restrict__ blk_mask, uint32_t mask0, uint32_t allow, int stride,
+                FoldOut O) {
+  extern __shared__ float fold_sm[];
+  const int lane = threadIdx.x & 31;
+  float* acc = fold_sm + (threadIdx.x >> 5) * stride;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t s = slot0 + ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
+       s < slot0 + slots; s += warps) {
+    const int b = (int)(s / kBlockRows), rr = (int)(s % kBlockRows);
+    const uint32_t mask = (blk_mask ? (uint32_t)blk_mask[b] : mask0) & allow;
+    if (!mask) continue;
+    const int32_t r = rowmap[s];
+    const int64_t lo = r >= 0 ? rp[r] : 0;
+    const int len = r >= 0 ? (int)(rp[r + 1] - lo) : 0;
+    fold_level<0>(mask, O, acc, col, val, perm, lo, len, b, rr, lane);
+    fold_level<1>(mask, O, acc, col, val, perm, lo, len, b, rr, lane);
+    fold_level<2>(mask, O, acc, col, val, perm, lo, len, b, rr, lane);
+    fold_level<3>(mask, O, acc, col, val, perm, lo, len, b, rr, lane);
+    fold_level<4>(mask, O, acc, col, val, perm, lo, len, b, rr, lane);
+    fold_level<5>(mask, O, acc, col, val, perm, lo, len, b, rr, lane);
+    fold_level<6>(mask, O, acc, col, val, perm, lo, len, b, rr, lane);
+    fold_level<7>(mask, O, acc, col, val, perm, lo, len, b, rr, lane);
+  }
+}
+static_assert(kFoldLevels == 8 && kFoldK[7] == 2048, "one fold_level call per level");
+
+constexpr uint32_t kNarrowLevels = 0x3f;  // K <= 512
+
+// Folds the places of [0, slots) with the levels of masks (host, per block;
+// empty: mask0 everywhere) into O.
+cuapss_status fold_side(const DevCsr& x, const int32_t* rowmap, int64_t slots,
+                        const std::vector<uint8_t>& masks, uint32_t mask0, const int32_t* perm,
+                        const FoldOut& O, Workspace& ws, const std::string& tag, cudaStream_t st) {
+  uint8_t* d_mask = nullptr;
+  uint32_t all = mask0;
+  int64_t wide0 = 0, wide1 = slots / kBlockRows;  // blocks with a wide level
+  if (!masks.empty()) {
+    ST_TRY(ws.get(tag + ":mask", masks.size(), &d_mask));
+    CU_TRY(cudaMemcpyAsync(d_mask, masks.data(), masks.size(), cudaMemcpyHostToDevice, st));
+    all = 0;
+    wide0 = (int64_t)masks.size();
+    wide1 = 0;
+    for (size_t b = 0; b < masks.size(); ++b) {
+      all |= masks[b];
+      if (masks[b] & ~kNarrowLevels) {
+        wide0 = std::min(wide0, (int64_t)b);
+        wide1 = (int64_t)b + 1;
+      }
+    }
+  }
+  // the wide levels take 4 times the shared memory: a launch of their own,
+  // over their blocks
+  for (int pass = 0; pass < 2; ++pass) {
+    const uint32_t allow = pass == 0 ? kNarrowLevels : ~kNarrowLevels;
+    if (!(all & allow)) continue;
+    int stride = 0;
+    for (int l = 0; l < kFoldLevels; ++l)
+      if ((all & allow) >> l & 1u) stride = std::max(stride, kFoldK[l]);
+    const int64_t s0 = pass == 0 ? 0 : wide0 * kBlockRows;
+    const int64_t s1 = pass == 0 ? slots : wide1 * kBlockRows;
+    const size_t smem = (size_t)stride * 4 * (kThreads / 32);
+    CU_TRY(cudaFuncSetAttribute(k_fold_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                2048 * 4 * (kThreads / 32)));
+    k_fold_rows<<<grid_for((s1 - s0) * 32, kThreads), kThreads, smem, st>>>(
+        rowmap, s0, s1 - s0, x.rp, x.col, x.val, perm, d_mask, mask0, allow, stride, O);
+    LAUNCH_CHECK();
+  }
+  return CUAPSS_OK;
+}
+
+float fold_eps(int level, double nrm2) {
+  // BF16 rounding of the head columns, FP32 accumulation of K / 16 steps
+  const double head = std::ldexp(1.0, -7) + std::ldexp(1.0, -16);
+  const double acc = (kFoldK[level] / 16.0 + 2.0) * std::ldexp(1.0, -20) * 1.02;
+  return (float)((head + acc) * nrm2 * 1.001 + 1e-6);
+}
+
+struct FoldSide {
+  DevCsr x;
+  int nb = 0;
+  int32_t* rowmap = nullptr;      // [128 nb] place -> caller's row, -1 past n
+  int edge[kClasses + 1] = {};    // first block of each class (even), nb at the end
+  double len[kClasses] = {};      // mean row length of each class
+  int32_t* sample = nullptr;
+  std::vector<uint8_t> masks;     // levels of each block
+  FoldOut out{};
+};
+
+// Row order and class edges.
+cuapss_status order_side(FoldSide& s, bool by_length, Workspace& ws, const std::string& tag,
+                         cudaStream_t st) {
+  s.nb = (int)ceil_div(s.x.n, kBlockRows);
+  const int64_t slots = (int64_t)s.nb * kBlockRows;
+  ST_TRY(ws.get(tag + ":map", (size_t)slots, &s.rowmap));
+  uint32_t* vals = nullptr;
+  if (by_length) {
+    uint64_t* keys = nullptr;
+    ST_TRY(ws.get(tag + ":keys", (size_t)s.x.n, &keys));
+    ST_TRY(ws.get(tag + ":vals", (size_t)s.x.n, &vals));
+    k_len_keys<<<grid_for(s.x.n, kThreads), kThreads, 0, st>>>(s.x.rp, s.x.n, keys, vals);
+    LAUNCH_CHECK();
+    ST_TRY(radix_sort_pairs(keys, vals, s.x.n, 8, ws, tag, st));
+  }
+  k_order<<<grid_for(slots, kThreads), kThreads, 0, st>>>(vals, s.x.n, slots, s.rowmap);
+  LAUNCH_CHECK();
+  for (int c = 0; c < kClasses; ++c)
+    s.edge[c + 1] = c + 1 == kClasses ? s.nb : std::min(s.nb, (int)(kClassEdge[c] * s.nb) & ~1);
+  return CUAPSS_OK;
+}
+
+ClassRows class_rows(const FoldSide& s) {
+  ClassRows c;
+  for (int k = 0; k <= kClasses; ++k)
+    c.row[k] = std::min<int64_t>(s.x.n, (int64_t)s.edge[k] * kBlockRows);
+  return c;
+}
+
+// The width of every pair of classes, from the products of sampled rows.
+// level[a][b] (I class a, J class b; self: b >= a) and the modelled cost of
+// the join in SM-nanoseconds, with its expected candidates.
+cuapss_status plan_levels(cuapss_ctx* ctx, FoldSide& I, FoldSide& J, bool self, float t,
+                          const int32_t* perm, double nrm2, int (*level)[kClasses], double* cost,
+                          double* cands) {
+  Workspace& ws = ctx->ws;
+  cudaStream_t st = ctx->stream;
+  const int64_t slots = (int64_t)kClasses * kBlockRows;
+  const size_t ncnt = (size_t)kFoldLevels * kClasses * kClasses;
+  unsigned long long* stats = nullptr;  // row length sums, then pair counts
+  ST_TRY(ws.get("fold:stats", 2 * kClasses + ncnt / 2, &stats));
+  uint32_t* cnt = reinterpret_cast<uint32_t*>(stats + 2 * kClasses);
+  CU_TRY(cudaMemsetAsync(stats, 0, 8 * (2 * kClasses) + 4 * ncnt, st));
+  FoldTileArgs ta;
+  FoldSide* side[2] = {&I, &J};
+  for (int k = 0; k < (self ? 1 : 2); ++k) {
+    FoldSide& s = *side[k];
+    const std::string tag = k == 0 ? "fold:sI" : "fold:sJ";
+    ST_TRY(ws.get(tag, (size_t)slots, &s.sample));
+    k_sample_rows<<<kClasses, kBlockRows, 0, st>>>(s.rowmap, s.x.rp, class_rows(s), s.sample,
+                                                   stats + k * kClasses);
+    LAUNCH_CHECK();
+    FoldOut o{};
+    for (int l = 0; l < kFoldLevels; ++l)
+      ST_TRY(ws.get(tag + std::to_string(l), (size_t)slots * kFoldK[l], &o.base[l]));
+    ST_TRY(fold_side(s.x, s.sample, slots, {}, (1u << kFoldLevels) - 1u, perm, o, ws, tag, st));
+    for (int l = 0; l < kFoldLevels; ++l) {
+      const uint8_t* p = reinterpret_cast<const uint8_t*>(o.base[l]);
+      if (k == 0) ta.lev[l].I = p;
+      if (k == 1 || self) ta.lev[l].J = p;
+    }
+  }
+  std::vector<int4> units;
+  for (int l = kFoldLevels - 1; l >= 0; --l) {
+    ta.lev[l].nkc = kFoldK[l] / 64;
+    ta.lev[l].eps = fold_eps(l, nrm2);
+    for (int a = 0; a < kClasses; a += 2)
+      for (int b = self ? a : 0; b < kClasses; ++b) units.push_back(make_int4(a, b, b + 1, l));
+  }
+  int4* d_units = nullptr;
+  int* ctl = nullptr;
+  ST_TRY(ws.get("fold:sunits", units.size(), &d_units));
+  ST_TRY(ws.get("fold:sctl", 2, &ctl));
+  CU_TRY(cudaMemcpyAsync(d_units, units.data(), sizeof(int4) * units.size(),
+                         cudaMemcpyHostToDevice, st));
+  CU_TRY(cudaMemsetAsync(ctl, 0, 2 * sizeof(int), st));
+  ta.nI = ta.nJ = slots;
+  ta.nbI = ta.nbJ = kClasses;
+  ta.t = t;
+  ta.units = d_units;
+  ta.nunits = (int)units.size();
+  ta.unit_counter = ctl;
+  ta.err = ctl + 1;
+  ta.class_count = cnt;
+  ST_TRY(launch_tiles_fold(ta, std::min(ctx->sms, (int)units.size()), st, true));
+  std::vector<uint8_t> h(8 * 2 * kClasses + 4 * ncnt);
+  int herr = 0;
+  CU_TRY(cudaMemcpyAsync(h.data(), stats, h.size(), cudaMemcpyDeviceToHost, st));
+  CU_TRY(cudaMemcpyAsync(&herr, ctl + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+  CU_TRY(cudaStreamSynchronize(st));
+  if (herr & kErrTimeout) return CUAPSS_ETIMEOUT;
+  if (herr) return CUAPSS_ECUDA;
+  const unsigned long long* hl = reinterpret_cast<const unsigned long long*>(h.data());
+  const uint32_t* hc = reinterpret_cast<const uint32_t*>(hl + 2 * kClasses);
+  ClassRows cr[2] = {class_rows(I), class_rows(J)};
+  double rows[2][kClasses];
+  for (int k = 0; k < 2; ++k)
+    for (int c = 0; c < kClasses; ++c) {
+      rows[k][c] = (double)std::min<int64_t>(kBlockRows, cr[k].row[c + 1] - cr[k].row[c]);
+      const int src = self ? 0 : k;
+      side[k]->len[c] = rows[k][c] > 0 ? (double)hl[src * kClasses + c] / rows[k][c] : 0.0;
+    }
+  *cost = *cands = 0.0;
+  for (int a = 0; a < kClasses; ++a)
+    for (int b = self ? a : 0; b < kClasses; ++b) {
+      const double sampled = rows[0][a] * rows[1][b] - (self && a == b ? rows[0][a] : 0.0);
+      const double nI = (double)(cr[0].row[a + 1] - cr[0].row[a]);
+      const double nJ = (double)(cr[1].row[b + 1] - cr[1].row[b]);
+      const double pairs = self && a == b ? nI * (nI - 1) / 2 : nI * nJ;
+      double best = 1e300, best_cand = 0.0;
+      level[a][b] = 0;
+      for (int l = 0; l < kFoldLevels; ++l) {
+        double c = (double)hc[((size_t)l * kClasses + a) * kClasses + b];
+        if (self && a == b) c = std::max(0.0, c - rows[0][a]);  // a row with itself
+        // a count of zero is not a share of zero: half a pair
+        const double share = sampled > 0 ? std::max(c, 0.5) / sampled : 0.0;
+        const double tiles = pairs / (2.0 * kBlockRows * kBlockRows);
+        const double tile_ns = std::max(kTileMinNs, kTileChunkNs * (kFoldK[l] / 64));
+        const double cand_ns =
+            kCandNs + kCandEntryNs * std::max(side[0]->len[a], side[1]->len[b]);
+        const double ns = tiles * tile_ns + share * pairs * cand_ns;
+        if (ns < best) {
+          best = ns;
+          best_cand = share * pairs;
+          level[a][b] = l;
+        }
+      }
+      *cost += best;
+      *cands += best_cand;
+    }
+  return CUAPSS_OK;
+}
+
+int class_of(const FoldSide& s, int block) {
+  int c = 0;
+  while (c + 1 < kClasses && block >= s.edge[c + 1]) ++c;
+  return c;
+}
+
+// Allocates and builds the folded levels a side needs.
+cuapss_status build_levels(FoldSide& s, const uint32_t (&need)[kClasses], const int32_t* perm,
+                           Workspace& ws, const std::string& tag, cudaStream_t st) {
+  uint32_t all = 0;
+  for (int c = 0; c < kClasses; ++c)
+    if (s.edge[c + 1] > s.edge[c]) all |= need[c];
+  for (int l = 0; l < kFoldLevels; ++l) {
+    if (!((all >> l) & 1u)) continue;
+    int lo = s.nb, hi = 0;
+    for (int c = 0; c < kClasses; ++c)
+      if (s.edge[c + 1] > s.edge[c] && ((need[c] >> l) & 1u)) {
+        lo = std::min(lo, s.edge[c]);
+        hi = std::max(hi, s.edge[c + 1]);
+      }
+    s.out.first[l] = lo;
+    ST_TRY(ws.get(tag + ":lev" + std::to_string(l), (size_t)(hi - lo) * kFoldK[l] * kBlockRows,
+                  &s.out.base[l]));
+  }
+  s.masks.assign((size_t)s.nb, 0);
+  for (int c = 0; c < kClasses; ++c)
+    for (int b = s.edge[c]; b < s.edge[c + 1]; ++b) s.masks[(size_t)b] = (uint8_t)need[c];
+  return fold_side(s.x, s.rowmap, (int64_t)s.nb * kBlockRows, s.masks, 0, perm, s.out, ws, tag, st);
+}
+
+// Units: windows of J blocks from the long rows down (the costly units
+// first), in each window every I pair against each class's part of it, so
+// that the CTAs running at one time share a window's chunks in L2. Wider
+// folds get proportionally shorter ranges.
+void make_units(const FoldSide& I, const FoldSide& J, bool self, const int (*level)[kClasses],
+                int sms, std::vector<int4>* units, int64_t* tiles) {
+  const int nbJ = J.nb;
+  const double total = self ? 0.25 * nbJ * (nbJ + 2.0) : 0.5 * (double)I.nb * nbJ;
+  const int w = (int)std::max(1.0, std::min(128.0, total / (sms * 16.0)));
+  for (int j1 = nbJ; j1 > 0; j1 -= w) {
+    const int j0 = std::max(0, j1 - w);
+    for (int b = class_of(J, j1 - 1); b >= 0 && J.edge[b + 1] > j0; --b) {
+      const int s0 = std::max(j0, J.edge[b]), s1 = std::min(j1, J.edge[b + 1]);
+      if (s0 >= s1) continue;
+      int a = 0;
+      for (int i = 0; i < (self ? std::min(I.nb, s1) : I.nb); i += 2) {
+        while (i >= I.edge[a + 1]) ++a;
+        const int lv = level[a][b];
+        const int f0 = self ? std::max(s0, i) : s0;
+        const int step = std::max(1, w * 2 / std::max(2, kFoldK[lv] / 64));
+        for (int f = f0; f < s1; f += step)
+          units->push_back(make_int4(i, f, std::min(s1, f + step), lv));
+      }
+    }
+  }
+  *tiles = self ? (int64_t)nbJ * (nbJ + 1) / 2 : (int64_t)I.nb * nbJ;
+}
+
+}  // namespace
+
+cuapss_status join_fold(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float t,
+                        const int32_t* perm, double nrm2, double other_ns, FoldResult* r,
+                        bool* done) {
+  *done = false;
+  const bool self = b == nullptr;
+  Workspace& ws = ctx->ws;
+  cudaStream_t st = ctx->stream;
+  FoldSide SI, SJ;
+  SI.x = a;
+  if (!self) SJ.x = *b;
+  FoldSide& J = self ? SI : SJ;
+  const int64_t nbI = ceil_div(SI.x.n, kBlockRows), nbJ = ceil_div(J.x.n, kBlockRows);
+  const double tiles128 = self ? 0.5 * nbI * (nbI + 1.0) : (double)nbI * nbJ;
+  const bool sampled = tiles128 >= 0.5 * kSampleMinBlocks * kSampleMinBlocks;
+  ST_TRY(order_side(SI, sampled, ws, "fold:I", st));
+  if (!self) ST_TRY(order_side(SJ, sampled, ws, "fold:J", st));
+  int level[kClasses][kClasses];
+  double cands = 0.0;
+  if (sampled) {
+    double cost = 0.0;
+    ST_TRY(plan_levels(ctx, SI, J, self, t, perm, nrm2, level, &cost, &cands));
+    if (cost >= tiles128 * other_ns) return CUAPSS_OK;
+  } else {
+    for (auto& row : level)
+      for (int& l : row) l = kSmallLevel;
+  }
+  // ---- folded operands
+  uint32_t needI[kClasses] = {}, needJ[kClasses] = {};
+  for (int x = 0; x < kClasses; ++x)
+    for (int y = self ? x : 0; y < kClasses; ++y) {
+      if (SI.edge[x + 1] <= SI.edge[x] || J.edge[y + 1] <= J.edge[y]) continue;
+      needI[x] |= 1u << level[x][y];
+      needJ[y] |= 1u << level[x][y];
+    }
+  if (self)
+    for (int c = 0; c < kClasses; ++c) needI[c] |= needJ[c];
+  ST_TRY(build_levels(SI, needI, perm, ws, "fold:I", st));
+  if (!self) ST_TRY(build_levels(SJ, needJ, perm, ws, "fold:J", st));
+  // ---- units
+  std::vector<int4> units;
+  make_units(SI, J, self, level, ctx->sms, &units, &r->tiles);
+  int4* d_units = nullptr;
+  ST_TRY(ws.get("tiles:units", std::max<size_t>(units.size(), 1), &d_units));
+  if (!units.empty())
+    CU_TRY(cudaMemcpyAsync(d_units, units.data(), sizeof(int4) * units.size(),
+                           cudaMemcpyHostToDevice, st));
+  // control words: candidates, pairs found, unit counter, error flags
+  unsigned long long* ctl = nullptr;
+  ST_TRY(ws.get("fold:ctl", 4, &ctl));
+  FoldTileArgs ta;
+  for (int l = 0; l < kFoldLevels; ++l) {
+    FoldLevel& L = ta.lev[l];
+    L.I = reinterpret_cast<const uint8_t*>(SI.out.base[l]);
+    L.J = reinterpret_cast<const uint8_t*>(J.out.base[l]);
+    L.firstI = SI.out.first[l];
+    L.firstJ = J.out.first[l];
+    L.nkc = kFoldK[l] / 64;
+    L.eps = fold_eps(l, nrm2);
+    if (SI.out.base[l]) r->max_band = std::max(r->max_band, (double)L.eps);
+  }
+  ta.nI = SI.x.n;
+  ta.nJ = J.x.n;
+  ta.nbI = SI.nb;
+  ta.nbJ = J.nb;
+  ta.self = self ? 1 : 0;
+  ta.t = t;
+  ta.units = d_units;
+  ta.nunits = (int)units.size();
+  ta.cand_count = ctl;
+  ta.unit_counter = reinterpret_cast<int*>(ctl + 2);
+  ta.err = reinterpret_cast<int*>(ctl + 3);
+  r->rbitsI = std::max(1, bits_for((uint64_t)SI.x.n));
+  r->rbitsJ = std::max(1, bits_for((uint64_t)J.x.n));
+  VerifyArgs va;
+  va.permI = SI.rowmap;
+  va.permJ = J.rowmap;
+  va.rpI = SI.x.rp;
+  va.colI = SI.x.col;
+  va.valI = SI.x.val;
+  va.rpJ = J.x.rp;
+  va.colJ = J.x.col;
+  va.valJ = J.x.val;
+  va.t = t;
+  va.self = ta.self;
+  va.rbits = r->rbitsJ;
+  va.ncand = ctl;
+  va.out_count = ctl + 1;
+  int64_t cap = std::max<int64_t>(sampled ? (int64_t)(1.5 * cands) : 0,
+                                  std::max<int64_t>(1 << 20, SI.x.n + J.x.n));
+  for (int attempt = 0; attempt < 3; ++attempt) {
+    ST_TRY(ws.get("fold:cand", (size_t)cap, &ta.cand));
+    ST_TRY(ws.get("out:key", (size_t)cap, &r->okey));
+    ST_TRY(ws.get("out:idx", (size_t)cap, &r->oidx));
+    ST_TRY(ws.get("out:sim", (size_t)cap, &r->osim));
+    ta.cand_cap = cap;
+    CU_TRY(cudaMemsetAsync(ctl, 0, 4 * sizeof(unsigned long long), st));
+    ST_TRY(launch_tiles_fold(ta, std::max(1, std::min((int)units.size(), ctx->sms)), st, false));
+    va.cand = ta.cand;
+    va.cap = cap;
+    va.out_key = r->okey;
+    va.out_idx = r->oidx;
+    va.out_sim = r->osim;
+    ST_TRY(launch_verify(va, st));
+    unsigned long long h[4] = {0, 0, 0, 0};
+    CU_TRY(cudaMemcpyAsync(h, ctl, sizeof(h), cudaMemcpyDeviceToHost, st));
+    CU_TRY(cudaStreamSynchronize(st));
+    if (h[3] & kErrTimeout) return CUAPSS_ETIMEOUT;
+    if (h[3]) return CUAPSS_ECUDA;
+    r->ncand = (int64_t)h[0];
+    r->npairs = (int64_t)h[1];
+    if (r->ncand <= cap) {
+      *done = true;
+      return CUAPSS_OK;
+    }
+    // an unsampled join that the bound does not prune, or one whose sample
+    // misjudged it: the probing path takes it
+    if (r->ncand > (sampled ? 4 * cap : kSmallMaxCand)) return CUAPSS_OK;
+    cap = r->ncand;
+  }
+  return CUAPSS_OK;
+}
+
+}  // namespace cuapss
