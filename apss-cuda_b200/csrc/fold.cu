@@ -28,11 +28,15 @@ constexpr int kSampleMinBlocks = 64;
 constexpr int kSmallLevel = 3;  // K = 256
 constexpr int64_t kSmallMaxCand = 1 << 21;
 
-// Cost model, SM-nanoseconds. A 256 x 128 tile takes kTileChunkNs per 64
-// columns (512 tensor-core cycles) and at least kTileMinNs (its epilogue);
-// a candidate kCandNs + kCandEntryNs per entry of its longer row in verify.
-constexpr double kTileChunkNs = 300.0, kTileMinNs = 330.0;
-constexpr double kCandNs = 60.0, kCandEntryNs = 0.6;
+// Cost model, SM-nanoseconds, measured on 200,000 and 400,000 rows of the
+// d = 50,000 workload. A 256 x 128 tile whose I chunks stay resident takes
+// kTileNs + kChunkNs per 64 columns (K = 64: 616, 128: 873, 256: 1,446; the
+// tensor cores alone 260 per 64 columns), a streamed one kStreamNs per 64
+// columns (L2 bandwidth; K = 512: 3,212). A candidate takes kCandNs (its
+// listing in the tile kernel, and verify) + kCandEntryNs per entry of its
+// longer row.
+constexpr double kTileNs = 340.0, kChunkNs = 275.0, kStreamNs = 400.0;
+constexpr double kCandNs = 45.0, kCandEntryNs = 0.25;
 
 inline unsigned grid_for(int64_t work, int per_block) {
   const int64_t g = ceil_div(std::max<int64_t>(work, 1), per_block);
@@ -75,99 +79,127 @@ __global__ void k_sample_rows(const int32_t* __restrict__ rowmap, const int64_t*
 }
 
 // ---- folded rows ---------------------------------------------------------
-// One warp per place: the row's entries are summed per column in the warp's
-// shared-memory row (squares in the shared columns) and written as BF16, in
-// the 128-byte-swizzled chunk layout of the tensor cores (prep.cu). Head
-// values are rounded to nearest, which the margin covers; shared columns are
-// rounded up after widening by the largest error their FP32 sums can have
-// (2^-24 per addition), so their products bound the exact ones.
+// A row's entries are summed per column of every wanted width in shared
+// memory (squares in the shared columns), in one pass over the row, and
+// written as BF16 in the 128-byte-swizzled chunk layout of the tensor cores
+// (prep.cu). Head values are rounded to nearest, which the margin covers;
+// shared columns are rounded up after widening by the largest error their
+// FP32 sums can have (2^-24 per addition), so their products bound the exact
+// ones.
 struct FoldOut {
   __nv_bfloat16* base[kFoldLevels];  // null: not built
   int first[kFoldLevels];            // block at offset 0
 };
 
-template <int K>
-__device__ __forceinline__ void fold_row(float* __restrict__ acc, const int32_t* __restrict__ col,
-                                         const float* __restrict__ val,
-                                         const int32_t* __restrict__ perm, int64_t lo, int len,
-                                         __nv_bfloat16* __restrict__ out, int rr, int lane) {
-  constexpr int P = K / 4, M = K - P;
-  for (int k = lane; k < K; k += 32) acc[k] = 0.0f;
-  __syncwarp();
-  for (int e = lane; e < len; e += 32) {
-    const uint32_t r = (uint32_t)perm[col[lo + e]];
-    const float v = val[lo + e];
-    if (r < (uint32_t)P) acc[r] = v;
-    else atomicAdd(&acc[P + (r - P) % (uint32_t)M], v * v);
-  }
-  __syncwarp();
-  const float widen = 1.0f + (float)(len + 16) * 5.9604645e-8f * 1.01f;
-  for (int c8 = lane; c8 < K / 8; c8 += 32) {
+// First accumulator column of level l when the levels of `allow` lie one
+// after another, and their total.
+__host__ __device__ constexpr int fold_offset(uint32_t allow, int l) {
+  constexpr int K[kFoldLevels] = {kFoldK[0], kFoldK[1], kFoldK[2], kFoldK[3],
+                                  kFoldK[4], kFoldK[5], kFoldK[6], kFoldK[7]};
+  int o = 0;
+  for (int k = 0; k < l; ++k)
+    if ((allow >> k) & 1u) o += K[k];
+  return o;
+}
+
+template <int LEV>
+__device__ __forceinline__ void fold_add(uint32_t mask, float* acc, uint32_t allow, uint32_t r,
+                                         float v) {
+  constexpr uint32_t P = kFoldK[LEV] / 4, M = kFoldK[LEV] - P;
+  if (!((mask >> LEV) & 1u)) return;  // uniform over the row's threads
+  float* a = acc + fold_offset(allow, LEV);
+  if (r < P) a[r] = v;
+  else atomicAdd(&a[P + (r - P) % M], v * v);
+}
+
+template <int LEV>
+__device__ __forceinline__ void fold_write(uint32_t mask, const float* acc, uint32_t allow,
+                                           const FoldOut& O, float widen, int b, int rr, int tid,
+                                           int nt) {
+  constexpr int K = kFoldK[LEV], P = K / 4;
+  if (!((mask >> LEV) & 1u)) return;
+  const float* a = acc + fold_offset(allow, LEV);
+  uint4* out = reinterpret_cast<uint4*>(O.base[LEV] + (size_t)(b - O.first[LEV]) * K * kBlockRows);
+  for (int c8 = tid; c8 < K / 8; c8 += nt) {
     __nv_bfloat162 w[4];
+    const float4 x = reinterpret_cast<const float4*>(a)[2 * c8];
+    const float4 y = reinterpret_cast<const float4*>(a)[2 * c8 + 1];
+    const float f[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const float x = acc[c8 * 8 + 2 * q], y = acc[c8 * 8 + 2 * q + 1];
       if (c8 * 8 < P) {  // P is a multiple of 8
-        w[q].x = __float2bfloat16_rn(x);
-        w[q].y = __float2bfloat16_rn(y);
+        w[q].x = __float2bfloat16_rn(f[2 * q]);
+        w[q].y = __float2bfloat16_rn(f[2 * q + 1]);
       } else {
-        w[q].x = __float2bfloat16_ru(__fsqrt_ru(x) * widen);
-        w[q].y = __float2bfloat16_ru(__fsqrt_ru(y) * widen);
+        w[q].x = __float2bfloat16_ru(__fsqrt_ru(f[2 * q]) * widen);
+        w[q].y = __float2bfloat16_ru(__fsqrt_ru(f[2 * q + 1]) * widen);
       }
     }
     const int kc = c8 >> 3, c = c8 & 7;
     uint4 u;
     memcpy(&u, w, 16);
-    reinterpret_cast<uint4*>(out)[((size_t)kc * kBlockRows + rr) * 8 + (c ^ (rr & 7))] = u;
+    out[((size_t)kc * kBlockRows + rr) * 8 + (c ^ (rr & 7))] = u;
   }
-  __syncwarp();
 }
 
-template <int LEV>
-__device__ __forceinline__ void fold_level(uint32_t mask, const FoldOut& O, float* acc,
-                                           const int32_t* col, const float* val,
-                                           const int32_t* perm, int64_t lo, int len, int b, int rr,
-                                           int lane) {
-  if (!((mask >> LEV) & 1u)) return;  // warp-uniform
-  constexpr int K = kFoldK[LEV];
-  fold_row<K>(acc, col, val, perm, lo, len,
-              O.base[LEV] + (size_t)(b - O.first[LEV]) * K * kBlockRows, rr, lane);
-}
+// GROUP threads per row (a warp, or the whole CTA for long rows). Blocks
+// [b0, b1) of rowmap; blk_mask[b]: levels of block b (null: mask0 for all);
+// only blocks whose levels are all in `allow` (wide: some level is not
+// narrow) are taken. Shared memory: the columns of `allow` per row.
+constexpr uint32_t kNarrowLevels = 0x3f;  // K <= 512
 
-// Places [slot0, slot0 + slots) of rowmap; blk_mask[b]: levels of block b
-// (null: mask0 for all). stride: floats of shared memory per warp, the widest
-// level's columns.
+template <int GROUP>
 __global__ void __launch_bounds__(kThreads)
-    k_fold_rows(const int32_t* __restrict__ rowmap, int64_t slot0, int64_t slots,
+    k_fold_rows(const int32_t* __restrict__ rowmap, int64_t slot0, int64_t slot1,
                 const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
                 const float* __restrict__ val, const int32_t* __restrict__ perm,
-                const uint8_t* __restrict__ blk_mask, uint32_t mask0, uint32_t allow, int stride,
+                const uint8_t* __restrict__ blk_mask, uint32_t mask0, uint32_t allow, bool wide,
                 FoldOut O) {
-  extern __shared__ float fold_sm[];
-  const int lane = threadIdx.x & 31;
-  float* acc = fold_sm + (threadIdx.x >> 5) * stride;
-  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t s = slot0 + ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
-       s < slot0 + slots; s += warps) {
+  extern __shared__ __align__(16) float fold_sm[];
+  constexpr int kGroups = kThreads / GROUP;
+  const int tid = threadIdx.x % GROUP;
+  const int ncol = fold_offset(allow, kFoldLevels);
+  float* acc = fold_sm + (threadIdx.x / GROUP) * ncol;
+  for (int64_t s = slot0 + (int64_t)blockIdx.x * kGroups + threadIdx.x / GROUP; s < slot1;
+       s += (int64_t)gridDim.x * kGroups) {
     const int b = (int)(s / kBlockRows), rr = (int)(s % kBlockRows);
-    const uint32_t mask = (blk_mask ? (uint32_t)blk_mask[b] : mask0) & allow;
-    if (!mask) continue;
+    const uint32_t mask = blk_mask ? (uint32_t)blk_mask[b] : mask0;
+    if (mask == 0 || ((mask & ~kNarrowLevels) != 0) != wide) continue;  // same for all of GROUP
     const int32_t r = rowmap[s];
     const int64_t lo = r >= 0 ? rp[r] : 0;
     const int len = r >= 0 ? (int)(rp[r + 1] - lo) : 0;
-    fold_level<0>(mask, O, acc, col, val, perm, lo, len, b, rr, lane);
-    fold_level<1>(mask, O, acc, col, val, perm, lo, len, b, rr, lane);
-    fold_level<2>(mask, O, acc, col, val, perm, lo, len, b, rr, lane);
-    fold_level<3>(mask, O, acc, col, val, perm, lo, len, b, rr, lane);
-    fold_level<4>(mask, O, acc, col, val, perm, lo, len, b, rr, lane);
-    fold_level<5>(mask, O, acc, col, val, perm, lo, len, b, rr, lane);
-    fold_level<6>(mask, O, acc, col, val, perm, lo, len, b, rr, lane);
-    fold_level<7>(mask, O, acc, col, val, perm, lo, len, b, rr, lane);
+    for (int k = tid; k < ncol / 4; k += GROUP)
+      reinterpret_cast<float4*>(acc)[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (GROUP == 32) __syncwarp();
+    else __syncthreads();
+    for (int e = tid; e < len; e += GROUP) {
+      const uint32_t f = (uint32_t)perm[col[lo + e]];
+      const float v = val[lo + e];
+      fold_add<0>(mask, acc, allow, f, v);
+      fold_add<1>(mask, acc, allow, f, v);
+      fold_add<2>(mask, acc, allow, f, v);
+      fold_add<3>(mask, acc, allow, f, v);
+      fold_add<4>(mask, acc, allow, f, v);
+      fold_add<5>(mask, acc, allow, f, v);
+      fold_add<6>(mask, acc, allow, f, v);
+      fold_add<7>(mask, acc, allow, f, v);
+    }
+    if (GROUP == 32) __syncwarp();
+    else __syncthreads();
+    const float widen = 1.0f + (float)(len + 16) * 5.9604645e-8f * 1.01f;
+    fold_write<0>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
+    fold_write<1>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
+    fold_write<2>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
+    fold_write<3>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
+    fold_write<4>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
+    fold_write<5>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
+    fold_write<6>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
+    fold_write<7>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
+    if (GROUP == 32) __syncwarp();
+    else __syncthreads();
   }
 }
-static_assert(kFoldLevels == 8 && kFoldK[7] == 2048, "one fold_level call per level");
-
-constexpr uint32_t kNarrowLevels = 0x3f;  // K <= 512
+static_assert(kFoldLevels == 8, "one fold_add / fold_write call per level");
 
 // Folds the places of [0, slots) with the levels of masks (host, per block;
 // empty: mask0 everywhere) into O.
@@ -175,37 +207,37 @@ cuapss_status fold_side(const DevCsr& x, const int32_t* rowmap, int64_t slots,
                         const std::vector<uint8_t>& masks, uint32_t mask0, const int32_t* perm,
                         const FoldOut& O, Workspace& ws, const std::string& tag, cudaStream_t st) {
   uint8_t* d_mask = nullptr;
-  uint32_t all = mask0;
-  int64_t wide0 = 0, wide1 = slots / kBlockRows;  // blocks with a wide level
-  if (!masks.empty()) {
+  // levels, and blocks, with and without a wide level
+  uint32_t all[2] = {0, 0};
+  int64_t b0[2] = {0, 0}, b1[2] = {0, 0};
+  if (masks.empty()) {
+    const int w = (mask0 & ~kNarrowLevels) ? 1 : 0;
+    all[w] = mask0;
+    b1[w] = slots / kBlockRows;
+  } else {
     ST_TRY(ws.get(tag + ":mask", masks.size(), &d_mask));
     CU_TRY(cudaMemcpyAsync(d_mask, masks.data(), masks.size(), cudaMemcpyHostToDevice, st));
-    all = 0;
-    wide0 = (int64_t)masks.size();
-    wide1 = 0;
     for (size_t b = 0; b < masks.size(); ++b) {
-      all |= masks[b];
-      if (masks[b] & ~kNarrowLevels) {
-        wide0 = std::min(wide0, (int64_t)b);
-        wide1 = (int64_t)b + 1;
-      }
+      const int w = (masks[b] & ~kNarrowLevels) ? 1 : 0;
+      if (!all[w]) b0[w] = (int64_t)b;
+      all[w] |= masks[b];
+      if (masks[b]) b1[w] = (int64_t)b + 1;
     }
   }
-  // the wide levels take 4 times the shared memory: a launch of their own,
-  // over their blocks
-  for (int pass = 0; pass < 2; ++pass) {
-    const uint32_t allow = pass == 0 ? kNarrowLevels : ~kNarrowLevels;
-    if (!(all & allow)) continue;
-    int stride = 0;
-    for (int l = 0; l < kFoldLevels; ++l)
-      if ((all & allow) >> l & 1u) stride = std::max(stride, kFoldK[l]);
-    const int64_t s0 = pass == 0 ? 0 : wide0 * kBlockRows;
-    const int64_t s1 = pass == 0 ? slots : wide1 * kBlockRows;
-    const size_t smem = (size_t)stride * 4 * (kThreads / 32);
-    CU_TRY(cudaFuncSetAttribute(k_fold_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                2048 * 4 * (kThreads / 32)));
-    k_fold_rows<<<grid_for((s1 - s0) * 32, kThreads), kThreads, smem, st>>>(
-        rowmap, s0, s1 - s0, x.rp, x.col, x.val, perm, d_mask, mask0, allow, stride, O);
+  if (all[0]) {  // a warp per row
+    const size_t smem = (size_t)fold_offset(all[0], kFoldLevels) * 4 * (kThreads / 32);
+    CU_TRY(cudaFuncSetAttribute(k_fold_rows<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                fold_offset(kNarrowLevels, kFoldLevels) * 4 * (kThreads / 32)));
+    k_fold_rows<32><<<grid_for((b1[0] - b0[0]) * kBlockRows, kThreads / 32), kThreads, smem, st>>>(
+        rowmap, b0[0] * kBlockRows, b1[0] * kBlockRows, x.rp, x.col, x.val, perm, d_mask, mask0,
+        all[0], false, O);
+    LAUNCH_CHECK();
+  }
+  if (all[1]) {  // blocks of long rows (and the samples): a CTA per row
+    const size_t smem = (size_t)fold_offset(all[1], kFoldLevels) * 4;
+    k_fold_rows<kThreads><<<grid_for((b1[1] - b0[1]) * kBlockRows, 1), kThreads, smem, st>>>(
+        rowmap, b0[1] * kBlockRows, b1[1] * kBlockRows, x.rp, x.col, x.val, perm, d_mask, mask0,
+        all[1], true, O);
     LAUNCH_CHECK();
   }
   return CUAPSS_OK;
@@ -346,7 +378,9 @@ cuapss_status plan_levels(cuapss_ctx* ctx, FoldSide& I, FoldSide& J, bool self, 
         // a count of zero is not a share of zero: half a pair
         const double share = sampled > 0 ? std::max(c, 0.5) / sampled : 0.0;
         const double tiles = pairs / (2.0 * kBlockRows * kBlockRows);
-        const double tile_ns = std::max(kTileMinNs, kTileChunkNs * (kFoldK[l] / 64));
+        const int nkc = kFoldK[l] / 64;
+        const double tile_ns =
+            kFoldK[l] <= kFoldResidentK ? kTileNs + kChunkNs * nkc : kStreamNs * nkc;
         const double cand_ns =
             kCandNs + kCandEntryNs * std::max(side[0]->len[a], side[1]->len[b]);
         const double ns = tiles * tile_ns + share * pairs * cand_ns;
@@ -412,8 +446,12 @@ void make_units(const FoldSide& I, const FoldSide& J, bool self, const int (*lev
         const int lv = level[a][b];
         const int f0 = self ? std::max(s0, i) : s0;
         const int step = std::max(1, w * 2 / std::max(2, kFoldK[lv] / 64));
-        for (int f = f0; f < s1; f += step)
-          units->push_back(make_int4(i, f, std::min(s1, f + step), lv));
+        for (int f = f0; f < s1; f += step) {
+          const int len = std::min(s1 - f, step);
+          // spread the starts of neighbouring units over the range
+          const int turn = (int)(((int64_t)(units->size() % 16) * len) / 16);
+          units->push_back(make_int4(i, f, f + len, lv | turn << 8));
+        }
       }
     }
   }
@@ -468,7 +506,8 @@ cuapss_status join_fold(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float
   if (!units.empty())
     CU_TRY(cudaMemcpyAsync(d_units, units.data(), sizeof(int4) * units.size(),
                            cudaMemcpyHostToDevice, st));
-  // control words: candidates, pairs found, unit counter, error flags
+  // control words: candidates, pairs found, {unit counter, verify's group
+  // counter}, error flags
   unsigned long long* ctl = nullptr;
   ST_TRY(ws.get("fold:ctl", 4, &ctl));
   FoldTileArgs ta;
@@ -509,6 +548,7 @@ cuapss_status join_fold(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float
   va.rbits = r->rbitsJ;
   va.ncand = ctl;
   va.out_count = ctl + 1;
+  va.work = reinterpret_cast<unsigned*>(ctl + 2) + 1;
   int64_t cap = std::max<int64_t>(sampled ? (int64_t)(1.5 * cands) : 0,
                                   std::max<int64_t>(1 << 20, SI.x.n + J.x.n));
   for (int attempt = 0; attempt < 3; ++attempt) {

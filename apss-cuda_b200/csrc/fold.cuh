@@ -28,6 +28,7 @@ namespace cuapss {
 
 constexpr int kFoldLevels = 8;
 constexpr int kFoldK[kFoldLevels] = {64, 128, 192, 256, 384, 512, 1024, 2048};
+constexpr int kFoldResidentK = 256;  // widest fold whose I chunks stay in shared memory
 constexpr int kFoldTileBytes = kBlockRows * 64 * 2;  // a 64-column BF16 chunk of a row block
 
 // One folded width of the two operands of a launch: [blocks][K / 64] chunks
@@ -47,7 +48,8 @@ struct FoldTileArgs {
   int self = 0;                  // pairs i < j of one side only
   float t = 0.f;
   const float* t_row = nullptr;  // threshold of each J row, or null: t
-  const int4* units = nullptr;   // {I block (even), J0, J1, level}: blocks I, I + 1 x [J0, J1)
+  const int4* units = nullptr;   // {I block (even), J0, J1, level | turn << 8}: blocks I, I + 1 x
+                                 // [J0, J1), from J0 + turn on (0 <= turn < J1 - J0)
   int nunits = 0;
   int* unit_counter = nullptr;
   uint64_t* cand = nullptr;      // {I row << 32 | J row}
@@ -65,6 +67,7 @@ struct VerifyArgs {
   const uint64_t* cand = nullptr;
   const unsigned long long* ncand = nullptr;  // device count (may exceed cap: nothing is done)
   int64_t cap = 0;
+  unsigned* work = nullptr;  // group counter, zero at the launch
   const int32_t* permI = nullptr;  // place -> caller's row, or null: identity
   const int32_t* permJ = nullptr;
   const int64_t* rpI = nullptr;

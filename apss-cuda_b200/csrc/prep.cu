@@ -1231,7 +1231,8 @@ cuapss_status rare_feature_candidates(const int32_t* counts, int64_t d, Workspac
   unsigned long long* out = nullptr;
   ST_TRY(ws.get("rare:stats", 3 * kRareCands, &out));
   CU_TRY(cudaMemsetAsync(out, 0, sizeof(unsigned long long) * 3 * kRareCands, st));
-  k_rare_stats<<<grid_for(d, kThreads), kThreads, 0, st>>>(counts, d, out);
+  // few CTAs: every warp ends with 24 atomics on the same words
+  k_rare_stats<<<std::min(grid_for(d, kThreads), 148u), kThreads, 0, st>>>(counts, d, out);
   LAUNCH_CHECK();
   unsigned long long h[3 * kRareCands];
   CU_TRY(cudaMemcpyAsync(h, out, sizeof(h), cudaMemcpyDeviceToHost, st));

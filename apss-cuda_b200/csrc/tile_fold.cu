@@ -7,12 +7,16 @@
 //   warp 0     producer: bulk copies of pre-swizzled 16 KB chunks (128 rows x
 //              64 columns) into two rings, A (J chunks, kA slots of 16 KB)
 //              and B (I chunk pairs, kB slots of 32 KB);
-//   warp 1     MMA: one thread issues M = 128, N = 256, K = 16 MMAs into two
-//              alternating accumulators of 256 columns (all of tensor memory);
-//   warps 2-9  epilogue, two per lane quarter (one I block each): the largest
-//              of each J row's 128 products is compared with t - eps; only
-//              32-column groups in which some row reaches it are read again
-//              and listed.
+//   warps 1-2  MMA: each issues the M = 128, N = 256, K = 16 MMAs of every
+//              other tile into its own accumulator of 256 columns (the two
+//              are all of tensor memory);
+//   warps 4-11 epilogue, two per lane quarter (one I block each): the largest
+//              of each J row's 32 products of a column group is compared with
+//              t - eps; only groups in which some row reaches it are looked
+//              at column by column. Candidates gather in shared memory, so
+//              that a warp reserves list room once per about 100 of them (one
+//              reservation per group cost a global atomic's latency each:
+//              n = 400,000, 3 candidates a tile, 29 ms).
 // Up to kB chunks wide (K <= 256), the I chunks stay in the B ring for a
 // whole unit (I pair x range of J blocks) and only 16 KB per 64 columns move
 // from L2 per tile, a third of what streaming both operands takes; wider
@@ -36,16 +40,20 @@ namespace cuapss {
 
 namespace {
 
-constexpr int kA = 6;                     // A ring slots (16 KB)
-constexpr int kB = 4;                     // B ring slots (32 KB)
+constexpr int kA = 5;                     // A ring slots (16 KB)
+constexpr int kB = kFoldResidentK / 64;   // B ring slots (32 KB)
+constexpr int kMW = 2;                    // MMA warps, one per accumulator
 constexpr int kEW = 8;                    // epilogue warps
-constexpr int kThreads = 64 + 32 * kEW;
+constexpr int kFirstEpi = 4;              // a multiple of 4: lane quarter = warp % 4
+constexpr int kThreads = 32 * (kFirstEpi + kEW);
 constexpr int kRing = 4;                  // unit ids published ahead
-constexpr int kReaders = 1 + kEW;         // MMA thread + epilogue warps
+constexpr int kReaders = kMW + kEW;       // MMA and epilogue warps
 constexpr int kColsPerAcc = 256;
-constexpr int kBars = 2 * kA + 2 * kB + 4 + 2 * kRing + 1;
+constexpr int kBars = (kMW + 1) * kA + 2 * kB + 4 + 2 * kRing + kMW;
 constexpr size_t kOffB = (size_t)kA * kFoldTileBytes;
-constexpr size_t kOffBar = kOffB + (size_t)kB * 2 * kFoldTileBytes;
+constexpr int kHits = 128;                 // candidates an epilogue warp holds back
+constexpr size_t kOffHits = kOffB + (size_t)kB * 2 * kFoldTileBytes;
+constexpr size_t kOffBar = kOffHits + (size_t)kEW * kHits * 8;
 constexpr size_t kOffUnit = kOffBar + (size_t)kBars * 8;
 constexpr size_t kOffMisc = kOffUnit + (size_t)kRing * 16 + 8;
 constexpr size_t kSmem = kOffMisc + 16 + 1024;  // + alignment slack
@@ -78,8 +86,49 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volati
   return live && got;
 }
 
+// Appends a warp's held candidates to the list: one reservation for up to
+// kHits of them.
+__device__ __forceinline__ void flush_hits(const FoldTileArgs& A, const uint64_t* hits, int n,
+                                           int lane) {
+  __syncwarp();
+  unsigned long long w = 0;
+  if (lane == 0) w = atomicAdd(A.cand_count, (unsigned long long)n);
+  w = __shfl_sync(0xffffffffu, w, 0);
+  for (int k = lane; k < n; k += 32)
+    if ((int64_t)w + k < A.cand_cap) A.cand[w + k] = hits[k];
+  __syncwarp();
+}
+
+// One 32-column group of a J row's products: the columns at or above thr
+// (bit j of the result), c of which exist (and, in a self-join, lie below
+// the J row).
+__device__ __forceinline__ uint32_t passing(const uint32_t (&v)[32], float thr, int c) {
+  uint32_t pass = 0;
+#pragma unroll
+  for (int j = 0; j < 32; ++j) pass |= (uint32_t)(__uint_as_float(v[j]) >= thr) << j;
+  return pass & (c >= 32 ? 0xffffffffu : c <= 0 ? 0u : (1u << c) - 1u);
+}
+
+__device__ __forceinline__ float largest(const uint32_t (&v)[32]) {
+  float m[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) m[q] = __uint_as_float(v[q]);
+#pragma unroll
+  for (int j = 4; j < 32; ++j) m[j & 3] = fmaxf(m[j & 3], __uint_as_float(v[j]));
+  return fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
+}
+
+// A unit {I, J0, J1, level | turn << 8}: its tiles in order, starting at
+// J0 + turn and wrapping around, so that CTAs that work on the same J blocks
+// at one time do not read the same L2 lines in step.
 struct Unit {
-  int I, J0, J1, lev;
+  int I, J0, len, lev, turn;
+  __device__ explicit Unit(const int4& u)
+      : I(u.x), J0(u.y), len(u.z - u.y), lev(u.w & 0xff), turn(u.w >> 8) {}
+  __device__ int J(int k) const {
+    const int j = k + turn;
+    return J0 + (j < len ? j : j - len);
+  }
 };
 
 template <bool COUNT>
@@ -88,8 +137,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<size_t>(smem_raw) + 1023) & ~(size_t)1023);
   uint8_t* ringA = base;
   uint8_t* ringB = base + kOffB;
+  // afull[m kA + s]: slot s was filled for MMA warp m. A barrier per warp and
+  // slot, so that a warp sees every phase of the barriers it waits on (a wait
+  // on a phase's parity is only meaningful one phase ahead).
   uint64_t* afull = reinterpret_cast<uint64_t*>(base + kOffBar);
-  uint64_t* aempty = afull + kA;
+  uint64_t* aempty = afull + kMW * kA;
   uint64_t* bfull = aempty + kA;
   uint64_t* bempty = bfull + kB;
   uint64_t* tfull = bempty + kB;
@@ -102,13 +154,11 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
   volatile int* abort = reinterpret_cast<volatile int*>(base + kOffMisc + 8);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kA; ++s) {
-      mbar_init(&afull[s], 1);
-      mbar_init(&aempty[s], 1);
-    }
+    for (int s = 0; s < kMW * kA; ++s) mbar_init(&afull[s], 1);
+    for (int s = 0; s < kA; ++s) mbar_init(&aempty[s], 1);
     for (int s = 0; s < kB; ++s) {
       mbar_init(&bfull[s], 1);
-      mbar_init(&bempty[s], 1);
+      mbar_init(&bempty[s], kMW);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tfull[b], 1);
@@ -118,7 +168,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
       mbar_init(&ufull[k], 1);
       mbar_init(&uempty[k], kReaders);
     }
-    mbar_init(drain, 1);
+    for (int m = 0; m < kMW; ++m) mbar_init(&drain[m], 1);
     *abort = 0;
     fence_mbar_init();
   }
@@ -135,7 +185,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
   if (warp == 0) {
     // ------------------------------------------------------------ producer
     if (lane == 0) {
-      uint32_t ia = 0, ib = 0;  // chunks copied into each ring
+      uint32_t ia = 0, ib = 0, tt = 0;  // chunks copied into each ring, tiles
+      uint32_t use[kMW] = {};           // bit s: parity of the next use of afull[m kA + s]
+      uint32_t last_m = 0, last_p = 0;  // bit s: warp and parity of slot s's last use
       bool ok = true;
       for (uint32_t k = 0; ok; ++k) {
         const uint32_t slot = k % kRing, ur = k / kRing;
@@ -147,14 +199,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
         uring[slot] = u;
         mbar_arrive(&ufull[slot]);
         if (u >= A.nunits) break;
-        const int4 U = A.units[u];
-        const FoldLevel& L = A.lev[U.w];
+        const Unit U(A.units[u]);
+        const FoldLevel& L = A.lev[U.lev];
         const int nkc = L.nkc;
-        const int wI = U.x + 1 < A.nbI ? 2 : 1;
-        const uint8_t* srcI = L.I + (size_t)(U.x - L.firstI) * nkc * kFoldTileBytes;
-        const uint8_t* srcJ = L.J + (size_t)(U.y - L.firstJ) * nkc * kFoldTileBytes;
-        for (int J = U.y; ok && J < U.z; ++J) {
-          const bool loadB = J == U.y || nkc > kB;
+        const int wI = U.I + 1 < A.nbI ? 2 : 1;
+        const uint8_t* srcI = L.I + (size_t)(U.I - L.firstI) * nkc * kFoldTileBytes;
+        for (int j = 0; ok && j < U.len; ++j, ++tt) {
+          const uint32_t m = tt & 1u;
+          const bool loadB = j == 0 || nkc > kB;
+          const uint8_t* srcJ = L.J + (size_t)(U.J(j) - L.firstJ) * nkc * kFoldTileBytes;
           for (int kc = 0; kc < nkc; ++kc) {
             if (loadB) {
               const uint32_t s = ib % kB, r = ib / kB;
@@ -177,88 +230,109 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
               ok = false;
               break;
             }
-            mbar_arrive_expect_tx(&afull[s], kFoldTileBytes);
-            bulk_g2s(ringA + (size_t)s * kFoldTileBytes, srcJ, kFoldTileBytes, &afull[s]);
+            mbar_arrive_expect_tx(&afull[m * kA + s], kFoldTileBytes);
+            bulk_g2s(ringA + (size_t)s * kFoldTileBytes, srcJ, kFoldTileBytes, &afull[m * kA + s]);
             srcJ += kFoldTileBytes;
+            const uint32_t bit = 1u << s, p = (m ? use[1] : use[0]) & bit;
+            last_m = (last_m & ~bit) | (m << s);
+            last_p = (last_p & ~bit) | p;
+            if (m) use[1] ^= bit;
+            else use[0] ^= bit;
             ++ia;
           }
         }
       }
       // the last copies issued must have landed before the CTA exits
-      for (uint32_t q = ia > kA ? ia - kA : 0u; q < ia; ++q)
-        if (!mbar_wait(&afull[q % kA], (q / kA) & 1u)) give_up(A.err, abort);
+      for (uint32_t s = 0; s < (ia < kA ? ia : (uint32_t)kA); ++s)
+        if (!mbar_wait(&afull[((last_m >> s) & 1u) * kA + s], (last_p >> s) & 1u))
+          give_up(A.err, abort);
       for (uint32_t q = ib > kB ? ib - kB : 0u; q < ib; ++q)
         if (!mbar_wait(&bfull[q % kB], (q / kB) & 1u)) give_up(A.err, abort);
     }
     __syncwarp();
-  } else if (warp == 1) {
+  } else if (warp <= kMW) {
     // ----------------------------------------------------------------- MMA
-    if (lane == 0) {
-      const uint32_t idesc1 = umma_idesc_bf16(kBlockRows, kBlockRows);
-      const uint32_t idesc2 = umma_idesc_bf16(kBlockRows, 2 * kBlockRows);
-      uint32_t ia = 0, ib = 0, tt = 0;  // A chunks used, first B chunk of the unit or tile, tiles
-      bool ok = true;
-      for (uint32_t k = 0; ok; ++k) {
-        const uint32_t slot = k % kRing, ur = k / kRing;
-        if (!wait_abort(&ufull[slot], ur & 1u, abort)) {
-          give_up(A.err, abort);
-          break;
-        }
-        const int u = uring[slot];
-        mbar_arrive(&uempty[slot]);
-        if (u >= A.nunits) break;
-        const int4 U = A.units[u];
-        const int nkc = A.lev[U.w].nkc;
-        const bool stream = nkc > kB;
-        const uint32_t idesc = U.x + 1 < A.nbI ? idesc2 : idesc1;
-        for (int J = U.y; ok && J < U.z; ++J, ++tt) {
-          const bool first = J == U.y, last = J + 1 == U.z;
-          const uint32_t b = tt & 1u, tr = tt >> 1;
-          if (!wait_abort(&tempty[b], (tr & 1u) ^ 1u, abort)) {
-            give_up(A.err, abort);
-            ok = false;
-            break;
-          }
+    // MMA warp m takes tiles m, m + 2, ... (accumulator m): issuing a tile's
+    // MMAs, waits and commits takes its warp about as long as the tensor
+    // cores take to run them, so two warps keep the cores fed
+    const uint32_t m = (uint32_t)warp - 1u;
+    const uint32_t idesc1 = umma_idesc_bf16(kBlockRows, kBlockRows);
+    const uint32_t idesc2 = umma_idesc_bf16(kBlockRows, 2 * kBlockRows);
+    const uint64_t descA = umma_desc_sw128(ringA), descB = umma_desc_sw128(ringB);
+    const uint32_t d = tmem + m * (uint32_t)kColsPerAcc;
+    uint32_t ia = 0;          // A chunks before this tile
+    uint32_t ib = 0, tt = 0;  // first B chunk of the unit or tile, tiles
+    uint32_t use = 0;         // bit s: parity of the next use of afull[m kA + s]
+    bool live = true;
+    for (uint32_t k = 0;; ++k) {
+      const uint32_t slot = k % kRing, ur = k / kRing;
+      live = warp_wait(&ufull[slot], ur & 1u, abort, A.err, live);
+      const int u = live ? uring[slot] : A.nunits;
+      __syncwarp();
+      if (live && lane == 0) mbar_arrive(&uempty[slot]);
+      if (u >= A.nunits) break;
+      const Unit U(A.units[u]);
+      const int nkc = A.lev[U.lev].nkc;
+      const bool stream = nkc > kB;
+      const uint32_t idesc = U.I + 1 < A.nbI ? idesc2 : idesc1;
+      bool fresh = true;  // this warp has not waited for the unit's B chunks
+      for (int j = 0; live && j < U.len; ++j, ++tt, ia += (uint32_t)nkc) {
+        if ((tt & 1u) == m) {
+          // the warp's last tile of the unit releases the resident B chunks
+          const bool last = j + kMW >= U.len;
+          live = warp_wait(&tempty[m], ((tt >> 1) & 1u) ^ 1u, abort, A.err, live);
           tc_fence_after();
-          const uint32_t d = tmem + b * (uint32_t)kColsPerAcc;
-          for (int kc = 0; kc < nkc; ++kc, ++ia) {
-            const uint32_t qb = ib + (uint32_t)kc;
-            if ((first || stream) && !wait_abort(&bfull[qb % kB], (qb / kB) & 1u, abort)) {
-              give_up(A.err, abort);
-              ok = false;
-              break;
-            }
-            const uint32_t s = ia % kA;
-            if (!wait_abort(&afull[s], (ia / kA) & 1u, abort)) {
-              give_up(A.err, abort);
-              ok = false;
-              break;
-            }
+          for (int kc = 0; kc < nkc; ++kc) {
+            const uint32_t qb = ib + (uint32_t)kc, sb = qb % kB, sa = (ia + (uint32_t)kc) % kA;
+            if (fresh || stream)
+              live = warp_wait(&bfull[sb], (qb / kB) & 1u, abort, A.err, live);
+            live = warp_wait(&afull[m * kA + sa], (use >> sa) & 1u, abort, A.err, live);
+            if (!live) break;
+            use ^= 1u << sa;
             tc_fence_after();
-            const uint64_t ad = umma_desc_sw128(ringA + (size_t)s * kFoldTileBytes);
-            const uint64_t bd = umma_desc_sw128(ringB + (size_t)(qb % kB) * 2 * kFoldTileBytes);
+            const uint64_t ad = descA + (uint64_t)(sa * (kFoldTileBytes >> 4));
+            const uint64_t bd = descB + (uint64_t)(sb * (2 * kFoldTileBytes >> 4));
 #pragma unroll
             for (int q = 0; q < 4; ++q)
-              umma_bf16(d, ad + 2u * q, bd + 2u * q, idesc, (kc | q) != 0 ? 1u : 0u);
-            umma_commit(&aempty[s]);
-            if (last || stream) umma_commit(&bempty[qb % kB]);
+              umma_bf16_warp(d, ad + 2u * q, bd + 2u * q, idesc, (kc | q) != 0 ? 1u : 0u);
+            umma_commit_warp(&aempty[sa]);
+            if (last || stream) umma_commit_warp(&bempty[sb]);
           }
-          if (ok) umma_commit(&tfull[b]);
-          if (stream || last) ib += (uint32_t)nkc;
+          if (live) umma_commit_warp(&tfull[m]);
+          fresh = false;
+        } else if (stream) {
+          // the other warp's tile: its B chunks are seen and released here too
+          for (int kc = 0; kc < nkc; ++kc) {
+            const uint32_t qb = ib + (uint32_t)kc, sb = qb % kB;
+            live = warp_wait(&bfull[sb], (qb / kB) & 1u, abort, A.err, live);
+            if (live && lane == 0) mbar_arrive(&bempty[sb]);
+          }
         }
+        if (stream) ib += (uint32_t)nkc;
       }
-      // every MMA issued must be complete before tensor memory is freed
-      if (ia > 0) {
-        umma_commit(drain);
-        if (!mbar_wait(drain, 0)) give_up(A.err, abort);
+      if (!stream) {
+        // a unit of one tile leaves the other warp without one: it sees and
+        // releases the B chunks all the same
+        if (fresh)
+          for (int kc = 0; kc < nkc; ++kc) {
+            const uint32_t qb = ib + (uint32_t)kc, sb = qb % kB;
+            live = warp_wait(&bfull[sb], (qb / kB) & 1u, abort, A.err, live);
+            if (live && lane == 0) mbar_arrive(&bempty[sb]);
+          }
+        ib += (uint32_t)nkc;
       }
     }
+    // every MMA issued must be complete before tensor memory is freed
+    umma_commit_warp(&drain[m]);
+    if (!mbar_wait(&drain[m], 0) && lane == 0) give_up(A.err, abort);
     __syncwarp();
-  } else {
+  } else if (warp >= kFirstEpi) {
     // ------------------------------------------------------------- epilogue
     const int q4 = warp & 3;             // tensor-memory lane quarter of this warp
-    const int half = (warp - 2) >> 2;    // which of the two I blocks
+    const int half = (warp - kFirstEpi) >> 2;    // which of the two I blocks
     const int row = 32 * q4 + lane;      // J row within its block
+    uint64_t* hits = reinterpret_cast<uint64_t*>(base + kOffHits) + (warp - kFirstEpi) * kHits;
+    int held = 0;                        // candidates in hits, the same in every lane
     bool live = true;
     uint32_t tt = 0;
     for (uint32_t k = 0;; ++k) {
@@ -268,13 +342,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
       __syncwarp();
       if (live && lane == 0) mbar_arrive(&uempty[slot]);
       if (u >= A.nunits) break;
-      const int4 U = A.units[u];
-      const float eps = A.lev[U.w].eps;
-      const int I = U.x + half;
+      const Unit U(A.units[u]);
+      const float eps = A.lev[U.lev].eps;
+      const int I = U.I + half;
       const bool haveI = I < A.nbI;
       const int64_t irow0 = (int64_t)I * kBlockRows;
       const int icols = haveI ? (int)(A.nI - irow0 < kBlockRows ? A.nI - irow0 : kBlockRows) : 0;
-      for (int J = U.y; J < U.z; ++J, ++tt) {
+      for (int j = 0; j < U.len; ++j, ++tt) {
+        const int J = U.J(j);
         const uint32_t b = tt & 1u, tr = tt >> 1;
         const int64_t jrow = (int64_t)J * kBlockRows + row;
         const float thr =
@@ -284,59 +359,44 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
         const uint32_t taddr = tmem + b * (uint32_t)kColsPerAcc + (uint32_t)(half * kBlockRows) +
                                ((uint32_t)(32 * q4) << 16);
         if (live && haveI && !(A.self && J < I)) {
-          uint32_t hit = 0;  // bit g: some product of columns 32 g .. reaches thr
+          // columns that exist; for a self-join only those below the J row
+          int64_t lim = icols;
+          if (A.self && jrow - irow0 < lim) lim = jrow - irow0;
+          uint32_t v[2][32];
+          tmem_ld32_async(taddr, v[0]);
+          uint32_t n_hits = 0;
 #pragma unroll
           for (int g = 0; g < 4; ++g) {
-            uint32_t v[32];
-            tmem_ld32(taddr + 32u * g, v);
-            float m = __uint_as_float(v[0]);
-#pragma unroll
-            for (int j = 1; j < 32; ++j) m = fmaxf(m, __uint_as_float(v[j]));
-            hit |= (uint32_t)(m >= thr) << g;
-          }
-          const uint32_t any = __reduce_or_sync(0xffffffffu, hit);
-          if (any) {
-            uint32_t n_hits = 0;
-            const int64_t jmin = A.self ? jrow : INT64_MAX;  // self: I rows below the J row only
-            for (int g = 0; g < 4; ++g) {
-              if (!((any >> g) & 1u)) continue;  // warp-uniform
-              uint32_t v[32];
-              tmem_ld32(taddr + 32u * g, v);
-              uint32_t pass = 0;
-#pragma unroll
-              for (int j = 0; j < 32; ++j)
-                pass |= (uint32_t)(__uint_as_float(v[j]) >= thr) << j;
-              // columns that exist, and for a self-join lie below the J row
-              int64_t lim = jmin - irow0 < (int64_t)icols ? jmin - irow0 : (int64_t)icols;
-              const int c = (int)lim - 32 * g;
-              pass &= c >= 32 ? 0xffffffffu : c <= 0 ? 0u : (1u << c) - 1u;
-              const int mine = __popc(pass);
-              if (COUNT) {
-                n_hits += (uint32_t)mine;
-              } else if (__any_sync(0xffffffffu, mine != 0)) {
-                int incl = mine;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                  const int x = __shfl_up_sync(0xffffffffu, incl, o);
-                  if (lane >= o) incl += x;
-                }
-                unsigned long long w = 0;
-                if (lane == 31) w = atomicAdd(A.cand_count, (unsigned long long)incl);
-                w = __shfl_sync(0xffffffffu, w, 31) + (unsigned long long)(incl - mine);
-                while (pass) {
-                  const int j = __ffs(pass) - 1;
-                  pass &= pass - 1;
-                  if ((int64_t)w < A.cand_cap)
-                    A.cand[w] = ((uint64_t)(irow0 + 32 * g + j) << 32) | (uint64_t)jrow;
-                  ++w;
-                }
-              }
-            }
+            // group g is worked on while group g + 1 loads
+            uint32_t(&x)[32] = v[g & 1];
+            tmem_wait(x);
+            if (g < 3) tmem_ld32_async(taddr + 32u * (g + 1), v[(g + 1) & 1]);
+            if (!__any_sync(0xffffffffu, largest(x) >= thr)) continue;
+            uint32_t pass = passing(x, thr, (int)lim - 32 * g);
             if (COUNT) {
-              const uint32_t total = __reduce_add_sync(0xffffffffu, n_hits);
-              if (lane == 0 && total)
-                atomicAdd(&A.class_count[((size_t)U.w * A.nbI + I) * A.nbJ + J], total);
+              n_hits += (uint32_t)__popc(pass);
+              continue;
             }
+            for (;;) {  // one candidate of each row that has some left
+              const unsigned some = __ballot_sync(0xffffffffu, pass != 0u);
+              if (!some) break;
+              if (held > kHits - 32) {
+                flush_hits(A, hits, held, lane);
+                held = 0;
+              }
+              if (pass) {
+                const int j = __ffs(pass) - 1;
+                pass &= pass - 1;
+                hits[held + __popc(some & ((1u << lane) - 1u))] =
+                    ((uint64_t)(irow0 + 32 * g + j) << 32) | (uint64_t)jrow;
+              }
+              held += __popc(some);
+            }
+          }
+          if (COUNT) {
+            const uint32_t total = __reduce_add_sync(0xffffffffu, n_hits);
+            if (lane == 0 && total)
+              atomicAdd(&A.class_count[((size_t)U.lev * A.nbI + I) * A.nbJ + J], total);
           }
         }
         tc_fence_before();
@@ -344,6 +404,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
         if (live && lane == 0) mbar_arrive(&tempty[b]);
       }
     }
+    if (!COUNT && held > 0) flush_hits(A, hits, held, lane);
   }
   tc_fence_before();
   __syncthreads();

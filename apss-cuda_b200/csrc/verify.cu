@@ -2,9 +2,8 @@
 // similarity in FP64 from the caller's CSR, kept if >= t.
 //
 // A warp takes up to 32 consecutive candidates: their row numbers and row
-// pointers load one candidate per lane, then the warp computes them in turn,
-// the lanes running over the shorter row and searching the longer one. The
-// sum's order differs from the oracle's ascending feature order, so a sum
+// pointers load one candidate per lane, then the warp computes them in turn
+// (warp_dot). The sum's order differs from the oracle's ascending feature order, so a sum
 // within the FP64 rounding of t is redone in that order by one lane; every
 // decision is then the oracle's. The order depends on the two rows alone, so
 // a pair's value does not depend on how the join was cut.
@@ -36,15 +35,97 @@ __device__ double dot_ordered(const int32_t* __restrict__ ca, const float* __res
   return s;
 }
 
+// Warp dot product of rows S (shorter) and L: lane l sums the products of
+// S's entries l, l + 32, ... in ascending order, the lanes' sums are added in
+// a fixed tree.
+//
+// Rows of similar length are merged in chunks of 32 entries held in
+// registers: every lane finds its S entry among the 32 L entries by shuffles,
+// then the chunk that ends first moves on (its successor is already loaded).
+// A much longer L is searched in place instead, kSearch entries of S a lane
+// at a time so that the searches' loads overlap.
+constexpr int kSearch = 4;
+constexpr int kSearchRatio = 12;  // L at least this many times longer: searched
+
+__device__ __forceinline__ double warp_dot(const int32_t* __restrict__ cs,
+                                           const float* __restrict__ vs, int sl,
+                                           const int32_t* __restrict__ cl,
+                                           const float* __restrict__ vl, int ll, int lane) {
+  double s = 0.0;
+  if (ll >= kSearchRatio * sl) {
+    for (int e0 = lane; e0 < sl; e0 += 32 * kSearch) {
+      int32_t c[kSearch];
+      int x[kSearch];
+#pragma unroll
+      for (int q = 0; q < kSearch; ++q) {
+        c[q] = e0 + 32 * q < sl ? cs[e0 + 32 * q] : INT32_MAX;
+        x[q] = 0;
+      }
+      for (int n = ll; n > 0;) {  // lower bounds of c in cl: each in [x, x + n]
+        const int h = (n + 1) >> 1;
+#pragma unroll
+        for (int q = 0; q < kSearch; ++q)
+          if (cl[x[q] + h - 1] < c[q]) x[q] += h;
+        n -= h;
+      }
+#pragma unroll
+      for (int q = 0; q < kSearch; ++q)
+        if (e0 + 32 * q < sl && x[q] < ll && cl[x[q]] == c[q])
+          s += (double)vs[e0 + 32 * q] * (double)vl[x[q]];
+    }
+  } else {
+    int i = 32, j = 32;  // next chunk of S and L
+    int32_t a = lane < sl ? cs[lane] : INT32_MAX, b = lane < ll ? cl[lane] : INT32_MAX;
+    float av = lane < sl ? vs[lane] : 0.0f, bv = lane < ll ? vl[lane] : 0.0f;
+    int32_t a2 = i + lane < sl ? cs[i + lane] : INT32_MAX;
+    int32_t b2 = j + lane < ll ? cl[j + lane] : INT32_MAX;
+    float av2 = i + lane < sl ? vs[i + lane] : 0.0f, bv2 = j + lane < ll ? vl[j + lane] : 0.0f;
+    for (;;) {
+      int p = 0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+        if (__shfl_sync(kFull, b, p + o - 1) < a) p += o;
+      const int32_t y = __shfl_sync(kFull, b, p);
+      const float w = __shfl_sync(kFull, bv, p);
+      if (y == a && a != INT32_MAX) s += (double)av * (double)w;
+      const int32_t amax = __shfl_sync(kFull, a, 31), bmax = __shfl_sync(kFull, b, 31);
+      if (amax <= bmax) {
+        if (i >= sl) break;
+        a = a2;
+        av = av2;
+        i += 32;
+        a2 = i + lane < sl ? cs[i + lane] : INT32_MAX;
+        av2 = i + lane < sl ? vs[i + lane] : 0.0f;
+      }
+      if (bmax <= amax) {
+        if (j >= ll) break;
+        b = b2;
+        bv = bv2;
+        j += 32;
+        b2 = j + lane < ll ? cl[j + lane] : INT32_MAX;
+        bv2 = j + lane < ll ? vl[j + lane] : 0.0f;
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
+  return s;
+}
+
 __global__ void __launch_bounds__(kThreads) k_verify(const VerifyArgs A) {
   const int64_t nc = (int64_t)*A.ncand;
   if (nc > A.cap) return;  // incomplete list: the host runs again with room
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  const int64_t wid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-  int g = 32;  // candidates a warp takes at a time: fewer when there are few
-  while (g > 1 && (int64_t)g * warps > nc) g >>= 1;
-  for (int64_t base = wid * g; base < nc; base += warps * g) {
+  // candidates a warp takes at a time, from a counter: rows differ in length
+  // by orders of magnitude
+  int g = 32;
+  while (g > 1 && (int64_t)g * 4 * warps > nc) g >>= 1;
+  for (;;) {
+    unsigned grp = 0;
+    if (lane == 0) grp = atomicAdd(A.work, 1u);
+    const int64_t base = (int64_t)__shfl_sync(kFull, grp, 0) * g;
+    if (base >= nc) break;
     const int m = (int)(nc - base < g ? nc - base : g);
     uint32_t pi = 0, pj = 0;  // caller's rows
     uint32_t so = 0, lo = 0;  // first entry of the shorter and the longer row
@@ -71,24 +152,9 @@ __global__ void __launch_bounds__(kThreads) k_verify(const VerifyArgs A) {
       const uint32_t so_k = __shfl_sync(kFull, so, k), lo_k = __shfl_sync(kFull, lo, k);
       const int sl_k = __shfl_sync(kFull, sl, k), ll_k = __shfl_sync(kFull, ll, k);
       const bool sw_k = __shfl_sync(kFull, (int)swapped, k) != 0;
-      const int32_t* __restrict__ cs = (sw_k ? A.colJ : A.colI) + so_k;
-      const float* __restrict__ vs = (sw_k ? A.valJ : A.valI) + so_k;
-      const int32_t* __restrict__ cl = (sw_k ? A.colI : A.colJ) + lo_k;
-      const float* __restrict__ vl = (sw_k ? A.valI : A.valJ) + lo_k;
-      double s = 0.0;
-      for (int e = lane; e < sl_k; e += 32) {
-        const int32_t c = cs[e];
-        int x = 0, n = ll_k;  // lower bound of c in cl
-        while (n > 0) {
-          const int h = n >> 1;
-          const bool right = cl[x + h] < c;
-          x = right ? x + h + 1 : x;
-          n = right ? n - h - 1 : h;
-        }
-        if (x < ll_k && cl[x] == c) s += (double)vs[e] * (double)vl[x];
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
+      const double s = warp_dot((sw_k ? A.colJ : A.colI) + so_k, (sw_k ? A.valJ : A.valI) + so_k,
+                                sl_k, (sw_k ? A.colI : A.colJ) + lo_k,
+                                (sw_k ? A.valI : A.valJ) + lo_k, ll_k, lane);
       if (lane == k) mine = s;
     }
     bool in = false;

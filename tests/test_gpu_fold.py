@@ -1,0 +1,79 @@
+"""GPU parity of the folded-bound joins against the FP64 oracle, where their
+kernels change behaviour: one I block without a partner, a partial last
+block, the sampled choice of widths (from 64 row blocks on) with rows long
+enough for the streamed and the widest folds, signed values, and inputs whose
+bound prunes nothing (the join falls back to the probing path).
+
+Pair sets are exact; similarities are FP64 sums rounded once to FP32, so they
+lie within 2^-24 (half an ulp below 1, values up to 1 + 1e-4) of the oracle's:
+1.2e-7 allows for both roundings."""
+import numpy as np
+import pytest
+
+import cuapss
+from cuapss import synth
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+SIM_TOL = 1.2e-7
+
+
+def _check(got, want):
+    gi, gj, gs = got
+    wi, wj, ws = want
+    assert len(gi) == len(wi)
+    assert np.array_equal(gi, wi) and np.array_equal(gj, wj)
+    if len(gs):
+        assert float(np.max(np.abs(gs.astype(np.float64) - ws))) <= SIM_TOL
+
+
+def _signed(x, seed):
+    sign = np.random.default_rng(seed).choice(np.array([-1, 1], np.float32), size=x.nnz)
+    return synth.Csr(x.rowptr, x.col, x.val * sign, x.d)
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    with cuapss.Context(precision=cuapss.PREC_MIXED) as c:
+        yield c
+
+
+@pytest.mark.parametrize("cfg,n,t", [
+    ("plain_20k", 129, 0.5), ("plain_20k", 384, 0.6), ("batch_instance", 8064, 0.6),
+    ("batch_instance", 8193, 0.5), ("mixed_1m", 8320, 0.5), ("plain_800k", 12_345, 0.3),
+    ("serve_5m", 9999, 0.95)])
+def test_self_join(ctx, cfg, n, t):
+    x = synth.generate(cfg, n=n, seed=n)
+    _check(ctx.run(x, t, capacity=1 << 22), oracle.apss(x, t))
+
+
+@pytest.mark.parametrize("n,m", [(100, 9000), (9000, 100), (5001, 4097), (257, 129)])
+def test_cross_join(ctx, n, m):
+    x = synth.generate("plain_800k", n=n + m, seed=3)
+    a, b = x.rows(0, n), x.rows(n, n + m)
+    _check(ctx.join(a, b, 0.5, capacity=1 << 20), oracle.join(a, b, 0.5))
+
+
+def test_signed_values(ctx):
+    x = _signed(synth.generate("plain_20k", n=9000, seed=4), 5)
+    _check(ctx.run(x, 0.3, capacity=1 << 20), oracle.apss(x, 0.3))
+
+
+def test_device_capacity_and_determinism(ctx):
+    x = synth.generate("plain_800k", n=9000, seed=6)
+    a = ctx.run(x, 0.5, capacity=1)  # EOVERFLOW, then the required room
+    b = ctx.run(x, 0.5, capacity=1 << 20)
+    assert all(np.array_equal(p, q) for p, q in zip(a, b))
+
+
+def test_no_pruning_falls_back(ctx):
+    # 2,200 near-identical rows: 2.4M candidates, more than a small folded
+    # join takes
+    rng = np.random.default_rng(7)
+    n, m = 2200, 20
+    col = np.tile(np.arange(m, dtype=np.int32) * 3, n)
+    val = (1.0 + 0.05 * rng.standard_normal((n, m)))
+    val = (val / np.linalg.norm(val, axis=1, keepdims=True)).astype(np.float32).ravel()
+    x = synth.Csr(np.arange(n + 1, dtype=np.int64) * m, col, val, 3 * m)
+    _check(ctx.run(x, 0.95, capacity=1 << 22), oracle.apss(x, 0.95))
