@@ -84,6 +84,9 @@ constexpr int kMaxModelHead = 8192;
 // Lowest threshold of the folded join: its margins (about 0.01) stay small
 // against t, and empty rows stay below it.
 constexpr float kFoldMinT = 0.05f;
+// SM-nanoseconds of an FP32 probing tile: the head, and per non-zero of the J
+// block (n = 800,000, 75 a row: 22 us; n = d = 1M, 120 a row: 32 us).
+constexpr double kPlainHeadNs = 5000.0, kPlainPostingNs = 1.75;
 constexpr double kUnitCostCap = 512.0;  // unit cost cap (tile weights, 1 + tail / mean)
 
 namespace {
@@ -384,9 +387,11 @@ cuapss_status join_device(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, flo
     }
   }
   const int64_t n_all = a.n + (self ? 0 : bb.n), nnz_all = a.nnz + (self ? 0 : bb.nnz);
+  // (the FP32 path without rare features only counts its head's postings)
   std::vector<int64_t> prefix;
-  if (precision == CUAPSS_PREC_MIXED || !rare.empty())
-    ST_TRY(rank_count_prefix(counts, d, ctx->opts.remap, kMaxModelHead, ws, st, &prefix));
+  const bool model = precision == CUAPSS_PREC_MIXED || !rare.empty();
+  ST_TRY(rank_count_prefix(counts, d, ctx->opts.remap, model ? kMaxModelHead : 64, ws, st,
+                           &prefix));
   int64_t max_pairs = 0;
   if (!rare.empty()) {
     size_t free_b = 0, total_b = 0;
@@ -395,8 +400,9 @@ cuapss_status join_device(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, flo
         kMaxExplicitPairs, (int64_t)((double)free_b * kExplicitMemShare / kExplicitPairBytes));
   }
   if (forced_rare > 0 && !rare.empty() && rare[0].pairs > max_pairs) return CUAPSS_ENOMEM;
-  const TilePlan plan = plan_tiles(precision, n_all, d, nnz_all, prefix, rare, max_pairs,
-                                   ctx->opts.head_width, forced_rare > 0);
+  const TilePlan plan =
+      plan_tiles(precision, n_all, d, nnz_all, model ? prefix : std::vector<int64_t>(), rare,
+                 max_pairs, ctx->opts.head_width, forced_rare > 0);
   int p = plan.p;
   const bool mixed = precision == CUAPSS_PREC_MIXED;
   const int pq = mixed ? 64 : 32;  // head width granularity of the tile kernels
@@ -427,13 +433,17 @@ cuapss_status join_device(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, flo
   // The folded join, unless the options fix how the probing path works (a
   // head width, a rare-feature threshold, no remap) or a shard owns rows by
   // their place.
-  if (mixed && ctx->opts.head_width == 0 && forced_rare == 0 && ctx->opts.remap && nshards == 1 &&
+  if (ctx->opts.head_width == 0 && forced_rare == 0 && ctx->opts.remap && nshards == 1 &&
       a.n > 0 && bb.n > 0 && t >= kFoldMinT) {
     nvtx.next("cuapss_run:tiles");
     cudaEventRecord(ctx->ev[1], st);
     FoldResult fr;
     bool done = false;
-    ST_TRY(join_fold(ctx, a, b, t, perm, nrm2, plan.tile_ns, &fr, &done));
+    // the FP32 probing tiles: their head at p = 64, and their probes
+    const double probing_ns =
+        mixed ? plan.tile_ns
+              : kPlainHeadNs + kPlainPostingNs * kBlockRows * ((double)nnz_all / (double)n_all);
+    ST_TRY(join_fold(ctx, a, b, t, perm, nrm2, probing_ns, &fr, &done));
     if (done) {
       cudaEventRecord(ctx->ev[2], st);
       nvtx.next("cuapss_run:finalize");

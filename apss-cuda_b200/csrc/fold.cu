@@ -25,7 +25,7 @@ constexpr double kClassEdge[kClasses] = {0.125, 0.25, 0.375, 0.5,  0.625, 0.75, 
 // Sides of fewer blocks keep the caller's order and one width, whose
 // candidates are few or, past kSmallMaxCand, make the join fall back.
 constexpr int kSampleMinBlocks = 64;
-constexpr int kSmallLevel = 3;  // K = 256
+constexpr int kSmallLevel = 3;
 constexpr int64_t kSmallMaxCand = 1 << 21;
 
 // Cost model, SM-nanoseconds, measured on 200,000 and 400,000 rows of the
@@ -36,7 +36,26 @@ constexpr int64_t kSmallMaxCand = 1 << 21;
 // listing in the tile kernel, and verify) + kCandEntryNs per entry of its
 // longer row.
 constexpr double kTileNs = 340.0, kChunkNs = 275.0, kStreamNs = 400.0;
-constexpr double kCandNs = 45.0, kCandEntryNs = 0.25;
+constexpr double kCandNs = 45.0, kCandEntryNs = 0.3;
+// FP32, 128 x 128 tiles.
+constexpr double kTile32Ns = 380.0, kColumn32Ns = 92.0;
+
+template <bool MIXED>
+constexpr int kPair = MIXED ? 2 : 1;  // I blocks of a tile
+template <bool MIXED>
+constexpr int kChunk = MIXED ? kFoldChunk16 : kFoldChunk32;
+
+template <bool MIXED>
+double tile_cost(int level) {
+  const int K = fold_k(MIXED, level);
+  if (!MIXED) return kTile32Ns + kColumn32Ns * K;
+  return K <= kFoldResident16 ? kTileNs + kChunkNs * (K / 64) : kStreamNs * (K / 64);
+}
+
+template <bool MIXED>
+cuapss_status launch_fold(const FoldTileArgs& a, int sms, cudaStream_t st, bool count) {
+  return MIXED ? launch_tiles_fold(a, sms, st, count) : launch_tiles_fold32(a, sms, st, count);
+}
 
 inline unsigned grid_for(int64_t work, int per_block) {
   const int64_t g = ceil_div(std::max<int64_t>(work, 1), per_block);
@@ -87,39 +106,48 @@ __global__ void k_sample_rows(const int32_t* __restrict__ rowmap, const int64_t*
 // FP32 sums can have (2^-24 per addition), so their products bound the exact
 // ones.
 struct FoldOut {
-  __nv_bfloat16* base[kFoldLevels];  // null: not built
-  int first[kFoldLevels];            // block at offset 0
+  uint8_t* base[kFoldLevels];  // null: not built
+  int first[kFoldLevels];      // block at offset 0
 };
+
+__host__ __device__ constexpr size_t fold_bytes(bool mixed, int level) {  // of a row block
+  return (size_t)fold_k(mixed, level) * kBlockRows * (mixed ? 2 : 4);
+}
 
 // First accumulator column of level l when the levels of `allow` lie one
 // after another, and their total.
-__host__ __device__ constexpr int fold_offset(uint32_t allow, int l) {
-  constexpr int K[kFoldLevels] = {kFoldK[0], kFoldK[1], kFoldK[2], kFoldK[3],
-                                  kFoldK[4], kFoldK[5], kFoldK[6], kFoldK[7]};
+__host__ __device__ constexpr int fold_offset(bool mixed, uint32_t allow, int l) {
   int o = 0;
   for (int k = 0; k < l; ++k)
-    if ((allow >> k) & 1u) o += K[k];
+    if ((allow >> k) & 1u) o += fold_k(mixed, k);
   return o;
 }
 
-template <int LEV>
+template <bool MIXED, int LEV>
 __device__ __forceinline__ void fold_add(uint32_t mask, float* acc, uint32_t allow, uint32_t r,
                                          float v) {
-  constexpr uint32_t P = kFoldK[LEV] / 4, M = kFoldK[LEV] - P;
+  constexpr uint32_t P = fold_k(MIXED, LEV) / 4, M = fold_k(MIXED, LEV) - P;
   if (!((mask >> LEV) & 1u)) return;  // uniform over the row's threads
-  float* a = acc + fold_offset(allow, LEV);
+  float* a = acc + fold_offset(MIXED, allow, LEV);
   if (r < P) a[r] = v;
   else atomicAdd(&a[P + (r - P) % M], v * v);
 }
 
-template <int LEV>
+template <bool MIXED, int LEV>
 __device__ __forceinline__ void fold_write(uint32_t mask, const float* acc, uint32_t allow,
                                            const FoldOut& O, float widen, int b, int rr, int tid,
                                            int nt) {
-  constexpr int K = kFoldK[LEV], P = K / 4;
+  constexpr int K = fold_k(MIXED, LEV), P = K / 4;
   if (!((mask >> LEV) & 1u)) return;
-  const float* a = acc + fold_offset(allow, LEV);
-  uint4* out = reinterpret_cast<uint4*>(O.base[LEV] + (size_t)(b - O.first[LEV]) * K * kBlockRows);
+  const float* a = acc + fold_offset(MIXED, allow, LEV);
+  uint8_t* dst = O.base[LEV] + (size_t)(b - O.first[LEV]) * fold_bytes(MIXED, LEV);
+  if (!MIXED) {  // [column][row]
+    for (int c = tid; c < K; c += nt)
+      reinterpret_cast<float*>(dst)[c * kBlockRows + rr] =
+          c < P ? a[c] : __fmul_ru(__fsqrt_ru(a[c]), widen);
+    return;
+  }
+  uint4* out = reinterpret_cast<uint4*>(dst);
   for (int c8 = tid; c8 < K / 8; c8 += nt) {
     __nv_bfloat162 w[4];
     const float4 x = reinterpret_cast<const float4*>(a)[2 * c8];
@@ -146,19 +174,19 @@ __device__ __forceinline__ void fold_write(uint32_t mask, const float* acc, uint
 // [b0, b1) of rowmap; blk_mask[b]: levels of block b (null: mask0 for all);
 // only blocks whose levels are all in `allow` (wide: some level is not
 // narrow) are taken. Shared memory: the columns of `allow` per row.
-constexpr uint32_t kNarrowLevels = 0x3f;  // K <= 512
+constexpr uint32_t kNarrowLevels = 0x7f;  // K <= 512 (mixed), 192 (FP32)
 
-template <int GROUP>
+template <bool MIXED, int GROUP>
 __global__ void __launch_bounds__(kThreads)
     k_fold_rows(const int32_t* __restrict__ rowmap, int64_t slot0, int64_t slot1,
                 const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
                 const float* __restrict__ val, const int32_t* __restrict__ perm,
-                const uint8_t* __restrict__ blk_mask, uint32_t mask0, uint32_t allow, bool wide,
+                const uint16_t* __restrict__ blk_mask, uint32_t mask0, uint32_t allow, bool wide,
                 FoldOut O) {
   extern __shared__ __align__(16) float fold_sm[];
   constexpr int kGroups = kThreads / GROUP;
   const int tid = threadIdx.x % GROUP;
-  const int ncol = fold_offset(allow, kFoldLevels);
+  const int ncol = fold_offset(MIXED, allow, kFoldLevels);
   float* acc = fold_sm + (threadIdx.x / GROUP) * ncol;
   for (int64_t s = slot0 + (int64_t)blockIdx.x * kGroups + threadIdx.x / GROUP; s < slot1;
        s += (int64_t)gridDim.x * kGroups) {
@@ -175,38 +203,43 @@ __global__ void __launch_bounds__(kThreads)
     for (int e = tid; e < len; e += GROUP) {
       const uint32_t f = (uint32_t)perm[col[lo + e]];
       const float v = val[lo + e];
-      fold_add<0>(mask, acc, allow, f, v);
-      fold_add<1>(mask, acc, allow, f, v);
-      fold_add<2>(mask, acc, allow, f, v);
-      fold_add<3>(mask, acc, allow, f, v);
-      fold_add<4>(mask, acc, allow, f, v);
-      fold_add<5>(mask, acc, allow, f, v);
-      fold_add<6>(mask, acc, allow, f, v);
-      fold_add<7>(mask, acc, allow, f, v);
+      fold_add<MIXED, 0>(mask, acc, allow, f, v);
+      fold_add<MIXED, 1>(mask, acc, allow, f, v);
+      fold_add<MIXED, 2>(mask, acc, allow, f, v);
+      fold_add<MIXED, 3>(mask, acc, allow, f, v);
+      fold_add<MIXED, 4>(mask, acc, allow, f, v);
+      fold_add<MIXED, 5>(mask, acc, allow, f, v);
+      fold_add<MIXED, 6>(mask, acc, allow, f, v);
+      fold_add<MIXED, 7>(mask, acc, allow, f, v);
+      fold_add<MIXED, 8>(mask, acc, allow, f, v);
+      fold_add<MIXED, 9>(mask, acc, allow, f, v);
     }
     if (GROUP == 32) __syncwarp();
     else __syncthreads();
     const float widen = 1.0f + (float)(len + 16) * 5.9604645e-8f * 1.01f;
-    fold_write<0>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
-    fold_write<1>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
-    fold_write<2>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
-    fold_write<3>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
-    fold_write<4>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
-    fold_write<5>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
-    fold_write<6>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
-    fold_write<7>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
+    fold_write<MIXED, 0>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
+    fold_write<MIXED, 1>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
+    fold_write<MIXED, 2>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
+    fold_write<MIXED, 3>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
+    fold_write<MIXED, 4>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
+    fold_write<MIXED, 5>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
+    fold_write<MIXED, 6>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
+    fold_write<MIXED, 7>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
+    fold_write<MIXED, 8>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
+    fold_write<MIXED, 9>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
     if (GROUP == 32) __syncwarp();
     else __syncthreads();
   }
 }
-static_assert(kFoldLevels == 8, "one fold_add / fold_write call per level");
+static_assert(kFoldLevels == 10, "one fold_add / fold_write call per level");
 
 // Folds the places of [0, slots) with the levels of masks (host, per block;
 // empty: mask0 everywhere) into O.
+template <bool MIXED>
 cuapss_status fold_side(const DevCsr& x, const int32_t* rowmap, int64_t slots,
-                        const std::vector<uint8_t>& masks, uint32_t mask0, const int32_t* perm,
+                        const std::vector<uint16_t>& masks, uint32_t mask0, const int32_t* perm,
                         const FoldOut& O, Workspace& ws, const std::string& tag, cudaStream_t st) {
-  uint8_t* d_mask = nullptr;
+  uint16_t* d_mask = nullptr;
   // levels, and blocks, with and without a wide level
   uint32_t all[2] = {0, 0};
   int64_t b0[2] = {0, 0}, b1[2] = {0, 0};
@@ -216,7 +249,7 @@ cuapss_status fold_side(const DevCsr& x, const int32_t* rowmap, int64_t slots,
     b1[w] = slots / kBlockRows;
   } else {
     ST_TRY(ws.get(tag + ":mask", masks.size(), &d_mask));
-    CU_TRY(cudaMemcpyAsync(d_mask, masks.data(), masks.size(), cudaMemcpyHostToDevice, st));
+    CU_TRY(cudaMemcpyAsync(d_mask, masks.data(), 2 * masks.size(), cudaMemcpyHostToDevice, st));
     for (size_t b = 0; b < masks.size(); ++b) {
       const int w = (masks[b] & ~kNarrowLevels) ? 1 : 0;
       if (!all[w]) b0[w] = (int64_t)b;
@@ -225,17 +258,19 @@ cuapss_status fold_side(const DevCsr& x, const int32_t* rowmap, int64_t slots,
     }
   }
   if (all[0]) {  // a warp per row
-    const size_t smem = (size_t)fold_offset(all[0], kFoldLevels) * 4 * (kThreads / 32);
-    CU_TRY(cudaFuncSetAttribute(k_fold_rows<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                fold_offset(kNarrowLevels, kFoldLevels) * 4 * (kThreads / 32)));
-    k_fold_rows<32><<<grid_for((b1[0] - b0[0]) * kBlockRows, kThreads / 32), kThreads, smem, st>>>(
+    const size_t smem = (size_t)fold_offset(MIXED, all[0], kFoldLevels) * 4 * (kThreads / 32);
+    CU_TRY(cudaFuncSetAttribute((const void*)k_fold_rows<MIXED, 32>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                fold_offset(MIXED, kNarrowLevels, kFoldLevels) * 4 *
+                                    (kThreads / 32)));
+    k_fold_rows<MIXED, 32><<<grid_for((b1[0] - b0[0]) * kBlockRows, kThreads / 32), kThreads, smem, st>>>(
         rowmap, b0[0] * kBlockRows, b1[0] * kBlockRows, x.rp, x.col, x.val, perm, d_mask, mask0,
         all[0], false, O);
     LAUNCH_CHECK();
   }
   if (all[1]) {  // blocks of long rows (and the samples): a CTA per row
-    const size_t smem = (size_t)fold_offset(all[1], kFoldLevels) * 4;
-    k_fold_rows<kThreads><<<grid_for((b1[1] - b0[1]) * kBlockRows, 1), kThreads, smem, st>>>(
+    const size_t smem = (size_t)fold_offset(MIXED, all[1], kFoldLevels) * 4;
+    k_fold_rows<MIXED, kThreads><<<grid_for((b1[1] - b0[1]) * kBlockRows, 1), kThreads, smem, st>>>(
         rowmap, b0[1] * kBlockRows, b1[1] * kBlockRows, x.rp, x.col, x.val, perm, d_mask, mask0,
         all[1], true, O);
     LAUNCH_CHECK();
@@ -243,10 +278,13 @@ cuapss_status fold_side(const DevCsr& x, const int32_t* rowmap, int64_t slots,
   return CUAPSS_OK;
 }
 
-float fold_eps(int level, double nrm2) {
-  // BF16 rounding of the head columns, FP32 accumulation of K / 16 steps
-  const double head = std::ldexp(1.0, -7) + std::ldexp(1.0, -16);
-  const double acc = (kFoldK[level] / 16.0 + 2.0) * std::ldexp(1.0, -20) * 1.02;
+float fold_eps(bool mixed, int level, double nrm2) {
+  // mixed: BF16 rounding of the head columns, FP32 accumulation of K / 16
+  // steps; FP32: a chain of K FMAs
+  const int K = fold_k(mixed, level);
+  const double head = mixed ? std::ldexp(1.0, -7) + std::ldexp(1.0, -16) : 0.0;
+  const double acc =
+      (mixed ? (K / 16.0 + 2.0) * std::ldexp(1.0, -20) : (K + 4.0) * std::ldexp(1.0, -24)) * 1.02;
   return (float)((head + acc) * nrm2 * 1.001 + 1e-6);
 }
 
@@ -257,7 +295,7 @@ struct FoldSide {
   int edge[kClasses + 1] = {};    // first block of each class (even), nb at the end
   double len[kClasses] = {};      // mean row length of each class
   int32_t* sample = nullptr;
-  std::vector<uint8_t> masks;     // levels of each block
+  std::vector<uint16_t> masks;     // levels of each block
   FoldOut out{};
 };
 
@@ -293,6 +331,7 @@ ClassRows class_rows(const FoldSide& s) {
 // The width of every pair of classes, from the products of sampled rows.
 // level[a][b] (I class a, J class b; self: b >= a) and the modelled cost of
 // the join in SM-nanoseconds, with its expected candidates.
+template <bool MIXED>
 cuapss_status plan_levels(cuapss_ctx* ctx, FoldSide& I, FoldSide& J, bool self, float t,
                           const int32_t* perm, double nrm2, int (*level)[kClasses], double* cost,
                           double* cands) {
@@ -315,19 +354,18 @@ cuapss_status plan_levels(cuapss_ctx* ctx, FoldSide& I, FoldSide& J, bool self, 
     LAUNCH_CHECK();
     FoldOut o{};
     for (int l = 0; l < kFoldLevels; ++l)
-      ST_TRY(ws.get(tag + std::to_string(l), (size_t)slots * kFoldK[l], &o.base[l]));
-    ST_TRY(fold_side(s.x, s.sample, slots, {}, (1u << kFoldLevels) - 1u, perm, o, ws, tag, st));
+      ST_TRY(ws.get(tag + std::to_string(l), kClasses * fold_bytes(MIXED, l), &o.base[l]));
+    ST_TRY(fold_side<MIXED>(s.x, s.sample, slots, {}, (1u << kFoldLevels) - 1u, perm, o, ws, tag, st));
     for (int l = 0; l < kFoldLevels; ++l) {
-      const uint8_t* p = reinterpret_cast<const uint8_t*>(o.base[l]);
-      if (k == 0) ta.lev[l].I = p;
-      if (k == 1 || self) ta.lev[l].J = p;
+      if (k == 0) ta.lev[l].I = o.base[l];
+      if (k == 1 || self) ta.lev[l].J = o.base[l];
     }
   }
   std::vector<int4> units;
   for (int l = kFoldLevels - 1; l >= 0; --l) {
-    ta.lev[l].nkc = kFoldK[l] / 64;
-    ta.lev[l].eps = fold_eps(l, nrm2);
-    for (int a = 0; a < kClasses; a += 2)
+    ta.lev[l].nkc = fold_k(MIXED, l) / kChunk<MIXED>;
+    ta.lev[l].eps = fold_eps(MIXED, l, nrm2);
+    for (int a = 0; a < kClasses; a += kPair<MIXED>)
       for (int b = self ? a : 0; b < kClasses; ++b) units.push_back(make_int4(a, b, b + 1, l));
   }
   int4* d_units = nullptr;
@@ -345,7 +383,7 @@ cuapss_status plan_levels(cuapss_ctx* ctx, FoldSide& I, FoldSide& J, bool self, 
   ta.unit_counter = ctl;
   ta.err = ctl + 1;
   ta.class_count = cnt;
-  ST_TRY(launch_tiles_fold(ta, std::min(ctx->sms, (int)units.size()), st, true));
+  ST_TRY(launch_fold<MIXED>(ta, ctx->sms, st, true));
   std::vector<uint8_t> h(8 * 2 * kClasses + 4 * ncnt);
   int herr = 0;
   CU_TRY(cudaMemcpyAsync(h.data(), stats, h.size(), cudaMemcpyDeviceToHost, st));
@@ -377,13 +415,10 @@ cuapss_status plan_levels(cuapss_ctx* ctx, FoldSide& I, FoldSide& J, bool self, 
         if (self && a == b) c = std::max(0.0, c - rows[0][a]);  // a row with itself
         // a count of zero is not a share of zero: half a pair
         const double share = sampled > 0 ? std::max(c, 0.5) / sampled : 0.0;
-        const double tiles = pairs / (2.0 * kBlockRows * kBlockRows);
-        const int nkc = kFoldK[l] / 64;
-        const double tile_ns =
-            kFoldK[l] <= kFoldResidentK ? kTileNs + kChunkNs * nkc : kStreamNs * nkc;
+        const double tiles = pairs / ((double)kPair<MIXED> * kBlockRows * kBlockRows);
         const double cand_ns =
             kCandNs + kCandEntryNs * std::max(side[0]->len[a], side[1]->len[b]);
-        const double ns = tiles * tile_ns + share * pairs * cand_ns;
+        const double ns = tiles * tile_cost<MIXED>(l) + share * pairs * cand_ns;
         if (ns < best) {
           best = ns;
           best_cand = share * pairs;
@@ -403,6 +438,7 @@ int class_of(const FoldSide& s, int block) {
 }
 
 // Allocates and builds the folded levels a side needs.
+template <bool MIXED>
 cuapss_status build_levels(FoldSide& s, const uint32_t (&need)[kClasses], const int32_t* perm,
                            Workspace& ws, const std::string& tag, cudaStream_t st) {
   uint32_t all = 0;
@@ -417,35 +453,39 @@ cuapss_status build_levels(FoldSide& s, const uint32_t (&need)[kClasses], const 
         hi = std::max(hi, s.edge[c + 1]);
       }
     s.out.first[l] = lo;
-    ST_TRY(ws.get(tag + ":lev" + std::to_string(l), (size_t)(hi - lo) * kFoldK[l] * kBlockRows,
+    ST_TRY(ws.get(tag + ":lev" + std::to_string(l), (size_t)(hi - lo) * fold_bytes(MIXED, l),
                   &s.out.base[l]));
   }
   s.masks.assign((size_t)s.nb, 0);
   for (int c = 0; c < kClasses; ++c)
-    for (int b = s.edge[c]; b < s.edge[c + 1]; ++b) s.masks[(size_t)b] = (uint8_t)need[c];
-  return fold_side(s.x, s.rowmap, (int64_t)s.nb * kBlockRows, s.masks, 0, perm, s.out, ws, tag, st);
+    for (int b = s.edge[c]; b < s.edge[c + 1]; ++b) s.masks[(size_t)b] = (uint16_t)need[c];
+  return fold_side<MIXED>(s.x, s.rowmap, (int64_t)s.nb * kBlockRows, s.masks, 0, perm, s.out, ws,
+                          tag, st);
 }
 
 // Units: windows of J blocks from the long rows down (the costly units
 // first), in each window every I pair against each class's part of it, so
 // that the CTAs running at one time share a window's chunks in L2. Wider
 // folds get proportionally shorter ranges.
+template <bool MIXED>
 void make_units(const FoldSide& I, const FoldSide& J, bool self, const int (*level)[kClasses],
                 int sms, std::vector<int4>* units, int64_t* tiles) {
   const int nbJ = J.nb;
-  const double total = self ? 0.25 * nbJ * (nbJ + 2.0) : 0.5 * (double)I.nb * nbJ;
-  const int w = (int)std::max(1.0, std::min(128.0, total / (sms * 16.0)));
+  const int pair = kPair<MIXED>;
+  const double total = (self ? 0.5 * nbJ * (nbJ + 2.0) : (double)I.nb * nbJ) / pair;
+  const int w = (int)std::max(1.0, std::min(MIXED ? 128.0 : 32.0, total / (sms * 16.0)));
   for (int j1 = nbJ; j1 > 0; j1 -= w) {
     const int j0 = std::max(0, j1 - w);
     for (int b = class_of(J, j1 - 1); b >= 0 && J.edge[b + 1] > j0; --b) {
       const int s0 = std::max(j0, J.edge[b]), s1 = std::min(j1, J.edge[b + 1]);
       if (s0 >= s1) continue;
       int a = 0;
-      for (int i = 0; i < (self ? std::min(I.nb, s1) : I.nb); i += 2) {
+      for (int i = 0; i < (self ? std::min(I.nb, s1) : I.nb); i += pair) {
         while (i >= I.edge[a + 1]) ++a;
         const int lv = level[a][b];
         const int f0 = self ? std::max(s0, i) : s0;
-        const int step = std::max(1, w * 2 / std::max(2, kFoldK[lv] / 64));
+        const double rel = tile_cost<MIXED>(lv) / tile_cost<MIXED>(MIXED ? 1 : 3);
+        const int step = std::max(1, (int)(w / std::max(1.0, rel)));
         for (int f = f0; f < s1; f += step) {
           const int len = std::min(s1 - f, step);
           // spread the starts of neighbouring units over the range
@@ -458,11 +498,10 @@ void make_units(const FoldSide& I, const FoldSide& J, bool self, const int (*lev
   *tiles = self ? (int64_t)nbJ * (nbJ + 1) / 2 : (int64_t)I.nb * nbJ;
 }
 
-}  // namespace
-
-cuapss_status join_fold(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float t,
-                        const int32_t* perm, double nrm2, double other_ns, FoldResult* r,
-                        bool* done) {
+template <bool MIXED>
+cuapss_status join_fold_as(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float t,
+                           const int32_t* perm, double nrm2, double other_ns, FoldResult* r,
+                           bool* done) {
   *done = false;
   const bool self = b == nullptr;
   Workspace& ws = ctx->ws;
@@ -480,11 +519,11 @@ cuapss_status join_fold(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float
   double cands = 0.0;
   if (sampled) {
     double cost = 0.0;
-    ST_TRY(plan_levels(ctx, SI, J, self, t, perm, nrm2, level, &cost, &cands));
+    ST_TRY(plan_levels<MIXED>(ctx, SI, J, self, t, perm, nrm2, level, &cost, &cands));
     if (cost >= tiles128 * other_ns) return CUAPSS_OK;
   } else {
     for (auto& row : level)
-      for (int& l : row) l = kSmallLevel;
+      for (int& l : row) l = kSmallLevel;  // K = 256 or 64
   }
   // ---- folded operands
   uint32_t needI[kClasses] = {}, needJ[kClasses] = {};
@@ -496,11 +535,11 @@ cuapss_status join_fold(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float
     }
   if (self)
     for (int c = 0; c < kClasses; ++c) needI[c] |= needJ[c];
-  ST_TRY(build_levels(SI, needI, perm, ws, "fold:I", st));
-  if (!self) ST_TRY(build_levels(SJ, needJ, perm, ws, "fold:J", st));
+  ST_TRY(build_levels<MIXED>(SI, needI, perm, ws, "fold:I", st));
+  if (!self) ST_TRY(build_levels<MIXED>(SJ, needJ, perm, ws, "fold:J", st));
   // ---- units
   std::vector<int4> units;
-  make_units(SI, J, self, level, ctx->sms, &units, &r->tiles);
+  make_units<MIXED>(SI, J, self, level, ctx->sms, &units, &r->tiles);
   int4* d_units = nullptr;
   ST_TRY(ws.get("tiles:units", std::max<size_t>(units.size(), 1), &d_units));
   if (!units.empty())
@@ -513,12 +552,12 @@ cuapss_status join_fold(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float
   FoldTileArgs ta;
   for (int l = 0; l < kFoldLevels; ++l) {
     FoldLevel& L = ta.lev[l];
-    L.I = reinterpret_cast<const uint8_t*>(SI.out.base[l]);
-    L.J = reinterpret_cast<const uint8_t*>(J.out.base[l]);
+    L.I = SI.out.base[l];
+    L.J = J.out.base[l];
     L.firstI = SI.out.first[l];
     L.firstJ = J.out.first[l];
-    L.nkc = kFoldK[l] / 64;
-    L.eps = fold_eps(l, nrm2);
+    L.nkc = fold_k(MIXED, l) / kChunk<MIXED>;
+    L.eps = fold_eps(MIXED, l, nrm2);
     if (SI.out.base[l]) r->max_band = std::max(r->max_band, (double)L.eps);
   }
   ta.nI = SI.x.n;
@@ -558,7 +597,7 @@ cuapss_status join_fold(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float
     ST_TRY(ws.get("out:sim", (size_t)cap, &r->osim));
     ta.cand_cap = cap;
     CU_TRY(cudaMemsetAsync(ctl, 0, 4 * sizeof(unsigned long long), st));
-    ST_TRY(launch_tiles_fold(ta, std::max(1, std::min((int)units.size(), ctx->sms)), st, false));
+    ST_TRY(launch_fold<MIXED>(ta, ctx->sms, st, false));
     va.cand = ta.cand;
     va.cap = cap;
     va.out_key = r->okey;
@@ -582,6 +621,16 @@ cuapss_status join_fold(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float
     cap = r->ncand;
   }
   return CUAPSS_OK;
+}
+
+}  // namespace
+
+cuapss_status join_fold(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float t,
+                        const int32_t* perm, double nrm2, double other_ns, FoldResult* r,
+                        bool* done) {
+  return ctx->opts.precision == CUAPSS_PREC_MIXED
+             ? join_fold_as<true>(ctx, a, b, t, perm, nrm2, other_ns, r, done)
+             : join_fold_as<false>(ctx, a, b, t, perm, nrm2, other_ns, r, done);
 }
 
 }  // namespace cuapss

@@ -11,6 +11,8 @@
 // be in the answer. The others (candidates) are computed in FP64 from the
 // caller's CSR (verify.cu): the folding decides only what is looked at.
 //
+// The FP32 form keeps FP32 columns and products throughout.
+//
 // Rows are sorted by length, and the width K is chosen per pair of length
 // classes from sampled rows (fold.cu): two short rows need few columns, two
 // long ones many.
@@ -26,18 +28,31 @@
 
 namespace cuapss {
 
-constexpr int kFoldLevels = 8;
-constexpr int kFoldK[kFoldLevels] = {64, 128, 192, 256, 384, 512, 1024, 2048};
-constexpr int kFoldResidentK = 256;  // widest fold whose I chunks stay in shared memory
-constexpr int kFoldTileBytes = kBlockRows * 64 * 2;  // a 64-column BF16 chunk of a row block
+// Widths. Mixed precision: BF16 folds multiplied on the tensor cores, in
+// 64-column chunks. FP32: FP32 folds multiplied on the CUDA cores, whose time
+// is proportional to K (65 ns per column and 128 x 128 tile), so the widths
+// are narrower and more candidates are computed.
+constexpr int kFoldLevels = 10;
+__host__ __device__ constexpr int fold_k(bool mixed, int level) {
+  constexpr int k16[kFoldLevels] = {64, 128, 192, 256, 320, 384, 512, 768, 1024, 2048};
+  constexpr int k32[kFoldLevels] = {16, 32, 48, 64, 96, 128, 192, 256, 512, 1024};
+  return mixed ? k16[level] : k32[level];
+}
+// Columns per chunk (one bulk copy per chunk and row block), and the widest
+// fold whose I chunks stay in shared memory.
+constexpr int kFoldChunk16 = 64, kFoldResident16 = 256;
+constexpr int kFoldChunk32 = 16, kFoldResident32 = 128;
+constexpr int kFoldTileBytes = kBlockRows * kFoldChunk16 * 2;  // 16 KB
+constexpr int kFoldSliceBytes = kBlockRows * kFoldChunk32 * 4;  // 8 KB
 
-// One folded width of the two operands of a launch: [blocks][K / 64] chunks
-// of 16 KB, block `first` of the side at offset 0.
+// One folded width of the two operands of a launch: [blocks][chunks], block
+// `first` of the side at offset 0. BF16 chunks are 128 rows x 64 columns in
+// the tensor cores' swizzled layout, FP32 chunks 16 columns x 128 rows.
 struct FoldLevel {
   const uint8_t* I = nullptr;
   const uint8_t* J = nullptr;
   int firstI = 0, firstJ = 0;
-  int nkc = 0;      // K / 64
+  int nkc = 0;      // chunks
   float eps = 0.f;  // margin of the bound at this width
 };
 
@@ -48,7 +63,7 @@ struct FoldTileArgs {
   int self = 0;                  // pairs i < j of one side only
   float t = 0.f;
   const float* t_row = nullptr;  // threshold of each J row, or null: t
-  const int4* units = nullptr;   // {I block (even), J0, J1, level | turn << 8}: blocks I, I + 1 x
+  const int4* units = nullptr;   // mixed: {I block (even), J0, J1, level | turn << 8}: blocks I, I + 1 x
                                  // [J0, J1), from J0 + turn on (0 <= turn < J1 - J0)
   int nunits = 0;
   int* unit_counter = nullptr;
@@ -59,8 +74,23 @@ struct FoldTileArgs {
   uint32_t* class_count = nullptr;  // sampling: [level][I block][J block] pairs at or above t - eps
 };
 
-// count: adds to class_count instead of listing candidates.
-cuapss_status launch_tiles_fold(const FoldTileArgs& a, int grid, cudaStream_t st, bool count);
+// A unit's tiles in order, starting at J0 + turn and wrapping around, so that
+// CTAs that work on the same J blocks at one time do not read the same L2
+// lines in step (n = 200,000, K = 128: 993 -> 873 ns a tile).
+struct FoldUnit {
+  int I, J0, len, lev, turn;
+  __device__ explicit FoldUnit(const int4& u)
+      : I(u.x), J0(u.y), len(u.z - u.y), lev(u.w & 0xff), turn(u.w >> 8) {}
+  __device__ int J(int k) const {
+    const int j = k + turn;
+    return J0 + (j < len ? j : j - len);
+  }
+};
+
+// count: adds to class_count instead of listing candidates. sms: SMs to fill.
+cuapss_status launch_tiles_fold(const FoldTileArgs& a, int sms, cudaStream_t st, bool count);
+// The FP32 form: units of one I block.
+cuapss_status launch_tiles_fold32(const FoldTileArgs& a, int sms, cudaStream_t st, bool count);
 
 // Exact decision of candidates (verify.cu).
 struct VerifyArgs {
@@ -97,7 +127,8 @@ struct FoldResult {
   double max_band = 0.0;  // widest margin of the widths used
 };
 
-// The folded join of validated device matrices (b == nullptr: self-join).
+// The folded join of validated device matrices (b == nullptr: self-join), in
+// the context's precision.
 // *done = false: the probing path is the better one here and nothing was
 // produced. other_ns: that path's modelled SM-nanoseconds per tile.
 cuapss_status join_fold(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float t,

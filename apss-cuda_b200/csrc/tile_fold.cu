@@ -31,9 +31,11 @@
 // is freed and the kernel returns.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "fold.cuh"
+#include "fold_tile.cuh"
 #include "ptx.cuh"
 
 namespace cuapss {
@@ -41,7 +43,7 @@ namespace cuapss {
 namespace {
 
 constexpr int kA = 5;                     // A ring slots (16 KB)
-constexpr int kB = kFoldResidentK / 64;   // B ring slots (32 KB)
+constexpr int kB = kFoldResident16 / kFoldChunk16;   // B ring slots (32 KB)
 constexpr int kMW = 2;                    // MMA warps, one per accumulator
 constexpr int kEW = 8;                    // epilogue warps
 constexpr int kFirstEpi = 4;              // a multiple of 4: lane quarter = warp % 4
@@ -59,45 +61,6 @@ constexpr size_t kOffMisc = kOffUnit + (size_t)kRing * 16 + 8;
 constexpr size_t kSmem = kOffMisc + 16 + 1024;  // + alignment slack
 static_assert(kSmem <= 232448, "shared memory budget");
 static_assert(kOffUnit % 8 == 0, "unit ring alignment");
-
-__device__ __forceinline__ bool wait_abort(uint64_t* bar, uint32_t parity,
-                                           const volatile int* abort) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = globaltimer_ns();
-  for (uint32_t i = 0; i < kMaxPolls; ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if (*abort || globaltimer_ns() - t0 >= kWaitLimitNs) return false;
-  }
-  return false;
-}
-
-__device__ __forceinline__ void give_up(int* err, volatile int* abort) {
-  if (!*abort) {
-    *abort = 1;
-    atomicOr(err, kErrTimeout);
-  }
-}
-
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort,
-                                          int* err, bool live) {
-  bool got = live ? wait_abort(bar, parity, abort) : true;
-  got = __all_sync(0xffffffffu, got);
-  if (live && !got && (threadIdx.x & 31) == 0) give_up(err, abort);
-  return live && got;
-}
-
-// Appends a warp's held candidates to the list: one reservation for up to
-// kHits of them.
-__device__ __forceinline__ void flush_hits(const FoldTileArgs& A, const uint64_t* hits, int n,
-                                           int lane) {
-  __syncwarp();
-  unsigned long long w = 0;
-  if (lane == 0) w = atomicAdd(A.cand_count, (unsigned long long)n);
-  w = __shfl_sync(0xffffffffu, w, 0);
-  for (int k = lane; k < n; k += 32)
-    if ((int64_t)w + k < A.cand_cap) A.cand[w + k] = hits[k];
-  __syncwarp();
-}
 
 // One 32-column group of a J row's products: the columns at or above thr
 // (bit j of the result), c of which exist (and, in a self-join, lie below
@@ -117,19 +80,6 @@ __device__ __forceinline__ float largest(const uint32_t (&v)[32]) {
   for (int j = 4; j < 32; ++j) m[j & 3] = fmaxf(m[j & 3], __uint_as_float(v[j]));
   return fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
 }
-
-// A unit {I, J0, J1, level | turn << 8}: its tiles in order, starting at
-// J0 + turn and wrapping around, so that CTAs that work on the same J blocks
-// at one time do not read the same L2 lines in step.
-struct Unit {
-  int I, J0, len, lev, turn;
-  __device__ explicit Unit(const int4& u)
-      : I(u.x), J0(u.y), len(u.z - u.y), lev(u.w & 0xff), turn(u.w >> 8) {}
-  __device__ int J(int k) const {
-    const int j = k + turn;
-    return J0 + (j < len ? j : j - len);
-  }
-};
 
 template <bool COUNT>
 __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constant__ FoldTileArgs A) {
@@ -199,7 +149,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
         uring[slot] = u;
         mbar_arrive(&ufull[slot]);
         if (u >= A.nunits) break;
-        const Unit U(A.units[u]);
+        const FoldUnit U(A.units[u]);
         const FoldLevel& L = A.lev[U.lev];
         const int nkc = L.nkc;
         const int wI = U.I + 1 < A.nbI ? 2 : 1;
@@ -271,7 +221,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
       __syncwarp();
       if (live && lane == 0) mbar_arrive(&uempty[slot]);
       if (u >= A.nunits) break;
-      const Unit U(A.units[u]);
+      const FoldUnit U(A.units[u]);
       const int nkc = A.lev[U.lev].nkc;
       const bool stream = nkc > kB;
       const uint32_t idesc = U.I + 1 < A.nbI ? idesc2 : idesc1;
@@ -342,7 +292,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
       __syncwarp();
       if (live && lane == 0) mbar_arrive(&uempty[slot]);
       if (u >= A.nunits) break;
-      const Unit U(A.units[u]);
+      const FoldUnit U(A.units[u]);
       const float eps = A.lev[U.lev].eps;
       const int I = U.I + half;
       const bool haveI = I < A.nbI;
@@ -431,9 +381,10 @@ cuapss_status tiles_fold_init() {
 
 }  // namespace
 
-cuapss_status launch_tiles_fold(const FoldTileArgs& a, int grid, cudaStream_t st, bool count) {
+cuapss_status launch_tiles_fold(const FoldTileArgs& a, int sms, cudaStream_t st, bool count) {
   ST_TRY(tiles_fold_init());
   if (a.nunits <= 0) return CUAPSS_OK;
+  const int grid = std::min(a.nunits, sms);
   if (count) k_tiles_fold<true><<<grid, kThreads, kSmem, st>>>(a);
   else k_tiles_fold<false><<<grid, kThreads, kSmem, st>>>(a);
   LAUNCH_CHECK();

@@ -33,9 +33,10 @@ def _signed(x, seed):
     return synth.Csr(x.rowptr, x.col, x.val * sign, x.d)
 
 
-@pytest.fixture(scope="module")
-def ctx():
-    with cuapss.Context(precision=cuapss.PREC_MIXED) as c:
+@pytest.fixture(scope="module", params=[cuapss.PREC_MIXED, cuapss.PREC_FP32],
+                ids=["mixed", "fp32"])
+def ctx(request):
+    with cuapss.Context(precision=request.param) as c:
         yield c
 
 
