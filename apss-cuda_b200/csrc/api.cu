@@ -81,9 +81,6 @@ struct TileCostModel {
 constexpr TileCostModel kProbedTail{388.0, 1.6, 0.06};
 constexpr TileCostModel kRarePaired{340.0, 1.84, 0.3};
 constexpr int kMaxModelHead = 8192;
-// Lowest threshold of the folded join: its margins (about 0.01) stay small
-// against t, and empty rows stay below it.
-constexpr float kFoldMinT = 0.05f;
 // SM-nanoseconds of an FP32 probing tile: the head, and per non-zero of the J
 // block (n = 800,000, 75 a row: 22 us; n = d = 1M, 120 a row: 32 us).
 constexpr double kPlainHeadNs = 5000.0, kPlainPostingNs = 1.75;
@@ -141,6 +138,10 @@ int choose_head_width(int precision, int64_t n, int64_t d, int64_t nnz,
   if (n <= 0 || prefix.size() < 2) return (int)std::min<int64_t>(1024, ((d + 63) / 64) * 64);
   double cost = 0.0;
   return best_head_width(n, nnz, prefix, rare_rank, rare_postings, &cost);
+}
+
+double plain_tile_ns(int64_t nnz, int64_t n) {
+  return kPlainHeadNs + kPlainPostingNs * kBlockRows * ((double)nnz / (double)std::max<int64_t>(n, 1));
 }
 
 bool head_bound_plan(int64_t p, int64_t n, int64_t nnz, const std::vector<int64_t>& prefix,
@@ -439,10 +440,7 @@ cuapss_status join_device(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, flo
     cudaEventRecord(ctx->ev[1], st);
     FoldResult fr;
     bool done = false;
-    // the FP32 probing tiles: their head at p = 64, and their probes
-    const double probing_ns =
-        mixed ? plan.tile_ns
-              : kPlainHeadNs + kPlainPostingNs * kBlockRows * ((double)nnz_all / (double)n_all);
+    const double probing_ns = mixed ? plan.tile_ns : plain_tile_ns(nnz_all, n_all);
     ST_TRY(join_fold(ctx, a, b, t, perm, nrm2, probing_ns, &fr, &done));
     if (done) {
       cudaEventRecord(ctx->ev[2], st);

@@ -82,4 +82,8 @@ TilePlan plan_tiles(int precision, int64_t n, int64_t d, int64_t nnz,
                     const std::vector<RareCandidate>& cands, int64_t max_pairs, int fixed_p,
                     bool forced = false);
 
+// Modelled SM-nanoseconds of an FP32 probing tile of rows with nnz / n
+// non-zeros each.
+double plain_tile_ns(int64_t nnz, int64_t n);
+
 }  // namespace cuapss

@@ -17,14 +17,14 @@ namespace cuapss {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kClasses = 16;  // length classes of a side
+constexpr int kClasses = kFoldClasses;
 // Upper edges of the classes as shares of the sorted rows: finer towards the
 // long rows, whose folded products spread the most.
 constexpr double kClassEdge[kClasses] = {0.125, 0.25, 0.375, 0.5,  0.625, 0.75,  0.8125, 0.875,
                                          0.92,  0.95, 0.97,  0.98, 0.988, 0.994, 0.998,  1.0};
-// Sides of fewer blocks keep the caller's order and one width, whose
+// Joins of fewer 128 x 128 tiles keep the caller's order and one width, whose
 // candidates are few or, past kSmallMaxCand, make the join fall back.
-constexpr int kSampleMinBlocks = 64;
+constexpr double kSampleMinTiles = 2048.0;
 constexpr int kSmallLevel = 3;
 constexpr int64_t kSmallMaxCand = 1 << 21;
 
@@ -63,11 +63,18 @@ inline unsigned grid_for(int64_t work, int per_block) {
 }
 
 // ---- row order: by length, in 256 classes of about 1/16 octave -----------
-__global__ void k_len_keys(const int64_t* __restrict__ rp, int64_t n, uint64_t* __restrict__ keys,
-                           uint32_t* __restrict__ vals) {
+// Rows with thresholds of their own are ordered by length over the squared
+// room between t and the usual product of unrelated rows: both make folded
+// products pass.
+__global__ void k_len_keys(const int64_t* __restrict__ rp, const float* __restrict__ t_row,
+                           int64_t n, uint64_t* __restrict__ keys, uint32_t* __restrict__ vals) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x) {
-    const float len = (float)(rp[i + 1] - rp[i]);
+    float len = (float)(rp[i + 1] - rp[i]);
+    if (t_row) {
+      const float room = fmaxf(t_row[i] - 0.15f, 0.1f);
+      len *= 0.1f / (room * room);
+    }
     keys[i] = (uint64_t)min(255, (int)(16.0f * __log2f(fmaxf(len, 1.0f))));
     vals[i] = (uint32_t)i;
   }
@@ -105,11 +112,6 @@ __global__ void k_sample_rows(const int32_t* __restrict__ rowmap, const int64_t*
 // shared columns are rounded up after widening by the largest error their
 // FP32 sums can have (2^-24 per addition), so their products bound the exact
 // ones.
-struct FoldOut {
-  uint8_t* base[kFoldLevels];  // null: not built
-  int first[kFoldLevels];      // block at offset 0
-};
-
 __host__ __device__ constexpr size_t fold_bytes(bool mixed, int level) {  // of a row block
   return (size_t)fold_k(mixed, level) * kBlockRows * (mixed ? 2 : 4);
 }
@@ -170,6 +172,8 @@ __device__ __forceinline__ void fold_write(uint32_t mask, const float* acc, uint
   }
 }
 
+// t_row (per caller's row, may be null): the row is folded divided by its
+// threshold, so that one threshold of 1 serves rows of different ones.
 // GROUP threads per row (a warp, or the whole CTA for long rows). Blocks
 // [b0, b1) of rowmap; blk_mask[b]: levels of block b (null: mask0 for all);
 // only blocks whose levels are all in `allow` (wide: some level is not
@@ -181,8 +185,8 @@ __global__ void __launch_bounds__(kThreads)
     k_fold_rows(const int32_t* __restrict__ rowmap, int64_t slot0, int64_t slot1,
                 const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
                 const float* __restrict__ val, const int32_t* __restrict__ perm,
-                const uint16_t* __restrict__ blk_mask, uint32_t mask0, uint32_t allow, bool wide,
-                FoldOut O) {
+                const float* __restrict__ t_row, const uint16_t* __restrict__ blk_mask,
+                uint32_t mask0, uint32_t allow, bool wide, FoldOut O) {
   extern __shared__ __align__(16) float fold_sm[];
   constexpr int kGroups = kThreads / GROUP;
   const int tid = threadIdx.x % GROUP;
@@ -200,9 +204,10 @@ __global__ void __launch_bounds__(kThreads)
       reinterpret_cast<float4*>(acc)[k] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (GROUP == 32) __syncwarp();
     else __syncthreads();
+    const float scale = t_row && r >= 0 ? __frcp_ru(t_row[r]) : 1.0f;
     for (int e = tid; e < len; e += GROUP) {
       const uint32_t f = (uint32_t)perm[col[lo + e]];
-      const float v = val[lo + e];
+      const float v = val[lo + e] * scale;
       fold_add<MIXED, 0>(mask, acc, allow, f, v);
       fold_add<MIXED, 1>(mask, acc, allow, f, v);
       fold_add<MIXED, 2>(mask, acc, allow, f, v);
@@ -236,9 +241,10 @@ static_assert(kFoldLevels == 10, "one fold_add / fold_write call per level");
 // Folds the places of [0, slots) with the levels of masks (host, per block;
 // empty: mask0 everywhere) into O.
 template <bool MIXED>
-cuapss_status fold_side(const DevCsr& x, const int32_t* rowmap, int64_t slots,
-                        const std::vector<uint16_t>& masks, uint32_t mask0, const int32_t* perm,
-                        const FoldOut& O, Workspace& ws, const std::string& tag, cudaStream_t st) {
+cuapss_status fold_places(const FoldSide& s, const int32_t* rowmap, int64_t slots,
+                          const std::vector<uint16_t>& masks, uint32_t mask0, const int32_t* perm,
+                          const FoldOut& O, Workspace& ws, const std::string& tag,
+                          cudaStream_t st) {
   uint16_t* d_mask = nullptr;
   // levels, and blocks, with and without a wide level
   uint32_t all[2] = {0, 0};
@@ -257,60 +263,56 @@ cuapss_status fold_side(const DevCsr& x, const int32_t* rowmap, int64_t slots,
       if (masks[b]) b1[w] = (int64_t)b + 1;
     }
   }
+  const DevCsr& x = s.x;
   if (all[0]) {  // a warp per row
     const size_t smem = (size_t)fold_offset(MIXED, all[0], kFoldLevels) * 4 * (kThreads / 32);
     CU_TRY(cudaFuncSetAttribute((const void*)k_fold_rows<MIXED, 32>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 fold_offset(MIXED, kNarrowLevels, kFoldLevels) * 4 *
                                     (kThreads / 32)));
-    k_fold_rows<MIXED, 32><<<grid_for((b1[0] - b0[0]) * kBlockRows, kThreads / 32), kThreads, smem, st>>>(
-        rowmap, b0[0] * kBlockRows, b1[0] * kBlockRows, x.rp, x.col, x.val, perm, d_mask, mask0,
-        all[0], false, O);
+    k_fold_rows<MIXED, 32>
+        <<<grid_for((b1[0] - b0[0]) * kBlockRows, kThreads / 32), kThreads, smem, st>>>(
+            rowmap, b0[0] * kBlockRows, b1[0] * kBlockRows, x.rp, x.col, x.val, perm, s.t_row,
+            d_mask, mask0, all[0], false, O);
     LAUNCH_CHECK();
   }
   if (all[1]) {  // blocks of long rows (and the samples): a CTA per row
     const size_t smem = (size_t)fold_offset(MIXED, all[1], kFoldLevels) * 4;
-    k_fold_rows<MIXED, kThreads><<<grid_for((b1[1] - b0[1]) * kBlockRows, 1), kThreads, smem, st>>>(
-        rowmap, b0[1] * kBlockRows, b1[1] * kBlockRows, x.rp, x.col, x.val, perm, d_mask, mask0,
-        all[1], true, O);
+    k_fold_rows<MIXED, kThreads>
+        <<<grid_for((b1[1] - b0[1]) * kBlockRows, 1), kThreads, smem, st>>>(
+            rowmap, b0[1] * kBlockRows, b1[1] * kBlockRows, x.rp, x.col, x.val, perm, s.t_row,
+            d_mask, mask0, all[1], true, O);
     LAUNCH_CHECK();
   }
   return CUAPSS_OK;
 }
 
-float fold_eps(bool mixed, int level, double nrm2) {
+// Margin of the bound at a level, for rows folded as they are (t_min = 1:
+// thresholds compare directly) or divided by thresholds of at least t_min.
+float fold_eps(bool mixed, int level, double nrm2, double t_min) {
   // mixed: BF16 rounding of the head columns, FP32 accumulation of K / 16
   // steps; FP32: a chain of K FMAs
   const int K = fold_k(mixed, level);
   const double head = mixed ? std::ldexp(1.0, -7) + std::ldexp(1.0, -16) : 0.0;
   const double acc =
       (mixed ? (K / 16.0 + 2.0) * std::ldexp(1.0, -20) : (K + 4.0) * std::ldexp(1.0, -24)) * 1.02;
-  return (float)((head + acc) * nrm2 * 1.001 + 1e-6);
+  return (float)(((head + acc) * nrm2 * 1.001 + 1e-6) / t_min);
 }
 
-struct FoldSide {
-  DevCsr x;
-  int nb = 0;
-  int32_t* rowmap = nullptr;      // [128 nb] place -> caller's row, -1 past n
-  int edge[kClasses + 1] = {};    // first block of each class (even), nb at the end
-  double len[kClasses] = {};      // mean row length of each class
-  int32_t* sample = nullptr;
-  std::vector<uint16_t> masks;     // levels of each block
-  FoldOut out{};
-};
-
-// Row order and class edges.
-cuapss_status order_side(FoldSide& s, bool by_length, Workspace& ws, const std::string& tag,
-                         cudaStream_t st) {
+// Row order (by length, or as given) and class edges.
+cuapss_status order_side(FoldSide& s, bool by_length, const FoldAlloc& alloc, Workspace& ws,
+                         const std::string& tag, cudaStream_t st) {
   s.nb = (int)ceil_div(s.x.n, kBlockRows);
   const int64_t slots = (int64_t)s.nb * kBlockRows;
-  ST_TRY(ws.get(tag + ":map", (size_t)slots, &s.rowmap));
+  void* map = nullptr;
+  ST_TRY(alloc("map", (size_t)slots * 4, &map));
+  s.rowmap = static_cast<int32_t*>(map);
   uint32_t* vals = nullptr;
   if (by_length) {
     uint64_t* keys = nullptr;
     ST_TRY(ws.get(tag + ":keys", (size_t)s.x.n, &keys));
     ST_TRY(ws.get(tag + ":vals", (size_t)s.x.n, &vals));
-    k_len_keys<<<grid_for(s.x.n, kThreads), kThreads, 0, st>>>(s.x.rp, s.x.n, keys, vals);
+    k_len_keys<<<grid_for(s.x.n, kThreads), kThreads, 0, st>>>(s.x.rp, s.t_row, s.x.n, keys, vals);
     LAUNCH_CHECK();
     ST_TRY(radix_sort_pairs(keys, vals, s.x.n, 8, ws, tag, st));
   }
@@ -328,105 +330,144 @@ ClassRows class_rows(const FoldSide& s) {
   return c;
 }
 
-// The width of every pair of classes, from the products of sampled rows.
-// level[a][b] (I class a, J class b; self: b >= a) and the modelled cost of
-// the join in SM-nanoseconds, with its expected candidates.
+constexpr int64_t kSampleSlots = (int64_t)kClasses * kBlockRows;
+
+// Samples a side's classes and folds the samples at every level of `levels`.
+// len_sum (device, kClasses words, zeroed) receives the sampled rows' lengths.
 template <bool MIXED>
-cuapss_status plan_levels(cuapss_ctx* ctx, FoldSide& I, FoldSide& J, bool self, float t,
-                          const int32_t* perm, double nrm2, int (*level)[kClasses], double* cost,
-                          double* cands) {
+cuapss_status sample_side(FoldSide& s, uint32_t levels, unsigned long long* len_sum,
+                          const int32_t* perm, const FoldAlloc& alloc, Workspace& ws,
+                          const std::string& tag, cudaStream_t st) {
+  void* p = nullptr;
+  ST_TRY(alloc("sample", (size_t)kSampleSlots * 4, &p));
+  s.sample = static_cast<int32_t*>(p);
+  k_sample_rows<<<kClasses, kBlockRows, 0, st>>>(s.rowmap, s.x.rp, class_rows(s), s.sample,
+                                                 len_sum);
+  LAUNCH_CHECK();
+  for (int l = 0; l < kFoldLevels; ++l) {
+    if (!((levels >> l) & 1u)) continue;
+    ST_TRY(alloc("sample" + std::to_string(l), kClasses * fold_bytes(MIXED, l), &p));
+    s.sample_out.base[l] = static_cast<uint8_t*>(p);
+  }
+  return fold_places<MIXED>(s, s.sample, kSampleSlots, {}, levels, perm, s.sample_out, ws, tag, st);
+}
+
+// One join of two sides (or of a side with itself) through the tile kernel.
+struct FoldTask {
+  FoldSide* I = nullptr;
+  FoldSide* J = nullptr;
+  bool self = false;
+  float t = 1.0f;           // threshold of the folded products
+  double t_min = 1.0;       // lowest threshold the I rows were divided by
+  int64_t j_offset = 0;     // added to the J row of every pair
+  int level[kClasses][kClasses] = {};  // width of each pair of classes
+  double cost = 0.0, cands = 0.0;      // modelled SM-nanoseconds, expected candidates
+  std::vector<int4> units;
+  int64_t tiles = 0;
+  int4* d_units = nullptr;
+  int64_t cap = 0;
+};
+
+// The width of every pair of classes, from the products of sampled rows, the
+// modelled cost of the join and its expected candidates. Levels the J side
+// does not hold (FoldSide::levels) are left out.
+template <bool MIXED>
+cuapss_status plan_levels(cuapss_ctx* ctx, FoldTask& k, const int32_t* perm, double nrm2) {
   Workspace& ws = ctx->ws;
   cudaStream_t st = ctx->stream;
-  const int64_t slots = (int64_t)kClasses * kBlockRows;
+  FoldSide& I = *k.I;
+  FoldSide& J = *k.J;
   const size_t ncnt = (size_t)kFoldLevels * kClasses * kClasses;
-  unsigned long long* stats = nullptr;  // row length sums, then pair counts
-  ST_TRY(ws.get("fold:stats", 2 * kClasses + ncnt / 2, &stats));
-  uint32_t* cnt = reinterpret_cast<uint32_t*>(stats + 2 * kClasses);
-  CU_TRY(cudaMemsetAsync(stats, 0, 8 * (2 * kClasses) + 4 * ncnt, st));
+  unsigned long long* stats = nullptr;  // row length sums, control words, pair counts
+  ST_TRY(ws.get("fold:stats", 2 * kClasses + 1 + ncnt / 2, &stats));
+  int* ctl = reinterpret_cast<int*>(stats + 2 * kClasses);
+  uint32_t* cnt = reinterpret_cast<uint32_t*>(stats + 2 * kClasses + 1);
+  const size_t stat_bytes = 8 * (2 * kClasses + 1) + 4 * ncnt;
+  CU_TRY(cudaMemsetAsync(stats, 0, stat_bytes, st));
+  uint32_t all = 0;
+  for (uint32_t m : J.levels) all |= m;
+  auto temp = [&](const char* tag) {
+    return [&ws, tag](const std::string& name, size_t bytes, void** out) {
+      return ws.get(tag + name, bytes, out);
+    };
+  };
+  ST_TRY(sample_side<MIXED>(I, all, stats, perm, temp("fold:sI:"), ws, "fold:sI", st));
+  if (!k.self && !J.sample)
+    ST_TRY(sample_side<MIXED>(J, all, stats + kClasses, perm, temp("fold:sJ:"), ws, "fold:sJ", st));
   FoldTileArgs ta;
-  FoldSide* side[2] = {&I, &J};
-  for (int k = 0; k < (self ? 1 : 2); ++k) {
-    FoldSide& s = *side[k];
-    const std::string tag = k == 0 ? "fold:sI" : "fold:sJ";
-    ST_TRY(ws.get(tag, (size_t)slots, &s.sample));
-    k_sample_rows<<<kClasses, kBlockRows, 0, st>>>(s.rowmap, s.x.rp, class_rows(s), s.sample,
-                                                   stats + k * kClasses);
-    LAUNCH_CHECK();
-    FoldOut o{};
-    for (int l = 0; l < kFoldLevels; ++l)
-      ST_TRY(ws.get(tag + std::to_string(l), kClasses * fold_bytes(MIXED, l), &o.base[l]));
-    ST_TRY(fold_side<MIXED>(s.x, s.sample, slots, {}, (1u << kFoldLevels) - 1u, perm, o, ws, tag, st));
-    for (int l = 0; l < kFoldLevels; ++l) {
-      if (k == 0) ta.lev[l].I = o.base[l];
-      if (k == 1 || self) ta.lev[l].J = o.base[l];
-    }
-  }
   std::vector<int4> units;
   for (int l = kFoldLevels - 1; l >= 0; --l) {
+    if (!((all >> l) & 1u)) continue;
+    ta.lev[l].I = I.sample_out.base[l];
+    ta.lev[l].J = J.sample_out.base[l];
     ta.lev[l].nkc = fold_k(MIXED, l) / kChunk<MIXED>;
-    ta.lev[l].eps = fold_eps(MIXED, l, nrm2);
-    for (int a = 0; a < kClasses; a += kPair<MIXED>)
-      for (int b = self ? a : 0; b < kClasses; ++b) units.push_back(make_int4(a, b, b + 1, l));
+    ta.lev[l].eps = fold_eps(MIXED, l, nrm2, k.t_min);
+    for (int a = 0; a < kClasses; a += kPair<MIXED>) {
+      if (I.edge[std::min(kClasses, a + kPair<MIXED>)] == I.edge[a]) continue;  // no rows
+      for (int b = k.self ? a : 0; b < kClasses; ++b)
+        if (J.edge[b + 1] > J.edge[b]) units.push_back(make_int4(a, b, b + 1, l));
+    }
   }
   int4* d_units = nullptr;
-  int* ctl = nullptr;
   ST_TRY(ws.get("fold:sunits", units.size(), &d_units));
-  ST_TRY(ws.get("fold:sctl", 2, &ctl));
   CU_TRY(cudaMemcpyAsync(d_units, units.data(), sizeof(int4) * units.size(),
                          cudaMemcpyHostToDevice, st));
-  CU_TRY(cudaMemsetAsync(ctl, 0, 2 * sizeof(int), st));
-  ta.nI = ta.nJ = slots;
+  ta.nI = ta.nJ = kSampleSlots;
   ta.nbI = ta.nbJ = kClasses;
-  ta.t = t;
+  ta.t = k.t;
   ta.units = d_units;
   ta.nunits = (int)units.size();
   ta.unit_counter = ctl;
   ta.err = ctl + 1;
   ta.class_count = cnt;
   ST_TRY(launch_fold<MIXED>(ta, ctx->sms, st, true));
-  std::vector<uint8_t> h(8 * 2 * kClasses + 4 * ncnt);
-  int herr = 0;
-  CU_TRY(cudaMemcpyAsync(h.data(), stats, h.size(), cudaMemcpyDeviceToHost, st));
-  CU_TRY(cudaMemcpyAsync(&herr, ctl + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+  std::vector<unsigned long long> h(stat_bytes / 8);
+  CU_TRY(cudaMemcpyAsync(h.data(), stats, stat_bytes, cudaMemcpyDeviceToHost, st));
   CU_TRY(cudaStreamSynchronize(st));
+  const int herr = (int)(h[2 * kClasses] >> 32);
   if (herr & kErrTimeout) return CUAPSS_ETIMEOUT;
   if (herr) return CUAPSS_ECUDA;
-  const unsigned long long* hl = reinterpret_cast<const unsigned long long*>(h.data());
-  const uint32_t* hc = reinterpret_cast<const uint32_t*>(hl + 2 * kClasses);
-  ClassRows cr[2] = {class_rows(I), class_rows(J)};
+  const uint32_t* hc = reinterpret_cast<const uint32_t*>(h.data() + 2 * kClasses + 1);
+  const ClassRows cr[2] = {class_rows(I), class_rows(J)};
   double rows[2][kClasses];
-  for (int k = 0; k < 2; ++k)
+  FoldSide* side[2] = {&I, &J};
+  for (int q = 0; q < 2; ++q)
     for (int c = 0; c < kClasses; ++c) {
-      rows[k][c] = (double)std::min<int64_t>(kBlockRows, cr[k].row[c + 1] - cr[k].row[c]);
-      const int src = self ? 0 : k;
-      side[k]->len[c] = rows[k][c] > 0 ? (double)hl[src * kClasses + c] / rows[k][c] : 0.0;
+      rows[q][c] = (double)std::min<int64_t>(kBlockRows, cr[q].row[c + 1] - cr[q].row[c]);
+      if (q == 1 && (k.self || J.prepared)) continue;  // known already
+      side[q]->len[c] = rows[q][c] > 0 ? (double)h[q * kClasses + c] / rows[q][c] : 0.0;
     }
-  *cost = *cands = 0.0;
+  // J chunks of a prepared index come from HBM: its bandwidth, an SM's share
+  const double load_ns_per_byte = J.prepared ? ctx->sms / 6500.0 : 0.0;
+  k.cost = k.cands = 0.0;
   for (int a = 0; a < kClasses; ++a)
-    for (int b = self ? a : 0; b < kClasses; ++b) {
-      const double sampled = rows[0][a] * rows[1][b] - (self && a == b ? rows[0][a] : 0.0);
+    for (int b = k.self ? a : 0; b < kClasses; ++b) {
+      const double sampled = rows[0][a] * rows[1][b] - (k.self && a == b ? rows[0][a] : 0.0);
       const double nI = (double)(cr[0].row[a + 1] - cr[0].row[a]);
       const double nJ = (double)(cr[1].row[b + 1] - cr[1].row[b]);
-      const double pairs = self && a == b ? nI * (nI - 1) / 2 : nI * nJ;
+      const double pairs = k.self && a == b ? nI * (nI - 1) / 2 : nI * nJ;
+      const double tiles = k.self ? pairs / ((double)kPair<MIXED> * kBlockRows * kBlockRows)
+                                  : std::ceil(nI / (kPair<MIXED> * kBlockRows)) *
+                                        std::ceil(nJ / kBlockRows);
       double best = 1e300, best_cand = 0.0;
-      level[a][b] = 0;
       for (int l = 0; l < kFoldLevels; ++l) {
+        if (!((J.levels[b] >> l) & 1u)) continue;
         double c = (double)hc[((size_t)l * kClasses + a) * kClasses + b];
-        if (self && a == b) c = std::max(0.0, c - rows[0][a]);  // a row with itself
+        if (k.self && a == b) c = std::max(0.0, c - rows[0][a]);  // a row with itself
         // a count of zero is not a share of zero: half a pair
         const double share = sampled > 0 ? std::max(c, 0.5) / sampled : 0.0;
-        const double tiles = pairs / ((double)kPair<MIXED> * kBlockRows * kBlockRows);
-        const double cand_ns =
-            kCandNs + kCandEntryNs * std::max(side[0]->len[a], side[1]->len[b]);
-        const double ns = tiles * tile_cost<MIXED>(l) + share * pairs * cand_ns;
+        const double cand_ns = kCandNs + kCandEntryNs * std::max(I.len[a], J.len[b]);
+        const double load = (double)fold_bytes(MIXED, l) * load_ns_per_byte;
+        const double ns = tiles * std::max(tile_cost<MIXED>(l), load) + share * pairs * cand_ns;
         if (ns < best) {
           best = ns;
           best_cand = share * pairs;
-          level[a][b] = l;
+          k.level[a][b] = l;
         }
       }
-      *cost += best;
-      *cands += best_cand;
+      if (pairs <= 0) continue;
+      k.cost += best;
+      k.cands += best_cand;
     }
   return CUAPSS_OK;
 }
@@ -437,10 +478,11 @@ int class_of(const FoldSide& s, int block) {
   return c;
 }
 
-// Allocates and builds the folded levels a side needs.
+// Allocates and builds the folded levels a side needs, per class.
 template <bool MIXED>
 cuapss_status build_levels(FoldSide& s, const uint32_t (&need)[kClasses], const int32_t* perm,
-                           Workspace& ws, const std::string& tag, cudaStream_t st) {
+                           const FoldAlloc& alloc, Workspace& ws, const std::string& tag,
+                           cudaStream_t st) {
   uint32_t all = 0;
   for (int c = 0; c < kClasses; ++c)
     if (s.edge[c + 1] > s.edge[c]) all |= need[c];
@@ -453,14 +495,15 @@ cuapss_status build_levels(FoldSide& s, const uint32_t (&need)[kClasses], const 
         hi = std::max(hi, s.edge[c + 1]);
       }
     s.out.first[l] = lo;
-    ST_TRY(ws.get(tag + ":lev" + std::to_string(l), (size_t)(hi - lo) * fold_bytes(MIXED, l),
-                  &s.out.base[l]));
+    void* p = nullptr;
+    ST_TRY(alloc("lev" + std::to_string(l), (size_t)(hi - lo) * fold_bytes(MIXED, l), &p));
+    s.out.base[l] = static_cast<uint8_t*>(p);
   }
-  s.masks.assign((size_t)s.nb, 0);
+  std::vector<uint16_t> masks((size_t)s.nb, 0);
   for (int c = 0; c < kClasses; ++c)
-    for (int b = s.edge[c]; b < s.edge[c + 1]; ++b) s.masks[(size_t)b] = (uint16_t)need[c];
-  return fold_side<MIXED>(s.x, s.rowmap, (int64_t)s.nb * kBlockRows, s.masks, 0, perm, s.out, ws,
-                          tag, st);
+    for (int b = s.edge[c]; b < s.edge[c + 1]; ++b) masks[(size_t)b] = (uint16_t)need[c];
+  return fold_places<MIXED>(s, s.rowmap, (int64_t)s.nb * kBlockRows, masks, 0, perm, s.out, ws,
+                            tag, st);
 }
 
 // Units: windows of J blocks from the long rows down (the costly units
@@ -468,11 +511,12 @@ cuapss_status build_levels(FoldSide& s, const uint32_t (&need)[kClasses], const 
 // that the CTAs running at one time share a window's chunks in L2. Wider
 // folds get proportionally shorter ranges.
 template <bool MIXED>
-void make_units(const FoldSide& I, const FoldSide& J, bool self, const int (*level)[kClasses],
-                int sms, std::vector<int4>* units, int64_t* tiles) {
+void make_units(FoldTask& k, int sms) {
+  const FoldSide& I = *k.I;
+  const FoldSide& J = *k.J;
   const int nbJ = J.nb;
   const int pair = kPair<MIXED>;
-  const double total = (self ? 0.5 * nbJ * (nbJ + 2.0) : (double)I.nb * nbJ) / pair;
+  const double total = k.self ? 0.5 * nbJ * (nbJ + 2.0) / pair : std::ceil((double)I.nb / pair) * nbJ;
   const int w = (int)std::max(1.0, std::min(MIXED ? 128.0 : 32.0, total / (sms * 16.0)));
   for (int j1 = nbJ; j1 > 0; j1 -= w) {
     const int j0 = std::max(0, j1 - w);
@@ -480,22 +524,153 @@ void make_units(const FoldSide& I, const FoldSide& J, bool self, const int (*lev
       const int s0 = std::max(j0, J.edge[b]), s1 = std::min(j1, J.edge[b + 1]);
       if (s0 >= s1) continue;
       int a = 0;
-      for (int i = 0; i < (self ? std::min(I.nb, s1) : I.nb); i += pair) {
+      for (int i = 0; i < (k.self ? std::min(I.nb, s1) : I.nb); i += pair) {
         while (i >= I.edge[a + 1]) ++a;
-        const int lv = level[a][b];
-        const int f0 = self ? std::max(s0, i) : s0;
+        const int lv = k.level[a][b];
+        const int f0 = k.self ? std::max(s0, i) : s0;
         const double rel = tile_cost<MIXED>(lv) / tile_cost<MIXED>(MIXED ? 1 : 3);
         const int step = std::max(1, (int)(w / std::max(1.0, rel)));
         for (int f = f0; f < s1; f += step) {
           const int len = std::min(s1 - f, step);
           // spread the starts of neighbouring units over the range
-          const int turn = (int)(((int64_t)(units->size() % 16) * len) / 16);
-          units->push_back(make_int4(i, f, f + len, lv | turn << 8));
+          const int turn = (int)(((int64_t)(k.units.size() % 16) * len) / 16);
+          k.units.push_back(make_int4(i, f, f + len, lv | turn << 8));
         }
       }
     }
   }
-  *tiles = self ? (int64_t)nbJ * (nbJ + 1) / 2 : (int64_t)I.nb * nbJ;
+  k.tiles = k.self ? (int64_t)nbJ * (nbJ + 1) / 2 : (int64_t)I.nb * nbJ;
+}
+
+// Widths for sides too small to sample: one for all.
+void one_level(FoldTask& k) {
+  for (auto& row : k.level)
+    for (int& l : row) l = kSmallLevel;  // K = 256 or 64
+}
+
+// The levels the sides of a task need, per class.
+void needed(const FoldTask& k, uint32_t (&needI)[kClasses], uint32_t (&needJ)[kClasses]) {
+  for (int x = 0; x < kClasses; ++x)
+    for (int y = k.self ? x : 0; y < kClasses; ++y) {
+      if (k.I->edge[x + 1] <= k.I->edge[x] || k.J->edge[y + 1] <= k.J->edge[y]) continue;
+      needI[x] |= 1u << k.level[x][y];
+      needJ[y] |= 1u << k.level[x][y];
+    }
+  if (k.self)
+    for (int c = 0; c < kClasses; ++c) needI[c] |= needJ[c];
+}
+
+cuapss_status upload_units(std::vector<FoldTask>& tasks, Workspace& ws, cudaStream_t st) {
+  std::vector<int4> all;
+  for (FoldTask& k : tasks) all.insert(all.end(), k.units.begin(), k.units.end());
+  int4* d = nullptr;
+  ST_TRY(ws.get("tiles:units", std::max<size_t>(all.size(), 1), &d));
+  if (!all.empty())
+    CU_TRY(cudaMemcpyAsync(d, all.data(), sizeof(int4) * all.size(), cudaMemcpyHostToDevice, st));
+  for (FoldTask& k : tasks) {
+    k.d_units = d;
+    d += k.units.size();
+  }
+  return CUAPSS_OK;
+}
+
+// Tiles and verification of all tasks into one unsorted pair list. *done =
+// false: the candidates do not fit what a folded join may take.
+template <bool MIXED>
+cuapss_status run_tasks(cuapss_ctx* ctx, std::vector<FoldTask>& tasks, double nrm2,
+                        const VerifyArgs& common, int64_t max_cand, FoldResult* r, bool* done) {
+  *done = false;
+  Workspace& ws = ctx->ws;
+  cudaStream_t st = ctx->stream;
+  const size_t nt = tasks.size();
+  // control words: pairs found, then per task candidates, {unit counter,
+  // verify's group counter}, error flags
+  unsigned long long* ctl = nullptr;
+  ST_TRY(ws.get("fold:ctl", 1 + 3 * nt, &ctl));
+  std::vector<unsigned long long> h(1 + 3 * nt);
+  for (int attempt = 0; attempt < 3; ++attempt) {
+    int64_t most = 1, room = 0;
+    for (FoldTask& k : tasks) {
+      most = std::max(most, k.cap);
+      room += k.cap;
+    }
+    uint64_t* cand = nullptr;
+    ST_TRY(ws.get("fold:cand", (size_t)most, &cand));  // the tasks run one after another
+    ST_TRY(ws.get("out:key", (size_t)room, &r->okey));
+    ST_TRY(ws.get("out:idx", (size_t)room, &r->oidx));
+    ST_TRY(ws.get("out:sim", (size_t)room, &r->osim));
+    CU_TRY(cudaMemsetAsync(ctl, 0, 8 * (1 + 3 * nt), st));
+    for (size_t i = 0; i < nt; ++i) {
+      FoldTask& k = tasks[i];
+      FoldTileArgs ta;
+      for (int l = 0; l < kFoldLevels; ++l) {
+        FoldLevel& L = ta.lev[l];
+        L.I = k.I->out.base[l];
+        L.J = k.J->out.base[l];
+        L.firstI = k.I->out.first[l];
+        L.firstJ = k.J->out.first[l];
+        L.nkc = fold_k(MIXED, l) / kChunk<MIXED>;
+        L.eps = fold_eps(MIXED, l, nrm2, k.t_min);
+        if (L.I) r->max_band = std::max(r->max_band, (double)L.eps);
+      }
+      ta.nI = k.I->slots ? k.I->slots : k.I->x.n;
+      ta.nJ = k.J->slots ? k.J->slots : k.J->x.n;
+      ta.nbI = k.I->nb;
+      ta.nbJ = k.J->nb;
+      ta.self = k.self ? 1 : 0;
+      ta.t = k.t;
+      ta.t_row = k.J->t_place;
+      ta.units = k.d_units;
+      ta.nunits = (int)k.units.size();
+      ta.cand = cand;
+      ta.cand_cap = k.cap;
+      ta.cand_count = ctl + 1 + 3 * i;
+      ta.unit_counter = reinterpret_cast<int*>(ctl + 2 + 3 * i);
+      ta.err = reinterpret_cast<int*>(ctl + 3 + 3 * i);
+      ST_TRY(launch_fold<MIXED>(ta, ctx->sms, st, false));
+      VerifyArgs va = common;
+      va.cand = cand;
+      va.ncand = ctl + 1 + 3 * i;
+      va.cap = k.cap;
+      va.work = reinterpret_cast<unsigned*>(ctl + 2 + 3 * i) + 1;
+      va.permI = k.I->rowmap;
+      va.permJ = k.J->rowmap;
+      va.rpI = k.I->x.rp;
+      va.colI = k.I->x.col;
+      va.valI = k.I->x.val;
+      va.rpJ = k.J->x.rp;
+      va.colJ = k.J->x.col;
+      va.valJ = k.J->x.val;
+      va.self = ta.self;
+      va.j_offset = k.j_offset;
+      va.out_key = r->okey;
+      va.out_idx = r->oidx;
+      va.out_sim = r->osim;
+      va.out_count = ctl;
+      ST_TRY(launch_verify(va, st));
+    }
+    CU_TRY(cudaMemcpyAsync(h.data(), ctl, 8 * (1 + 3 * nt), cudaMemcpyDeviceToHost, st));
+    CU_TRY(cudaStreamSynchronize(st));
+    bool over = false;
+    int64_t want = 0;
+    for (size_t i = 0; i < nt; ++i) {
+      const int herr = (int)h[3 + 3 * i];
+      if (herr & kErrTimeout) return CUAPSS_ETIMEOUT;
+      if (herr) return CUAPSS_ECUDA;
+      const int64_t c = (int64_t)h[1 + 3 * i];
+      want += c;
+      over = over || c > tasks[i].cap;
+      tasks[i].cap = std::max(tasks[i].cap, c);
+    }
+    r->npairs = (int64_t)h[0];
+    r->ncand = want;
+    if (!over) {
+      *done = true;
+      return CUAPSS_OK;
+    }
+    if (want > max_cand) return CUAPSS_OK;
+  }
+  return CUAPSS_OK;
 }
 
 template <bool MIXED>
@@ -509,118 +684,145 @@ cuapss_status join_fold_as(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, fl
   FoldSide SI, SJ;
   SI.x = a;
   if (!self) SJ.x = *b;
-  FoldSide& J = self ? SI : SJ;
-  const int64_t nbI = ceil_div(SI.x.n, kBlockRows), nbJ = ceil_div(J.x.n, kBlockRows);
+  std::vector<FoldTask> tasks(1);
+  FoldTask& k = tasks[0];
+  k.I = &SI;
+  k.J = self ? &SI : &SJ;
+  k.self = self;
+  k.t = t;
+  const int64_t nbI = ceil_div(SI.x.n, kBlockRows), nbJ = ceil_div(k.J->x.n, kBlockRows);
   const double tiles128 = self ? 0.5 * nbI * (nbI + 1.0) : (double)nbI * nbJ;
-  const bool sampled = tiles128 >= 0.5 * kSampleMinBlocks * kSampleMinBlocks;
-  ST_TRY(order_side(SI, sampled, ws, "fold:I", st));
-  if (!self) ST_TRY(order_side(SJ, sampled, ws, "fold:J", st));
-  int level[kClasses][kClasses];
-  double cands = 0.0;
+  const bool sampled = tiles128 >= kSampleMinTiles;
+  auto allocI = [&ws](const std::string& name, size_t bytes, void** out) {
+    return ws.get("fold:I:" + name, bytes, out);
+  };
+  auto allocJ = [&ws](const std::string& name, size_t bytes, void** out) {
+    return ws.get("fold:J:" + name, bytes, out);
+  };
+  ST_TRY(order_side(SI, sampled, allocI, ws, "fold:I", st));
+  if (!self) ST_TRY(order_side(SJ, sampled, allocJ, ws, "fold:J", st));
   if (sampled) {
-    double cost = 0.0;
-    ST_TRY(plan_levels<MIXED>(ctx, SI, J, self, t, perm, nrm2, level, &cost, &cands));
-    if (cost >= tiles128 * other_ns) return CUAPSS_OK;
+    ST_TRY(plan_levels<MIXED>(ctx, k, perm, nrm2));
+    if (k.cost >= tiles128 * other_ns) return CUAPSS_OK;
   } else {
-    for (auto& row : level)
-      for (int& l : row) l = kSmallLevel;  // K = 256 or 64
+    one_level(k);
   }
-  // ---- folded operands
   uint32_t needI[kClasses] = {}, needJ[kClasses] = {};
-  for (int x = 0; x < kClasses; ++x)
-    for (int y = self ? x : 0; y < kClasses; ++y) {
-      if (SI.edge[x + 1] <= SI.edge[x] || J.edge[y + 1] <= J.edge[y]) continue;
-      needI[x] |= 1u << level[x][y];
-      needJ[y] |= 1u << level[x][y];
-    }
-  if (self)
-    for (int c = 0; c < kClasses; ++c) needI[c] |= needJ[c];
-  ST_TRY(build_levels<MIXED>(SI, needI, perm, ws, "fold:I", st));
-  if (!self) ST_TRY(build_levels<MIXED>(SJ, needJ, perm, ws, "fold:J", st));
-  // ---- units
-  std::vector<int4> units;
-  make_units<MIXED>(SI, J, self, level, ctx->sms, &units, &r->tiles);
-  int4* d_units = nullptr;
-  ST_TRY(ws.get("tiles:units", std::max<size_t>(units.size(), 1), &d_units));
-  if (!units.empty())
-    CU_TRY(cudaMemcpyAsync(d_units, units.data(), sizeof(int4) * units.size(),
-                           cudaMemcpyHostToDevice, st));
-  // control words: candidates, pairs found, {unit counter, verify's group
-  // counter}, error flags
-  unsigned long long* ctl = nullptr;
-  ST_TRY(ws.get("fold:ctl", 4, &ctl));
-  FoldTileArgs ta;
-  for (int l = 0; l < kFoldLevels; ++l) {
-    FoldLevel& L = ta.lev[l];
-    L.I = SI.out.base[l];
-    L.J = J.out.base[l];
-    L.firstI = SI.out.first[l];
-    L.firstJ = J.out.first[l];
-    L.nkc = fold_k(MIXED, l) / kChunk<MIXED>;
-    L.eps = fold_eps(MIXED, l, nrm2);
-    if (SI.out.base[l]) r->max_band = std::max(r->max_band, (double)L.eps);
-  }
-  ta.nI = SI.x.n;
-  ta.nJ = J.x.n;
-  ta.nbI = SI.nb;
-  ta.nbJ = J.nb;
-  ta.self = self ? 1 : 0;
-  ta.t = t;
-  ta.units = d_units;
-  ta.nunits = (int)units.size();
-  ta.cand_count = ctl;
-  ta.unit_counter = reinterpret_cast<int*>(ctl + 2);
-  ta.err = reinterpret_cast<int*>(ctl + 3);
+  needed(k, needI, needJ);
+  ST_TRY(build_levels<MIXED>(SI, needI, perm, allocI, ws, "fold:I", st));
+  if (!self) ST_TRY(build_levels<MIXED>(SJ, needJ, perm, allocJ, ws, "fold:J", st));
+  make_units<MIXED>(k, ctx->sms);
+  ST_TRY(upload_units(tasks, ws, st));
+  r->tiles = k.tiles;
   r->rbitsI = std::max(1, bits_for((uint64_t)SI.x.n));
-  r->rbitsJ = std::max(1, bits_for((uint64_t)J.x.n));
+  r->rbitsJ = std::max(1, bits_for((uint64_t)k.J->x.n));
+  k.cap = std::max<int64_t>(sampled ? (int64_t)(1.5 * k.cands) : 0,
+                            std::max<int64_t>(1 << 20, SI.x.n + k.J->x.n));
   VerifyArgs va;
-  va.permI = SI.rowmap;
-  va.permJ = J.rowmap;
-  va.rpI = SI.x.rp;
-  va.colI = SI.x.col;
-  va.valI = SI.x.val;
-  va.rpJ = J.x.rp;
-  va.colJ = J.x.col;
-  va.valJ = J.x.val;
   va.t = t;
-  va.self = ta.self;
   va.rbits = r->rbitsJ;
-  va.ncand = ctl;
-  va.out_count = ctl + 1;
-  va.work = reinterpret_cast<unsigned*>(ctl + 2) + 1;
-  int64_t cap = std::max<int64_t>(sampled ? (int64_t)(1.5 * cands) : 0,
-                                  std::max<int64_t>(1 << 20, SI.x.n + J.x.n));
-  for (int attempt = 0; attempt < 3; ++attempt) {
-    ST_TRY(ws.get("fold:cand", (size_t)cap, &ta.cand));
-    ST_TRY(ws.get("out:key", (size_t)cap, &r->okey));
-    ST_TRY(ws.get("out:idx", (size_t)cap, &r->oidx));
-    ST_TRY(ws.get("out:sim", (size_t)cap, &r->osim));
-    ta.cand_cap = cap;
-    CU_TRY(cudaMemsetAsync(ctl, 0, 4 * sizeof(unsigned long long), st));
-    ST_TRY(launch_fold<MIXED>(ta, ctx->sms, st, false));
-    va.cand = ta.cand;
-    va.cap = cap;
-    va.out_key = r->okey;
-    va.out_idx = r->oidx;
-    va.out_sim = r->osim;
-    ST_TRY(launch_verify(va, st));
-    unsigned long long h[4] = {0, 0, 0, 0};
-    CU_TRY(cudaMemcpyAsync(h, ctl, sizeof(h), cudaMemcpyDeviceToHost, st));
-    CU_TRY(cudaStreamSynchronize(st));
-    if (h[3] & kErrTimeout) return CUAPSS_ETIMEOUT;
-    if (h[3]) return CUAPSS_ECUDA;
-    r->ncand = (int64_t)h[0];
-    r->npairs = (int64_t)h[1];
-    if (r->ncand <= cap) {
-      *done = true;
-      return CUAPSS_OK;
-    }
-    // an unsampled join that the bound does not prune, or one whose sample
-    // misjudged it: the probing path takes it
-    if (r->ncand > (sampled ? 4 * cap : kSmallMaxCand)) return CUAPSS_OK;
-    cap = r->ncand;
+  // an unsampled join that the bound does not prune, or one whose sample
+  // misjudged it, is left to the probing path
+  return run_tasks<MIXED>(ctx, tasks, nrm2, va, sampled ? 4 * k.cap : kSmallMaxCand, r, done);
+}
+
+// ---- resident index -------------------------------------------------------
+// Levels a segment holds for its classes: narrow ones for every row, wide
+// ones for the long rows.
+template <bool MIXED>
+uint32_t index_levels(int c, bool sampled) {
+  if (!sampled) return 1u << kSmallLevel;
+  // mixed: 64, 128, 256 | 512 | 1,024 | 2,048; FP32: 32, 64, 128 | 256 | 512 | 1,024
+  const uint32_t base = MIXED ? 0x0bu : 0x2au;
+  const uint32_t wide[3] = {MIXED ? 1u << 6 : 1u << 7, 1u << 8, 1u << 9};
+  return base | (c >= 4 ? wide[0] : 0) | (c >= 9 ? wide[1] : 0) | (c >= 13 ? wide[2] : 0);
+}
+
+template <bool MIXED>
+cuapss_status fold_index_as(cuapss_ctx* ctx, const DevCsr& x, const int32_t* perm,
+                            const FoldAlloc& alloc, FoldSide* s) {
+  Workspace& ws = ctx->ws;
+  cudaStream_t st = ctx->stream;
+  s->x = x;
+  s->prepared = true;
+  const bool sampled = ceil_div(x.n, kBlockRows) >= 2 * kClasses;
+  ST_TRY(order_side(*s, sampled, alloc, ws, "fold:X", st));
+  uint32_t need[kClasses];
+  uint32_t all = 0;
+  for (int c = 0; c < kClasses; ++c) {
+    need[c] = s->levels[c] = index_levels<MIXED>(c, sampled);
+    all |= need[c];
+  }
+  ST_TRY(build_levels<MIXED>(*s, need, perm, alloc, ws, "fold:X", st));
+  if (!sampled) return CUAPSS_OK;
+  unsigned long long* len_sum = nullptr;
+  ST_TRY(ws.get("fold:xlen", kClasses, &len_sum));
+  CU_TRY(cudaMemsetAsync(len_sum, 0, 8 * kClasses, st));
+  ST_TRY(sample_side<MIXED>(*s, all, len_sum, perm, alloc, ws, "fold:X", st));
+  unsigned long long h[kClasses];
+  CU_TRY(cudaMemcpyAsync(h, len_sum, sizeof(h), cudaMemcpyDeviceToHost, st));
+  CU_TRY(cudaStreamSynchronize(st));
+  const ClassRows cr = class_rows(*s);
+  for (int c = 0; c < kClasses; ++c) {
+    const int64_t m = std::min<int64_t>(kBlockRows, cr.row[c + 1] - cr.row[c]);
+    s->len[c] = m > 0 ? (double)h[c] / (double)m : 0.0;
   }
   return CUAPSS_OK;
+}
+
+template <bool MIXED>
+cuapss_status fold_query_as(cuapss_ctx* ctx, const std::vector<FoldSegment>& segs,
+                            const DevCsr& q, const float* t_row, float t_min, const int32_t* perm,
+                            double nrm2, double other_ns, int64_t rows, FoldResult* r,
+                            bool* done) {
+  *done = false;
+  Workspace& ws = ctx->ws;
+  cudaStream_t st = ctx->stream;
+  FoldSide Q;
+  Q.x = q;
+  Q.t_row = t_row;
+  auto alloc = [&ws](const std::string& name, size_t bytes, void** out) {
+    return ws.get("fold:Q:" + name, bytes, out);
+  };
+  // several blocks of queries: those with much to compare together
+  ST_TRY(order_side(Q, q.n > 2 * kBlockRows, alloc, ws, "fold:Q", st));
+  std::vector<FoldTask> tasks(segs.size());
+  uint32_t needQ[kClasses] = {};
+  double cost = 0.0;
+  r->tiles = 0;
+  for (size_t i = 0; i < segs.size(); ++i) {
+    FoldTask& k = tasks[i];
+    k.I = &Q;
+    k.J = segs[i].side;
+    k.t = 1.0f;
+    k.t_min = t_min;
+    k.j_offset = segs[i].row0;
+    const double tiles128 = (double)Q.nb * k.J->nb;
+    const bool sampled = k.J->sample != nullptr && tiles128 >= kSampleMinTiles;
+    if (sampled) {
+      ST_TRY(plan_levels<MIXED>(ctx, k, perm, nrm2));
+      cost += k.cost;
+    } else {
+      one_level(k);
+      cost += tiles128 * tile_cost<MIXED>(kSmallLevel) / kPair<MIXED>;
+    }
+    uint32_t needJ[kClasses] = {};
+    needed(k, needQ, needJ);
+    make_units<MIXED>(k, ctx->sms);
+    r->tiles += k.tiles;
+    k.cap = std::max<int64_t>(sampled ? (int64_t)(2.0 * k.cands) : 0, 1 << 18);
+  }
+  if (cost >= (double)r->tiles * other_ns) return CUAPSS_OK;
+  ST_TRY(build_levels<MIXED>(Q, needQ, perm, alloc, ws, "fold:Q", st));
+  ST_TRY(upload_units(tasks, ws, st));
+  r->rbitsI = std::max(1, bits_for((uint64_t)q.n));
+  r->rbitsJ = std::max(1, bits_for((uint64_t)std::max<int64_t>(rows, 1)));
+  VerifyArgs va;
+  va.t_of_i = t_row;
+  va.rbits = r->rbitsJ;
+  int64_t max_cand = kSmallMaxCand;
+  for (const FoldTask& k : tasks) max_cand = std::max(max_cand, 4 * k.cap);
+  return run_tasks<MIXED>(ctx, tasks, nrm2, va, max_cand, r, done);
 }
 
 }  // namespace
@@ -631,6 +833,20 @@ cuapss_status join_fold(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float
   return ctx->opts.precision == CUAPSS_PREC_MIXED
              ? join_fold_as<true>(ctx, a, b, t, perm, nrm2, other_ns, r, done)
              : join_fold_as<false>(ctx, a, b, t, perm, nrm2, other_ns, r, done);
+}
+
+cuapss_status fold_index(cuapss_ctx* ctx, bool mixed, const DevCsr& x, const int32_t* perm,
+                         const FoldAlloc& alloc, FoldSide* s) {
+  return mixed ? fold_index_as<true>(ctx, x, perm, alloc, s)
+               : fold_index_as<false>(ctx, x, perm, alloc, s);
+}
+
+cuapss_status fold_query(cuapss_ctx* ctx, bool mixed, const std::vector<FoldSegment>& segs,
+                         const DevCsr& q, const float* t_row, float t_min, const int32_t* perm,
+                         double nrm2, double other_ns, int64_t rows, FoldResult* r, bool* done) {
+  return mixed ? fold_query_as<true>(ctx, segs, q, t_row, t_min, perm, nrm2, other_ns, rows, r, done)
+               : fold_query_as<false>(ctx, segs, q, t_row, t_min, perm, nrm2, other_ns, rows, r,
+                                      done);
 }
 
 }  // namespace cuapss

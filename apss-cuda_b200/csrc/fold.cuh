@@ -21,12 +21,18 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <functional>
+#include <string>
 #include <vector>
 
 #include "common.cuh"
 #include "ctx.cuh"
 
 namespace cuapss {
+
+// Lowest threshold of a folded join: its margins (about 0.01) stay small
+// against t, and empty rows stay below it.
+constexpr float kFoldMinT = 0.05f;
 
 // Widths. Mixed precision: BF16 folds multiplied on the tensor cores, in
 // 64-column chunks. FP32: FP32 folds multiplied on the CUDA cores, whose time
@@ -92,6 +98,35 @@ cuapss_status launch_tiles_fold(const FoldTileArgs& a, int sms, cudaStream_t st,
 // The FP32 form: units of one I block.
 cuapss_status launch_tiles_fold32(const FoldTileArgs& a, int sms, cudaStream_t st, bool count);
 
+constexpr int kFoldClasses = 16;  // length classes of a side
+
+struct FoldOut {
+  uint8_t* base[kFoldLevels] = {};  // null: not built
+  int first[kFoldLevels] = {};      // block at offset 0
+};
+
+// One operand: its CSR, the order of its rows and its folded levels.
+struct FoldSide {
+  DevCsr x;
+  int nb = 0;
+  int64_t slots = 0;              // places, if some inside are empty (else x.n)
+  int32_t* rowmap = nullptr;      // [128 nb] place -> caller's row, -1: empty
+  const float* t_row = nullptr;   // per caller's row: rows are folded divided by it
+  const float* t_place = nullptr; // per place: threshold of the row's products
+  int edge[kFoldClasses + 1] = {};   // first block of each class (even), nb at the end
+  double len[kFoldClasses] = {};     // mean row length of each class
+  uint32_t levels[kFoldClasses];     // levels that may be used
+  bool prepared = false;          // a resident index's side
+  FoldOut out;
+  int32_t* sample = nullptr;      // sampled rows, up to 128 per class
+  FoldOut sample_out;
+  FoldSide() {
+    for (uint32_t& l : levels) l = (1u << kFoldLevels) - 1u;
+  }
+};
+
+using FoldAlloc = std::function<cuapss_status(const std::string& name, size_t bytes, void** out)>;
+
 // Exact decision of candidates (verify.cu).
 struct VerifyArgs {
   const uint64_t* cand = nullptr;
@@ -107,7 +142,9 @@ struct VerifyArgs {
   const int32_t* colJ = nullptr;
   const float* valJ = nullptr;
   float t = 0.f;
-  const float* t_row = nullptr;  // threshold of each J place, or null: t
+  const float* t_row = nullptr;   // threshold of each J place, or
+  const float* t_of_i = nullptr;  // of each of the I side's caller rows, or null: t
+  int64_t j_offset = 0;              // added to the J row of every pair
   int self = 0;
   int rbits = 0;  // output key = (i << rbits) | j
   uint64_t* out_key = nullptr;
@@ -134,5 +171,22 @@ struct FoldResult {
 cuapss_status join_fold(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float t,
                         const int32_t* perm, double nrm2, double other_ns, FoldResult* r,
                         bool* done);
+
+// A resident index segment's side: order, levels and samples of x's rows,
+// allocated through alloc.
+cuapss_status fold_index(cuapss_ctx* ctx, bool mixed, const DevCsr& x, const int32_t* perm,
+                         const FoldAlloc& alloc, FoldSide* s);
+
+struct FoldSegment {
+  FoldSide* side = nullptr;
+  int64_t row0 = 0;
+};
+
+// The folded join of query rows (thresholds t_row, device, at least t_min)
+// with the segments of an index of `rows` rows. *done and other_ns as in
+// join_fold.
+cuapss_status fold_query(cuapss_ctx* ctx, bool mixed, const std::vector<FoldSegment>& segs,
+                         const DevCsr& q, const float* t_row, float t_min, const int32_t* perm,
+                         double nrm2, double other_ns, int64_t rows, FoldResult* r, bool* done);
 
 }  // namespace cuapss

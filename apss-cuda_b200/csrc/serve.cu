@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "ctx.cuh"
+#include "fold.cuh"
 #include "prep.cuh"
 #include "serve.h"
 #include "prims.cuh"
@@ -120,6 +121,8 @@ struct Segment {
   int64_t* hptr = nullptr;
   uint2* rec = nullptr;
   int64_t ntail = 0;
+  // folded rows (fold.cuh), if the index has them
+  std::unique_ptr<FoldSide> fold;
 };
 
 using SegList = std::vector<std::shared_ptr<const Segment>>;
@@ -147,6 +150,8 @@ struct cuapss_index {
   cudaStream_t free_st = nullptr;  // stream-ordered frees of dropped segments
   bool mixed = false;
   int p = 0;
+  bool fold = false;      // queries go through the folded rows where those prune
+  double tile_ns = 0.0;   // modelled SM-nanoseconds of a probing tile
   int64_t d = 0;
   float norm_tol = 1e-4f;
   int validate = 1;
@@ -207,6 +212,20 @@ cuapss_status build_segment(cuapss_ctx* ctx, const cuapss_index* idx, const DevC
   }
   ST_TRY(H.copy(S.hptr, (size_t)kJSegs * nb + 1, &seg->hptr, st));
   ST_TRY(H.copy(S.bil_rec, (size_t)std::max<int64_t>(S.ntail, 1), &seg->rec, st));
+  if (idx->fold && x.n > 0) {
+    DevCsr own = x;
+    own.rp = seg->rp;
+    own.col = seg->col;
+    own.val = seg->val;
+    seg->fold = std::make_unique<FoldSide>();
+    auto alloc = [&H](const std::string&, size_t bytes, void** out) {
+      uint8_t* p = nullptr;
+      const cuapss_status r = H.alloc(bytes, &p);
+      *out = p;
+      return r;
+    };
+    ST_TRY(fold_index(ctx, idx->mixed, own, idx->perm, alloc, seg->fold.get()));
+  }
   CU_TRY(cudaStreamSynchronize(st));
   *out = std::move(seg);
   return CUAPSS_OK;
@@ -256,6 +275,18 @@ cuapss_status concat_segments(cuapss_ctx* ctx, const Segment& a, const Segment& 
 
 constexpr size_t kMaxSegments = 24;
 
+void query_times(cuapss_ctx* ctx, cuapss_stats* stats) {
+  float ms = 0.f;
+  cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
+  stats->ms_preprocess = ms;
+  cudaEventElapsedTime(&ms, ctx->ev[1], ctx->ev[2]);
+  stats->ms_tiles = ms;
+  cudaEventElapsedTime(&ms, ctx->ev[2], ctx->ev[3]);
+  stats->ms_finalize = ms;
+  cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[3]);
+  stats->ms_total = ms;
+}
+
 }  // namespace
 }  // namespace cuapss
 
@@ -296,7 +327,12 @@ extern "C" cuapss_status cuapss_index_create(cuapss_ctx* ctx, const cuapss_csr* 
     std::vector<int64_t> prefix;
     if (idx->mixed)
       ST_TRY(rank_count_prefix(counts, a.d, ctx->opts.remap, 8192, ctx->ws, ctx->stream, &prefix));
-    p = choose_head_width(ctx->opts.precision, a.n, a.d, a.nnz, prefix);
+    const TilePlan plan =
+        plan_tiles(ctx->opts.precision, a.n, a.d, a.nnz, prefix, {}, 0, 0);
+    p = plan.p;
+    idx->tile_ns = idx->mixed ? plan.tile_ns : plain_tile_ns(a.nnz, a.n);
+    // a given head width, or no remap, fix how the index is probed
+    idx->fold = ctx->opts.remap != 0;
   }
   const int pq = idx->mixed ? 64 : 32;
   p = (int)std::min<int64_t>(((int64_t)p + pq - 1) / pq * pq, ceil_div(a.d, pq) * pq);
@@ -453,6 +489,49 @@ cuapss_status cuapss::index_query_rows(cuapss_ctx* ctx, const cuapss_index* idx,
   ST_TRY(check_rows(ctx, idx, q, nullptr, &nrm_q, "QX"));
   const double nrm2 = nrm_q * nrm_idx;
   if (nrm2 >= 1.9) return CUAPSS_EINVAL;
+  float* t_row = nullptr;
+  ST_TRY(ws.get("Q:trow", (size_t)std::max<int64_t>(q.n, 1), &t_row));
+  if (q.n > 0)
+    CU_TRY(cudaMemcpyAsync(t_row, t, sizeof(float) * q.n, cudaMemcpyHostToDevice, st));
+  // ---- the folded rows, where they prune
+  const float t_min = q.n > 0 ? *std::min_element(t, t + q.n) : 0.0f;
+  if (idx->fold && q.n > 0 && rows > 0 && t_min >= kFoldMinT) {
+    nvtx.next("cuapss_index_query:tiles");
+    cudaEventRecord(ctx->ev[1], st);
+    std::vector<FoldSegment> fs;
+    for (const auto& g : segs)
+      if (g->fold) fs.push_back({g->fold.get(), g->row0});
+    // a probing tile also streams its J block's head and postings
+    const int64_t nbq = ceil_div(q.n, kBlockRows);
+    double block_bytes = (double)idx->p * kBlockRows * (idx->mixed ? 2.0 : 4.0);
+    for (const auto& g : segs) block_bytes += 8.0 * (double)g->ntail / ((double)rows / kBlockRows);
+    const double stream_ns = block_bytes * ctx->sms / 6500.0 / (double)nbq;
+    FoldResult fr;
+    bool done = false;
+    ST_TRY(fold_query(ctx, idx->mixed, fs, q, t_row, t_min, idx->perm, nrm2,
+                      std::max(idx->tile_ns, stream_ns), rows, &fr, &done));
+    if (done) {
+      cudaEventRecord(ctx->ev[2], st);
+      nvtx.next("cuapss_index_query:finalize");
+      const cuapss_status result = emit_pairs(ctx, fr.okey, fr.oidx, fr.osim, fr.npairs,
+                                              fr.rbitsI + fr.rbitsJ, fr.rbitsJ, out);
+      if (result != CUAPSS_OK && result != CUAPSS_EOVERFLOW) return result;
+      cudaEventRecord(ctx->ev[3], st);
+      CU_TRY(cudaStreamSynchronize(st));
+      if (stats) {
+        memset(stats, 0, sizeof(*stats));
+        stats->pairs = fr.npairs;
+        stats->candidates = stats->rescored = fr.ncand;
+        stats->tiles = fr.tiles;
+        stats->head_width = idx->p;
+        stats->max_band = fr.max_band;
+        query_times(ctx, stats);
+        stats->launches = g_launches.load() - launches0;
+      }
+      return result;
+    }
+    nvtx.next("cuapss_index_query:prepare");
+  }
   // ---- query side (I role)
   PrepOptions po;
   po.p = idx->p;
@@ -467,10 +546,6 @@ cuapss_status cuapss::index_query_rows(cuapss_ctx* ctx, const cuapss_index* idx,
   SQ.nnz = q.nnz;
   SQ.nrm_max = nrm_q;
   if (q.n > 0) ST_TRY(build_side(SQ, po, idx->perm, ws, "Q", st));
-  float* t_row = nullptr;
-  ST_TRY(ws.get("Q:trow", (size_t)std::max<int64_t>(q.n, 1), &t_row));
-  if (q.n > 0)
-    CU_TRY(cudaMemcpyAsync(t_row, t, sizeof(float) * q.n, cudaMemcpyHostToDevice, st));
   ST_TRY(tiles_init(idx->mixed));
   cudaEventRecord(ctx->ev[1], st);
   nvtx.next("cuapss_index_query:tiles");
@@ -659,26 +734,9 @@ cuapss_status cuapss::index_query_rows(cuapss_ctx* ctx, const cuapss_index* idx,
   CU_TRY(cudaMemcpyAsync(hcnt, ocount, sizeof(hcnt), cudaMemcpyDeviceToHost, st));
   CU_TRY(cudaStreamSynchronize(st));
   const int64_t npairs = (int64_t)hcnt[0];
-  ST_TRY(radix_sort_pairs(okey, oidx, npairs, rbitsI + rbitsJ, ws, "out", st));
-  out->count = npairs;
-  cuapss_status result = CUAPSS_OK;
-  if (npairs > out->capacity) {
-    result = CUAPSS_EOVERFLOW;
-  } else if (npairs > 0) {
-    if (out->on_device) {
-      ST_TRY(launch_split_pairs(okey, oidx, osim, npairs, rbitsJ, out->i, out->j, out->sim, st));
-    } else {
-      int32_t *di = nullptr, *dj = nullptr;
-      float* ds = nullptr;
-      ST_TRY(ws.get("out:i", (size_t)npairs, &di));
-      ST_TRY(ws.get("out:j", (size_t)npairs, &dj));
-      ST_TRY(ws.get("out:s", (size_t)npairs, &ds));
-      ST_TRY(launch_split_pairs(okey, oidx, osim, npairs, rbitsJ, di, dj, ds, st));
-      CU_TRY(cudaMemcpyAsync(out->i, di, sizeof(int32_t) * npairs, cudaMemcpyDeviceToHost, st));
-      CU_TRY(cudaMemcpyAsync(out->j, dj, sizeof(int32_t) * npairs, cudaMemcpyDeviceToHost, st));
-      CU_TRY(cudaMemcpyAsync(out->sim, ds, sizeof(float) * npairs, cudaMemcpyDeviceToHost, st));
-    }
-  }
+  const cuapss_status result =
+      emit_pairs(ctx, okey, oidx, osim, npairs, rbitsI + rbitsJ, rbitsJ, out);
+  if (result != CUAPSS_OK && result != CUAPSS_EOVERFLOW) return result;
   cudaEventRecord(ctx->ev[3], st);
   CU_TRY(cudaStreamSynchronize(st));
   if (stats) {
@@ -689,15 +747,7 @@ cuapss_status cuapss::index_query_rows(cuapss_ctx* ctx, const cuapss_index* idx,
     stats->tiles = ntiles;
     stats->head_width = idx->p;
     stats->tail_entries = SQ.ntail;
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
-    stats->ms_preprocess = ms;
-    cudaEventElapsedTime(&ms, ctx->ev[1], ctx->ev[2]);
-    stats->ms_tiles = ms;
-    cudaEventElapsedTime(&ms, ctx->ev[2], ctx->ev[3]);
-    stats->ms_finalize = ms;
-    cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[3]);
-    stats->ms_total = ms;
+    query_times(ctx, stats);
     stats->launches = g_launches.load() - launches0;
   }
   return result;

@@ -135,9 +135,9 @@ __global__ void __launch_bounds__(kThreads) k_verify(const VerifyArgs A) {
     if (lane < m) {
       const uint64_t key = A.cand[base + lane];
       const uint32_t ip = (uint32_t)(key >> 32), jp = (uint32_t)key;
-      t = A.t_row ? (double)A.t_row[jp] : (double)A.t;
       pi = A.permI ? (uint32_t)A.permI[ip] : ip;
       pj = A.permJ ? (uint32_t)A.permJ[jp] : jp;
+      t = A.t_of_i ? (double)A.t_of_i[pi] : A.t_row ? (double)A.t_row[jp] : (double)A.t;
       const int64_t a0 = A.rpI[pi], b0 = A.rpJ[pj];
       const int na = (int)(A.rpI[pi + 1] - a0), nb = (int)(A.rpJ[pj + 1] - b0);
       // equal lengths: the smaller row number of a self-join leads
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(kThreads) k_verify(const VerifyArgs A) {
     if (lane == 0) w = atomicAdd(A.out_count, (unsigned long long)__popc(found));
     w = __shfl_sync(kFull, w, 0) + (unsigned long long)__popc(found & ((1u << lane) - 1u));
     if (in) {  // w < nc <= cap
-      uint64_t x = pi, y = pj;
+      uint64_t x = pi, y = (uint64_t)pj + (uint64_t)A.j_offset;
       if (A.self && x > y) {
         x = pj;
         y = pi;
