@@ -736,6 +736,7 @@ cuapss_status cuapss_create(cuapss_ctx** out, const cuapss_opts* opts) {
     }
     c->own_stream = true;
   }
+  c->ws.set_stream(c->stream);
   for (auto& e : c->ev) cudaEventCreate(&e);
   *out = c;
   return CUAPSS_OK;

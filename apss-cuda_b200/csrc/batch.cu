@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "ctx.cuh"
+#include "fold.cuh"
 #include "prep.cuh"
 #include "prims.cuh"
 #include "tiles.cuh"
@@ -38,6 +39,9 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kNumBuckets = CUAPSS_BATCH_BUCKETS;
+// SM-nanoseconds of a mixed probing tile of the batched workload (512
+// instances of 64 .. 20,000 rows, 30 non-zeros: 21 ms over 0.55M tiles).
+constexpr double kBatchTileNs = 5600.0;
 constexpr int64_t kTuneRows = 65536;  // rows of a bucket's tuning sample
 
 inline int bucket_of(int64_t n) { return n <= 1024 ? 0 : (n <= 8192 ? 1 : 2); }
@@ -400,6 +404,52 @@ cuapss_status batch_device(cuapss_ctx* ctx, const DevCsr& x, int k, const int64_
                       counts, &nrm, ws, "A", st));
   if (nrm * nrm >= 1.9) return CUAPSS_EINVAL;  // fixed-point tail needs ~unit norms
   ST_TRY(feature_perm(counts, d, x.n, ctx->opts.remap, perm, ws, st));
+  // ---- the folded form, unless a head width or no remap fixes the probing
+  const float t_min = *std::min_element(tq, tq + k);
+  if (ctx->opts.head_width == 0 && ctx->opts.remap && x.n > 0 && t_min >= kFoldMinT) {
+    cudaEventRecord(ctx->ev[1], st);
+    nvtx.next("cuapss_batch_run:tiles");
+    // a mixed probing tile at p = 512 (its tuned width): 8 head chunks
+    const double other_ns = mixed ? kBatchTileNs : plain_tile_ns(x.nnz, x.n);
+    std::vector<int> width;
+    FoldResult fr;
+    bool done = false;
+    ST_TRY(fold_batch(ctx, x, k, inst_ptr, tq, perm, nrm * nrm, other_ns, &width, &fr, &done));
+    if (done) {
+      cudaEventRecord(ctx->ev[2], st);
+      nvtx.next("cuapss_batch_run:finalize");
+      const cuapss_status result = emit_pairs(ctx, fr.okey, fr.oidx, fr.osim, fr.npairs,
+                                              fr.rbitsI + fr.rbitsJ, fr.rbitsJ, out);
+      if (result != CUAPSS_OK && result != CUAPSS_EOVERFLOW) return result;
+      cudaEventRecord(ctx->ev[3], st);
+      CU_TRY(cudaStreamSynchronize(st));
+      int32_t widest[kNumBuckets] = {0, 0, 0};
+      int64_t tiles[kNumBuckets] = {0, 0, 0};
+      for (int q = 0; q < k; ++q) {
+        const int64_t n = inst_ptr[q + 1] - inst_ptr[q];
+        const int b = bucket_of(n);
+        widest[b] = std::max<int32_t>(widest[b], width[(size_t)q]);
+        tiles[b] += ceil_div(n, kBlockRows) * (ceil_div(n, kBlockRows) + 1) / 2;
+      }
+      if (bucket_p)
+        for (int b = 0; b < kNumBuckets; ++b) bucket_p[b] = widest[b];
+      if (stats) {
+        memset(stats, 0, sizeof(*stats));
+        stats->pairs = fr.npairs;
+        stats->candidates = stats->rescored = fr.ncand;
+        stats->tiles = fr.tiles;
+        stats->head_width = widest[std::max_element(tiles, tiles + kNumBuckets) - tiles];
+        stats->max_band = fr.max_band;
+        stats->ms_preprocess = elapsed_ms(ctx->ev[0], ctx->ev[1]);
+        stats->ms_tiles = elapsed_ms(ctx->ev[1], ctx->ev[2]);
+        stats->ms_finalize = elapsed_ms(ctx->ev[2], ctx->ev[3]);
+        stats->ms_total = elapsed_ms(ctx->ev[0], ctx->ev[3]);
+        stats->launches = g_launches.load() - launches0;
+      }
+      return result;
+    }
+    nvtx.next("cuapss_batch_run:prepare");
+  }
   BatchIn in;
   in.x = x;
   in.k = k;
@@ -565,26 +615,8 @@ cuapss_status batch_device(cuapss_ctx* ctx, const DevCsr& x, int k, const int64_
   CU_TRY(cudaMemcpyAsync(hcnt, ocount, sizeof(hcnt), cudaMemcpyDeviceToHost, st));
   CU_TRY(cudaStreamSynchronize(st));
   const int64_t npairs = (int64_t)hcnt[0];
-  ST_TRY(radix_sort_pairs(okey, oidx, npairs, 2 * rbits, ws, "out", st));
-  out->count = npairs;
-  cuapss_status result = CUAPSS_OK;
-  if (npairs > out->capacity) {
-    result = CUAPSS_EOVERFLOW;
-  } else if (npairs > 0) {
-    if (out->on_device) {
-      ST_TRY(launch_split_pairs(okey, oidx, osim, npairs, rbits, out->i, out->j, out->sim, st));
-    } else {
-      int32_t *di = nullptr, *dj = nullptr;
-      float* ds = nullptr;
-      ST_TRY(ws.get("out:i", (size_t)npairs, &di));
-      ST_TRY(ws.get("out:j", (size_t)npairs, &dj));
-      ST_TRY(ws.get("out:s", (size_t)npairs, &ds));
-      ST_TRY(launch_split_pairs(okey, oidx, osim, npairs, rbits, di, dj, ds, st));
-      CU_TRY(cudaMemcpyAsync(out->i, di, sizeof(int32_t) * npairs, cudaMemcpyDeviceToHost, st));
-      CU_TRY(cudaMemcpyAsync(out->j, dj, sizeof(int32_t) * npairs, cudaMemcpyDeviceToHost, st));
-      CU_TRY(cudaMemcpyAsync(out->sim, ds, sizeof(float) * npairs, cudaMemcpyDeviceToHost, st));
-    }
-  }
+  const cuapss_status result = emit_pairs(ctx, okey, oidx, osim, npairs, 2 * rbits, rbits, out);
+  if (result != CUAPSS_OK && result != CUAPSS_EOVERFLOW) return result;
   cudaEventRecord(ctx->ev[3], st);
   CU_TRY(cudaStreamSynchronize(st));
   if (stats) {

@@ -74,11 +74,15 @@ inline int bits_for(uint64_t v) {  // bits needed to represent values < v+1
   return b;
 }
 
-// Grow-only named device buffers owned by a context; avoids cudaMalloc on
-// every call.
+// Grow-only named device buffers owned by a context; avoids an allocation on
+// every call. Allocations and frees are ordered on the context's stream (all
+// its work runs there), so that neither waits for the device: building an
+// index of 200,000 rows spent 30 of 34 ms in cudaMalloc and cudaFree of its
+// temporaries.
 class Workspace {
  public:
   ~Workspace() { release(); }
+  void set_stream(cudaStream_t st) { st_ = st; }
   // Returns a device pointer with at least `bytes` bytes (256-byte aligned).
   cuapss_status get(const std::string& name, size_t bytes, void** out) {
     if (bytes == 0) bytes = 256;
@@ -88,15 +92,15 @@ class Workspace {
       return CUAPSS_OK;
     }
     if (it != bufs_.end()) {
-      cudaFree(it->second.ptr);
+      cudaFreeAsync(it->second.ptr, st_);
       bufs_.erase(it);
     }
     void* p = nullptr;
     size_t want = bytes + bytes / 8;  // headroom against regrowth
-    cudaError_t e = cudaMalloc(&p, want);
+    cudaError_t e = cudaMallocAsync(&p, want, st_);
     if (e != cudaSuccess) {
       cudaGetLastError();
-      e = cudaMalloc(&p, bytes);
+      e = cudaMallocAsync(&p, bytes, st_);
       want = bytes;
       if (e != cudaSuccess) {
         cudaGetLastError();
@@ -114,20 +118,26 @@ class Workspace {
     *out = static_cast<T*>(p);
     return s;
   }
+  // Bytes a buffer holds already (0: none).
+  size_t held(const std::string& name) const {
+    auto it = bufs_.find(name);
+    return it == bufs_.end() ? 0 : it->second.size;
+  }
   size_t bytes_held() const {
     size_t s = 0;
     for (auto& kv : bufs_) s += kv.second.size;
     return s;
   }
   void release() {
-    for (auto& kv : bufs_) cudaFree(kv.second.ptr);
+    for (auto& kv : bufs_) cudaFreeAsync(kv.second.ptr, st_);
+    if (!bufs_.empty()) cudaStreamSynchronize(st_);
     bufs_.clear();
   }
   // Frees the buffers whose names start with prefix.
   void release_prefix(const std::string& prefix) {
     for (auto it = bufs_.begin(); it != bufs_.end();) {
       if (it->first.compare(0, prefix.size(), prefix) == 0) {
-        cudaFree(it->second.ptr);
+        cudaFreeAsync(it->second.ptr, st_);
         it = bufs_.erase(it);
       } else {
         ++it;
@@ -141,6 +151,7 @@ class Workspace {
     size_t size;
   };
   std::map<std::string, Buf> bufs_;
+  cudaStream_t st_ = nullptr;
 };
 
 // NVTX ranges of a call's host-side stages (prepare, tiles, finalize), for

@@ -37,6 +37,8 @@ constexpr int64_t kSmallMaxCand = 1 << 21;
 // longer row.
 constexpr double kTileNs = 340.0, kChunkNs = 275.0, kStreamNs = 400.0;
 constexpr double kCandNs = 45.0, kCandEntryNs = 0.3;
+// Building a folded row, per column.
+constexpr double kFoldColumnNs = 0.05;
 // FP32, 128 x 128 tiles.
 constexpr double kTile32Ns = 380.0, kColumn32Ns = 92.0;
 
@@ -85,6 +87,34 @@ __global__ void k_order(const uint32_t* __restrict__ sorted, int64_t n, int64_t 
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < slots;
        i += (int64_t)gridDim.x * blockDim.x)
     rowmap[i] = i < n ? (sorted ? (int32_t)sorted[i] : (int32_t)i) : -1;
+}
+
+// ---- batches: each instance's rows from a block boundary on ---------------
+// tab[4 q ..] = {first place, first row, rows, threshold bits} of instance q;
+// places past its rows up to the next block boundary are empty.
+__global__ void k_batch_places(const int64_t* __restrict__ tab, int k, int32_t* __restrict__ rowmap,
+                               float* __restrict__ t_place) {
+  for (int q = blockIdx.x; q < k; q += gridDim.x) {
+    const int64_t S = tab[4 * q], R = tab[4 * q + 1], n = tab[4 * q + 2];
+    const float t = __int_as_float((int)tab[4 * q + 3]);
+    const int64_t npad = (n + kBlockRows - 1) / kBlockRows * kBlockRows;
+    for (int64_t r = threadIdx.x; r < npad; r += blockDim.x) {
+      rowmap[S + r] = r < n ? (int32_t)(R + r) : -1;
+      t_place[S + r] = t;
+    }
+  }
+}
+
+// kBatchSample rows evenly spaced over all n (rows past n: none).
+__global__ void k_spread_rows(const int64_t* __restrict__ rp, int64_t n, int slots,
+                              int32_t* __restrict__ sample, unsigned long long* __restrict__ len_sum) {
+  unsigned long long len = 0;
+  for (int i = threadIdx.x; i < slots; i += blockDim.x) {
+    const int64_t r = n >= slots ? (int64_t)i * n / slots : i;
+    sample[i] = r < n ? (int32_t)r : -1;
+    if (r < n) len += (unsigned long long)(rp[r + 1] - rp[r]);
+  }
+  if (len) atomicAdd(len_sum, len);
 }
 
 // ---- sampled rows: up to 128 of each class, evenly spaced ----------------
@@ -588,6 +618,11 @@ cuapss_status run_tasks(cuapss_ctx* ctx, std::vector<FoldTask>& tasks, double nr
   unsigned long long* ctl = nullptr;
   ST_TRY(ws.get("fold:ctl", 1 + 3 * nt, &ctl));
   std::vector<unsigned long long> h(1 + 3 * nt);
+  // room that earlier calls left is room to use
+  if (nt == 1)
+    tasks[0].cap = std::max<int64_t>(
+        tasks[0].cap, (int64_t)std::min({ws.held("fold:cand") / 8, ws.held("out:key") / 8,
+                                         ws.held("out:idx") / 4, ws.held("out:sim") / 4}));
   for (int attempt = 0; attempt < 3; ++attempt) {
     int64_t most = 1, room = 0;
     for (FoldTask& k : tasks) {
@@ -716,14 +751,15 @@ cuapss_status join_fold_as(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, fl
   r->tiles = k.tiles;
   r->rbitsI = std::max(1, bits_for((uint64_t)SI.x.n));
   r->rbitsJ = std::max(1, bits_for((uint64_t)k.J->x.n));
-  k.cap = std::max<int64_t>(sampled ? (int64_t)(1.5 * k.cands) : 0,
-                            std::max<int64_t>(1 << 20, SI.x.n + k.J->x.n));
+  // twice what the sample promises: a run that does not fit is run again
+  const int64_t expect = std::max<int64_t>(sampled ? (int64_t)(2.0 * k.cands) : 0, 1 << 20);
+  k.cap = expect + SI.x.n + k.J->x.n;
   VerifyArgs va;
   va.t = t;
   va.rbits = r->rbitsJ;
   // an unsampled join that the bound does not prune, or one whose sample
   // misjudged it, is left to the probing path
-  return run_tasks<MIXED>(ctx, tasks, nrm2, va, sampled ? 4 * k.cap : kSmallMaxCand, r, done);
+  return run_tasks<MIXED>(ctx, tasks, nrm2, va, sampled ? 4 * expect : kSmallMaxCand, r, done);
 }
 
 // ---- resident index -------------------------------------------------------
@@ -789,6 +825,7 @@ cuapss_status fold_query_as(cuapss_ctx* ctx, const std::vector<FoldSegment>& seg
   std::vector<FoldTask> tasks(segs.size());
   uint32_t needQ[kClasses] = {};
   double cost = 0.0;
+  int64_t max_cand = kSmallMaxCand;
   r->tiles = 0;
   for (size_t i = 0; i < segs.size(); ++i) {
     FoldTask& k = tasks[i];
@@ -811,6 +848,7 @@ cuapss_status fold_query_as(cuapss_ctx* ctx, const std::vector<FoldSegment>& seg
     make_units<MIXED>(k, ctx->sms);
     r->tiles += k.tiles;
     k.cap = std::max<int64_t>(sampled ? (int64_t)(2.0 * k.cands) : 0, 1 << 18);
+    max_cand = std::max(max_cand, 4 * k.cap);
   }
   if (cost >= (double)r->tiles * other_ns) return CUAPSS_OK;
   ST_TRY(build_levels<MIXED>(Q, needQ, perm, alloc, ws, "fold:Q", st));
@@ -820,9 +858,199 @@ cuapss_status fold_query_as(cuapss_ctx* ctx, const std::vector<FoldSegment>& seg
   VerifyArgs va;
   va.t_of_i = t_row;
   va.rbits = r->rbitsJ;
-  int64_t max_cand = kSmallMaxCand;
-  for (const FoldTask& k : tasks) max_cand = std::max(max_cand, 4 * k.cap);
   return run_tasks<MIXED>(ctx, tasks, nrm2, va, max_cand, r, done);
+}
+
+// ---- batches ---------------------------------------------------------------
+// Thresholds the sample is compared at: an instance takes the shares of the
+// highest of them that does not exceed its own.
+constexpr int kBatchT = kClasses;
+constexpr int kBatchI = 4;  // sampled I blocks
+
+template <bool MIXED>
+cuapss_status fold_batch_as(cuapss_ctx* ctx, const DevCsr& x, int k, const int64_t* inst_ptr,
+                            const float* t, const int32_t* perm, double nrm2, double other_ns,
+                            std::vector<int>* width, FoldResult* r, bool* done) {
+  *done = false;
+  Workspace& ws = ctx->ws;
+  cudaStream_t st = ctx->stream;
+  const int pair = kPair<MIXED>;
+  // ---- instances with pairs, by threshold
+  std::vector<int> inst;
+  double all_pairs = 0.0;
+  for (int q = 0; q < k; ++q) {
+    const double n = (double)(inst_ptr[q + 1] - inst_ptr[q]);
+    if (n < 2) continue;
+    inst.push_back(q);
+    all_pairs += n * n;
+  }
+  width->assign((size_t)k, 0);
+  if (inst.empty()) return CUAPSS_OK;
+  std::sort(inst.begin(), inst.end(), [&](int a, int b) { return t[a] != t[b] ? t[a] < t[b] : a < b; });
+  float grid[kBatchT];  // thresholds at equal shares of the pairs, the lowest first
+  {
+    double seen = 0.0;
+    int g = 0;
+    for (int q : inst) {
+      const double n = (double)(inst_ptr[q + 1] - inst_ptr[q]);
+      while (g < kBatchT && seen >= all_pairs * g / kBatchT) grid[g++] = t[q];
+      seen += n * n;
+    }
+    while (g < kBatchT) grid[g++] = t[inst.back()];
+  }
+  // ---- shares of sampled pairs at or above each of them, per level
+  const int64_t slots = kSampleSlots;
+  const size_t ncnt = (size_t)kFoldLevels * kBatchI * kBatchT;
+  unsigned long long* stats = nullptr;  // length sum, control words, counts
+  ST_TRY(ws.get("fold:stats", 2 + ncnt / 2, &stats));
+  CU_TRY(cudaMemsetAsync(stats, 0, 8 * 2 + 4 * ncnt, st));
+  FoldSide B;
+  B.x = x;
+  int32_t* sample = nullptr;
+  float* sample_t = nullptr;
+  ST_TRY(ws.get("fold:sI:sample", (size_t)slots, &sample));
+  ST_TRY(ws.get("fold:sI:t", (size_t)slots, &sample_t));
+  k_spread_rows<<<1, 1024, 0, st>>>(x.rp, x.n, (int)slots, sample, stats);
+  LAUNCH_CHECK();
+  std::vector<float> ht((size_t)slots);
+  for (int64_t i = 0; i < slots; ++i) ht[(size_t)i] = grid[i / kBlockRows];
+  CU_TRY(cudaMemcpyAsync(sample_t, ht.data(), 4 * (size_t)slots, cudaMemcpyHostToDevice, st));
+  FoldOut so;
+  for (int l = 0; l < kFoldLevels; ++l)
+    ST_TRY(ws.get("fold:sI:sample" + std::to_string(l), kClasses * fold_bytes(MIXED, l),
+                  &so.base[l]));
+  const uint32_t every = (1u << kFoldLevels) - 1u;
+  ST_TRY(fold_places<MIXED>(B, sample, slots, {}, every, perm, so, ws, "fold:sI", st));
+  FoldTileArgs ta;
+  std::vector<int4> units;
+  for (int l = kFoldLevels - 1; l >= 0; --l) {
+    ta.lev[l].I = ta.lev[l].J = so.base[l];
+    ta.lev[l].nkc = fold_k(MIXED, l) / kChunk<MIXED>;
+    ta.lev[l].eps = fold_eps(MIXED, l, nrm2, 1.0);
+    for (int a = 0; a < kBatchI; a += pair)
+      for (int b = 0; b < kBatchT; ++b) units.push_back(make_int4(a, b, b + 1, l));
+  }
+  int4* d_units = nullptr;
+  ST_TRY(ws.get("fold:sunits", units.size(), &d_units));
+  CU_TRY(cudaMemcpyAsync(d_units, units.data(), sizeof(int4) * units.size(),
+                         cudaMemcpyHostToDevice, st));
+  ta.nI = kBatchI * kBlockRows;
+  ta.nJ = slots;
+  ta.nbI = kBatchI;
+  ta.nbJ = kBatchT;
+  ta.t_row = sample_t;
+  ta.units = d_units;
+  ta.nunits = (int)units.size();
+  ta.unit_counter = reinterpret_cast<int*>(stats + 1);
+  ta.err = ta.unit_counter + 1;
+  ta.class_count = reinterpret_cast<uint32_t*>(stats + 2);
+  ST_TRY(launch_fold<MIXED>(ta, ctx->sms, st, true));
+  std::vector<unsigned long long> h(2 + ncnt / 2);
+  CU_TRY(cudaMemcpyAsync(h.data(), stats, 8 * h.size(), cudaMemcpyDeviceToHost, st));
+  CU_TRY(cudaStreamSynchronize(st));
+  const int herr = (int)(h[1] >> 32);
+  if (herr & kErrTimeout) return CUAPSS_ETIMEOUT;
+  if (herr) return CUAPSS_ECUDA;
+  const uint32_t* hc = reinterpret_cast<const uint32_t*>(h.data() + 2);
+  const int64_t have = std::min<int64_t>(slots, x.n);  // sampled rows
+  const double mean_len = have > 0 ? (double)h[0] / (double)have : 0.0;
+  double share[kFoldLevels][kBatchT];
+  for (int l = 0; l < kFoldLevels; ++l)
+    for (int b = 0; b < kBatchT; ++b) {
+      const double rowsJ = (double)std::max<int64_t>(0, std::min<int64_t>(kBlockRows, have - b * kBlockRows));
+      const double rowsI = (double)std::min<int64_t>(kBatchI * kBlockRows, have);
+      double c = 0.0;
+      for (int a = 0; a < kBatchI; ++a) c += (double)hc[((size_t)l * kBatchI + a) * kBatchT + b];
+      if (b < kBatchI) c -= rowsJ;  // rows with themselves
+      share[l][b] = rowsJ > 0 ? std::max(c, 0.5) / (rowsI * rowsJ) : 1.0;
+    }
+  // a sample short of blocks knows nothing of the last thresholds: take the
+  // lowest one's shares, which are no smaller
+  for (int l = 0; l < kFoldLevels; ++l)
+    for (int b = 1; b < kBatchT; ++b)
+      if (have < (b + 1) * kBlockRows) share[l][b] = share[l][0];
+  // ---- a level per instance; instances laid out level by level
+  std::vector<int> lev((size_t)k, 0);
+  double cost = 0.0, cands = 0.0, tiles = 0.0;
+  std::vector<int> by_level[kFoldLevels];
+  int g = 0;
+  for (int q : inst) {
+    while (g + 1 < kBatchT && grid[g + 1] <= t[q]) ++g;
+    const int64_t n = inst_ptr[q + 1] - inst_ptr[q];
+    const double nb = (double)ceil_div(n, kBlockRows);
+    const double pairs = 0.5 * (double)n * (double)(n - 1);
+    double best = 1e300, best_cand = 0.0;
+    for (int l = 0; l < kFoldLevels; ++l) {
+      const double cand = share[l][g] * pairs;
+      const double ns = std::ceil(nb / pair) * (nb + 1.0) * 0.5 * tile_cost<MIXED>(l) +
+                        cand * (kCandNs + kCandEntryNs * mean_len) +
+                        (double)n * fold_k(MIXED, l) * kFoldColumnNs;
+      if (ns < best) {
+        best = ns;
+        best_cand = cand;
+        lev[(size_t)q] = l;
+      }
+    }
+    cost += best;
+    cands += best_cand;
+    tiles += 0.5 * nb * (nb + 1.0);
+    by_level[lev[(size_t)q]].push_back(q);
+  }
+  if (cost >= tiles * other_ns) return CUAPSS_OK;
+  std::vector<int64_t> tab;
+  std::vector<FoldTask> tasks(1);
+  FoldTask& task = tasks[0];
+  int64_t S = 0;
+  std::vector<uint16_t> masks;
+  const int most = (int)std::max(1.0, std::min(64.0, tiles / pair / (ctx->sms * 16.0)));
+  for (int l = kFoldLevels - 1; l >= 0; --l) {  // the costly ones first
+    B.out.first[l] = (int)(S / kBlockRows);
+    for (int q : by_level[l]) {
+      const int64_t n = inst_ptr[q + 1] - inst_ptr[q];
+      int tbits = 0;
+      memcpy(&tbits, &t[q], sizeof(float));
+      tab.insert(tab.end(), {S, inst_ptr[q], n, (int64_t)tbits});
+      const int b0 = (int)(S / kBlockRows), b1 = b0 + (int)ceil_div(n, kBlockRows);
+      for (int i = b0; i < b1; i += pair) {
+        const int single = MIXED && i + 1 >= b1 ? kFoldSingle : 0;
+        for (int f = i; f < b1; f += most)
+          task.units.push_back(make_int4(i, f, std::min(b1, f + most), l | single));
+      }
+      task.tiles += (int64_t)(b1 - b0) * (b1 - b0 + 1) / 2;
+      (*width)[(size_t)q] = fold_k(MIXED, l);
+      masks.insert(masks.end(), (size_t)(b1 - b0), (uint16_t)(1u << l));
+      S += (int64_t)(b1 - b0) * kBlockRows;
+      if (S >= INT32_MAX) return CUAPSS_EINVAL;
+    }
+    const int64_t blocks = S / kBlockRows - B.out.first[l];
+    if (blocks > 0)
+      ST_TRY(ws.get("fold:B:lev" + std::to_string(l), (size_t)blocks * fold_bytes(MIXED, l),
+                    &B.out.base[l]));
+  }
+  B.nb = (int)(S / kBlockRows);
+  B.slots = S;
+  const int kq = (int)inst.size();
+  int64_t* d_tab = nullptr;
+  float* t_place = nullptr;
+  ST_TRY(ws.get("fold:B:tab", tab.size(), &d_tab));
+  ST_TRY(ws.get("fold:B:map", (size_t)S, &B.rowmap));
+  ST_TRY(ws.get("fold:B:t", (size_t)S, &t_place));
+  CU_TRY(cudaMemcpyAsync(d_tab, tab.data(), 8 * tab.size(), cudaMemcpyHostToDevice, st));
+  k_batch_places<<<grid_for((int64_t)kq, 1), kThreads, 0, st>>>(d_tab, kq, B.rowmap, t_place);
+  LAUNCH_CHECK();
+  B.t_place = t_place;
+  ST_TRY(fold_places<MIXED>(B, B.rowmap, S, masks, 0, perm, B.out, ws, "fold:B", st));
+  task.I = task.J = &B;
+  task.self = true;
+  const int64_t expect = std::max<int64_t>((int64_t)(2.0 * cands), 1 << 20);
+  task.cap = expect + x.n;
+  ST_TRY(upload_units(tasks, ws, st));
+  r->tiles = task.tiles;
+  r->rbitsI = r->rbitsJ = std::max(1, bits_for((uint64_t)x.n));
+  VerifyArgs va;
+  va.t_row = t_place;
+  va.rbits = r->rbitsJ;
+  return run_tasks<MIXED>(ctx, tasks, nrm2, va, 4 * expect, r, done);
 }
 
 }  // namespace
@@ -833,6 +1061,14 @@ cuapss_status join_fold(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float
   return ctx->opts.precision == CUAPSS_PREC_MIXED
              ? join_fold_as<true>(ctx, a, b, t, perm, nrm2, other_ns, r, done)
              : join_fold_as<false>(ctx, a, b, t, perm, nrm2, other_ns, r, done);
+}
+
+cuapss_status fold_batch(cuapss_ctx* ctx, const DevCsr& x, int k, const int64_t* inst_ptr,
+                         const float* t, const int32_t* perm, double nrm2, double other_ns,
+                         std::vector<int>* width, FoldResult* r, bool* done) {
+  return ctx->opts.precision == CUAPSS_PREC_MIXED
+             ? fold_batch_as<true>(ctx, x, k, inst_ptr, t, perm, nrm2, other_ns, width, r, done)
+             : fold_batch_as<false>(ctx, x, k, inst_ptr, t, perm, nrm2, other_ns, width, r, done);
 }
 
 cuapss_status fold_index(cuapss_ctx* ctx, bool mixed, const DevCsr& x, const int32_t* perm,

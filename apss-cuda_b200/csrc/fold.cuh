@@ -69,8 +69,9 @@ struct FoldTileArgs {
   int self = 0;                  // pairs i < j of one side only
   float t = 0.f;
   const float* t_row = nullptr;  // threshold of each J row, or null: t
-  const int4* units = nullptr;   // mixed: {I block (even), J0, J1, level | turn << 8}: blocks I, I + 1 x
-                                 // [J0, J1), from J0 + turn on (0 <= turn < J1 - J0)
+  // Mixed: {I block, J0, J1, level | single << 7 | turn << 8}: blocks I and
+  // I + 1 (single: I alone) x [J0, J1), from J0 + turn on, 0 <= turn < J1 - J0.
+  const int4* units = nullptr;
   int nunits = 0;
   int* unit_counter = nullptr;
   uint64_t* cand = nullptr;      // {I row << 32 | J row}
@@ -83,10 +84,13 @@ struct FoldTileArgs {
 // A unit's tiles in order, starting at J0 + turn and wrapping around, so that
 // CTAs that work on the same J blocks at one time do not read the same L2
 // lines in step (n = 200,000, K = 128: 993 -> 873 ns a tile).
+constexpr int kFoldSingle = 0x80;
 struct FoldUnit {
   int I, J0, len, lev, turn;
+  bool single;
   __device__ explicit FoldUnit(const int4& u)
-      : I(u.x), J0(u.y), len(u.z - u.y), lev(u.w & 0xff), turn(u.w >> 8) {}
+      : I(u.x), J0(u.y), len(u.z - u.y), lev(u.w & 0x7f), turn(u.w >> 8),
+        single((u.w & kFoldSingle) != 0) {}
   __device__ int J(int k) const {
     const int j = k + turn;
     return J0 + (j < len ? j : j - len);
@@ -188,5 +192,13 @@ struct FoldSegment {
 cuapss_status fold_query(cuapss_ctx* ctx, bool mixed, const std::vector<FoldSegment>& segs,
                          const DevCsr& q, const float* t_row, float t_min, const int32_t* perm,
                          double nrm2, double other_ns, int64_t rows, FoldResult* r, bool* done);
+
+// The folded form of a batch of self-joins: instance q is the rows
+// [inst_ptr[q], inst_ptr[q + 1]) of x at threshold t[q] (host arrays, all
+// at least kFoldMinT). (*width)[q] receives the width of its folded rows (0: no
+// pairs). *done and other_ns as in join_fold.
+cuapss_status fold_batch(cuapss_ctx* ctx, const DevCsr& x, int k, const int64_t* inst_ptr,
+                         const float* t, const int32_t* perm, double nrm2, double other_ns,
+                         std::vector<int>* width, FoldResult* r, bool* done);
 
 }  // namespace cuapss

@@ -72,7 +72,11 @@ class DevHeap {
   template <typename T>
   cuapss_status alloc(size_t count, T** out) {
     void* p = nullptr;
-    const size_t bytes = std::max<size_t>(count * sizeof(T), 256);
+    // sizes in steps of an eighth of their power of two, so that the pool's
+    // freed blocks fit the next object of a similar size
+    size_t bytes = std::max<size_t>(count * sizeof(T), 256), step = 256;
+    while (step * 16 <= bytes) step *= 2;
+    bytes = (bytes + step - 1) / step * step;
     const cudaError_t e = alloc_st_ ? cudaMallocAsync(&p, bytes, alloc_st_) : cudaMalloc(&p, bytes);
     if (e != cudaSuccess) {
       cudaGetLastError();
@@ -275,6 +279,18 @@ cuapss_status concat_segments(cuapss_ctx* ctx, const Segment& a, const Segment& 
 
 constexpr size_t kMaxSegments = 24;
 
+// The device's pool keeps at most kPoolSlack bytes that nobody uses (building
+// an index frees its temporaries there); the rest goes back to the device.
+constexpr uint64_t kPoolSlack = 2ull << 30;
+void trim_pool(int device) {
+  cudaMemPool_t pool = nullptr;
+  uint64_t used = 0;
+  if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess)
+    cudaMemPoolTrimTo(pool, (size_t)(used + kPoolSlack));
+  cudaGetLastError();
+}
+
 void query_times(cuapss_ctx* ctx, cuapss_stats* stats) {
   float ms = 0.f;
   cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[1]);
@@ -344,6 +360,8 @@ extern "C" cuapss_status cuapss_index_create(cuapss_ctx* ctx, const cuapss_csr* 
   idx->p = seg->p;
   ctx->ws.release_prefix("seg:");
   ctx->ws.release_prefix("IX:");
+  CU_TRY(cudaStreamSynchronize(ctx->stream));
+  trim_pool(ctx->device);
   idx->segs.push_back(seg);
   idx->rows = a.n;
   idx->nrm = nrm;
@@ -444,9 +462,11 @@ extern "C" cuapss_status cuapss_index_info(const cuapss_index* idx, int64_t* row
 
 extern "C" cuapss_status cuapss_index_destroy(cuapss_index* idx) {
   if (!idx) return CUAPSS_OK;
-  cudaSetDevice(idx->device);
+  const int device = idx->device;
+  cudaSetDevice(device);
   cudaDeviceSynchronize();
   delete idx;
+  trim_pool(device);
   return CUAPSS_OK;
 }
 

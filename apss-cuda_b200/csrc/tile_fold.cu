@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
         const FoldUnit U(A.units[u]);
         const FoldLevel& L = A.lev[U.lev];
         const int nkc = L.nkc;
-        const int wI = U.I + 1 < A.nbI ? 2 : 1;
+        const int wI = U.I + 1 < A.nbI && !U.single ? 2 : 1;
         const uint8_t* srcI = L.I + (size_t)(U.I - L.firstI) * nkc * kFoldTileBytes;
         for (int j = 0; ok && j < U.len; ++j, ++tt) {
           const uint32_t m = tt & 1u;
@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
       const FoldUnit U(A.units[u]);
       const int nkc = A.lev[U.lev].nkc;
       const bool stream = nkc > kB;
-      const uint32_t idesc = U.I + 1 < A.nbI ? idesc2 : idesc1;
+      const uint32_t idesc = U.I + 1 < A.nbI && !U.single ? idesc2 : idesc1;
       bool fresh = true;  // this warp has not waited for the unit's B chunks
       for (int j = 0; live && j < U.len; ++j, ++tt, ia += (uint32_t)nkc) {
         if ((tt & 1u) == m) {
@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
       const FoldUnit U(A.units[u]);
       const float eps = A.lev[U.lev].eps;
       const int I = U.I + half;
-      const bool haveI = I < A.nbI;
+      const bool haveI = I < A.nbI && !(half == 1 && U.single);
       const int64_t irow0 = (int64_t)I * kBlockRows;
       const int icols = haveI ? (int)(A.nI - irow0 < kBlockRows ? A.nI - irow0 : kBlockRows) : 0;
       for (int j = 0; j < U.len; ++j, ++tt) {
