@@ -316,18 +316,20 @@ cuapss_status emit_pairs(cuapss_ctx* ctx, uint64_t* key, uint32_t* idx, const fl
                          int64_t npairs, int keybits, int rbitsJ, cuapss_pairs* out) {
   cudaStream_t st = ctx->stream;
   Workspace& ws = ctx->ws;
-  ST_TRY(radix_sort_pairs(key, idx, npairs, keybits, ws, "out", st));
   out->count = npairs;
   if (npairs > out->capacity) return CUAPSS_EOVERFLOW;
   if (npairs == 0) return CUAPSS_OK;
+  const bool small = npairs <= kSmallSort;
+  if (!small) ST_TRY(radix_sort_pairs(key, idx, npairs, keybits, ws, "out", st));
+  auto split = small ? launch_sort_split_small : launch_split_pairs;
   if (out->on_device)
-    return launch_split_pairs(key, idx, sim, npairs, rbitsJ, out->i, out->j, out->sim, st);
+    return split(key, idx, sim, npairs, rbitsJ, out->i, out->j, out->sim, st);
   int32_t *di = nullptr, *dj = nullptr;
   float* ds = nullptr;
   ST_TRY(ws.get("out:i", (size_t)npairs, &di));
   ST_TRY(ws.get("out:j", (size_t)npairs, &dj));
   ST_TRY(ws.get("out:s", (size_t)npairs, &ds));
-  ST_TRY(launch_split_pairs(key, idx, sim, npairs, rbitsJ, di, dj, ds, st));
+  ST_TRY(split(key, idx, sim, npairs, rbitsJ, di, dj, ds, st));
   CU_TRY(cudaMemcpyAsync(out->i, di, sizeof(int32_t) * npairs, cudaMemcpyDeviceToHost, st));
   CU_TRY(cudaMemcpyAsync(out->j, dj, sizeof(int32_t) * npairs, cudaMemcpyDeviceToHost, st));
   CU_TRY(cudaMemcpyAsync(out->sim, ds, sizeof(float) * npairs, cudaMemcpyDeviceToHost, st));
@@ -373,42 +375,102 @@ cuapss_status join_device(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, flo
   // remap. The threshold and the head width are chosen together: the head
   // is sized against the tail that is still probed, each threshold's pairs
   // cost their build and their additions.
-  std::vector<RareCandidate> rare;
   const int forced_rare = ctx->opts.rare_max_count;
   // below kRareMinRows rows the pairs cannot pay for the planning's extra
   // host round trips (unless forced)
-  if (self && ctx->opts.remap &&
-      (forced_rare > 0 || (forced_rare == 0 && a.n >= kRareMinRows))) {
-    ST_TRY(rare_feature_candidates(counts, d, ws, st, &rare));
+  const bool want_rare = self && ctx->opts.remap &&
+                         (forced_rare > 0 || (forced_rare == 0 && a.n >= kRareMinRows));
+  const int64_t n_all = a.n + (self ? 0 : bb.n), nnz_all = a.nnz + (self ? 0 : bb.nnz);
+  const bool mixed = precision == CUAPSS_PREC_MIXED;
+  // The statistics are copied back without waiting; make_plan waits for them.
+  // (FP32 without rare features only counts its head's postings.)
+  const bool model = mixed || want_rare;
+  const int64_t ranks = std::min<int64_t>(d, model ? kMaxModelHead : 64);
+  auto* h_rare = static_cast<unsigned long long*>(ctx->pinned);
+  auto* h_counts = reinterpret_cast<int32_t*>(h_rare + kRareStats);
+  static_assert(kRareStats * 8 + kMaxModelHead * 4 <= kPinnedBytes, "pinned scratch");
+  if (want_rare) ST_TRY(rare_stats_launch(counts, d, ws, st, h_rare));
+  ST_TRY(rank_counts_launch(counts, ranks, d, ctx->opts.remap, ws, st, h_counts));
+  std::vector<int64_t> prefix;
+  TilePlan plan;
+  auto make_plan = [&]() -> cuapss_status {
+    if (!prefix.empty()) return CUAPSS_OK;  // made
+    CU_TRY(cudaStreamSynchronize(st));
+    prefix = count_prefix(h_counts, ranks);
+    std::vector<RareCandidate> rare;
+    if (want_rare) rare = rare_candidates(h_rare);
     if (forced_rare > 0) {
       std::vector<RareCandidate> keep;
       for (const RareCandidate& c : rare)
         if (c.max_count == forced_rare) keep.push_back(c);
       rare.swap(keep);
     }
+    int64_t max_pairs = 0;
+    if (!rare.empty()) {
+      size_t free_b = 0, total_b = 0;
+      CU_TRY(cudaMemGetInfo(&free_b, &total_b));
+      max_pairs = std::min<int64_t>(
+          kMaxExplicitPairs, (int64_t)((double)free_b * kExplicitMemShare / kExplicitPairBytes));
+    }
+    if (forced_rare > 0 && !rare.empty() && rare[0].pairs > max_pairs) return CUAPSS_ENOMEM;
+    plan = plan_tiles(precision, n_all, d, nnz_all, model ? prefix : std::vector<int64_t>(), rare,
+                      max_pairs, ctx->opts.head_width, forced_rare > 0);
+    const int pq = mixed ? 64 : 32;  // head width granularity of the tile kernels
+    plan.p = (int)std::min<int64_t>(((int64_t)plan.p + pq - 1) / pq * pq, ((d + pq - 1) / pq) * pq);
+    if (mixed && plan.p < 64) plan.p = 64;
+    return CUAPSS_OK;
+  };
+  const double nrm2 = nrm_a * nrm_b;
+  if (nrm2 >= 1.9) return CUAPSS_EINVAL;  // fixed-point tail needs ~unit norms
+  if (d > (int64_t)(1u << 20) - 2) {  // 20-bit tail feature keys
+    ST_TRY(make_plan());
+    if (d - plan.p > (int64_t)(1u << 20) - 2) return CUAPSS_EINVAL;
   }
-  const int64_t n_all = a.n + (self ? 0 : bb.n), nnz_all = a.nnz + (self ? 0 : bb.nnz);
-  // (the FP32 path without rare features only counts its head's postings)
-  std::vector<int64_t> prefix;
-  const bool model = precision == CUAPSS_PREC_MIXED || !rare.empty();
-  ST_TRY(rank_count_prefix(counts, d, ctx->opts.remap, model ? kMaxModelHead : 64, ws, st,
-                           &prefix));
-  int64_t max_pairs = 0;
-  if (!rare.empty()) {
-    size_t free_b = 0, total_b = 0;
-    CU_TRY(cudaMemGetInfo(&free_b, &total_b));
-    max_pairs = std::min<int64_t>(
-        kMaxExplicitPairs, (int64_t)((double)free_b * kExplicitMemShare / kExplicitPairBytes));
+  if (a.nnz >= (int64_t)UINT32_MAX - 1 || bb.nnz >= (int64_t)UINT32_MAX - 1) return CUAPSS_EINVAL;
+  // The folded join, unless the options fix how the probing path works (a
+  // head width, a rare-feature threshold, no remap) or a shard owns rows by
+  // their place.
+  if (ctx->opts.head_width == 0 && forced_rare == 0 && ctx->opts.remap && nshards == 1 &&
+      a.n > 0 && bb.n > 0 && t >= kFoldMinT) {
+    nvtx.next("cuapss_run:tiles");
+    cudaEventRecord(ctx->ev[1], st);
+    FoldResult fr;
+    bool done = false;
+    auto probing_ns = [&](double* ns) -> cuapss_status {
+      if (mixed) ST_TRY(make_plan());
+      *ns = mixed ? plan.tile_ns : plain_tile_ns(nnz_all, n_all);
+      return CUAPSS_OK;
+    };
+    ST_TRY(join_fold(ctx, a, b, t, perm, nrm2, probing_ns, &fr, &done));
+    if (done) {
+      cudaEventRecord(ctx->ev[2], st);
+      nvtx.next("cuapss_run:finalize");
+      const cuapss_status result = emit_pairs(ctx, fr.okey, fr.oidx, fr.osim, fr.npairs,
+                                              fr.rbitsI + fr.rbitsJ, fr.rbitsJ, out);
+      if (result != CUAPSS_OK && result != CUAPSS_EOVERFLOW) return result;
+      cudaEventRecord(ctx->ev[3], st);
+      CU_TRY(cudaStreamSynchronize(st));
+      if (stats) {
+        memset(stats, 0, sizeof(*stats));
+        stats->pairs = fr.npairs;
+        stats->candidates = stats->rescored = fr.ncand;
+        stats->tiles = fr.tiles;
+        ST_TRY(make_plan());
+        stats->head_width = plan.p;
+        plan_split_stats(plan, plan.p, nnz_all, prefix, stats);
+        stats->max_band = fr.max_band;
+        stats->ms_preprocess = elapsed(ctx->ev[0], ctx->ev[1]);
+        stats->ms_tiles = elapsed(ctx->ev[1], ctx->ev[2]);
+        stats->ms_finalize = elapsed(ctx->ev[2], ctx->ev[3]);
+        stats->ms_total = elapsed(ctx->ev[0], ctx->ev[3]);
+        stats->launches = g_launches.load() - launches0;
+      }
+      return result;
+    }
+    nvtx.next("cuapss_run:prepare");
   }
-  if (forced_rare > 0 && !rare.empty() && rare[0].pairs > max_pairs) return CUAPSS_ENOMEM;
-  const TilePlan plan =
-      plan_tiles(precision, n_all, d, nnz_all, model ? prefix : std::vector<int64_t>(), rare,
-                 max_pairs, ctx->opts.head_width, forced_rare > 0);
-  int p = plan.p;
-  const bool mixed = precision == CUAPSS_PREC_MIXED;
-  const int pq = mixed ? 64 : 32;  // head width granularity of the tile kernels
-  p = (int)std::min<int64_t>(((int64_t)p + pq - 1) / pq * pq, ((d + pq - 1) / pq) * pq);
-  if (mixed && p < 64) p = 64;
+  ST_TRY(make_plan());
+  const int p = plan.p;
   PrepOptions po;
   po.p = p;
   // Rows are dealt into 128-row blocks by their tail non-zeros, so every
@@ -426,47 +488,6 @@ cuapss_status join_device(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, flo
     po.rare_max_count = plan.rare.max_count;
     po.rare_shard = shard;
     po.rare_nshards = nshards;
-  }
-  const double nrm2 = nrm_a * nrm_b;
-  if (nrm2 >= 1.9) return CUAPSS_EINVAL;  // fixed-point tail needs ~unit norms
-  if (d - p > (int64_t)(1u << 20) - 2) return CUAPSS_EINVAL;  // 20-bit tail feature keys
-  if (a.nnz >= (int64_t)UINT32_MAX - 1 || bb.nnz >= (int64_t)UINT32_MAX - 1) return CUAPSS_EINVAL;
-  // The folded join, unless the options fix how the probing path works (a
-  // head width, a rare-feature threshold, no remap) or a shard owns rows by
-  // their place.
-  if (ctx->opts.head_width == 0 && forced_rare == 0 && ctx->opts.remap && nshards == 1 &&
-      a.n > 0 && bb.n > 0 && t >= kFoldMinT) {
-    nvtx.next("cuapss_run:tiles");
-    cudaEventRecord(ctx->ev[1], st);
-    FoldResult fr;
-    bool done = false;
-    const double probing_ns = mixed ? plan.tile_ns : plain_tile_ns(nnz_all, n_all);
-    ST_TRY(join_fold(ctx, a, b, t, perm, nrm2, probing_ns, &fr, &done));
-    if (done) {
-      cudaEventRecord(ctx->ev[2], st);
-      nvtx.next("cuapss_run:finalize");
-      const cuapss_status result = emit_pairs(ctx, fr.okey, fr.oidx, fr.osim, fr.npairs,
-                                              fr.rbitsI + fr.rbitsJ, fr.rbitsJ, out);
-      if (result != CUAPSS_OK && result != CUAPSS_EOVERFLOW) return result;
-      cudaEventRecord(ctx->ev[3], st);
-      CU_TRY(cudaStreamSynchronize(st));
-      if (stats) {
-        memset(stats, 0, sizeof(*stats));
-        stats->pairs = fr.npairs;
-        stats->candidates = stats->rescored = fr.ncand;
-        stats->tiles = fr.tiles;
-        stats->head_width = p;
-        plan_split_stats(plan, p, nnz_all, prefix, stats);
-        stats->max_band = fr.max_band;
-        stats->ms_preprocess = elapsed(ctx->ev[0], ctx->ev[1]);
-        stats->ms_tiles = elapsed(ctx->ev[1], ctx->ev[2]);
-        stats->ms_finalize = elapsed(ctx->ev[2], ctx->ev[3]);
-        stats->ms_total = elapsed(ctx->ev[0], ctx->ev[3]);
-        stats->launches = g_launches.load() - launches0;
-      }
-      return result;
-    }
-    nvtx.next("cuapss_run:prepare");
   }
   const bool head_bound = mixed && head_bound_plan(p, n_all, nnz_all, prefix, plan.rare);
   Side SA, SB;
@@ -737,6 +758,11 @@ cuapss_status cuapss_create(cuapss_ctx** out, const cuapss_opts* opts) {
     c->own_stream = true;
   }
   c->ws.set_stream(c->stream);
+  if (cudaHostAlloc(&c->pinned, kPinnedBytes, cudaHostAllocDefault) != cudaSuccess) {
+    cudaGetLastError();
+    cuapss_destroy(c);
+    return CUAPSS_ENOMEM;
+  }
   for (auto& e : c->ev) cudaEventCreate(&e);
   *out = c;
   return CUAPSS_OK;
@@ -749,6 +775,7 @@ cuapss_status cuapss_destroy(cuapss_ctx* c) {
   if (c->batch_exec) cudaGraphExecDestroy(c->batch_exec);
   if (c->batch_graph) cudaGraphDestroy(c->batch_graph);
   c->ws.release();
+  if (c->pinned) cudaFreeHost(c->pinned);
   for (auto& e : c->ev)
     if (e) cudaEventDestroy(e);
   if (c->own_stream) cudaStreamDestroy(c->stream);

@@ -21,6 +21,7 @@ struct cuapss_ctx {
   cuapss::Workspace ws;
   cudaEvent_t ev[6] = {};
   int64_t cand_cap = 0;
+  void* pinned = nullptr;  // kPinnedBytes of host memory for small copies back
   // batched joins: the captured tile launches (updated in place when the
   // next batch has the same launch topology) and the tuner's choices
   cudaGraph_t batch_graph = nullptr;
@@ -29,6 +30,8 @@ struct cuapss_ctx {
 };
 
 namespace cuapss {
+
+constexpr size_t kPinnedBytes = 64 * 1024;
 
 struct DevCsr {
   int64_t n = 0, d = 0, nnz = 0;

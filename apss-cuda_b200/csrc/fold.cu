@@ -710,7 +710,7 @@ cuapss_status run_tasks(cuapss_ctx* ctx, std::vector<FoldTask>& tasks, double nr
 
 template <bool MIXED>
 cuapss_status join_fold_as(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float t,
-                           const int32_t* perm, double nrm2, double other_ns, FoldResult* r,
+                           const int32_t* perm, double nrm2, const CostFn& other_ns, FoldResult* r,
                            bool* done) {
   *done = false;
   const bool self = b == nullptr;
@@ -738,7 +738,9 @@ cuapss_status join_fold_as(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, fl
   if (!self) ST_TRY(order_side(SJ, sampled, allocJ, ws, "fold:J", st));
   if (sampled) {
     ST_TRY(plan_levels<MIXED>(ctx, k, perm, nrm2));
-    if (k.cost >= tiles128 * other_ns) return CUAPSS_OK;
+    double ns = 0.0;
+    ST_TRY(other_ns(&ns));
+    if (k.cost >= tiles128 * ns) return CUAPSS_OK;
   } else {
     one_level(k);
   }
@@ -1056,7 +1058,7 @@ cuapss_status fold_batch_as(cuapss_ctx* ctx, const DevCsr& x, int k, const int64
 }  // namespace
 
 cuapss_status join_fold(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float t,
-                        const int32_t* perm, double nrm2, double other_ns, FoldResult* r,
+                        const int32_t* perm, double nrm2, const CostFn& other_ns, FoldResult* r,
                         bool* done) {
   return ctx->opts.precision == CUAPSS_PREC_MIXED
              ? join_fold_as<true>(ctx, a, b, t, perm, nrm2, other_ns, r, done)

@@ -168,12 +168,15 @@ struct FoldResult {
   double max_band = 0.0;  // widest margin of the widths used
 };
 
+// Modelled cost, asked for only when it is needed.
+using CostFn = std::function<cuapss_status(double* ns)>;
+
 // The folded join of validated device matrices (b == nullptr: self-join), in
 // the context's precision.
 // *done = false: the probing path is the better one here and nothing was
 // produced. other_ns: that path's modelled SM-nanoseconds per tile.
 cuapss_status join_fold(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float t,
-                        const int32_t* perm, double nrm2, double other_ns, FoldResult* r,
+                        const int32_t* perm, double nrm2, const CostFn& other_ns, FoldResult* r,
                         bool* done);
 
 // A resident index segment's side: order, levels and samples of x's rows,

@@ -47,20 +47,9 @@ __device__ __forceinline__ int warp_or(int v) {
   return v;
 }
 
-__global__ void k_check_rowptr(const int64_t* __restrict__ rp, int64_t n, int64_t nnz, int* err) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i <= n;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t v = rp[i];
-    int bad = 0;
-    if (v < 0 || v > nnz) bad = 1;
-    if (i == 0 && v != 0) bad = 1;
-    if (i == n && v != nnz) bad = 1;
-    if (i < n && rp[i + 1] < v) bad = 1;
-    if (bad) atomicOr(err, kErrRowptr);
-  }
-}
-
-// One warp per row: id range/order, finite values, FP64 norm, posting counts.
+// One warp per row: row pointers, id range/order, finite values, FP64 norm,
+// posting counts. A row whose pointers are out of order or range is flagged
+// and not read.
 // Hot Zipf features would serialize on their global counters, so counts are
 // first gathered per CTA in shared memory and added to the global counts
 // once per CTA:
@@ -103,8 +92,8 @@ __device__ __forceinline__ void hist_add(int mode, int* hist, int32_t* __restric
 
 template <int MODE>
 __global__ void k_check_rows(const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
-                             const float* __restrict__ val, int64_t n, int64_t d, float tol,
-                             int check, int32_t* __restrict__ counts, int* err,
+                             const float* __restrict__ val, int64_t n, int64_t d, int64_t nnz,
+                             float tol, int check, int32_t* __restrict__ counts, int* err,
                              unsigned long long* nrm_max_bits) {
   extern __shared__ int hist[];
   if (MODE == kHistDirect) {
@@ -121,8 +110,13 @@ __global__ void k_check_rows(const int64_t* __restrict__ rp, const int32_t* __re
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   double nrm_max = 0.0;  // this warp's rows (one global atomic per warp at the end)
   int bad_all = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0 && (rp[0] != 0 || rp[n] != nnz)) bad_all = kErrRowptr;
   for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
     const int64_t lo = rp[i], hi = rp[i + 1];
+    if (lo < 0 || hi < lo || hi > nnz) {  // warp-uniform
+      bad_all |= kErrRowptr;
+      continue;
+    }
     double ss = 0.0;
     int bad = 0;
     for (int64_t e = lo + lane; e < hi; e += 32) {
@@ -1056,7 +1050,7 @@ cuapss_status build_explicit_pairs(Side& s, const PrepOptions& o, int64_t* rcoun
   k_rare_keys<<<grid_for(n * 32, kThreads), kThreads, 0, st>>>(s.rp2, s.col2, s.val2, rptr, n,
                                                                o.rare_from, rbits, keys, idx, vrm);
   LAUNCH_CHECK();
-  ST_TRY(radix_sort_pairs(keys, idx, m, rbits + fbits, ws, t + "rare", st));
+  ST_TRY(radix_sort_pairs(keys, idx, m, rbits + fbits, ws, t + "rare", st, rbits));
   k_rare_gather<<<grid_for(m, kThreads), kThreads, 0, st>>>(idx, vrm, m, vs, inv);
   LAUNCH_CHECK();
   CU_TRY(cudaMemsetAsync(total, 0, sizeof(unsigned long long), st));
@@ -1109,18 +1103,10 @@ cuapss_status validate_csr(const int64_t* rp, const int32_t* col, const float* v
                            int64_t d, int64_t nnz, float tol, int check, int32_t* counts,
                            double* nrm_max, Workspace& ws, const std::string& tag,
                            cudaStream_t st) {
-  int* err = nullptr;
-  unsigned long long* nm = nullptr;
-  ST_TRY(ws.get(tag + ":err", 1, &err));
-  ST_TRY(ws.get(tag + ":nrm", 1, &nm));
-  CU_TRY(cudaMemsetAsync(err, 0, sizeof(int), st));
-  CU_TRY(cudaMemsetAsync(nm, 0, sizeof(unsigned long long), st));
-  k_check_rowptr<<<grid_for(n + 1, kThreads), kThreads, 0, st>>>(rp, n, nnz, err);
-  LAUNCH_CHECK();
-  int h_err = 0;
-  CU_TRY(cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, st));
-  CU_TRY(cudaStreamSynchronize(st));
-  if (h_err) return CUAPSS_EINVAL;
+  unsigned long long* nm = nullptr;  // largest norm's bits, then the error flags
+  ST_TRY(ws.get(tag + ":check", 2, &nm));
+  int* err = reinterpret_cast<int*>(nm + 1);
+  CU_TRY(cudaMemsetAsync(nm, 0, 2 * sizeof(unsigned long long), st));
   const int mode = !counts ? kHistGlobal
                    : (d <= kHistMax && nnz >= 4 * d) ? kHistDirect
                    : (d > kHistMax && nnz >= ((int64_t)1 << 22)) ? kHistHashed
@@ -1147,22 +1133,21 @@ cuapss_status validate_csr(const int64_t* rp, const int32_t* col, const float* v
     const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>(sms, ceil_div(n, 32)));
     if (mode == kHistDirect)
       k_check_rows<kHistDirect><<<g, 1024, (size_t)d * sizeof(int), st>>>(
-          rp, col, val, n, d, tol, check, counts, err, nm);
+          rp, col, val, n, d, nnz, tol, check, counts, err, nm);
     else
       k_check_rows<kHistHashed><<<g, 1024, 2 * kHashSlots * sizeof(int), st>>>(
-          rp, col, val, n, d, tol, check, counts, err, nm);
+          rp, col, val, n, d, nnz, tol, check, counts, err, nm);
   } else {
     k_check_rows<kHistGlobal><<<grid_for(n * 32, kThreads), kThreads, 0, st>>>(
-        rp, col, val, n, d, tol, check, counts, err, nm);
+        rp, col, val, n, d, nnz, tol, check, counts, err, nm);
   }
   LAUNCH_CHECK();
-  unsigned long long h_nm = 0;
-  CU_TRY(cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, st));
-  CU_TRY(cudaMemcpyAsync(&h_nm, nm, sizeof(h_nm), cudaMemcpyDeviceToHost, st));
+  unsigned long long h[2] = {0, 0};
+  CU_TRY(cudaMemcpyAsync(h, nm, sizeof(h), cudaMemcpyDeviceToHost, st));
   CU_TRY(cudaStreamSynchronize(st));
-  if (h_err) return CUAPSS_EINVAL;
+  if (h[1]) return CUAPSS_EINVAL;
   double v;
-  memcpy(&v, &h_nm, sizeof(v));
+  memcpy(&v, &h[0], sizeof(v));
   if (nrm_max) *nrm_max = v;
   return CUAPSS_OK;
 }
@@ -1181,7 +1166,9 @@ cuapss_status feature_perm(const int32_t* counts, int64_t d, int64_t max_count, 
   const int fbits = bits_for((uint64_t)d);
   k_feat_keys<<<grid_for(d, kThreads), kThreads, 0, st>>>(counts, d, max_count, fbits, keys, vals);
   LAUNCH_CHECK();
-  ST_TRY(radix_sort_pairs(keys, vals, d, fbits + bits_for((uint64_t)max_count), ws, "perm", st));
+  // ids ascend already: the passes over the counts alone
+  ST_TRY(radix_sort_pairs(keys, vals, d, fbits + bits_for((uint64_t)max_count), ws, "perm", st,
+                          fbits));
   k_perm_from_sorted<<<grid_for(d, kThreads), kThreads, 0, st>>>(vals, d, perm);
   LAUNCH_CHECK();
   return CUAPSS_OK;
@@ -1225,45 +1212,61 @@ __global__ void k_rare_stats(const int32_t* __restrict__ counts, int64_t d,
   }
 }
 
-cuapss_status rare_feature_candidates(const int32_t* counts, int64_t d, Workspace& ws,
-                                      cudaStream_t st, std::vector<RareCandidate>* cands) {
-  cands->clear();
+cuapss_status rare_stats_launch(const int32_t* counts, int64_t d, Workspace& ws, cudaStream_t st,
+                                unsigned long long* host) {
   unsigned long long* out = nullptr;
-  ST_TRY(ws.get("rare:stats", 3 * kRareCands, &out));
-  CU_TRY(cudaMemsetAsync(out, 0, sizeof(unsigned long long) * 3 * kRareCands, st));
+  ST_TRY(ws.get("rare:stats", kRareStats, &out));
+  CU_TRY(cudaMemsetAsync(out, 0, sizeof(unsigned long long) * kRareStats, st));
   // few CTAs: every warp ends with 24 atomics on the same words
   k_rare_stats<<<std::min(grid_for(d, kThreads), 148u), kThreads, 0, st>>>(counts, d, out);
   LAUNCH_CHECK();
-  unsigned long long h[3 * kRareCands];
-  CU_TRY(cudaMemcpyAsync(h, out, sizeof(h), cudaMemcpyDeviceToHost, st));
-  CU_TRY(cudaStreamSynchronize(st));
+  CU_TRY(cudaMemcpyAsync(host, out, sizeof(unsigned long long) * kRareStats,
+                         cudaMemcpyDeviceToHost, st));
+  return CUAPSS_OK;
+}
+
+std::vector<RareCandidate> rare_candidates(const unsigned long long* host) {
+  static_assert(kRareStats == 3 * kRareCands, "three words per threshold");
+  std::vector<RareCandidate> cands;
   for (int k = 0; k < kRareCands; ++k) {
     // the features of count <= C hold the ranks from (features above C) on
     RareCandidate c;
     c.max_count = rare_cand(k);
-    c.rank = (int64_t)h[3 * k];
-    c.pairs = (int64_t)h[3 * k + 1];
-    c.postings = (int64_t)h[3 * k + 2];
-    if (c.postings > 0) cands->push_back(c);
+    c.rank = (int64_t)host[3 * k];
+    c.pairs = (int64_t)host[3 * k + 1];
+    c.postings = (int64_t)host[3 * k + 2];
+    if (c.postings > 0) cands.push_back(c);
   }
-  return CUAPSS_OK;
+  return cands;
 }
 
-cuapss_status rank_count_prefix(const int32_t* counts, int64_t d, int remap, int64_t m,
-                                Workspace& ws, cudaStream_t st, std::vector<int64_t>* prefix) {
-  m = std::max<int64_t>(0, std::min(m, d));
-  prefix->assign((size_t)m + 1, 0);
-  if (m == 0) return CUAPSS_OK;
+cuapss_status rank_counts_launch(const int32_t* counts, int64_t m, int64_t d, int remap,
+                                 Workspace& ws, cudaStream_t st, int32_t* host) {
   uint32_t* vals = nullptr;
   if (remap) ST_TRY(ws.get("perm:vals", (size_t)d, &vals));  // ids by rank (feature_perm)
   int32_t* out = nullptr;
   ST_TRY(ws.get("perm:rank_counts", (size_t)m, &out));
   k_rank_counts<<<grid_for(m, kThreads), kThreads, 0, st>>>(remap ? vals : nullptr, counts, m, out);
   LAUNCH_CHECK();
+  CU_TRY(cudaMemcpyAsync(host, out, sizeof(int32_t) * m, cudaMemcpyDeviceToHost, st));
+  return CUAPSS_OK;
+}
+
+std::vector<int64_t> count_prefix(const int32_t* host, int64_t m) {
+  std::vector<int64_t> prefix((size_t)m + 1, 0);
+  for (int64_t r = 0; r < m; ++r) prefix[(size_t)r + 1] = prefix[(size_t)r] + host[r];
+  return prefix;
+}
+
+cuapss_status rank_count_prefix(const int32_t* counts, int64_t d, int remap, int64_t m,
+                                Workspace& ws, cudaStream_t st, std::vector<int64_t>* prefix) {
+  m = std::max<int64_t>(0, std::min(m, d));
   std::vector<int32_t> h((size_t)m);
-  CU_TRY(cudaMemcpyAsync(h.data(), out, sizeof(int32_t) * m, cudaMemcpyDeviceToHost, st));
-  CU_TRY(cudaStreamSynchronize(st));
-  for (int64_t r = 0; r < m; ++r) (*prefix)[(size_t)r + 1] = (*prefix)[(size_t)r] + h[(size_t)r];
+  if (m > 0) {
+    ST_TRY(rank_counts_launch(counts, m, d, remap, ws, st, h.data()));
+    CU_TRY(cudaStreamSynchronize(st));
+  }
+  *prefix = count_prefix(h.data(), m);
   return CUAPSS_OK;
 }
 
@@ -1301,7 +1304,7 @@ cuapss_status build_side(Side& s, const PrepOptions& o, const int32_t* perm, Wor
     // tail counts are < 2^31: rbits + 31 key bits at most (the sort takes the
     // bits of the largest possible count, bounded by d)
     ST_TRY(radix_sort_pairs(keys, vals, n, rbits + std::max(1, bits_for((uint64_t)d)), ws,
-                            t + "bal", st));
+                            t + "bal", st, rbits));
     k_deal_rows<<<grid_for(n, kThreads), kThreads, 0, st>>>(vals, s.rp0, n, full_blocks,
                                                             s.rowperm, newlen);
     LAUNCH_CHECK();
@@ -1441,7 +1444,7 @@ cuapss_status build_side(Side& s, const PrepOptions& o, const int32_t* perm, Wor
     ST_TRY(ws.get(t + "entpos", (size_t)T, &entpos));
     ST_TRY(ws.get(t + "cptr", (size_t)nf + 1, &s.cptr));
     ST_TRY(ws.get(t + "csc", (size_t)T, &s.csc));
-    ST_TRY(radix_sort_pairs(ckeys, cvals, T, rbits + fb, ws, t + "csc", st));
+    ST_TRY(radix_sort_pairs(ckeys, cvals, T, rbits + fb, ws, t + "csc", st, rbits));
     k_csc_fill<<<grid_for(T, kThreads), kThreads, 0, st>>>(ckeys, cvals, s.tk, s.val2, T, rmask,
                                                           s.csc, entpos);
     LAUNCH_CHECK();

@@ -42,6 +42,12 @@ cuapss_status feature_perm(const int32_t* counts, int64_t d, int64_t max_count, 
 cuapss_status rank_count_prefix(const int32_t* counts, int64_t d, int remap, int64_t m,
                                 Workspace& ws, cudaStream_t st, std::vector<int64_t>* prefix);
 
+// The same in two steps: the m <= d largest counts copied to host (pinned: the
+// copy is not waited for), and their prefix sums.
+cuapss_status rank_counts_launch(const int32_t* counts, int64_t m, int64_t d, int remap,
+                                 Workspace& ws, cudaStream_t st, int32_t* host);
+std::vector<int64_t> count_prefix(const int32_t* host, int64_t m);
+
 // Rare features of a self-join (explicit pairs instead of probes), for each
 // threshold C in {2048, 1024, ..., 16}: the features occurring in at most C
 // rows, which under the frequency remap hold the ranks from `rank` on, their
@@ -53,8 +59,12 @@ struct RareCandidate {
   int64_t pairs = 0;      // sum of count (count - 1) / 2 over them
   int64_t postings = 0;   // sum of count over them
 };
-cuapss_status rare_feature_candidates(const int32_t* counts, int64_t d, Workspace& ws,
-                                      cudaStream_t st, std::vector<RareCandidate>* cands);
+// The statistics are copied to host (kRareStats words, pinned: the copy is
+// not waited for), from which rare_candidates makes the list.
+constexpr int kRareStats = 24;
+cuapss_status rare_stats_launch(const int32_t* counts, int64_t d, Workspace& ws, cudaStream_t st,
+                                unsigned long long* host);
+std::vector<RareCandidate> rare_candidates(const unsigned long long* host);
 
 // Builds every array of `s` (s.rp0/col0/val0/n/d/nnz must be set).
 cuapss_status build_side(Side& s, const PrepOptions& o, const int32_t* perm, Workspace& ws,

@@ -225,10 +225,12 @@ static __global__ void __launch_bounds__(kRsThreads) k_rs_downsweep(const uint64
   }
 }
 
-// Sorts (keys, vals) in place by keys' bits [0, nbits), stable.
+// Sorts (keys, vals) in place by keys' bits [first, nbits), stable: bits below
+// `first` that the input order follows already need no pass of their own.
 inline cuapss_status radix_sort_pairs(uint64_t* keys, uint32_t* vals, int64_t n, int nbits,
-                                      Workspace& ws, const std::string& tag, cudaStream_t st) {
-  if (n <= 1 || nbits <= 0) return CUAPSS_OK;
+                                      Workspace& ws, const std::string& tag, cudaStream_t st,
+                                      int first = 0) {
+  if (n <= 1 || nbits <= first) return CUAPSS_OK;
   if (n >= (int64_t)UINT32_MAX) return CUAPSS_EINVAL;
   const int nblocks = (int)ceil_div(n, kRsTile);
   uint64_t* k2 = nullptr;
@@ -242,7 +244,7 @@ inline cuapss_status radix_sort_pairs(uint64_t* keys, uint32_t* vals, int64_t n,
   uint64_t* kb = k2;
   uint32_t* vb = v2;
   int passes = 0;
-  for (int shift = 0; shift < nbits; shift += 8, ++passes) {
+  for (int shift = first; shift < nbits; shift += 8, ++passes) {
     k_rs_upsweep<<<nblocks, kRsThreads, 0, st>>>(ka, n, shift, hist, nblocks);
     LAUNCH_CHECK();
     ST_TRY(exclusive_scan<uint32_t>(hist, hist, (int64_t)nblocks * 256, nullptr, ws, tag + ":rs", st));

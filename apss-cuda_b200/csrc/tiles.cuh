@@ -159,4 +159,11 @@ cuapss_status launch_split_pairs(const uint64_t* key, const uint32_t* idx, const
                                  int64_t m, int rbits, int32_t* oi, int32_t* oj, float* os,
                                  cudaStream_t st);
 
+// The same for up to kSmallSort unsorted keys, sorted on the way, in one
+// launch (the radix sort takes three launches per 8 key bits).
+constexpr int64_t kSmallSort = 4096;
+cuapss_status launch_sort_split_small(const uint64_t* key, const uint32_t* idx, const float* sim_in,
+                                      int64_t m, int rbits, int32_t* oi, int32_t* oj, float* os,
+                                      cudaStream_t st);
+
 }  // namespace cuapss
