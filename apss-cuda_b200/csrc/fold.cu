@@ -30,12 +30,11 @@ constexpr int64_t kSmallMaxCand = 1 << 21;
 
 // Cost model, SM-nanoseconds, measured on 200,000 and 400,000 rows of the
 // d = 50,000 workload. A 256 x 128 tile whose I chunks stay resident takes
-// kTileNs + kChunkNs per 64 columns (K = 64: 616, 128: 873, 256: 1,446; the
-// tensor cores alone 260 per 64 columns), a streamed one kStreamNs per 64
-// columns (L2 bandwidth; K = 512: 3,212). A candidate takes kCandNs (its
-// listing in the tile kernel, and verify) + kCandEntryNs per entry of its
-// longer row.
-constexpr double kTileNs = 340.0, kChunkNs = 275.0, kStreamNs = 400.0;
+// kTileNs + kChunkNs per 64 columns and at least kTileMinNs (K = 64: 613, 128:
+// 709, 256: 1,371), a streamed one kStreamNs per 64 columns (K = 384: 2,441,
+// 1,024: 6,768). A candidate takes kCandNs (its listing in the tile kernel,
+// and verify) + kCandEntryNs per entry of its longer row.
+constexpr double kTileNs = 55.0, kChunkNs = 328.0, kTileMinNs = 610.0, kStreamNs = 415.0;
 constexpr double kCandNs = 45.0, kCandEntryNs = 0.3;
 // Building a folded row, per column.
 constexpr double kFoldColumnNs = 0.05;
@@ -51,7 +50,8 @@ template <bool MIXED>
 double tile_cost(int level) {
   const int K = fold_k(MIXED, level);
   if (!MIXED) return kTile32Ns + kColumn32Ns * K;
-  return K <= kFoldResident16 ? kTileNs + kChunkNs * (K / 64) : kStreamNs * (K / 64);
+  return K <= kFoldResident16 ? std::max(kTileMinNs, kTileNs + kChunkNs * (K / 64))
+                              : kStreamNs * (K / 64);
 }
 
 template <bool MIXED>
@@ -773,7 +773,7 @@ uint32_t index_levels(int c, bool sampled) {
   // mixed: 64, 128, 256 | 512 | 1,024 | 2,048; FP32: 32, 64, 128 | 256 | 512 | 1,024
   const uint32_t base = MIXED ? 0x0bu : 0x2au;
   const uint32_t wide[3] = {MIXED ? 1u << 6 : 1u << 7, 1u << 8, 1u << 9};
-  return base | (c >= 4 ? wide[0] : 0) | (c >= 9 ? wide[1] : 0) | (c >= 13 ? wide[2] : 0);
+  return base | (c >= 6 ? wide[0] : 0) | (c >= 9 ? wide[1] : 0) | (c >= 13 ? wide[2] : 0);
 }
 
 template <bool MIXED>

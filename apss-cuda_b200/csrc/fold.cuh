@@ -83,7 +83,7 @@ struct FoldTileArgs {
 
 // A unit's tiles in order, starting at J0 + turn and wrapping around, so that
 // CTAs that work on the same J blocks at one time do not read the same L2
-// lines in step (n = 200,000, K = 128: 993 -> 873 ns a tile).
+// lines in step (n = 200,000, K = 128: 993 -> 873 ns a tile when measured).
 constexpr int kFoldSingle = 0x80;
 struct FoldUnit {
   int I, J0, len, lev, turn;

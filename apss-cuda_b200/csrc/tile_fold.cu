@@ -10,11 +10,12 @@
 //   warps 1-2  MMA: each issues the M = 128, N = 256, K = 16 MMAs of every
 //              other tile into its own accumulator of 256 columns (the two
 //              are all of tensor memory);
-//   warps 4-11 epilogue, two per lane quarter (one I block each): the largest
-//              of each J row's 32 products of a column group is compared with
-//              t - eps; only groups in which some row reaches it are looked
-//              at column by column. Candidates gather in shared memory, so
-//              that a warp reserves list room once per about 100 of them (one
+//   warps 4-11 epilogue, two per lane quarter (one I block each): a warp
+//              loads its 128 columns, gives the accumulator back, and votes
+//              once on the largest of each J row's products against t - eps;
+//              only where that passes are the column groups looked at one by
+//              one. Candidates gather in shared memory, so that a warp
+//              reserves list room once per about 100 of them (one
 //              reservation per group cost a global atomic's latency each:
 //              n = 400,000, 3 candidates a tile, 29 ms).
 // Up to kB chunks wide (K <= 256), the I chunks stay in the B ring for a
@@ -22,9 +23,15 @@
 // from L2 per tile, a third of what streaming both operands takes; wider
 // folds stream both.
 //
-// Bound: the tensor cores (K / 64 x 512 cycles per tile) down to K = 128; at
-// K = 64 the epilogue's 256 tensor-memory columns per lane quarter cost
-// about as much as the MMAs.
+// Bound: the tensor cores from K = 128 on (260 ns per 64 columns and tile at
+// their peak; measured 709 ns at K = 128, 1,371 at 256, of which the loads and
+// hand-offs hide all but 60); at K = 64 (613 ns) the hand-off of the two
+// accumulators: tensor cores, epilogue loads and waits in turn, tensor pipe
+// 51% active; above K = 256 the operand stream from L2 (about 410 ns per 64
+// columns). Holding the accumulator until a warp was done, voting per column
+// group: 616, 873 and 1,446 ns at K = 64, 128 and 256. Sixteen epilogue warps
+// of 64 columns each: 630, 825, 1,453 (more warps wait and poll, the loads are
+// no faster).
 //
 // Every wait is bounded as in tile_mma.cu: a timeout raises kErrTimeout and
 // a shared abort flag, copies and MMAs in flight are drained, tensor memory
@@ -46,6 +53,7 @@ constexpr int kA = 5;                     // A ring slots (16 KB)
 constexpr int kB = kFoldResident16 / kFoldChunk16;   // B ring slots (32 KB)
 constexpr int kMW = 2;                    // MMA warps, one per accumulator
 constexpr int kEW = 8;                    // epilogue warps
+constexpr int kEpiCols = 1024 / kEW;      // accumulator columns of an epilogue warp
 constexpr int kFirstEpi = 4;              // a multiple of 4: lane quarter = warp % 4
 constexpr int kThreads = 32 * (kFirstEpi + kEW);
 constexpr int kRing = 4;                  // unit ids published ahead
@@ -53,7 +61,7 @@ constexpr int kReaders = kMW + kEW;       // MMA and epilogue warps
 constexpr int kColsPerAcc = 256;
 constexpr int kBars = (kMW + 1) * kA + 2 * kB + 4 + 2 * kRing + kMW;
 constexpr size_t kOffB = (size_t)kA * kFoldTileBytes;
-constexpr int kHits = 128;                 // candidates an epilogue warp holds back
+constexpr int kHits = 1024 / kEW;               // candidates an epilogue warp holds back
 constexpr size_t kOffHits = kOffB + (size_t)kB * 2 * kFoldTileBytes;
 constexpr size_t kOffBar = kOffHits + (size_t)kEW * kHits * 8;
 constexpr size_t kOffUnit = kOffBar + (size_t)kBars * 8;
@@ -72,13 +80,20 @@ __device__ __forceinline__ uint32_t passing(const uint32_t (&v)[32], float thr, 
   return pass & (c >= 32 ? 0xffffffffu : c <= 0 ? 0u : (1u << c) - 1u);
 }
 
+__device__ __forceinline__ float max3(float a, uint32_t b, uint32_t c) {
+  float d;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(__uint_as_float(b)), "f"(__uint_as_float(c)));
+  return d;
+}
+
+// Three-input maxima: half the instructions of the epilogue's main loop.
 __device__ __forceinline__ float largest(const uint32_t (&v)[32]) {
-  float m[4];
+  float m[2];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) m[q] = __uint_as_float(v[q]);
+  for (int q = 0; q < 2; ++q) m[q] = __uint_as_float(v[q]);
 #pragma unroll
-  for (int j = 4; j < 32; ++j) m[j & 3] = fmaxf(m[j & 3], __uint_as_float(v[j]));
-  return fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
+  for (int j = 2; j + 1 < 32; j += 2) m[(j >> 1) & 1] = max3(m[(j >> 1) & 1], v[j], v[j + 1]);
+  return fmaxf(m[0], m[1]);
 }
 
 template <bool COUNT>
@@ -279,7 +294,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
   } else if (warp >= kFirstEpi) {
     // ------------------------------------------------------------- epilogue
     const int q4 = warp & 3;             // tensor-memory lane quarter of this warp
-    const int half = (warp - kFirstEpi) >> 2;    // which of the two I blocks
+    const int strip = (warp - kFirstEpi) >> 2;      // which kEpiCols columns
+    const int half = strip * kEpiCols / kBlockRows; // which of the two I blocks
+    const int col0 = strip * kEpiCols % kBlockRows; // first column within it
     const int row = 32 * q4 + lane;      // J row within its block
     uint64_t* hits = reinterpret_cast<uint64_t*>(base + kOffHits) + (warp - kFirstEpi) * kHits;
     int held = 0;                        // candidates in hits, the same in every lane
@@ -296,8 +313,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
       const float eps = A.lev[U.lev].eps;
       const int I = U.I + half;
       const bool haveI = I < A.nbI && !(half == 1 && U.single);
-      const int64_t irow0 = (int64_t)I * kBlockRows;
-      const int icols = haveI ? (int)(A.nI - irow0 < kBlockRows ? A.nI - irow0 : kBlockRows) : 0;
+      const int64_t irow0 = (int64_t)I * kBlockRows + col0;  // I row of this warp's first column
+      const int icols =
+          haveI && A.nI > irow0 ? (int)(A.nI - irow0 < kEpiCols ? A.nI - irow0 : kEpiCols) : 0;
       for (int j = 0; j < U.len; ++j, ++tt) {
         const int J = U.J(j);
         const uint32_t b = tt & 1u, tr = tt >> 1;
@@ -306,23 +324,39 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
             jrow < A.nJ ? __fsub_rd(A.t_row ? A.t_row[jrow] : A.t, eps) : __int_as_float(0x7f800000);
         live = warp_wait(&tfull[b], tr & 1u, abort, A.err, live);
         tc_fence_after();
-        const uint32_t taddr = tmem + b * (uint32_t)kColsPerAcc + (uint32_t)(half * kBlockRows) +
+        const uint32_t taddr = tmem + b * (uint32_t)kColsPerAcc + (uint32_t)(strip * kEpiCols) +
                                ((uint32_t)(32 * q4) << 16);
-        if (live && haveI && !(A.self && J < I)) {
+        const bool work = live && haveI && !(A.self && J < I);
+        uint32_t v[kEpiCols / 32][32];
+        if (work) {
+#pragma unroll
+          for (int g = 0; g < kEpiCols / 32; ++g) tmem_ld32_async(taddr + 32u * g, v[g]);
+#pragma unroll
+          for (int g = 0; g < kEpiCols / 32; ++g) tmem_wait(v[g]);
+        }
+        // the products are in registers: the accumulator is free again
+        tc_fence_before();
+        __syncwarp();
+        if (live && lane == 0) mbar_arrive(&tempty[b]);
+        if (!work) continue;
+        // the groups' maxima first, and one vote: nearly all tiles end here
+        float m[kEpiCols / 32];
+        float top = largest(v[0]);
+        m[0] = top;
+#pragma unroll
+        for (int g = 1; g < kEpiCols / 32; ++g) {
+          m[g] = largest(v[g]);
+          top = fmaxf(top, m[g]);
+        }
+        if (__any_sync(0xffffffffu, top >= thr)) {
           // columns that exist; for a self-join only those below the J row
           int64_t lim = icols;
           if (A.self && jrow - irow0 < lim) lim = jrow - irow0;
-          uint32_t v[2][32];
-          tmem_ld32_async(taddr, v[0]);
           uint32_t n_hits = 0;
 #pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            // group g is worked on while group g + 1 loads
-            uint32_t(&x)[32] = v[g & 1];
-            tmem_wait(x);
-            if (g < 3) tmem_ld32_async(taddr + 32u * (g + 1), v[(g + 1) & 1]);
-            if (!__any_sync(0xffffffffu, largest(x) >= thr)) continue;
-            uint32_t pass = passing(x, thr, (int)lim - 32 * g);
+          for (int g = 0; g < kEpiCols / 32; ++g) {
+            if (!__any_sync(0xffffffffu, m[g] >= thr)) continue;
+            uint32_t pass = passing(v[g], thr, (int)lim - 32 * g);
             if (COUNT) {
               n_hits += (uint32_t)__popc(pass);
               continue;
@@ -349,9 +383,6 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
               atomicAdd(&A.class_count[((size_t)U.lev * A.nbI + I) * A.nbJ + J], total);
           }
         }
-        tc_fence_before();
-        __syncwarp();
-        if (live && lane == 0) mbar_arrive(&tempty[b]);
       }
     }
     if (!COUNT && held > 0) flush_hits(A, hits, held, lane);
