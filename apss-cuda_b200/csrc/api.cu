@@ -431,7 +431,7 @@ cuapss_status join_device(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, flo
   // head width, a rare-feature threshold, no remap) or a shard owns rows by
   // their place.
   if (ctx->opts.head_width == 0 && forced_rare == 0 && ctx->opts.remap && nshards == 1 &&
-      a.n > 0 && bb.n > 0 && t >= kFoldMinT) {
+      a.n > 0 && bb.n > 0 && t >= kFoldMinT && nrm_a * nrm_a < 1.9 && nrm_b * nrm_b < 1.9) {
     nvtx.next("cuapss_run:tiles");
     cudaEventRecord(ctx->ev[1], st);
     FoldResult fr;

@@ -133,43 +133,29 @@ __global__ void k_split_pairs(const uint64_t* __restrict__ key, const uint32_t* 
   }
 }
 
-// One CTA: bitonic sort of m <= kSmallSort unique keys in shared memory (48 KB:
-// keys and payload indexes), then the split. Up to 4,096 keys take 78 exchange
-// steps of two pairs a thread.
-constexpr int kSmallThreads = 1024;
-__global__ void __launch_bounds__(kSmallThreads)
+// m <= kSmallSort unique keys by their ranks: every CTA holds all keys in
+// shared memory, a warp counts the keys below each of its own (the lanes
+// stride over all of them) and writes that pair to its place.
+__global__ void __launch_bounds__(kThreads)
     k_sort_split_small(const uint64_t* __restrict__ key, const uint32_t* __restrict__ idx,
-                       const float* __restrict__ sim_in, int m, int size, int rbits,
+                       const float* __restrict__ sim_in, int m, int rbits,
                        int32_t* __restrict__ oi, int32_t* __restrict__ oj, float* __restrict__ os) {
   __shared__ uint64_t k[kSmallSort];
-  __shared__ uint32_t v[kSmallSort];
-  for (int q = threadIdx.x; q < size; q += kSmallThreads) {
-    k[q] = q < m ? key[q] : ~0ull;
-    v[q] = q < m ? idx[q] : 0u;
-  }
+  for (int q = threadIdx.x; q < m; q += kThreads) k[q] = key[q];
   __syncthreads();
-  for (int run = 2; run <= size; run <<= 1) {
-    for (int gap = run >> 1; gap > 0; gap >>= 1) {
-      for (int q = threadIdx.x; q < size / 2; q += kSmallThreads) {
-        const int a = 2 * q - (q & (gap - 1)), b = a + gap;
-        const bool up = (a & run) == 0;
-        const uint64_t x = k[a], y = k[b];
-        if ((x > y) == up) {
-          k[a] = y;
-          k[b] = x;
-          const uint32_t w = v[a];
-          v[a] = v[b];
-          v[b] = w;
-        }
-      }
-      __syncthreads();
-    }
-  }
+  const int lane = threadIdx.x & 31;
   const uint64_t mask = (1ull << rbits) - 1ull;
-  for (int q = threadIdx.x; q < m; q += kSmallThreads) {
-    oi[q] = (int32_t)(k[q] >> rbits);
-    oj[q] = (int32_t)(k[q] & mask);
-    os[q] = sim_in[v[q]];
+  for (int q = (blockIdx.x * kThreads + threadIdx.x) >> 5; q < m;
+       q += (gridDim.x * kThreads) >> 5) {
+    const uint64_t x = k[q];
+    int below = 0;
+    for (int o = lane; o < m; o += 32) below += k[o] < x;
+    below = __reduce_add_sync(0xffffffffu, below);
+    if (lane == 0) {
+      oi[below] = (int32_t)(x >> rbits);
+      oj[below] = (int32_t)(x & mask);
+      os[below] = sim_in[idx[q]];
+    }
   }
 }
 
@@ -180,9 +166,8 @@ cuapss_status launch_sort_split_small(const uint64_t* key, const uint32_t* idx, 
                                       cudaStream_t st) {
   if (m <= 0) return CUAPSS_OK;
   if (m > kSmallSort) return CUAPSS_EINVAL;
-  int size = 1;
-  while (size < m) size <<= 1;
-  k_sort_split_small<<<1, kSmallThreads, 0, st>>>(key, idx, sim_in, (int)m, size, rbits, oi, oj, os);
+  const int64_t g = std::min<int64_t>(ceil_div(m, kThreads / 32), 148);
+  k_sort_split_small<<<(unsigned)g, kThreads, 0, st>>>(key, idx, sim_in, (int)m, rbits, oi, oj, os);
   LAUNCH_CHECK();
   return CUAPSS_OK;
 }

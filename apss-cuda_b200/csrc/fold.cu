@@ -36,8 +36,8 @@ constexpr int64_t kSmallMaxCand = 1 << 21;
 // and verify) + kCandEntryNs per entry of its longer row.
 constexpr double kTileNs = 55.0, kChunkNs = 328.0, kTileMinNs = 610.0, kStreamNs = 415.0;
 constexpr double kCandNs = 45.0, kCandEntryNs = 0.3;
-// Building a folded row, per column.
-constexpr double kFoldColumnNs = 0.05;
+// Folding a row at a width, per entry and per column.
+constexpr double kFoldEntryNs = 0.35, kFoldColumnNs = 0.05;
 // FP32, 128 x 128 tiles.
 constexpr double kTile32Ns = 380.0, kColumn32Ns = 92.0;
 
@@ -136,12 +136,17 @@ __global__ void k_sample_rows(const int32_t* __restrict__ rowmap, const int64_t*
 
 // ---- folded rows ---------------------------------------------------------
 // A row's entries are summed per column of every wanted width in shared
-// memory (squares in the shared columns), in one pass over the row, and
-// written as BF16 in the 128-byte-swizzled chunk layout of the tensor cores
-// (prep.cu). Head values are rounded to nearest, which the margin covers;
-// shared columns are rounded up after widening by the largest error their
-// FP32 sums can have (2^-24 per addition), so their products bound the exact
-// ones.
+// memory, in one pass over the row, and written as BF16 in the
+// 128-byte-swizzled chunk layout of the tensor cores (prep.cu), or as FP32.
+// Shared columns sum the squares, each rounded up to a multiple of 2^-31, as
+// integers (a row's squared norm is below 1.9; integer shared-memory atomics
+// run at 12 a clock and SM against 3.4 for FP32: 200,000 rows of the d = 1M
+// workload, 619 -> 394 us together with leaving out the widths that do not
+// pay), and every step from there on rounds up, so their products bound the
+// exact ones. Head values are rounded
+// to nearest, which the margin covers.
+constexpr float kSquareScale = 2147483648.0f;  // 2^31
+
 __host__ __device__ constexpr size_t fold_bytes(bool mixed, int level) {  // of a row block
   return (size_t)fold_k(mixed, level) * kBlockRows * (mixed ? 2 : 4);
 }
@@ -156,49 +161,64 @@ __host__ __device__ constexpr int fold_offset(bool mixed, uint32_t allow, int l)
 }
 
 template <bool MIXED, int LEV>
-__device__ __forceinline__ void fold_add(uint32_t mask, float* acc, uint32_t allow, uint32_t r,
-                                         float v) {
+__device__ __forceinline__ void fold_add(uint32_t mask, uint32_t* acc, uint32_t allow, uint32_t r,
+                                         float v, uint32_t square) {
   constexpr uint32_t P = fold_k(MIXED, LEV) / 4, M = fold_k(MIXED, LEV) - P;
   if (!((mask >> LEV) & 1u)) return;  // uniform over the row's threads
-  float* a = acc + fold_offset(MIXED, allow, LEV);
-  if (r < P) a[r] = v;
-  else atomicAdd(&a[P + (r - P) % M], v * v);
+  uint32_t* a = acc + fold_offset(MIXED, allow, LEV);
+  if (r < P) a[r] = __float_as_uint(v);
+  else atomicAdd(&a[P + (r - P) % M], square);
+}
+
+// Norm of a shared column from its fixed-point squares, times scale: an upper
+// bound (sqrt.approx is within 2^-23 of the root; scale carries a factor
+// 1 + 2^-21 for it). The IEEE root and the software round-up conversion to
+// BF16 took most of the instructions of folding short rows (1.6M rows of 30:
+// 1,348 -> 961 us; 200,000 rows of 120: 394 -> 301 us).
+__device__ __forceinline__ float fold_norm(uint32_t squares, float scale) {
+  float r;
+  asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(__uint2float_ru(squares) * (1.0f / kSquareScale)));
+  return __fmul_ru(r, scale);
+}
+
+// Two non-negative floats rounded up to BF16, packed.
+__device__ __forceinline__ uint32_t bf16x2_up(float lo, float hi) {
+  return __byte_perm(__float_as_uint(lo) + 0xffffu, __float_as_uint(hi) + 0xffffu, 0x7632);
 }
 
 template <bool MIXED, int LEV>
-__device__ __forceinline__ void fold_write(uint32_t mask, const float* acc, uint32_t allow,
-                                           const FoldOut& O, float widen, int b, int rr, int tid,
+__device__ __forceinline__ void fold_write(uint32_t mask, const uint32_t* acc, uint32_t allow,
+                                           const FoldOut& O, float scale, int b, int rr, int tid,
                                            int nt) {
   constexpr int K = fold_k(MIXED, LEV), P = K / 4;
   if (!((mask >> LEV) & 1u)) return;
-  const float* a = acc + fold_offset(MIXED, allow, LEV);
+  const uint32_t* a = acc + fold_offset(MIXED, allow, LEV);
   uint8_t* dst = O.base[LEV] + (size_t)(b - O.first[LEV]) * fold_bytes(MIXED, LEV);
+  const float up = __fmul_ru(scale, 1.0f + 4.76837158e-7f);  // 1 + 2^-21
   if (!MIXED) {  // [column][row]
     for (int c = tid; c < K; c += nt)
       reinterpret_cast<float*>(dst)[c * kBlockRows + rr] =
-          c < P ? a[c] : __fmul_ru(__fsqrt_ru(a[c]), widen);
+          c < P ? __uint_as_float(a[c]) * scale : fold_norm(a[c], up);
     return;
   }
   uint4* out = reinterpret_cast<uint4*>(dst);
   for (int c8 = tid; c8 < K / 8; c8 += nt) {
-    __nv_bfloat162 w[4];
-    const float4 x = reinterpret_cast<const float4*>(a)[2 * c8];
-    const float4 y = reinterpret_cast<const float4*>(a)[2 * c8 + 1];
-    const float f[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+    const uint4 x = reinterpret_cast<const uint4*>(a)[2 * c8];
+    const uint4 y = reinterpret_cast<const uint4*>(a)[2 * c8 + 1];
+    const uint32_t f[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+    uint32_t w[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       if (c8 * 8 < P) {  // P is a multiple of 8
-        w[q].x = __float2bfloat16_rn(f[2 * q]);
-        w[q].y = __float2bfloat16_rn(f[2 * q + 1]);
+        const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(f[2 * q]) * scale,
+                                                       __uint_as_float(f[2 * q + 1]) * scale);
+        memcpy(&w[q], &h, 4);
       } else {
-        w[q].x = __float2bfloat16_ru(__fsqrt_ru(f[2 * q]) * widen);
-        w[q].y = __float2bfloat16_ru(__fsqrt_ru(f[2 * q + 1]) * widen);
+        w[q] = bf16x2_up(fold_norm(f[2 * q], up), fold_norm(f[2 * q + 1], up));
       }
     }
     const int kc = c8 >> 3, c = c8 & 7;
-    uint4 u;
-    memcpy(&u, w, 16);
-    out[((size_t)kc * kBlockRows + rr) * 8 + (c ^ (rr & 7))] = u;
+    out[((size_t)kc * kBlockRows + rr) * 8 + (c ^ (rr & 7))] = make_uint4(w[0], w[1], w[2], w[3]);
   }
 }
 
@@ -217,11 +237,11 @@ __global__ void __launch_bounds__(kThreads)
                 const float* __restrict__ val, const int32_t* __restrict__ perm,
                 const float* __restrict__ t_row, const uint16_t* __restrict__ blk_mask,
                 uint32_t mask0, uint32_t allow, bool wide, FoldOut O) {
-  extern __shared__ __align__(16) float fold_sm[];
+  extern __shared__ __align__(16) uint32_t fold_sm[];
   constexpr int kGroups = kThreads / GROUP;
   const int tid = threadIdx.x % GROUP;
   const int ncol = fold_offset(MIXED, allow, kFoldLevels);
-  float* acc = fold_sm + (threadIdx.x / GROUP) * ncol;
+  uint32_t* acc = fold_sm + (threadIdx.x / GROUP) * ncol;
   for (int64_t s = slot0 + (int64_t)blockIdx.x * kGroups + threadIdx.x / GROUP; s < slot1;
        s += (int64_t)gridDim.x * kGroups) {
     const int b = (int)(s / kBlockRows), rr = (int)(s % kBlockRows);
@@ -231,37 +251,37 @@ __global__ void __launch_bounds__(kThreads)
     const int64_t lo = r >= 0 ? rp[r] : 0;
     const int len = r >= 0 ? (int)(rp[r + 1] - lo) : 0;
     for (int k = tid; k < ncol / 4; k += GROUP)
-      reinterpret_cast<float4*>(acc)[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      reinterpret_cast<uint4*>(acc)[k] = make_uint4(0u, 0u, 0u, 0u);
     if (GROUP == 32) __syncwarp();
     else __syncthreads();
-    const float scale = t_row && r >= 0 ? __frcp_ru(t_row[r]) : 1.0f;
     for (int e = tid; e < len; e += GROUP) {
       const uint32_t f = (uint32_t)perm[col[lo + e]];
-      const float v = val[lo + e] * scale;
-      fold_add<MIXED, 0>(mask, acc, allow, f, v);
-      fold_add<MIXED, 1>(mask, acc, allow, f, v);
-      fold_add<MIXED, 2>(mask, acc, allow, f, v);
-      fold_add<MIXED, 3>(mask, acc, allow, f, v);
-      fold_add<MIXED, 4>(mask, acc, allow, f, v);
-      fold_add<MIXED, 5>(mask, acc, allow, f, v);
-      fold_add<MIXED, 6>(mask, acc, allow, f, v);
-      fold_add<MIXED, 7>(mask, acc, allow, f, v);
-      fold_add<MIXED, 8>(mask, acc, allow, f, v);
-      fold_add<MIXED, 9>(mask, acc, allow, f, v);
+      const float v = val[lo + e];
+      const uint32_t square = __float2uint_ru(__fmul_ru(v, v) * kSquareScale);
+      fold_add<MIXED, 0>(mask, acc, allow, f, v, square);
+      fold_add<MIXED, 1>(mask, acc, allow, f, v, square);
+      fold_add<MIXED, 2>(mask, acc, allow, f, v, square);
+      fold_add<MIXED, 3>(mask, acc, allow, f, v, square);
+      fold_add<MIXED, 4>(mask, acc, allow, f, v, square);
+      fold_add<MIXED, 5>(mask, acc, allow, f, v, square);
+      fold_add<MIXED, 6>(mask, acc, allow, f, v, square);
+      fold_add<MIXED, 7>(mask, acc, allow, f, v, square);
+      fold_add<MIXED, 8>(mask, acc, allow, f, v, square);
+      fold_add<MIXED, 9>(mask, acc, allow, f, v, square);
     }
     if (GROUP == 32) __syncwarp();
     else __syncthreads();
-    const float widen = 1.0f + (float)(len + 16) * 5.9604645e-8f * 1.01f;
-    fold_write<MIXED, 0>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
-    fold_write<MIXED, 1>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
-    fold_write<MIXED, 2>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
-    fold_write<MIXED, 3>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
-    fold_write<MIXED, 4>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
-    fold_write<MIXED, 5>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
-    fold_write<MIXED, 6>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
-    fold_write<MIXED, 7>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
-    fold_write<MIXED, 8>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
-    fold_write<MIXED, 9>(mask, acc, allow, O, widen, b, rr, tid, GROUP);
+    const float scale = t_row && r >= 0 ? __frcp_ru(t_row[r]) : 1.0f;
+    fold_write<MIXED, 0>(mask, acc, allow, O, scale, b, rr, tid, GROUP);
+    fold_write<MIXED, 1>(mask, acc, allow, O, scale, b, rr, tid, GROUP);
+    fold_write<MIXED, 2>(mask, acc, allow, O, scale, b, rr, tid, GROUP);
+    fold_write<MIXED, 3>(mask, acc, allow, O, scale, b, rr, tid, GROUP);
+    fold_write<MIXED, 4>(mask, acc, allow, O, scale, b, rr, tid, GROUP);
+    fold_write<MIXED, 5>(mask, acc, allow, O, scale, b, rr, tid, GROUP);
+    fold_write<MIXED, 6>(mask, acc, allow, O, scale, b, rr, tid, GROUP);
+    fold_write<MIXED, 7>(mask, acc, allow, O, scale, b, rr, tid, GROUP);
+    fold_write<MIXED, 8>(mask, acc, allow, O, scale, b, rr, tid, GROUP);
+    fold_write<MIXED, 9>(mask, acc, allow, O, scale, b, rr, tid, GROUP);
     if (GROUP == 32) __syncwarp();
     else __syncthreads();
   }
@@ -398,6 +418,14 @@ struct FoldTask {
   int64_t cap = 0;
 };
 
+// Whether a level is sampled for a pair of classes: the widest ones only pay
+// where both rows are long (all of them for all pairs took 212 us of a 1.5 ms
+// FP32 join of 20,000 rows).
+bool sampled_level(int l, int a, int b) {
+  const int lo = std::min(a, b), sum = a + b;
+  return l < 7 || (l == 7 && sum >= 10) || (l == 8 && sum >= 16) || (l == 9 && lo >= 9);
+}
+
 // The width of every pair of classes, from the products of sampled rows, the
 // modelled cost of the join and its expected candidates. Levels the J side
 // does not hold (FoldSide::levels) are left out.
@@ -416,6 +444,11 @@ cuapss_status plan_levels(cuapss_ctx* ctx, FoldTask& k, const int32_t* perm, dou
   CU_TRY(cudaMemsetAsync(stats, 0, stat_bytes, st));
   uint32_t all = 0;
   for (uint32_t m : J.levels) all |= m;
+  // a sampled tile of a wide level may not take more than a tenth of a small
+  // join (an FP32 tile of 1,024 columns takes 190 us beside another)
+  const double whole = (k.self ? 0.5 : 1.0) * I.nb * J.nb / kPair<MIXED> * tile_cost<MIXED>(kSmallLevel);
+  for (int l = kSmallLevel + 1; l < kFoldLevels; ++l)
+    if ((MIXED ? 1.0 : 2.0) * tile_cost<MIXED>(l) > 0.1 * whole / ctx->sms) all &= ~(1u << l);
   auto temp = [&](const char* tag) {
     return [&ws, tag](const std::string& name, size_t bytes, void** out) {
       return ws.get(tag + name, bytes, out);
@@ -435,7 +468,8 @@ cuapss_status plan_levels(cuapss_ctx* ctx, FoldTask& k, const int32_t* perm, dou
     for (int a = 0; a < kClasses; a += kPair<MIXED>) {
       if (I.edge[std::min(kClasses, a + kPair<MIXED>)] == I.edge[a]) continue;  // no rows
       for (int b = k.self ? a : 0; b < kClasses; ++b)
-        if (J.edge[b + 1] > J.edge[b]) units.push_back(make_int4(a, b, b + 1, l));
+        if (J.edge[b + 1] > J.edge[b] && sampled_level(l, a + kPair<MIXED> - 1, b))
+          units.push_back(make_int4(a, b, b + 1, l));
     }
   }
   int4* d_units = nullptr;
@@ -469,36 +503,81 @@ cuapss_status plan_levels(cuapss_ctx* ctx, FoldTask& k, const int32_t* perm, dou
     }
   // J chunks of a prepared index come from HBM: its bandwidth, an SM's share
   const double load_ns_per_byte = J.prepared ? ctx->sms / 6500.0 : 0.0;
-  k.cost = k.cands = 0.0;
+  // cost[l][a][b], share[l][a][b] of every level that was sampled
+  const double kNever = 1e300;
+  std::vector<double> cost(ncnt, kNever), found(ncnt, 0.0);
+  auto at = [](int l, int a, int b) { return ((size_t)l * kClasses + a) * kClasses + b; };
   for (int a = 0; a < kClasses; ++a)
     for (int b = k.self ? a : 0; b < kClasses; ++b) {
       const double sampled = rows[0][a] * rows[1][b] - (k.self && a == b ? rows[0][a] : 0.0);
       const double nI = (double)(cr[0].row[a + 1] - cr[0].row[a]);
       const double nJ = (double)(cr[1].row[b + 1] - cr[1].row[b]);
       const double pairs = k.self && a == b ? nI * (nI - 1) / 2 : nI * nJ;
+      if (pairs <= 0) continue;
       const double tiles = k.self ? pairs / ((double)kPair<MIXED> * kBlockRows * kBlockRows)
                                   : std::ceil(nI / (kPair<MIXED> * kBlockRows)) *
                                         std::ceil(nJ / kBlockRows);
-      double best = 1e300, best_cand = 0.0;
       for (int l = 0; l < kFoldLevels; ++l) {
-        if (!((J.levels[b] >> l) & 1u)) continue;
-        double c = (double)hc[((size_t)l * kClasses + a) * kClasses + b];
+        // (a mixed sample tile spans the classes a, a + 1 of an even a)
+        if (!((all & J.levels[b]) >> l & 1u) || !sampled_level(l, a | (kPair<MIXED> - 1), b)) continue;
+        double c = (double)hc[at(l, a, b)];
         if (k.self && a == b) c = std::max(0.0, c - rows[0][a]);  // a row with itself
         // a count of zero is not a share of zero: half a pair
         const double share = sampled > 0 ? std::max(c, 0.5) / sampled : 0.0;
         const double cand_ns = kCandNs + kCandEntryNs * std::max(I.len[a], J.len[b]);
         const double load = (double)fold_bytes(MIXED, l) * load_ns_per_byte;
-        const double ns = tiles * std::max(tile_cost<MIXED>(l), load) + share * pairs * cand_ns;
-        if (ns < best) {
-          best = ns;
-          best_cand = share * pairs;
-          k.level[a][b] = l;
+        found[at(l, a, b)] = share * pairs;
+        cost[at(l, a, b)] = tiles * std::max(tile_cost<MIXED>(l), load) + share * pairs * cand_ns;
+      }
+    }
+  // the best level of each pair of classes among `use`, and what folding the
+  // rows at the levels taken costs
+  auto choose = [&](uint32_t use, bool write) {
+    double sum = 0.0;
+    uint32_t needI[kClasses] = {}, needJ[kClasses] = {};
+    if (write) k.cands = 0.0;
+    for (int a = 0; a < kClasses; ++a)
+      for (int b = k.self ? a : 0; b < kClasses; ++b) {
+        int best = -1;
+        for (int l = 0; l < kFoldLevels; ++l)
+          if (((use >> l) & 1u) && cost[at(l, a, b)] < kNever &&
+              (best < 0 || cost[at(l, a, b)] < cost[at(best, a, b)]))
+            best = l;
+        if (best < 0) {
+          if (cost[at(0, a, b)] < kNever || cost[at(kSmallLevel, a, b)] < kNever) return kNever;
+          continue;  // no pairs
+        }
+        sum += cost[at(best, a, b)];
+        needI[a] |= 1u << best;
+        (k.self ? needI : needJ)[b] |= 1u << best;
+        if (write) {
+          k.level[a][b] = best;
+          k.cands += found[at(best, a, b)];
         }
       }
-      if (pairs <= 0) continue;
-      k.cost += best;
-      k.cands += best_cand;
+    for (int q = 0; q < (k.self || J.prepared ? 1 : 2); ++q)
+      for (int c = 0; c < kClasses; ++c) {
+        const double n = (double)(cr[q].row[c + 1] - cr[q].row[c]);
+        const double len = q == 0 ? I.len[c] : J.len[c];
+        for (int l = 0; l < kFoldLevels; ++l)
+          if (((q == 0 ? needI : needJ)[c] >> l) & 1u)
+            sum += n * (kFoldEntryNs * len + kFoldColumnNs * fold_k(MIXED, l));
+      }
+    return sum;
+  };
+  // levels whose tiles save less than folding the rows for them costs go
+  uint32_t use = all;
+  double total = choose(use, false);
+  for (int l = 0; l < kFoldLevels; ++l) {
+    const uint32_t fewer = use & ~(1u << l);
+    if (fewer == use || fewer == 0) continue;
+    const double c = choose(fewer, false);
+    if (c < total) {
+      total = c;
+      use = fewer;
     }
+  }
+  k.cost = choose(use, true);
   return CUAPSS_OK;
 }
 
@@ -986,7 +1065,7 @@ cuapss_status fold_batch_as(cuapss_ctx* ctx, const DevCsr& x, int k, const int64
       const double cand = share[l][g] * pairs;
       const double ns = std::ceil(nb / pair) * (nb + 1.0) * 0.5 * tile_cost<MIXED>(l) +
                         cand * (kCandNs + kCandEntryNs * mean_len) +
-                        (double)n * fold_k(MIXED, l) * kFoldColumnNs;
+                        (double)n * (mean_len * kFoldEntryNs + fold_k(MIXED, l) * kFoldColumnNs);
       if (ns < best) {
         best = ns;
         best_cand = cand;

@@ -90,7 +90,24 @@ __device__ __forceinline__ void hist_add(int mode, int* hist, int32_t* __restric
   atomicAdd(&counts[c], 1);
 }
 
-template <int MODE>
+// Sum over the warp of each of ROWS values, ROWS = 1 or 4; lane l gets the sum
+// of value (l >> 3) & 3 (ROWS = 4): six exchanges instead of twenty.
+template <int ROWS>
+__device__ __forceinline__ double warp_sums(const double (&v)[ROWS]) {
+  if (ROWS == 1) return warp_sum_d(v[0]);
+  const int lane = threadIdx.x & 31;
+  const bool h16 = lane & 16, h8 = lane & 8;
+  const double a0 = h16 ? v[2 % ROWS] : v[0], a1 = h16 ? v[3 % ROWS] : v[1 % ROWS];
+  const double b0 = h16 ? v[0] : v[2 % ROWS], b1 = h16 ? v[1 % ROWS] : v[3 % ROWS];
+  const double s0 = a0 + __shfl_xor_sync(0xffffffffu, b0, 16);
+  const double s1 = a1 + __shfl_xor_sync(0xffffffffu, b1, 16);
+  double s = (h8 ? s1 : s0) + __shfl_xor_sync(0xffffffffu, h8 ? s0 : s1, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  return s;
+}
+
+template <int MODE, int ROWS>
 __global__ void k_check_rows(const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
                              const float* __restrict__ val, int64_t n, int64_t d, int64_t nnz,
                              float tol, int check, int32_t* __restrict__ counts, int* err,
@@ -111,30 +128,68 @@ __global__ void k_check_rows(const int64_t* __restrict__ rp, const int32_t* __re
   double nrm_max = 0.0;  // this warp's rows (one global atomic per warp at the end)
   int bad_all = 0;
   if (blockIdx.x == 0 && threadIdx.x == 0 && (rp[0] != 0 || rp[n] != nnz)) bad_all = kErrRowptr;
-  for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
-    const int64_t lo = rp[i], hi = rp[i + 1];
-    if (lo < 0 || hi < lo || hi > nnz) {  // warp-uniform
-      bad_all |= kErrRowptr;
-      continue;
+  // ROWS rows at a time: their pointers, then the first 32 entries of
+  // each, load together, so that short rows do not wait for one load after
+  // another (49M non-zeros in rows of 30: 586 -> 412 us; small inputs, which
+  // have too few rows for it, keep one)
+  const int64_t w0 = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+  for (int64_t i0 = w0 * ROWS; i0 < n; i0 += warps * ROWS) {
+    int64_t lo[ROWS], hi[ROWS];
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) {
+      lo[q] = i0 + q < n ? rp[i0 + q] : 0;
+      hi[q] = i0 + q < n ? rp[i0 + q + 1] : 0;
+      if (lo[q] < 0 || hi[q] < lo[q] || hi[q] > nnz) {  // warp-uniform
+        bad_all |= kErrRowptr;
+        lo[q] = hi[q] = 0;
+      }
     }
-    double ss = 0.0;
-    int bad = 0;
-    for (int64_t e = lo + lane; e < hi; e += 32) {
-      const int32_t c = col[e];
-      const float v = val[e];
-      if (c < 0 || c >= d) bad |= kErrColRange;
-      if (e > lo && col[e - 1] >= c) bad |= kErrColOrder;
-      if (!isfinite(v)) bad |= kErrValue;
-      ss += (double)v * (double)v;
-      if (counts && c >= 0 && c < d) hist_add(MODE, hist, counts, c);
+    int32_t c0[ROWS];
+    float v0[ROWS];
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) {
+      const bool in = lo[q] + lane < hi[q];
+      c0[q] = in ? col[lo[q] + lane] : 0;
+      v0[q] = in ? val[lo[q] + lane] : 0.0f;
     }
-    ss = warp_sum_d(ss);
-    bad = warp_or(bad);
-    const double nrm = sqrt(ss);
-    if (check && hi > lo && fabs(nrm - 1.0) > (double)tol) bad |= kErrNorm;
-    bad_all |= bad;
+    double ss[ROWS];
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) {
+      ss[q] = 0.0;
+      int32_t last = -1;  // the id before this chunk
+      int32_t c = c0[q];
+      float v = v0[q];
+      for (int64_t base = lo[q]; base < hi[q]; base += 32) {  // warp-uniform
+        const int64_t e = base + lane;
+        const bool in = e < hi[q];
+        if (base > lo[q]) {
+          c = in ? col[e] : 0;
+          v = in ? val[e] : 0.0f;
+        }
+        int32_t before = __shfl_up_sync(0xffffffffu, c, 1);
+        if (lane == 0) before = last;
+        last = __shfl_sync(0xffffffffu, c, 31);
+        if (in) {
+          if (c < 0 || c >= d) bad_all |= kErrColRange;
+          if (e > lo[q] && before >= c) bad_all |= kErrColOrder;
+          if (!isfinite(v)) bad_all |= kErrValue;
+          ss[q] += (double)v * (double)v;
+          if (counts && c >= 0 && c < d) hist_add(MODE, hist, counts, c);
+        }
+      }
+    }
+    // each lane checks one of the rows' norms (empty rows have none)
+    const double nrm = sqrt(warp_sums<ROWS>(ss));
+    bool empty = hi[0] <= lo[0];
+#pragma unroll
+    for (int q = 1; q < ROWS; ++q)
+      if (((lane >> 3) & 3) == q) empty = hi[q] <= lo[q];
+    if (check && !empty && fabs(nrm - 1.0) > (double)tol) bad_all |= kErrNorm;
     nrm_max = fmax(nrm_max, nrm);
   }
+  bad_all = warp_or(bad_all);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) nrm_max = fmax(nrm_max, __shfl_xor_sync(0xffffffffu, nrm_max, o));
   if (lane == 0) {
     if (bad_all) atomicOr(err, bad_all);
     if (nrm_max > 0.0) atomicMax(nrm_max_bits, (unsigned long long)__double_as_longlong(nrm_max));
@@ -1119,10 +1174,10 @@ cuapss_status validate_csr(const int64_t* rp, const int32_t* col, const float* v
     {
       std::lock_guard<std::mutex> lk(mu);
       if (dev >= 64 || !((done >> dev) & 1ull)) {
-        CU_TRY(cudaFuncSetAttribute(k_check_rows<kHistDirect>,
+        CU_TRY(cudaFuncSetAttribute(k_check_rows<kHistDirect, 4>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)(kHistMax * sizeof(int))));
-        CU_TRY(cudaFuncSetAttribute(k_check_rows<kHistHashed>,
+        CU_TRY(cudaFuncSetAttribute(k_check_rows<kHistHashed, 4>,
                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)(2 * kHashSlots * sizeof(int))));
         if (dev < 64) done |= 1ull << dev;
@@ -1130,15 +1185,16 @@ cuapss_status validate_csr(const int64_t* rp, const int32_t* col, const float* v
     }
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>(sms, ceil_div(n, 32)));
+    const unsigned g =
+        (unsigned)std::max<int64_t>(1, std::min<int64_t>(sms, ceil_div(n, 32 * 4)));
     if (mode == kHistDirect)
-      k_check_rows<kHistDirect><<<g, 1024, (size_t)d * sizeof(int), st>>>(
+      k_check_rows<kHistDirect, 4><<<g, 1024, (size_t)d * sizeof(int), st>>>(
           rp, col, val, n, d, nnz, tol, check, counts, err, nm);
     else
-      k_check_rows<kHistHashed><<<g, 1024, 2 * kHashSlots * sizeof(int), st>>>(
+      k_check_rows<kHistHashed, 4><<<g, 1024, 2 * kHashSlots * sizeof(int), st>>>(
           rp, col, val, n, d, nnz, tol, check, counts, err, nm);
   } else {
-    k_check_rows<kHistGlobal><<<grid_for(n * 32, kThreads), kThreads, 0, st>>>(
+    k_check_rows<kHistGlobal, 1><<<grid_for(n * 32, kThreads), kThreads, 0, st>>>(
         rp, col, val, n, d, nnz, tol, check, counts, err, nm);
   }
   LAUNCH_CHECK();

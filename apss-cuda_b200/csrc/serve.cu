@@ -519,7 +519,7 @@ cuapss_status cuapss::index_query_rows(cuapss_ctx* ctx, const cuapss_index* idx,
     CU_TRY(cudaMemcpyAsync(t_row, t, sizeof(float) * q.n, cudaMemcpyHostToDevice, st));
   // ---- the folded rows, where they prune
   const float t_min = q.n > 0 ? *std::min_element(t, t + q.n) : 0.0f;
-  if (idx->fold && q.n > 0 && rows > 0 && t_min >= kFoldMinT) {
+  if (idx->fold && q.n > 0 && rows > 0 && t_min >= kFoldMinT && nrm_q * nrm_q < 1.9) {
     nvtx.next("cuapss_index_query:tiles");
     cudaEventRecord(ctx->ev[1], st);
     std::vector<FoldSegment> fs;
