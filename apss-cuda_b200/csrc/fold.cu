@@ -41,6 +41,9 @@ constexpr double kFoldEntryNs = 0.35, kFoldColumnNs = 0.05;
 // FP32, 128 x 128 tiles.
 constexpr double kTile32Ns = 380.0, kColumn32Ns = 92.0;
 
+// Joins of at least this long look for tiles too short for one another.
+constexpr double kReachMinNs = 500e3;
+
 template <bool MIXED>
 constexpr int kPair = MIXED ? 2 : 1;  // I blocks of a tile
 template <bool MIXED>
@@ -63,6 +66,8 @@ inline unsigned grid_for(int64_t work, int per_block) {
   const int64_t g = ceil_div(std::max<int64_t>(work, 1), per_block);
   return (unsigned)std::min<int64_t>(g, 148 * 32);
 }
+
+constexpr float kSquareScale = 2147483648.0f;  // 2^31, of fixed-point squares
 
 // ---- row order: by length, in 256 classes of about 1/16 octave -----------
 // Rows with thresholds of their own are ordered by length over the squared
@@ -117,6 +122,80 @@ __global__ void k_spread_rows(const int64_t* __restrict__ rp, int64_t n, int slo
   if (len) atomicAdd(len_sum, len);
 }
 
+// ---- rows too short for one another ---------------------------------------
+// A row with k entries shares at most k features with row b, so their product
+// is at most the first one's norm times the norm of b's k largest entries:
+// below need(b) = the k at which that reaches t, the pair cannot be in the
+// answer. One warp per place finds a lower bound of need(b): for a cut c, with
+// S and n the sum and number of b's squares above c and S < T = (t / norm)^2,
+// need >= n + (T - S) / c. Each block gets its smallest need and its longest
+// row.
+constexpr int kNeedRegs = 4;  // entries a lane keeps in registers
+__global__ void k_block_needs(const int32_t* __restrict__ rowmap, int64_t slots,
+                              const int64_t* __restrict__ rp, const float* __restrict__ val,
+                              uint32_t T, int* __restrict__ need, int* __restrict__ longest) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; s < slots; s += warps) {
+    const int32_t r = rowmap[s];
+    if (r < 0) continue;  // warp-uniform
+    const int64_t lo = rp[r];
+    const int len = (int)(rp[r + 1] - lo);
+    // squares in multiples of 2^-31, rounded up: sums of them are exact
+    uint32_t q[kNeedRegs];
+    auto square = [&](int e) {
+      const float v = val[lo + e];
+      return __float2uint_ru(__fmul_ru(v, v) * kSquareScale);
+    };
+    uint32_t top = 0;
+#pragma unroll
+    for (int k = 0; k < kNeedRegs; ++k) {
+      q[k] = lane + 32 * k < len ? square(lane + 32 * k) : 0u;
+      top = max(top, q[k]);
+    }
+    for (int e = lane + 32 * kNeedRegs; e < len; e += 32) top = max(top, square(e));
+    top = __reduce_max_sync(0xffffffffu, top);
+    // the largest cut (of eight halvings) whose sum above stays below T gives
+    // the bound; the cut at the top has nothing above it
+    uint32_t below = 0, above = top;  // sums: >= T at `below` or not known, < T at `above`
+    uint32_t S = 0;
+    int n = 0;
+    for (int it = 0; it < 8; ++it) {
+      const uint32_t c = below + (above - below) / 2;
+      uint32_t sum = 0;
+      int cnt = 0;
+#pragma unroll
+      for (int k = 0; k < kNeedRegs; ++k)
+        if (q[k] > c) {
+          sum += q[k];
+          ++cnt;
+        }
+      for (int e = lane + 32 * kNeedRegs; e < len; e += 32) {
+        const uint32_t x = square(e);
+        if (x > c) {
+          sum += x;
+          ++cnt;
+        }
+      }
+      sum = __reduce_add_sync(0xffffffffu, sum);
+      cnt = __reduce_add_sync(0xffffffffu, cnt);
+      if (sum < T) {
+        above = c;
+        S = sum;
+        n = cnt;
+      } else {
+        below = c;
+      }
+    }
+    if (lane == 0) {
+      const uint32_t c = max(above, 1u);
+      const int k = min(len, n + (int)min((T - S) / c, 0x3fffffffu));
+      atomicMin(&need[s / kBlockRows], k);
+      atomicMax(&longest[s / kBlockRows], len);
+    }
+  }
+}
+
 // ---- sampled rows: up to 128 of each class, evenly spaced ----------------
 struct ClassRows {
   int64_t row[kClasses + 1];  // first row of each class, n at the end
@@ -145,8 +224,6 @@ __global__ void k_sample_rows(const int32_t* __restrict__ rowmap, const int64_t*
 // pay), and every step from there on rounds up, so their products bound the
 // exact ones. Head values are rounded
 // to nearest, which the margin covers.
-constexpr float kSquareScale = 2147483648.0f;  // 2^31
-
 __host__ __device__ constexpr size_t fold_bytes(bool mixed, int level) {  // of a row block
   return (size_t)fold_k(mixed, level) * kBlockRows * (mixed ? 2 : 4);
 }
@@ -412,6 +489,9 @@ struct FoldTask {
   int64_t j_offset = 0;     // added to the J row of every pair
   int level[kClasses][kClasses] = {};  // width of each pair of classes
   double cost = 0.0, cands = 0.0;      // modelled SM-nanoseconds, expected candidates
+  // self-joins: the last J block whose rows can match rows as short as those
+  // of each I block (empty: all)
+  std::vector<int> last;
   std::vector<int4> units;
   int64_t tiles = 0;
   int4* d_units = nullptr;
@@ -637,10 +717,13 @@ void make_units(FoldTask& k, int sms) {
         while (i >= I.edge[a + 1]) ++a;
         const int lv = k.level[a][b];
         const int f0 = k.self ? std::max(s0, i) : s0;
+        // the pair's second block reaches at least as far
+        const int e1 = k.last.empty() ? s1
+                                      : std::min(s1, k.last[(size_t)std::min(I.nb, i + pair) - 1] + 1);
         const double rel = tile_cost<MIXED>(lv) / tile_cost<MIXED>(MIXED ? 1 : 3);
         const int step = std::max(1, (int)(w / std::max(1.0, rel)));
-        for (int f = f0; f < s1; f += step) {
-          const int len = std::min(s1 - f, step);
+        for (int f = f0; f < e1; f += step) {
+          const int len = std::min(e1 - f, step);
           // spread the starts of neighbouring units over the range
           const int turn = (int)(((int64_t)(k.units.size() % 16) * len) / 16);
           k.units.push_back(make_int4(i, f, f + len, lv | turn << 8));
@@ -787,6 +870,47 @@ cuapss_status run_tasks(cuapss_ctx* ctx, std::vector<FoldTask>& tasks, double nr
   return CUAPSS_OK;
 }
 
+// FoldTask::last of a self-join whose rows are sorted by length.
+cuapss_status block_reach(cuapss_ctx* ctx, FoldTask& k, double nrm2) {
+  Workspace& ws = ctx->ws;
+  cudaStream_t st = ctx->stream;
+  FoldSide& I = *k.I;
+  const int nb = I.nb;
+  // T = (t / norm)^2 with room for the rounding of t, of the norm and of the
+  // reported sums, in the fixed point of the squares
+  const double T = ((double)k.t - 1e-6) * ((double)k.t - 1e-6) / nrm2 * (1.0 - 1e-5);
+  if (!(T > 0.0) || T >= 1.9) return CUAPSS_OK;
+  int* d = nullptr;
+  ST_TRY(ws.get("fold:need", 2 * (size_t)nb, &d));
+  CU_TRY(cudaMemsetAsync(d, 0x3f, 4 * (size_t)nb, st));
+  CU_TRY(cudaMemsetAsync(d + nb, 0, 4 * (size_t)nb, st));
+  const int64_t slots = (int64_t)nb * kBlockRows;
+  k_block_needs<<<grid_for(slots * 32, kThreads), kThreads, 0, st>>>(
+      I.rowmap, slots, I.x.rp, I.x.val, (uint32_t)(T * kSquareScale), d, d + nb);
+  LAUNCH_CHECK();
+  std::vector<int> h(2 * (size_t)nb);
+  CU_TRY(cudaMemcpyAsync(h.data(), d, 8 * (size_t)nb, cudaMemcpyDeviceToHost, st));
+  CU_TRY(cudaStreamSynchronize(st));
+  // first[J]: the first I block with a row long enough for some row of J or of
+  // a later block
+  std::vector<int> first((size_t)nb);
+  int i = 0, longest = h[(size_t)nb];
+  std::vector<int> need(h.begin(), h.begin() + nb);
+  for (int j = nb - 2; j >= 0; --j) need[(size_t)j] = std::min(need[(size_t)j], need[(size_t)j + 1]);
+  for (int j = 0; j < nb; ++j) {
+    while (i < j && longest < need[(size_t)j]) longest = std::max(longest, h[(size_t)nb + ++i]);
+    first[(size_t)j] = i;
+  }
+  // first is non-decreasing: the last J of each I
+  k.last.assign((size_t)nb, nb - 1);
+  for (int q = 0, j = 0; q < nb; ++q) {
+    j = std::max(j, q);
+    while (j + 1 < nb && first[(size_t)j + 1] <= q) ++j;
+    k.last[(size_t)q] = j;
+  }
+  return CUAPSS_OK;
+}
+
 template <bool MIXED>
 cuapss_status join_fold_as(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float t,
                            const int32_t* perm, double nrm2, const CostFn& other_ns, FoldResult* r,
@@ -823,6 +947,8 @@ cuapss_status join_fold_as(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, fl
   } else {
     one_level(k);
   }
+  // (a launch and a round trip: 60 us)
+  if (self && sampled && k.cost > kReachMinNs * ctx->sms) ST_TRY(block_reach(ctx, k, nrm2));
   uint32_t needI[kClasses] = {}, needJ[kClasses] = {};
   needed(k, needI, needJ);
   ST_TRY(build_levels<MIXED>(SI, needI, perm, allocI, ws, "fold:I", st));

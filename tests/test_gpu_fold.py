@@ -78,3 +78,30 @@ def test_no_pruning_falls_back(ctx):
     val = (val / np.linalg.norm(val, axis=1, keepdims=True)).astype(np.float32).ravel()
     x = synth.Csr(np.arange(n + 1, dtype=np.int64) * m, col, val, 3 * m)
     _check(ctx.run(x, 0.95, capacity=1 << 22), oracle.apss(x, 0.95))
+
+
+@pytest.mark.parametrize("t", [0.5, 0.9])
+def test_rows_too_short_for_one_another(ctx, t):
+    # 40,000 rows whose lengths run from 1 to 400 with a few dominant values:
+    # tiles of short against long rows are skipped, and rows with one large
+    # value match much longer ones
+    rng = np.random.default_rng(11)
+    n, d = 40_000, 3000
+    lens = np.minimum(400, np.maximum(1, rng.lognormal(3.0, 1.3, size=n))).astype(np.int64)
+    rp = np.zeros(n + 1, np.int64)
+    np.cumsum(lens, out=rp[1:])
+    col = np.concatenate([np.sort(rng.choice(d, size=k, replace=False)) for k in lens]).astype(np.int32)
+    val = rng.uniform(0.5, 1.5, size=int(rp[-1]))
+    big = rng.random(n) < 0.3
+    val[rp[:-1][big]] *= 30.0
+    row = np.repeat(np.arange(n), lens)
+    val = (val / np.sqrt(np.bincount(row, weights=val * val))[row]).astype(np.float32)
+    x = synth.Csr(rp, col, val, d)
+    rows = np.concatenate([rng.choice(n, size=120, replace=False), np.argsort(lens)[-8:],
+                           np.argsort(lens)[:8]])
+    rows = np.unique(rows).astype(np.int32)
+    wi, wj, ws = oracle.rows(x, t, rows)
+    assert len(wi) > 100
+    gi, gj, gs = ctx.run(x, t, capacity=1 << 24)
+    sel = np.isin(gi, rows) | np.isin(gj, rows)
+    _check((gi[sel], gj[sel], gs[sel]), (wi, wj, ws))
