@@ -359,11 +359,12 @@ cuapss_status join_device(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, flo
   CU_TRY(cudaMemsetAsync(counts, 0, sizeof(int32_t) * d, st));
   double nrm_a = 1.0, nrm_b = 1.0;
   const int check = ctx->opts.validate;
+  bool neg_a = true, neg_b = true;
   ST_TRY(validate_csr(a.rp, a.col, a.val, a.n, d, a.nnz, ctx->opts.norm_tol, check, counts, &nrm_a,
-                      ws, "A", st));
+                      ws, "A", st, &neg_a));
   if (!self)
     ST_TRY(validate_csr(bb.rp, bb.col, bb.val, bb.n, d, bb.nnz, ctx->opts.norm_tol, check, counts,
-                        &nrm_b, ws, "B", st));
+                        &nrm_b, ws, "B", st, &neg_b));
   else
     nrm_b = nrm_a;
   ST_TRY(feature_perm(counts, d, a.n + (self ? 0 : bb.n), ctx->opts.remap, perm, ws, st));
@@ -441,7 +442,10 @@ cuapss_status join_device(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, flo
       *ns = mixed ? plan.tile_ns : plain_tile_ns(nnz_all, n_all);
       return CUAPSS_OK;
     };
-    ST_TRY(join_fold(ctx, a, b, t, perm, nrm2, probing_ns, &fr, &done));
+    DevCsr fa = a, fb = bb;
+    fa.nonneg = !neg_a;
+    fb.nonneg = !neg_b;
+    ST_TRY(join_fold(ctx, fa, self ? nullptr : &fb, t, perm, nrm2, probing_ns, &fr, &done));
     if (done) {
       cudaEventRecord(ctx->ev[2], st);
       nvtx.next("cuapss_run:finalize");

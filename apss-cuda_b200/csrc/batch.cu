@@ -400,8 +400,9 @@ cuapss_status batch_device(cuapss_ctx* ctx, const DevCsr& x, int k, const int64_
   ST_TRY(ws.get("perm", (size_t)d, &perm));
   CU_TRY(cudaMemsetAsync(counts, 0, sizeof(int32_t) * d, st));
   double nrm = 1.0;
+  bool negative = true;
   ST_TRY(validate_csr(x.rp, x.col, x.val, x.n, d, x.nnz, ctx->opts.norm_tol, ctx->opts.validate,
-                      counts, &nrm, ws, "A", st));
+                      counts, &nrm, ws, "A", st, &negative));
   if (nrm * nrm >= 1.9) return CUAPSS_EINVAL;  // fixed-point tail needs ~unit norms
   ST_TRY(feature_perm(counts, d, x.n, ctx->opts.remap, perm, ws, st));
   // ---- the folded form, unless a head width or no remap fixes the probing
@@ -414,7 +415,9 @@ cuapss_status batch_device(cuapss_ctx* ctx, const DevCsr& x, int k, const int64_
     std::vector<int> width;
     FoldResult fr;
     bool done = false;
-    ST_TRY(fold_batch(ctx, x, k, inst_ptr, tq, perm, nrm * nrm, other_ns, &width, &fr, &done));
+    DevCsr fx = x;
+    fx.nonneg = !negative;
+    ST_TRY(fold_batch(ctx, fx, k, inst_ptr, tq, perm, nrm * nrm, other_ns, &width, &fr, &done));
     if (done) {
       cudaEventRecord(ctx->ev[2], st);
       nvtx.next("cuapss_batch_run:finalize");

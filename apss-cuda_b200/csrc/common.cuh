@@ -51,6 +51,7 @@ enum : int {
   kErrNorm = 16,       // | ||x|| - 1 | > tol
   kErrTimeout = 32,    // a bounded wait gave up
   kErrInternal = 64,   // an internal capacity check failed
+  kNegative = 128,     // not an error: some value is negative
 };
 
 constexpr int kBlockRows = 128;  // rows per row block (tile edge)

@@ -38,6 +38,7 @@ struct DevCsr {
   const int64_t* rp = nullptr;
   const int32_t* col = nullptr;
   const float* val = nullptr;
+  bool nonneg = false;  // no value is negative (known after validation)
 };
 
 // Validates the descriptor and returns device pointers (staging host

@@ -173,6 +173,7 @@ __global__ void k_check_rows(const int64_t* __restrict__ rp, const int32_t* __re
           if (c < 0 || c >= d) bad_all |= kErrColRange;
           if (e > lo[q] && before >= c) bad_all |= kErrColOrder;
           if (!isfinite(v)) bad_all |= kErrValue;
+          if (v < 0.0f) bad_all |= kNegative;
           ss[q] += (double)v * (double)v;
           if (counts && c >= 0 && c < d) hist_add(MODE, hist, counts, c);
         }
@@ -1157,7 +1158,7 @@ cuapss_status build_explicit_pairs(Side& s, const PrepOptions& o, int64_t* rcoun
 cuapss_status validate_csr(const int64_t* rp, const int32_t* col, const float* val, int64_t n,
                            int64_t d, int64_t nnz, float tol, int check, int32_t* counts,
                            double* nrm_max, Workspace& ws, const std::string& tag,
-                           cudaStream_t st) {
+                           cudaStream_t st, bool* negative) {
   unsigned long long* nm = nullptr;  // largest norm's bits, then the error flags
   ST_TRY(ws.get(tag + ":check", 2, &nm));
   int* err = reinterpret_cast<int*>(nm + 1);
@@ -1201,7 +1202,8 @@ cuapss_status validate_csr(const int64_t* rp, const int32_t* col, const float* v
   unsigned long long h[2] = {0, 0};
   CU_TRY(cudaMemcpyAsync(h, nm, sizeof(h), cudaMemcpyDeviceToHost, st));
   CU_TRY(cudaStreamSynchronize(st));
-  if (h[1]) return CUAPSS_EINVAL;
+  if (h[1] & ~(unsigned long long)kNegative) return CUAPSS_EINVAL;
+  if (negative) *negative = (h[1] & kNegative) != 0;
   double v;
   memcpy(&v, &h[0], sizeof(v));
   if (nrm_max) *nrm_max = v;

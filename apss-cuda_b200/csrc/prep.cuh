@@ -27,11 +27,12 @@ struct PrepOptions {
 };
 
 // Validates a device CSR. counts (device, d entries, may be null) are
-// incremented per posting. *nrm_max receives the largest row norm.
+// incremented per posting. *nrm_max receives the largest row norm, *negative
+// (may be null) whether some value is negative.
 cuapss_status validate_csr(const int64_t* rp, const int32_t* col, const float* val, int64_t n,
                            int64_t d, int64_t nnz, float tol, int check, int32_t* counts,
                            double* nrm_max, Workspace& ws, const std::string& tag,
-                           cudaStream_t st);
+                           cudaStream_t st, bool* negative = nullptr);
 
 // perm[f] = rank of feature f by (count desc, id asc); identity if !remap.
 cuapss_status feature_perm(const int32_t* counts, int64_t d, int64_t max_count, int remap,

@@ -237,13 +237,15 @@ cuapss_status build_segment(cuapss_ctx* ctx, const cuapss_index* idx, const DevC
 
 // Validates x (device CSR) and returns its largest row norm; counts (d
 // entries) receives the posting counts when non-null.
-cuapss_status check_rows(cuapss_ctx* ctx, const cuapss_index* idx, const DevCsr& x,
+cuapss_status check_rows(cuapss_ctx* ctx, const cuapss_index* idx, DevCsr& x,
                          int32_t* counts, double* nrm, const std::string& tag) {
   int32_t* c = counts;
   if (!c) ST_TRY(ctx->ws.get(tag + ":counts", (size_t)idx->d, &c));
   CU_TRY(cudaMemsetAsync(c, 0, sizeof(int32_t) * idx->d, ctx->stream));
+  bool negative = true;
   ST_TRY(validate_csr(x.rp, x.col, x.val, x.n, idx->d, x.nnz, idx->norm_tol, idx->validate, c,
-                      nrm, ctx->ws, tag, ctx->stream));
+                      nrm, ctx->ws, tag, ctx->stream, &negative));
+  x.nonneg = !negative;
   return CUAPSS_OK;
 }
 
@@ -421,6 +423,7 @@ cuapss_status index_merge_step(cuapss_ctx* ctx, cuapss_index* idx, bool* merged)
   DevCsr m;
   ST_TRY(concat_segments(ctx, *A, *B, &m));
   m.d = idx->d;
+  m.nonneg = A->fold && A->fold->x.nonneg && B->fold && B->fold->x.nonneg;
   std::shared_ptr<Segment> ab;
   ST_TRY(build_segment(ctx, idx, m, A->row0, std::max(A->nrm, B->nrm), &ab));
   std::lock_guard<std::mutex> lk(idx->mu);
