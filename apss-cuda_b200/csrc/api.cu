@@ -761,7 +761,6 @@ cuapss_status cuapss_create(cuapss_ctx** out, const cuapss_opts* opts) {
     }
     c->own_stream = true;
   }
-  c->ws.set_stream(c->stream);
   if (cudaHostAlloc(&c->pinned, kPinnedBytes, cudaHostAllocDefault) != cudaSuccess) {
     cudaGetLastError();
     cuapss_destroy(c);

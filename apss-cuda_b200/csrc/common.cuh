@@ -75,15 +75,12 @@ inline int bits_for(uint64_t v) {  // bits needed to represent values < v+1
   return b;
 }
 
-// Grow-only named device buffers owned by a context; avoids an allocation on
-// every call. Allocations and frees are ordered on the context's stream (all
-// its work runs there), so that neither waits for the device: building an
-// index of 200,000 rows spent 30 of 34 ms in cudaMalloc and cudaFree of its
-// temporaries.
+// Grow-only named device buffers owned by a context; avoids cudaMalloc on
+// every call. (cudaMalloc maps a GB in about 1 ms, a stream-ordered pool that
+// has to grow in 6-30 ms.)
 class Workspace {
  public:
   ~Workspace() { release(); }
-  void set_stream(cudaStream_t st) { st_ = st; }
   // Returns a device pointer with at least `bytes` bytes (256-byte aligned).
   cuapss_status get(const std::string& name, size_t bytes, void** out) {
     if (bytes == 0) bytes = 256;
@@ -93,15 +90,15 @@ class Workspace {
       return CUAPSS_OK;
     }
     if (it != bufs_.end()) {
-      cudaFreeAsync(it->second.ptr, st_);
+      cudaFree(it->second.ptr);
       bufs_.erase(it);
     }
     void* p = nullptr;
     size_t want = bytes + bytes / 8;  // headroom against regrowth
-    cudaError_t e = cudaMallocAsync(&p, want, st_);
+    cudaError_t e = cudaMalloc(&p, want);
     if (e != cudaSuccess) {
       cudaGetLastError();
-      e = cudaMallocAsync(&p, bytes, st_);
+      e = cudaMalloc(&p, bytes);
       want = bytes;
       if (e != cudaSuccess) {
         cudaGetLastError();
@@ -124,21 +121,21 @@ class Workspace {
     auto it = bufs_.find(name);
     return it == bufs_.end() ? 0 : it->second.size;
   }
-  size_t bytes_held() const {
+  size_t bytes_held(const std::string& prefix = "") const {
     size_t s = 0;
-    for (auto& kv : bufs_) s += kv.second.size;
+    for (auto& kv : bufs_)
+      if (kv.first.compare(0, prefix.size(), prefix) == 0) s += kv.second.size;
     return s;
   }
   void release() {
-    for (auto& kv : bufs_) cudaFreeAsync(kv.second.ptr, st_);
-    if (!bufs_.empty()) cudaStreamSynchronize(st_);
+    for (auto& kv : bufs_) cudaFree(kv.second.ptr);
     bufs_.clear();
   }
   // Frees the buffers whose names start with prefix.
   void release_prefix(const std::string& prefix) {
     for (auto it = bufs_.begin(); it != bufs_.end();) {
       if (it->first.compare(0, prefix.size(), prefix) == 0) {
-        cudaFreeAsync(it->second.ptr, st_);
+        cudaFree(it->second.ptr);
         it = bufs_.erase(it);
       } else {
         ++it;
@@ -152,7 +149,6 @@ class Workspace {
     size_t size;
   };
   std::map<std::string, Buf> bufs_;
-  cudaStream_t st_ = nullptr;
 };
 
 // NVTX ranges of a call's host-side stages (prepare, tiles, finalize), for

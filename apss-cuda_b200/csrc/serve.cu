@@ -172,12 +172,20 @@ struct cuapss_index {
 namespace cuapss {
 namespace {
 
+constexpr double kPoolSegment = 2e9, kFoldRowBytes = 1400.0;
+constexpr size_t kKeepTemps = (size_t)2 << 30;
+
 // Builds a segment from device CSR x (rows become index rows row0..).
 cuapss_status build_segment(cuapss_ctx* ctx, const cuapss_index* idx, const DevCsr& x,
                             int64_t row0, double nrm, std::shared_ptr<Segment>* out) {
   cudaStream_t st = ctx->stream;
   auto seg = std::make_shared<Segment>();
-  seg->heap.set_streams(st, idx->free_st);
+  // Small segments come from the device's pool, which appends and merges
+  // return to without waiting for the device; a large one, made once, from
+  // cudaMalloc, which maps its memory ten times faster than a growing pool.
+  const double bytes = 16.0 * (double)x.nnz +
+                       (double)x.n * ((idx->mixed ? 2.0 : 4.0) * idx->p + kFoldRowBytes);
+  if (bytes <= kPoolSegment) seg->heap.set_streams(st, idx->free_st);
   seg->row0 = row0;
   seg->n = x.n;
   seg->nnz = x.nnz;
@@ -282,9 +290,8 @@ cuapss_status concat_segments(cuapss_ctx* ctx, const Segment& a, const Segment& 
 constexpr size_t kMaxSegments = 24;
 
 // The device's pool keeps at most a sixteenth of the device's memory that
-// nobody uses (building an index frees its temporaries there); the rest goes
-// back to the device. Mapping it anew costs about 15 ms a GB: with 2 GB kept,
-// building an index of 1M rows took 104 ms instead of 60.
+// nobody uses (destroyed indexes return their segments there); the rest goes
+// back to the device.
 constexpr uint64_t kPoolSlackShare = 16;
 void trim_pool(int device) {
   cudaMemPool_t pool = nullptr;
@@ -364,10 +371,13 @@ extern "C" cuapss_status cuapss_index_create(cuapss_ctx* ctx, const cuapss_csr* 
   std::shared_ptr<Segment> seg;
   ST_TRY(build_segment(ctx, idx.get(), a, 0, nrm, &seg));
   idx->p = seg->p;
-  ctx->ws.release_prefix("seg:");
-  ctx->ws.release_prefix("IX:");
-  CU_TRY(cudaStreamSynchronize(ctx->stream));
-  trim_pool(ctx->device);
+  // the temporaries of a small build stay in the context (its next index
+  // needs them again: freeing and allocating them took 20 of 34 ms at 200,000
+  // rows), those of a large one go back
+  if (ctx->ws.bytes_held("seg:") + ctx->ws.bytes_held("IX:") > kKeepTemps) {
+    ctx->ws.release_prefix("seg:");
+    ctx->ws.release_prefix("IX:");
+  }
   idx->segs.push_back(seg);
   idx->rows = a.n;
   idx->nrm = nrm;

@@ -305,12 +305,33 @@ def mean_stage(stats):
             for k in ("ms_preprocess", "ms_tiles", "ms_finalize", "ms_total")}
 
 
+def folded(s):
+    """Whether a call's join was folded: every candidate is then computed in
+    FP64 (the probing path rescores only its error band)."""
+    return s["candidates"] > 0 and s["rescored"] == s["candidates"]
+
+
+def folded_roofline(tile_ms, s, prec_mixed, bf16_sus, src):
+    """The folded join multiplies rows of 64 .. 2,048 (FP32: 16 .. 1,024)
+    columns, chosen per pair of length classes from sampled rows, and skips
+    tiles whose rows are too short for one another; the call does not report
+    that mix, so no rate is claimed for it here."""
+    return {"bound": "tensor" if prec_mixed else "fp32 fma", "achieved": None,
+            "peak": bf16_sus if prec_mixed else None, "unit": "TFLOP/s", "frac": None,
+            "traffic": None, "peak_source": src,
+            "kernel": "k_tiles_fold" if prec_mixed else "k_tiles_fold32",
+            "kernel_ms": tile_ms, "tiles": s["tiles"], "candidates": s["candidates"],
+            "note": "kernel_ms covers folding, tiles and verification; the tile kernel's "
+                    "tensor-pipe share is in profiles/k_tiles_fold.md"}
+
+
 def tile_roofline(stats, p, pairs, n, world, prec_mixed, x, peaks_):
     """Roofline of the pair-tile kernel from its CUDA-event time."""
     hbm, bf16, bf16_sus, src = peaks_
-    import cuapss
     tile_ms = sum(s["ms_tiles"] for s in stats) / len(stats)
     s0 = stats[-1]
+    if folded(s0):
+        return folded_roofline(tile_ms, s0, prec_mixed, bf16_sus, src)
     head_flops = 2.0 * p * pairs
     nb = (n + 127) // 128
     if world > 1:
@@ -478,7 +499,8 @@ def run_selfjoin(args, rank, world, local):
         "metric": METRIC, "value": value, "unit": "pairs/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms,
         "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
-        "dtype": "f32" if not mixed else "bf16 head + f32 tail + f64 band",
+        "dtype": "f32" if not mixed else "bf16 bounds + f64 candidates" if folded(s0)
+                 else "bf16 head + f32 tail + f64 band",
         "data": "synthetic (seeded generator, reference corpus not distributed)",
         "config": {"workload": workload, "n": x.n, "d": x.d, "nnz": x.nnz, "t": args.t,
                    "precision": args.precision, "head_width": p,
@@ -560,10 +582,8 @@ def run_selfjoin(args, rank, world, local):
                 "same_pair_set_as_headline": same_pairs(R4),
                 "roofline": tile_roofline(st4, int(st4[-1]["head_width"]), pairs_per_step, x.n,
                                           1, True, x, pk),
-                "note": f"the workload names a {ph}-feature dense head; the library's "
-                        f"cost model picks p = {p} and the rare-feature threshold together, "
-                        f"trading tensor-core head work (2p flops per pair) against sparse "
-                        f"tail work"}
+                "note": f"the workload names a {ph}-feature dense head (the probing path); by "
+                        f"itself the library folds rows and computes candidates only"}
             R4.close()
 
         # ---- the plain FP32 hybrid on the same data ----
@@ -711,7 +731,9 @@ def run_batch(args, rank, world, local):
     tile_ms = sum(s["ms_tiles"] for s in stats) / len(stats)
     s0 = stats[-1]
     tiles = int(s0["tiles"])
-    if prec == cuapss.PREC_MIXED:
+    if folded(s0):
+        roofline = folded_roofline(tile_ms, s0, prec == cuapss.PREC_MIXED, bf16, src)
+    elif prec == cuapss.PREC_MIXED:
         # head GEMM flops of the tiles actually run: 2 * 128 * 128 * p per
         # tile, p of the bucket that owns the most tiles (stats.head_width)
         flops = 2.0 * 128 * 128 * int(s0["head_width"]) * tiles
@@ -763,7 +785,8 @@ def run_batch(args, rank, world, local):
         "metric": METRIC, "value": value, "unit": "pairs/s", "n_gpus": world,
         "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms,
         "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": "f32" if prec == cuapss.PREC_FP32 else "bf16 head + f32 tail + f64 band",
+        "dtype": "f32" if prec == cuapss.PREC_FP32 else "bf16 bounds + f64 candidates"
+                 if folded(s0) else "bf16 head + f32 tail + f64 band",
         "data": "synthetic (seeded generator, independent row stream per instance)",
         "config": {"workload": "batch", "instances": int(len(tq)), "rows": x.n, "d": x.d,
                    "nnz": x.nnz, "n_range": [int(ns.min()), int(ns.max())],
@@ -955,7 +978,7 @@ def run_serve(args, rank, world, local):
                   "resident index; p50/p99 ms",
         "value": out["q256"]["queries_per_s"], "unit": "queries/s", "n_gpus": 1,
         "steps": args.serve_requests, "warmup": 3, "higher_is_better": True,
-        "scaling": "weak", "vs_baseline": None, "dtype": "bf16 head + f32 tail + f64 band",
+        "scaling": "weak", "vs_baseline": None, "dtype": "bf16 bounds + f64 candidates",
         "data": "synthetic (seeded generator; queries are fresh rows of the index's stream)",
         "config": {"workload": "serve", "index_rows": n_index, "d": x.d, "nnz": x.nnz,
                    "head_width": info0["head_width"], "lanes": 3,
