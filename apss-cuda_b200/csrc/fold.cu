@@ -238,6 +238,13 @@ __host__ __device__ constexpr int fold_offset(bool mixed, uint32_t allow, int l)
   return o;
 }
 
+// Bytes of a row block's levels below l.
+constexpr size_t fold_offset_bytes(bool mixed, int l) {
+  size_t o = 0;
+  for (int k = 0; k < l; ++k) o += fold_bytes(mixed, k);
+  return o;
+}
+
 template <bool MIXED, int LEV>
 __device__ __forceinline__ void fold_add(uint32_t mask, uint32_t* acc, uint32_t allow, uint32_t r,
                                          float v, uint32_t square) {
@@ -478,10 +485,15 @@ cuapss_status sample_side(FoldSide& s, uint32_t levels, unsigned long long* len_
   k_sample_rows<<<kClasses, kBlockRows, 0, st>>>(s.rowmap, s.x.rp, class_rows(s), s.sample,
                                                  len_sum);
   LAUNCH_CHECK();
+  size_t total = 0;
+  for (int l = 0; l < kFoldLevels; ++l)
+    if ((levels >> l) & 1u) total += kClasses * fold_bytes(MIXED, l);
+  ST_TRY(alloc("samples", total, &p));
+  uint8_t* at = static_cast<uint8_t*>(p);
   for (int l = 0; l < kFoldLevels; ++l) {
     if (!((levels >> l) & 1u)) continue;
-    ST_TRY(alloc("sample" + std::to_string(l), kClasses * fold_bytes(MIXED, l), &p));
-    s.sample_out.base[l] = static_cast<uint8_t*>(p);
+    s.sample_out.base[l] = at;
+    at += kClasses * fold_bytes(MIXED, l);
   }
   return fold_places<MIXED>(s, s.sample, kSampleSlots, {}, levels, perm, s.sample_out, ws, tag, st);
 }
@@ -679,21 +691,27 @@ template <bool MIXED>
 cuapss_status build_levels(FoldSide& s, const uint32_t (&need)[kClasses], const int32_t* perm,
                            const FoldAlloc& alloc, Workspace& ws, const std::string& tag,
                            cudaStream_t st) {
-  uint32_t all = 0;
-  for (int c = 0; c < kClasses; ++c)
-    if (s.edge[c + 1] > s.edge[c]) all |= need[c];
+  // one allocation for all levels: which levels a call takes varies from input
+  // to input more than their total does
+  size_t size[kFoldLevels] = {}, total = 0;
   for (int l = 0; l < kFoldLevels; ++l) {
-    if (!((all >> l) & 1u)) continue;
     int lo = s.nb, hi = 0;
     for (int c = 0; c < kClasses; ++c)
       if (s.edge[c + 1] > s.edge[c] && ((need[c] >> l) & 1u)) {
         lo = std::min(lo, s.edge[c]);
         hi = std::max(hi, s.edge[c + 1]);
       }
+    if (hi <= lo) continue;
     s.out.first[l] = lo;
-    void* p = nullptr;
-    ST_TRY(alloc("lev" + std::to_string(l), (size_t)(hi - lo) * fold_bytes(MIXED, l), &p));
-    s.out.base[l] = static_cast<uint8_t*>(p);
+    size[l] = (size_t)(hi - lo) * fold_bytes(MIXED, l);
+    total += size[l];
+  }
+  void* p = nullptr;
+  ST_TRY(alloc("levels", total, &p));
+  uint8_t* at = static_cast<uint8_t*>(p);
+  for (int l = 0; l < kFoldLevels; ++l) {
+    s.out.base[l] = size[l] ? at : nullptr;
+    at += size[l];
   }
   std::vector<uint16_t> masks((size_t)s.nb, 0);
   for (int c = 0; c < kClasses; ++c)
@@ -787,7 +805,14 @@ cuapss_status run_tasks(cuapss_ctx* ctx, std::vector<FoldTask>& tasks, double nr
   unsigned long long* ctl = nullptr;
   ST_TRY(ws.get("fold:ctl", 1 + 3 * nt, &ctl));
   std::vector<unsigned long long> h(1 + 3 * nt);
-  // room that earlier calls left is room to use
+  // sizes in steps of a quarter of their power of two, so that calls of similar
+  // inputs find their buffers large enough; room that earlier calls left is
+  // room to use (as it is: no call asks for more because of it)
+  for (FoldTask& k : tasks) {
+    int64_t step = 1 << 16;
+    while (step * 8 <= k.cap) step *= 2;
+    k.cap = (k.cap + step - 1) / step * step;
+  }
   if (nt == 1)
     tasks[0].cap = std::max<int64_t>(
         tasks[0].cap, (int64_t)std::min({ws.held("fold:cand") / 8, ws.held("out:key") / 8,
@@ -1130,9 +1155,10 @@ cuapss_status fold_batch_as(cuapss_ctx* ctx, const DevCsr& x, int k, const int64
   for (int64_t i = 0; i < slots; ++i) ht[(size_t)i] = grid[i / kBlockRows];
   CU_TRY(cudaMemcpyAsync(sample_t, ht.data(), 4 * (size_t)slots, cudaMemcpyHostToDevice, st));
   FoldOut so;
+  uint8_t* samples = nullptr;
+  ST_TRY(ws.get("fold:sI:samples", kClasses * fold_offset_bytes(MIXED, kFoldLevels), &samples));
   for (int l = 0; l < kFoldLevels; ++l)
-    ST_TRY(ws.get("fold:sI:sample" + std::to_string(l), kClasses * fold_bytes(MIXED, l),
-                  &so.base[l]));
+    so.base[l] = samples + kClasses * fold_offset_bytes(MIXED, l);
   const uint32_t every = (1u << kFoldLevels) - 1u;
   ST_TRY(fold_places<MIXED>(B, sample, slots, {}, every, perm, so, ws, "fold:sI", st));
   FoldTileArgs ta;
@@ -1215,6 +1241,7 @@ cuapss_status fold_batch_as(cuapss_ctx* ctx, const DevCsr& x, int k, const int64
   std::vector<FoldTask> tasks(1);
   FoldTask& task = tasks[0];
   int64_t S = 0;
+  size_t size[kFoldLevels] = {}, total = 0;
   std::vector<uint16_t> masks;
   const int most = (int)std::max(1.0, std::min(64.0, tiles / pair / (ctx->sms * 16.0)));
   for (int l = kFoldLevels - 1; l >= 0; --l) {  // the costly ones first
@@ -1236,10 +1263,14 @@ cuapss_status fold_batch_as(cuapss_ctx* ctx, const DevCsr& x, int k, const int64
       S += (int64_t)(b1 - b0) * kBlockRows;
       if (S >= INT32_MAX) return CUAPSS_EINVAL;
     }
-    const int64_t blocks = S / kBlockRows - B.out.first[l];
-    if (blocks > 0)
-      ST_TRY(ws.get("fold:B:lev" + std::to_string(l), (size_t)blocks * fold_bytes(MIXED, l),
-                    &B.out.base[l]));
+    size[l] = (size_t)(S / kBlockRows - B.out.first[l]) * fold_bytes(MIXED, l);
+    total += size[l];
+  }
+  uint8_t* levels = nullptr;
+  ST_TRY(ws.get("fold:B:levels", total, &levels));
+  for (int l = 0; l < kFoldLevels; ++l) {
+    if (size[l]) B.out.base[l] = levels;
+    levels += size[l];
   }
   B.nb = (int)(S / kBlockRows);
   B.slots = S;

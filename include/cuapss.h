@@ -95,14 +95,23 @@ typedef struct {
   int on_device;     /* 1: i, j, sim are device pointers */
 } cuapss_pairs;
 
+/* With default options a join is folded where that prunes (rows of 16 .. 2,048
+ * columns bound every pair, candidates are computed in FP64) and probes
+ * otherwise; a head_width, a rare_max_count, remap = 0 or a shard always
+ * probe. The result is the same. head_width, tail_entries, explicit_pairs and
+ * rare_max_count are the probing path's plan in either case, which
+ * cuapss_plan_self_join gives too (index queries and batches count no tail
+ * when folded, and a folded batch reports folded widths). */
 typedef struct {
   int64_t pairs;          /* pairs emitted (sim >= t) */
   int64_t candidates;     /* pairs that left the tile epilogue */
-  int64_t rescored;       /* candidates inside the error band, redone in FP64 */
-  int64_t tiles;          /* 128x128 pair tiles evaluated */
+  int64_t rescored;       /* candidates inside the error band, redone in FP64
+                             (folded: every candidate) */
+  int64_t tiles;          /* 128x128 pair tiles of the call (folded self-joins
+                             skip those whose rows are too short to match) */
   int64_t head_width;     /* p used */
   int64_t tail_entries;   /* non-zeros outside the head */
-  int64_t tail_products;  /* sum over tail features of L(L-1)/2 */
+  int64_t tail_products;  /* sum over tail features of L(L-1)/2 (folded: 0) */
   double max_band;        /* largest error margin used by the epilogue */
   double ms_preprocess;   /* validate + remap + row order + norms + layout */
   double ms_index;        /* inverted lists (block-local and global) */
