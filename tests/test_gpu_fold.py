@@ -105,3 +105,58 @@ def test_rows_too_short_for_one_another(ctx, t):
     gi, gj, gs = ctx.run(x, t, capacity=1 << 24)
     sel = np.isin(gi, rows) | np.isin(gj, rows)
     _check((gi[sel], gj[sel], gs[sel]), (wi, wj, ws))
+
+
+@pytest.mark.parametrize("signed", [False, True])
+def test_index_query_sampled_widths(ctx, signed):
+    # 157 x 16 tiles of 128 x 128: the widths come from samples (from 2,048
+    # tiles on); thresholds differ by query
+    x = synth.generate("plain_800k", n=20_000, seed=8)
+    q = synth.generate("plain_800k", n=2000, seed=8, row_offset=19_000)
+    if signed:
+        x, q = _signed(x, 9), _signed(q, 10)
+    t = np.random.default_rng(12).uniform(0.3, 0.9, size=q.n).astype(np.float32)
+    with cuapss.Index(ctx, x) as idx:
+        gi, gj, gs = idx.query(q, t)
+    wi, wj, ws = oracle.join(q, x, float(t.min()))
+    keep = ws >= t[wi].astype(np.float64)
+    assert keep.sum() >= 1000 * (not signed)  # 1,000 queries are index rows
+    _check((gi, gj, gs), (wi[keep], wj[keep], ws[keep]))
+
+
+def test_batch_signed_and_odd_blocks(ctx):
+    # instances of 1 .. 5 blocks: odd last blocks are multiplied alone
+    sizes = [1, 128, 129, 257, 384, 385, 640, 2]
+    x = _signed(synth.generate("plain_20k", n=sum(sizes), seed=13), 14)
+    ptr = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    t = np.linspace(0.2, 0.6, len(sizes)).astype(np.float32)
+    want = [oracle.apss(x.rows(a, b), float(tq)) for a, b, tq in zip(ptr, ptr[1:], t)]
+    want = [np.concatenate([w[k] + (a if k < 2 else 0) for a, w in zip(ptr, want)])
+            for k in range(3)]
+    assert len(want[0]) > 0
+    _check(ctx.batch_run(x, ptr, t), want)
+
+
+@pytest.mark.parametrize("groups", [2047, 2048, 2049])
+def test_result_sort_edge(ctx, groups):
+    # two pairs a group of near-duplicates: 4,094 / 4,096 / 4,098 results
+    # around the 4,096 that one launch ranks
+    rng = np.random.default_rng(groups)
+    d = 50_000
+    rows, cols, vals = [0], [], []
+    for g in range(groups):
+        base = np.sort(rng.choice(d, size=12, replace=False)).astype(np.int32)
+        v = rng.uniform(0.5, 1.5, size=12)
+        # the outer two share half of the middle's squares each and no feature
+        h = np.sqrt(np.sum(v[:6] ** 2) / np.sum(v[6:] ** 2))
+        v[6:] *= h
+        for sl in (slice(0, 6), slice(0, 12), slice(6, 12)):
+            w = v[sl] / np.linalg.norm(v[sl])
+            cols.append(base[sl])
+            vals.append(w)
+            rows.append(rows[-1] + len(w))
+    x = synth.Csr(np.array(rows, np.int64), np.concatenate(cols),
+                  np.concatenate(vals).astype(np.float32), d)
+    want = oracle.apss(x, 0.7)
+    assert len(want[0]) == 2 * groups
+    _check(ctx.run(x, 0.7, capacity=1 << 14), want)
