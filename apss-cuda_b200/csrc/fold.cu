@@ -229,12 +229,12 @@ __host__ __device__ constexpr size_t fold_bytes(bool mixed, int level) {  // of 
   return (size_t)fold_k(mixed, level) * kBlockRows * (mixed ? 2 : 4);
 }
 
-// First accumulator column of level l when the levels of `allow` lie one
+// First accumulator column of level l when the levels of `mask` lie one
 // after another, and their total.
-__host__ __device__ constexpr int fold_offset(bool mixed, uint32_t allow, int l) {
+__host__ __device__ constexpr int fold_offset(bool mixed, uint32_t mask, int l) {
   int o = 0;
   for (int k = 0; k < l; ++k)
-    if ((allow >> k) & 1u) o += fold_k(mixed, k);
+    if ((mask >> k) & 1u) o += fold_k(mixed, k);
   return o;
 }
 
@@ -245,14 +245,68 @@ constexpr size_t fold_offset_bytes(bool mixed, int l) {
   return o;
 }
 
-template <bool MIXED, int LEV>
-__device__ __forceinline__ void fold_add(uint32_t mask, uint32_t* acc, uint32_t allow, uint32_t r,
-                                         float v, uint32_t square) {
-  constexpr uint32_t P = fold_k(MIXED, LEV) / 4, M = fold_k(MIXED, LEV) - P;
-  if (!((mask >> LEV) & 1u)) return;  // uniform over the row's threads
-  uint32_t* a = acc + fold_offset(MIXED, allow, LEV);
-  if (r < P) a[r] = __float_as_uint(v);
-  else atomicAdd(&a[P + (r - P) % M], square);
+// A level's columns, for loops over the levels of a mask: k columns, p of them
+// exact, m = k - p shared; x / m = umulhi(x, magic) >> shift for x < 2^31
+// (magic = ceil(2^(31 + s) / m) with s = ceil(log2 m): the error x e / (m
+// 2^(31 + s)), e < m <= 2^s, is below 1 / m).
+struct FoldDiv {
+  uint32_t k, p, m, magic, shift;
+};
+struct FoldDivs {
+  FoldDiv d[2][kFoldLevels];
+};
+constexpr FoldDivs fold_divs() {
+  FoldDivs t{};
+  for (int f = 0; f < 2; ++f)
+    for (int l = 0; l < kFoldLevels; ++l) {
+      const uint32_t k = (uint32_t)fold_k(f == 1, l), m = k - k / 4;
+      uint32_t s = 0;
+      while ((1u << s) < m) ++s;
+      const uint64_t pow = 1ull << (31 + s);
+      t.d[f][l] = {k, k / 4, m, (uint32_t)((pow + m - 1) / m), s - 1};
+    }
+  return t;
+}
+__constant__ const FoldDivs kFoldDivs = fold_divs();
+
+// Runs f(l, D) for the levels l of mask (the row's threads take the same
+// branches): unrolled, with constants for D, or as a loop.
+template <bool MIXED, bool UNROLL, typename F>
+__device__ __forceinline__ void fold_for_levels(uint32_t mask, F&& f) {
+  if constexpr (UNROLL) {
+#pragma unroll
+    for (int l = 0; l < kFoldLevels; ++l)
+      if ((mask >> l) & 1u) {
+        const uint32_t k = (uint32_t)fold_k(MIXED, l);
+        f(l, FoldDiv{k, k / 4, k - k / 4, 0, 0});
+      }
+  } else {
+    for (uint32_t w = mask; w; w &= w - 1) {
+      const int l = __ffs(w) - 1;
+      f(l, kFoldDivs.d[MIXED][l]);
+    }
+  }
+}
+
+// N entries of a row into the columns of every level of mask (f: rank, < 0:
+// none).
+template <bool MIXED, int N, bool UNROLL>
+__device__ __forceinline__ void fold_add(uint32_t mask, uint32_t* acc, const int32_t (&f)[N],
+                                         const float (&v)[N]) {
+  uint32_t square[N];
+#pragma unroll
+  for (int q = 0; q < N; ++q) square[q] = __float2uint_ru(__fmul_ru(v[q], v[q]) * kSquareScale);
+  fold_for_levels<MIXED, UNROLL>(mask, [&](int, const FoldDiv D) {
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+      const uint32_t r = (uint32_t)f[q], x = r - D.p;
+      if (r < D.p) acc[r] = __float_as_uint(v[q]);
+      else if (f[q] >= 0)
+        atomicAdd(&acc[D.p + (UNROLL ? x % D.m : x - (__umulhi(x, D.magic) >> D.shift) * D.m)],
+                  square[q]);
+    }
+    acc += D.k;
+  });
 }
 
 // Norm of a shared column from its fixed-point squares, times scale: an upper
@@ -271,51 +325,62 @@ __device__ __forceinline__ uint32_t bf16x2_up(float lo, float hi) {
   return __byte_perm(__float_as_uint(lo) + 0xffffu, __float_as_uint(hi) + 0xffffu, 0x7632);
 }
 
-template <bool MIXED, int LEV>
-__device__ __forceinline__ void fold_write(uint32_t mask, const uint32_t* acc, uint32_t allow,
-                                           const FoldOut& O, float scale, bool nonneg, int b,
-                                           int rr, int tid, int nt) {
-  constexpr int K = fold_k(MIXED, LEV), P = K / 4;
-  if (!((mask >> LEV) & 1u)) return;
-  const uint32_t* a = acc + fold_offset(MIXED, allow, LEV);
-  uint8_t* dst = O.base[LEV] + (size_t)(b - O.first[LEV]) * fold_bytes(MIXED, LEV);
+// A row's sums to its place (block b, row rr) in every level of mask.
+template <bool MIXED, bool UNROLL>
+__device__ __forceinline__ void fold_write(uint32_t mask, const uint32_t* acc, const FoldOut& O,
+                                           float scale, bool nonneg, int b, int rr, int tid,
+                                           int nt) {
   const float up = __fmul_ru(scale, 1.0f + 4.76837158e-7f);  // 1 + 2^-21
-  if (!MIXED) {  // [column][row]
-    for (int c = tid; c < K; c += nt)
-      reinterpret_cast<float*>(dst)[c * kBlockRows + rr] =
-          c < P ? __uint_as_float(a[c]) * scale : fold_norm(a[c], up);
-    return;
-  }
-  uint4* out = reinterpret_cast<uint4*>(dst);
-  for (int c8 = tid; c8 < K / 8; c8 += nt) {
-    const uint4 x = reinterpret_cast<const uint4*>(a)[2 * c8];
-    const uint4 y = reinterpret_cast<const uint4*>(a)[2 * c8 + 1];
-    const uint32_t f[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
-    uint32_t w[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      if (c8 * 8 < P && nonneg) {  // P is a multiple of 8
-        w[q] = bf16x2_up(__fmul_ru(__uint_as_float(f[2 * q]), scale),
-                         __fmul_ru(__uint_as_float(f[2 * q + 1]), scale));
-      } else if (c8 * 8 < P) {
-        const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(f[2 * q]) * scale,
-                                                       __uint_as_float(f[2 * q + 1]) * scale);
-        memcpy(&w[q], &h, 4);
-      } else {
-        w[q] = bf16x2_up(fold_norm(f[2 * q], up), fold_norm(f[2 * q + 1], up));
-      }
+  fold_for_levels<MIXED, UNROLL>(mask, [&](int l, const FoldDiv D) {
+    const int K = (int)D.k, P = K / 4;
+    const uint32_t* a = acc;
+    acc += K;
+    uint8_t* dst = O.base[l] + (size_t)(b - O.first[l]) * ((size_t)K * kBlockRows * (MIXED ? 2 : 4));
+    if (!MIXED) {  // [column][row]
+      for (int c = tid; c < K; c += nt)
+        reinterpret_cast<float*>(dst)[c * kBlockRows + rr] =
+            c < P ? __uint_as_float(a[c]) * scale : fold_norm(a[c], up);
+      return;
     }
-    const int kc = c8 >> 3, c = c8 & 7;
-    out[((size_t)kc * kBlockRows + rr) * 8 + (c ^ (rr & 7))] = make_uint4(w[0], w[1], w[2], w[3]);
-  }
+    uint4* out = reinterpret_cast<uint4*>(dst);
+    for (int c8 = tid; c8 < K / 8; c8 += nt) {
+      const uint4 x = reinterpret_cast<const uint4*>(a)[2 * c8];
+      const uint4 y = reinterpret_cast<const uint4*>(a)[2 * c8 + 1];
+      const uint32_t f[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+      uint32_t w[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (c8 * 8 >= P) {  // P is a multiple of 8
+          w[q] = bf16x2_up(fold_norm(f[2 * q], up), fold_norm(f[2 * q + 1], up));
+        } else if (nonneg) {
+          w[q] = bf16x2_up(__fmul_ru(__uint_as_float(f[2 * q]), scale),
+                           __fmul_ru(__uint_as_float(f[2 * q + 1]), scale));
+        } else {
+          const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(f[2 * q]) * scale,
+                                                         __uint_as_float(f[2 * q + 1]) * scale);
+          memcpy(&w[q], &h, 4);
+        }
+      }
+      const int kc = c8 >> 3, c = c8 & 7;
+      out[((size_t)kc * kBlockRows + rr) * 8 + (c ^ (rr & 7))] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  });
 }
 
 // t_row (per caller's row, may be null): the row is folded divided by its
 // threshold, so that one threshold of 1 serves rows of different ones.
-// GROUP threads per row (a warp, or the whole CTA for long rows). Blocks
+// GROUP threads per row (8 .. 32, or the whole CTA for long rows). Blocks
 // [b0, b1) of rowmap; blk_mask[b]: levels of block b (null: mask0 for all);
-// only blocks whose levels are all in `allow` (wide: some level is not
-// narrow) are taken. Shared memory: the columns of `allow` per row.
+// only blocks with (wide) or without a level that is not narrow are taken.
+// Bound by instructions: 425 a row of 30 entries in 192 columns when every
+// entry went through ten unrolled level tests with their offsets; a loop over
+// the levels that the block has, 4 entries at a time, 8 threads a row, takes
+// 1,112 -> 594 us for 1.6M such rows (672 with the unrolled tests). Longer
+// rows keep the unrolled levels, whose divisions are constants, and take
+// several entries between the tests: 200,000 rows of 120, a warp each, 308 ->
+// 275 us; rows with wide levels 143 -> 130 us (170 as a loop).
+// Shared memory: max_col columns per row, the most that a block's levels
+// have.
 constexpr uint32_t kNarrowLevels = 0x7f;  // K <= 512 (mixed), 192 (FP32)
 
 template <bool MIXED, int GROUP>
@@ -324,57 +389,61 @@ __global__ void __launch_bounds__(kThreads)
                 const int64_t* __restrict__ rp, const int32_t* __restrict__ col,
                 const float* __restrict__ val, const int32_t* __restrict__ perm,
                 const float* __restrict__ t_row, bool nonneg,
-                const uint16_t* __restrict__ blk_mask, uint32_t mask0, uint32_t allow, bool wide, FoldOut O) {
+                const uint16_t* __restrict__ blk_mask, uint32_t mask0, int max_col, bool wide,
+                const __grid_constant__ FoldOut O) {
   extern __shared__ __align__(16) uint32_t fold_sm[];
   constexpr int kGroups = kThreads / GROUP;
+  constexpr bool kUnroll = GROUP >= 32;
+  constexpr int N = GROUP > 32 ? 2 : 4;
   const int tid = threadIdx.x % GROUP;
-  const int ncol = fold_offset(MIXED, allow, kFoldLevels);
-  uint32_t* acc = fold_sm + (threadIdx.x / GROUP) * ncol;
+  uint32_t* acc = fold_sm + (threadIdx.x / GROUP) * max_col;
   for (int64_t s = slot0 + (int64_t)blockIdx.x * kGroups + threadIdx.x / GROUP; s < slot1;
        s += (int64_t)gridDim.x * kGroups) {
     const int b = (int)(s / kBlockRows), rr = (int)(s % kBlockRows);
     const uint32_t mask = blk_mask ? (uint32_t)blk_mask[b] : mask0;
-    if (mask == 0 || ((mask & ~kNarrowLevels) != 0) != wide) continue;  // same for all of GROUP
+    if (mask == 0 || ((mask & ~kNarrowLevels) != 0) != wide) continue;  // same for the warp
+    const int ncol = fold_offset(MIXED, mask, kFoldLevels);
     const int32_t r = rowmap[s];
     const int64_t lo = r >= 0 ? rp[r] : 0;
     const int len = r >= 0 ? (int)(rp[r + 1] - lo) : 0;
     for (int k = tid; k < ncol / 4; k += GROUP)
       reinterpret_cast<uint4*>(acc)[k] = make_uint4(0u, 0u, 0u, 0u);
-    if (GROUP == 32) __syncwarp();
+    if (GROUP <= 32) __syncwarp();
     else __syncthreads();
-    for (int e = tid; e < len; e += GROUP) {
-      const uint32_t f = (uint32_t)perm[col[lo + e]];
-      const float v = val[lo + e];
-      const uint32_t square = __float2uint_ru(__fmul_ru(v, v) * kSquareScale);
-      fold_add<MIXED, 0>(mask, acc, allow, f, v, square);
-      fold_add<MIXED, 1>(mask, acc, allow, f, v, square);
-      fold_add<MIXED, 2>(mask, acc, allow, f, v, square);
-      fold_add<MIXED, 3>(mask, acc, allow, f, v, square);
-      fold_add<MIXED, 4>(mask, acc, allow, f, v, square);
-      fold_add<MIXED, 5>(mask, acc, allow, f, v, square);
-      fold_add<MIXED, 6>(mask, acc, allow, f, v, square);
-      fold_add<MIXED, 7>(mask, acc, allow, f, v, square);
-      fold_add<MIXED, 8>(mask, acc, allow, f, v, square);
-      fold_add<MIXED, 9>(mask, acc, allow, f, v, square);
+    for (int e0 = 0; e0 < len; e0 += N * GROUP) {
+      int32_t f[N];
+      float v[N];
+#pragma unroll
+      for (int q = 0; q < N; ++q) {
+        const int e = e0 + q * GROUP + tid;
+        f[q] = e < len ? perm[col[lo + e]] : -1;
+        v[q] = e < len ? val[lo + e] : 0.0f;
+      }
+      fold_add<MIXED, N, kUnroll>(mask, acc, f, v);
     }
-    if (GROUP == 32) __syncwarp();
+    if (GROUP <= 32) __syncwarp();
     else __syncthreads();
     const float scale = t_row && r >= 0 ? __frcp_ru(t_row[r]) : 1.0f;
-    fold_write<MIXED, 0>(mask, acc, allow, O, scale, nonneg, b, rr, tid, GROUP);
-    fold_write<MIXED, 1>(mask, acc, allow, O, scale, nonneg, b, rr, tid, GROUP);
-    fold_write<MIXED, 2>(mask, acc, allow, O, scale, nonneg, b, rr, tid, GROUP);
-    fold_write<MIXED, 3>(mask, acc, allow, O, scale, nonneg, b, rr, tid, GROUP);
-    fold_write<MIXED, 4>(mask, acc, allow, O, scale, nonneg, b, rr, tid, GROUP);
-    fold_write<MIXED, 5>(mask, acc, allow, O, scale, nonneg, b, rr, tid, GROUP);
-    fold_write<MIXED, 6>(mask, acc, allow, O, scale, nonneg, b, rr, tid, GROUP);
-    fold_write<MIXED, 7>(mask, acc, allow, O, scale, nonneg, b, rr, tid, GROUP);
-    fold_write<MIXED, 8>(mask, acc, allow, O, scale, nonneg, b, rr, tid, GROUP);
-    fold_write<MIXED, 9>(mask, acc, allow, O, scale, nonneg, b, rr, tid, GROUP);
-    if (GROUP == 32) __syncwarp();
+    fold_write<MIXED, kUnroll>(mask, acc, O, scale, nonneg, b, rr, tid, GROUP);
+    if (GROUP <= 32) __syncwarp();
     else __syncthreads();
   }
 }
-static_assert(kFoldLevels == 10, "one fold_add / fold_write call per level");
+
+// Threads per row. Short rows leave most of a warp idle, in their entries (30)
+// and in writing 64 columns (8 lanes): 8 or 16 threads take a row where its
+// columns leave room for the CTA's rows in shared memory (8 rows a warp of
+// 512 columns: 64 KB a CTA) and the rows fill 8 CTAs a SM (20,000 rows: 54 us
+// with 8 threads a row, 24 with 16, 30 with 32).
+constexpr int kFoldCols8 = 512;
+constexpr int64_t kFoldRows8 = 148 * 8 * (kThreads / 8);
+constexpr int kFoldSmem = 64 * 1024;
+static_assert(fold_offset(true, kNarrowLevels, kFoldLevels) * 8 * 4 <= kFoldSmem &&
+                  fold_offset(false, kNarrowLevels, kFoldLevels) * 8 * 4 <= kFoldSmem &&
+                  fold_offset(true, (1u << kFoldLevels) - 1, kFoldLevels) * 4 <= kFoldSmem &&
+                  fold_offset(false, (1u << kFoldLevels) - 1, kFoldLevels) * 4 <= kFoldSmem &&
+                  kFoldCols8 * (kThreads / 8) * 4 <= kFoldSmem,
+              "shared memory of folded rows");
 
 // Folds the places of [0, slots) with the levels of masks (host, per block;
 // empty: mask0 everywhere) into O.
@@ -384,43 +453,43 @@ cuapss_status fold_places(const FoldSide& s, const int32_t* rowmap, int64_t slot
                           const FoldOut& O, Workspace& ws, const std::string& tag,
                           cudaStream_t st) {
   uint16_t* d_mask = nullptr;
-  // levels, and blocks, with and without a wide level
-  uint32_t all[2] = {0, 0};
+  // most columns of a block, and blocks, without and with a wide level
+  int cols[2] = {0, 0};
   int64_t b0[2] = {0, 0}, b1[2] = {0, 0};
   if (masks.empty()) {
     const int w = (mask0 & ~kNarrowLevels) ? 1 : 0;
-    all[w] = mask0;
+    cols[w] = fold_offset(MIXED, mask0, kFoldLevels);
     b1[w] = slots / kBlockRows;
   } else {
     ST_TRY(ws.get(tag + ":mask", masks.size(), &d_mask));
     CU_TRY(cudaMemcpyAsync(d_mask, masks.data(), 2 * masks.size(), cudaMemcpyHostToDevice, st));
     for (size_t b = 0; b < masks.size(); ++b) {
+      if (!masks[b]) continue;
       const int w = (masks[b] & ~kNarrowLevels) ? 1 : 0;
-      if (!all[w]) b0[w] = (int64_t)b;
-      all[w] |= masks[b];
-      if (masks[b]) b1[w] = (int64_t)b + 1;
+      if (!cols[w]) b0[w] = (int64_t)b;
+      cols[w] = std::max(cols[w], fold_offset(MIXED, masks[b], kFoldLevels));
+      b1[w] = (int64_t)b + 1;
     }
   }
   const DevCsr& x = s.x;
-  if (all[0]) {  // a warp per row
-    const size_t smem = (size_t)fold_offset(MIXED, all[0], kFoldLevels) * 4 * (kThreads / 32);
-    CU_TRY(cudaFuncSetAttribute((const void*)k_fold_rows<MIXED, 32>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                fold_offset(MIXED, kNarrowLevels, kFoldLevels) * 4 *
-                                    (kThreads / 32)));
-    k_fold_rows<MIXED, 32>
-        <<<grid_for((b1[0] - b0[0]) * kBlockRows, kThreads / 32), kThreads, smem, st>>>(
-            rowmap, b0[0] * kBlockRows, b1[0] * kBlockRows, x.rp, x.col, x.val, perm, s.t_row,
-            x.nonneg, d_mask, mask0, all[0], false, O);
-    LAUNCH_CHECK();
-  }
-  if (all[1]) {  // blocks of long rows (and the samples): a CTA per row
-    const size_t smem = (size_t)fold_offset(MIXED, all[1], kFoldLevels) * 4;
-    k_fold_rows<MIXED, kThreads>
-        <<<grid_for((b1[1] - b0[1]) * kBlockRows, 1), kThreads, smem, st>>>(
-            rowmap, b0[1] * kBlockRows, b1[1] * kBlockRows, x.rp, x.col, x.val, perm, s.t_row,
-            x.nonneg, d_mask, mask0, all[1], true, O);
-    LAUNCH_CHECK();
+  for (int w = 0; w < 2; ++w) {
+    if (!cols[w]) continue;
+    const int64_t rows = (b1[w] - b0[w]) * kBlockRows;
+    auto run = [&](auto kernel, int group) -> cuapss_status {
+      const size_t smem = (size_t)cols[w] * 4 * (kThreads / group);
+      CU_TRY(cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  kFoldSmem));
+      kernel<<<grid_for(rows, kThreads / group), kThreads, smem, st>>>(
+          rowmap, b0[w] * kBlockRows, b1[w] * kBlockRows, x.rp, x.col, x.val, perm, s.t_row,
+          x.nonneg, d_mask, mask0, cols[w], w == 1, O);
+      LAUNCH_CHECK();
+      return CUAPSS_OK;
+    };
+    if (w == 1) ST_TRY(run(k_fold_rows<MIXED, kThreads>, kThreads));  // and the samples
+    else if (cols[w] <= kFoldCols8 && rows >= kFoldRows8) ST_TRY(run(k_fold_rows<MIXED, 8>, 8));
+    else if (cols[w] <= 2 * kFoldCols8 && rows >= kFoldRows8 / 2)
+      ST_TRY(run(k_fold_rows<MIXED, 16>, 16));
+    else ST_TRY(run(k_fold_rows<MIXED, 32>, 32));
   }
   return CUAPSS_OK;
 }

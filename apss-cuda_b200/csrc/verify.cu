@@ -8,8 +8,11 @@
 // decision is then the oracle's. The order depends on the two rows alone, so
 // a pair's value does not depend on how the join was cut.
 //
-// Bound: latency of the searches' loads (rows come from L2), hidden by 64
-// warps a SM.
+// Bound: instructions of the merge (n = 60k, d = 50k, t = 0.5 in FP32: 3.2M
+// candidates in 1.63 ms, 427 warp instructions each, 73% of the issue slots
+// at 32 warps a SM; more warps in fewer registers, votes in place of the
+// shuffles of the chunks' ends and sums of four candidates at a time change
+// nothing). Rows come from L2, which is at 12%.
 #include <cuda_runtime.h>
 
 #include "fold.cuh"

@@ -160,3 +160,15 @@ def test_result_sort_edge(ctx, groups):
     want = oracle.apss(x, 0.7)
     assert len(want[0]) == 2 * groups
     _check(ctx.run(x, 0.7, capacity=1 << 14), want)
+
+
+@pytest.mark.parametrize("n", [18_815, 18_817, 37_760, 37_761])
+def test_threads_per_row(ctx, n):
+    # folded rows take 32, 16 or 8 threads each from 148 and 296 blocks on
+    x = synth.generate("batch_instance", n=n, seed=n)
+    rows = np.unique(np.random.default_rng(n).choice(n, size=150)).astype(np.int32)
+    wi, wj, ws = oracle.rows(x, 0.4, rows)
+    assert len(wi) > 0
+    gi, gj, gs = ctx.run(x, 0.4, capacity=1 << 24)
+    sel = np.isin(gi, rows) | np.isin(gj, rows)
+    _check((gi[sel], gj[sel], gs[sel]), (wi, wj, ws))
