@@ -1367,11 +1367,17 @@ cuapss_status fold_batch_as(cuapss_ctx* ctx, const DevCsr& x, int k, const int64
   return run_tasks<MIXED>(ctx, tasks, nrm2, va, 4 * expect, r, done);
 }
 
+// Verification holds a row's first entry in 32 bits; a longer matrix is left
+// to the probing path, which compacts it (batches) or refuses it.
+bool verifiable(const DevCsr& x) { return x.nnz < (int64_t)UINT32_MAX; }
+
 }  // namespace
 
 cuapss_status join_fold(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float t,
                         const int32_t* perm, double nrm2, const CostFn& other_ns, FoldResult* r,
                         bool* done) {
+  *done = false;
+  if (!verifiable(a) || (b && !verifiable(*b))) return CUAPSS_OK;
   return ctx->opts.precision == CUAPSS_PREC_MIXED
              ? join_fold_as<true>(ctx, a, b, t, perm, nrm2, other_ns, r, done)
              : join_fold_as<false>(ctx, a, b, t, perm, nrm2, other_ns, r, done);
@@ -1380,6 +1386,8 @@ cuapss_status join_fold(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float
 cuapss_status fold_batch(cuapss_ctx* ctx, const DevCsr& x, int k, const int64_t* inst_ptr,
                          const float* t, const int32_t* perm, double nrm2, double other_ns,
                          std::vector<int>* width, FoldResult* r, bool* done) {
+  *done = false;
+  if (!verifiable(x)) return CUAPSS_OK;
   return ctx->opts.precision == CUAPSS_PREC_MIXED
              ? fold_batch_as<true>(ctx, x, k, inst_ptr, t, perm, nrm2, other_ns, width, r, done)
              : fold_batch_as<false>(ctx, x, k, inst_ptr, t, perm, nrm2, other_ns, width, r, done);
@@ -1394,6 +1402,10 @@ cuapss_status fold_index(cuapss_ctx* ctx, bool mixed, const DevCsr& x, const int
 cuapss_status fold_query(cuapss_ctx* ctx, bool mixed, const std::vector<FoldSegment>& segs,
                          const DevCsr& q, const float* t_row, float t_min, const int32_t* perm,
                          double nrm2, double other_ns, int64_t rows, FoldResult* r, bool* done) {
+  *done = false;
+  if (!verifiable(q)) return CUAPSS_OK;
+  for (const FoldSegment& g : segs)
+    if (!verifiable(g.side->x)) return CUAPSS_OK;
   return mixed ? fold_query_as<true>(ctx, segs, q, t_row, t_min, perm, nrm2, other_ns, rows, r, done)
                : fold_query_as<false>(ctx, segs, q, t_row, t_min, perm, nrm2, other_ns, rows, r,
                                       done);
