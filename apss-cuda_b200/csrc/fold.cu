@@ -876,12 +876,15 @@ cuapss_status run_tasks(cuapss_ctx* ctx, std::vector<FoldTask>& tasks, double nr
   std::vector<unsigned long long> h(1 + 3 * nt);
   // sizes in steps of a quarter of their power of two, so that calls of similar
   // inputs find their buffers large enough; room that earlier calls left is
-  // room to use (as it is: no call asks for more because of it)
+  // room to use (as it is: no call asks for more because of it), but the route
+  // is decided by the caps that a new context would have
   for (FoldTask& k : tasks) {
     int64_t step = 1 << 16;
     while (step * 8 <= k.cap) step *= 2;
     k.cap = (k.cap + step - 1) / step * step;
   }
+  std::vector<int64_t> own;
+  for (const FoldTask& k : tasks) own.push_back(k.cap);
   if (nt == 1)
     tasks[0].cap = std::max<int64_t>(
         tasks[0].cap, (int64_t)std::min({ws.held("fold:cand") / 8, ws.held("out:key") / 8,
@@ -949,7 +952,7 @@ cuapss_status run_tasks(cuapss_ctx* ctx, std::vector<FoldTask>& tasks, double nr
     }
     CU_TRY(cudaMemcpyAsync(h.data(), ctl, 8 * (1 + 3 * nt), cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaStreamSynchronize(st));
-    bool over = false;
+    bool over = false, past_own = false;
     int64_t want = 0;
     for (size_t i = 0; i < nt; ++i) {
       const int herr = (int)h[3 + 3 * i];
@@ -958,15 +961,16 @@ cuapss_status run_tasks(cuapss_ctx* ctx, std::vector<FoldTask>& tasks, double nr
       const int64_t c = (int64_t)h[1 + 3 * i];
       want += c;
       over = over || c > tasks[i].cap;
+      past_own = past_own || c > own[i];
       tasks[i].cap = std::max(tasks[i].cap, c);
     }
     r->npairs = (int64_t)h[0];
     r->ncand = want;
+    if (past_own && want > max_cand) return CUAPSS_OK;
     if (!over) {
       *done = true;
       return CUAPSS_OK;
     }
-    if (want > max_cand) return CUAPSS_OK;
   }
   return CUAPSS_OK;
 }

@@ -51,3 +51,32 @@ def test_batch_past_32_bit_offsets(precision):
         c = ctx.batch_run_device(a, ptr, t, out)
     gi, gj, gs = (out[q][:c].cpu().numpy() for q in ("i", "j", "sim"))
     _check((gi - k, gj - k, gs), want)
+
+
+def _near_identical(n, groups, m, seed):
+    """n rows in groups of one support of m features each, values within 5%."""
+    rng = np.random.default_rng(seed)
+    g = np.arange(n) % groups
+    col = (g[:, None] * m + np.arange(m)).astype(np.int32).ravel()
+    val = 1.0 + 0.05 * rng.standard_normal((n, m))
+    val = (val / np.linalg.norm(val, axis=1, keepdims=True)).astype(np.float32).ravel()
+    return synth.Csr(np.arange(n + 1, dtype=np.int64) * m, col, val, groups * m)
+
+
+@pytest.mark.parametrize("precision,n,t", [(cuapss.PREC_MIXED, 100_000, 0.4),
+                                           (cuapss.PREC_FP32, 60_000, 0.5)], ids=["mixed", "fp32"])
+def test_route_does_not_depend_on_earlier_calls(precision, n, t):
+    """2,100 near-identical rows are 2.2M candidates, which a small folded join
+    does not take, also where an earlier call left room for them."""
+    x = _near_identical(2100, 1, 20, 7)
+    runs = []
+    for warm in (False, True):
+        with cuapss.Context(precision=precision) as ctx:
+            if warm:
+                ctx.run(synth.generate("plain_800k", n=n, seed=1), t, capacity=1 << 22)
+                assert ctx.last_stats["rescored"] == ctx.last_stats["candidates"] > 3_000_000
+            got = ctx.run(x, 0.95, capacity=1 << 22)
+            runs.append((got, ctx.last_stats["candidates"], ctx.last_stats["rescored"]))
+    for a, b in zip(*(r[0] for r in runs)):
+        assert np.array_equal(a, b)
+    assert runs[0][1:] == runs[1][1:]
