@@ -446,11 +446,15 @@ cuapss_status join_device(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, flo
     fa.nonneg = !neg_a;
     fb.nonneg = !neg_b;
     ST_TRY(join_fold(ctx, fa, self ? nullptr : &fb, t, perm, nrm2, probing_ns, &fr, &done));
+    cuapss_status result = CUAPSS_ENOMEM;
     if (done) {
       cudaEventRecord(ctx->ev[2], st);
       nvtx.next("cuapss_run:finalize");
-      const cuapss_status result = emit_pairs(ctx, fr.okey, fr.oidx, fr.osim, fr.npairs,
-                                              fr.rbitsI + fr.rbitsJ, fr.rbitsJ, out);
+      result = emit_pairs(ctx, fr.okey, fr.oidx, fr.osim, fr.npairs, fr.rbitsI + fr.rbitsJ,
+                          fr.rbitsJ, out);
+      if (result == CUAPSS_ENOMEM) ws.release_prefix("out:");  // the probing path's are smaller
+    }
+    if (result != CUAPSS_ENOMEM) {
       if (result != CUAPSS_OK && result != CUAPSS_EOVERFLOW) return result;
       cudaEventRecord(ctx->ev[3], st);
       CU_TRY(cudaStreamSynchronize(st));

@@ -418,11 +418,15 @@ cuapss_status batch_device(cuapss_ctx* ctx, const DevCsr& x, int k, const int64_
     DevCsr fx = x;
     fx.nonneg = !negative;
     ST_TRY(fold_batch(ctx, fx, k, inst_ptr, tq, perm, nrm * nrm, other_ns, &width, &fr, &done));
+    cuapss_status result = CUAPSS_ENOMEM;
     if (done) {
       cudaEventRecord(ctx->ev[2], st);
       nvtx.next("cuapss_batch_run:finalize");
-      const cuapss_status result = emit_pairs(ctx, fr.okey, fr.oidx, fr.osim, fr.npairs,
-                                              fr.rbitsI + fr.rbitsJ, fr.rbitsJ, out);
+      result = emit_pairs(ctx, fr.okey, fr.oidx, fr.osim, fr.npairs, fr.rbitsI + fr.rbitsJ,
+                          fr.rbitsJ, out);
+      if (result == CUAPSS_ENOMEM) ws.release_prefix("out:");  // the probing path's are smaller
+    }
+    if (result != CUAPSS_ENOMEM) {
       if (result != CUAPSS_OK && result != CUAPSS_EOVERFLOW) return result;
       cudaEventRecord(ctx->ev[3], st);
       CU_TRY(cudaStreamSynchronize(st));

@@ -95,19 +95,25 @@ class Workspace {
     }
     void* p = nullptr;
     size_t want = bytes + bytes / 8;  // headroom against regrowth
-    cudaError_t e = cudaMalloc(&p, want);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      e = cudaMalloc(&p, bytes);
+    if (!alloc(&p, want)) {
       want = bytes;
-      if (e != cudaSuccess) {
-        cudaGetLastError();
-        return CUAPSS_ENOMEM;
+      if (!alloc(&p, want)) {
+        // buffers that this call does not use make room
+        if (spare_.empty() || bytes_held(spare_) == 0) return CUAPSS_ENOMEM;
+        release_prefix(spare_);
+        if (!alloc(&p, want)) return CUAPSS_ENOMEM;
       }
     }
     bufs_[name] = {p, want};
     *out = p;
     return CUAPSS_OK;
+  }
+  // Buffers whose names start with `prefix` may be freed when memory runs out
+  // (empty: none). Returns the prefix set before.
+  std::string set_spare(const std::string& prefix) {
+    std::string before = spare_;
+    spare_ = prefix;
+    return before;
   }
   template <typename T>
   cuapss_status get(const std::string& name, size_t count, T** out) {
@@ -148,7 +154,13 @@ class Workspace {
     void* ptr;
     size_t size;
   };
+  static bool alloc(void** p, size_t bytes) {
+    if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+  }
   std::map<std::string, Buf> bufs_;
+  std::string spare_;
 };
 
 // NVTX ranges of a call's host-side stages (prepare, tiles, finalize), for

@@ -860,6 +860,10 @@ cuapss_status upload_units(std::vector<FoldTask>& tasks, Workspace& ws, cudaStre
   return CUAPSS_OK;
 }
 
+// Candidate lists above this ask for the free memory first and take at most
+// this share of it.
+constexpr double kAskBytes = 1e9, kListShare = 0.6;
+
 // Tiles and verification of all tasks into one unsorted pair list. *done =
 // false: the candidates do not fit what a folded join may take.
 template <bool MIXED>
@@ -894,6 +898,16 @@ cuapss_status run_tasks(cuapss_ctx* ctx, std::vector<FoldTask>& tasks, double nr
     for (FoldTask& k : tasks) {
       most = std::max(most, k.cap);
       room += k.cap;
+    }
+    if (room >= (int64_t)UINT32_MAX) return CUAPSS_OK;  // out_idx
+    // large lists leave the sorted result its room (at most 24 bytes a pair,
+    // of which there are half as many as the first list's slots)
+    const double bytes = 8.0 * (double)most + 16.0 * (double)room;
+    if (bytes > kAskBytes) {
+      size_t free_b = 0, total_b = 0;
+      CU_TRY(cudaMemGetInfo(&free_b, &total_b));
+      const double held = (double)(ws.held("fold:cand") + ws.bytes_held("out:"));
+      if (bytes > kListShare * ((double)free_b + held)) return CUAPSS_OK;
     }
     uint64_t* cand = nullptr;
     ST_TRY(ws.get("fold:cand", (size_t)most, &cand));  // the tasks run one after another
@@ -1375,6 +1389,26 @@ cuapss_status fold_batch_as(cuapss_ctx* ctx, const DevCsr& x, int k, const int64
 // to the probing path, which compacts it (batches) or refuses it.
 bool verifiable(const DevCsr& x) { return x.nnz < (int64_t)UINT32_MAX; }
 
+// Folded joins take more working memory than probing ones where the bound
+// prunes less (24 bytes a candidate). One that does not get it frees what it
+// took and leaves the call to the probing path, during which its buffers may
+// go.
+class FoldMemory {
+ public:
+  explicit FoldMemory(Workspace& ws) : ws_(ws) { ws.set_spare(""); }
+  ~FoldMemory() { ws_.set_spare("fold:"); }
+  cuapss_status or_probe(cuapss_status s, bool* done) {
+    if (s != CUAPSS_ENOMEM) return s;
+    *done = false;
+    ws_.release_prefix("fold:");
+    ws_.release_prefix("out:");
+    return CUAPSS_OK;
+  }
+
+ private:
+  Workspace& ws_;
+};
+
 }  // namespace
 
 cuapss_status join_fold(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float t,
@@ -1382,9 +1416,11 @@ cuapss_status join_fold(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float
                         bool* done) {
   *done = false;
   if (!verifiable(a) || (b && !verifiable(*b))) return CUAPSS_OK;
-  return ctx->opts.precision == CUAPSS_PREC_MIXED
-             ? join_fold_as<true>(ctx, a, b, t, perm, nrm2, other_ns, r, done)
-             : join_fold_as<false>(ctx, a, b, t, perm, nrm2, other_ns, r, done);
+  FoldMemory mem(ctx->ws);
+  return mem.or_probe(ctx->opts.precision == CUAPSS_PREC_MIXED
+                          ? join_fold_as<true>(ctx, a, b, t, perm, nrm2, other_ns, r, done)
+                          : join_fold_as<false>(ctx, a, b, t, perm, nrm2, other_ns, r, done),
+                      done);
 }
 
 cuapss_status fold_batch(cuapss_ctx* ctx, const DevCsr& x, int k, const int64_t* inst_ptr,
@@ -1392,13 +1428,17 @@ cuapss_status fold_batch(cuapss_ctx* ctx, const DevCsr& x, int k, const int64_t*
                          std::vector<int>* width, FoldResult* r, bool* done) {
   *done = false;
   if (!verifiable(x)) return CUAPSS_OK;
-  return ctx->opts.precision == CUAPSS_PREC_MIXED
-             ? fold_batch_as<true>(ctx, x, k, inst_ptr, t, perm, nrm2, other_ns, width, r, done)
-             : fold_batch_as<false>(ctx, x, k, inst_ptr, t, perm, nrm2, other_ns, width, r, done);
+  FoldMemory mem(ctx->ws);
+  return mem.or_probe(
+      ctx->opts.precision == CUAPSS_PREC_MIXED
+          ? fold_batch_as<true>(ctx, x, k, inst_ptr, t, perm, nrm2, other_ns, width, r, done)
+          : fold_batch_as<false>(ctx, x, k, inst_ptr, t, perm, nrm2, other_ns, width, r, done),
+      done);
 }
 
 cuapss_status fold_index(cuapss_ctx* ctx, bool mixed, const DevCsr& x, const int32_t* perm,
                          const FoldAlloc& alloc, FoldSide* s) {
+  FoldMemory mem(ctx->ws);
   return mixed ? fold_index_as<true>(ctx, x, perm, alloc, s)
                : fold_index_as<false>(ctx, x, perm, alloc, s);
 }
@@ -1410,9 +1450,11 @@ cuapss_status fold_query(cuapss_ctx* ctx, bool mixed, const std::vector<FoldSegm
   if (!verifiable(q)) return CUAPSS_OK;
   for (const FoldSegment& g : segs)
     if (!verifiable(g.side->x)) return CUAPSS_OK;
-  return mixed ? fold_query_as<true>(ctx, segs, q, t_row, t_min, perm, nrm2, other_ns, rows, r, done)
-               : fold_query_as<false>(ctx, segs, q, t_row, t_min, perm, nrm2, other_ns, rows, r,
-                                      done);
+  FoldMemory mem(ctx->ws);
+  return mem.or_probe(
+      mixed ? fold_query_as<true>(ctx, segs, q, t_row, t_min, perm, nrm2, other_ns, rows, r, done)
+            : fold_query_as<false>(ctx, segs, q, t_row, t_min, perm, nrm2, other_ns, rows, r, done),
+      done);
 }
 
 }  // namespace cuapss

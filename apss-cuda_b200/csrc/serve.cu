@@ -549,11 +549,15 @@ cuapss_status cuapss::index_query_rows(cuapss_ctx* ctx, const cuapss_index* idx,
     bool done = false;
     ST_TRY(fold_query(ctx, idx->mixed, fs, q, t_row, t_min, idx->perm, nrm2,
                       std::max(idx->tile_ns, stream_ns), rows, &fr, &done));
+    cuapss_status result = CUAPSS_ENOMEM;
     if (done) {
       cudaEventRecord(ctx->ev[2], st);
       nvtx.next("cuapss_index_query:finalize");
-      const cuapss_status result = emit_pairs(ctx, fr.okey, fr.oidx, fr.osim, fr.npairs,
-                                              fr.rbitsI + fr.rbitsJ, fr.rbitsJ, out);
+      result = emit_pairs(ctx, fr.okey, fr.oidx, fr.osim, fr.npairs, fr.rbitsI + fr.rbitsJ,
+                          fr.rbitsJ, out);
+      if (result == CUAPSS_ENOMEM) ws.release_prefix("out:");  // the probing path's are smaller
+    }
+    if (result != CUAPSS_ENOMEM) {
       if (result != CUAPSS_OK && result != CUAPSS_EOVERFLOW) return result;
       cudaEventRecord(ctx->ev[3], st);
       CU_TRY(cudaStreamSynchronize(st));

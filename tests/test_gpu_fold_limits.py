@@ -80,3 +80,42 @@ def test_route_does_not_depend_on_earlier_calls(precision, n, t):
     for a, b in zip(*(r[0] for r in runs)):
         assert np.array_equal(a, b)
     assert runs[0][1:] == runs[1][1:]
+
+
+def _footprint(precision, x, t, **opts):
+    """Device bytes a context holds after one self-join, and its result."""
+    import torch
+    with cuapss.Context(precision=precision, **opts) as ctx:
+        got = ctx.run(x, t, capacity=1 << 22)
+        held = torch.cuda.mem_get_info()[0]
+    return torch.cuda.mem_get_info()[0] - held, got
+
+
+@pytest.mark.parametrize("precision,t,head", [(cuapss.PREC_FP32, 0.5, 64),
+                                              (cuapss.PREC_MIXED, 0.4, 512)], ids=["fp32", "mixed"])
+def test_short_of_memory_probes(precision, t, head):
+    """With room for the probing path's working memory but not for the folded
+    join's candidates, the call probes instead of failing."""
+    import torch
+    x = synth.generate("plain_20k", n=120_000, seed=1)
+    small = synth.generate("plain_20k", n=100, seed=1)
+    _footprint(precision, small, 0.5)  # module loading
+    probing, want = _footprint(precision, x, t, head_width=head)
+    folding, same = _footprint(precision, x, t)
+    leave = probing + (160 << 20)
+    assert folding > leave + (160 << 20)
+    free = torch.cuda.mem_get_info()[0]
+    rest = torch.empty(free - leave, dtype=torch.uint8, device="cuda")
+    try:
+        with cuapss.Context(precision=precision) as ctx:
+            got = ctx.run(x, t, capacity=1 << 22)
+            probed = ctx.last_stats["rescored"] < ctx.last_stats["candidates"]
+            again = ctx.run(x, t, capacity=1 << 22)
+    finally:
+        del rest
+        torch.cuda.empty_cache()
+    assert probed
+    for k in range(2):
+        assert np.array_equal(got[k], want[k]) and np.array_equal(got[k], same[k])
+    assert np.max(np.abs(got[2] - same[2])) <= SIM_TOL
+    assert all(np.array_equal(a, b) for a, b in zip(got, again))
