@@ -405,6 +405,13 @@ cuapss_status batch_device(cuapss_ctx* ctx, const DevCsr& x, int k, const int64_
                       counts, &nrm, ws, "A", st, &negative));
   if (nrm * nrm >= 1.9) return CUAPSS_EINVAL;  // fixed-point tail needs ~unit norms
   ST_TRY(feature_perm(counts, d, x.n, ctx->opts.remap, perm, ws, st));
+  // 20-bit tail keys: what the tuner's narrowest head leaves no keys for is
+  // refused on either route
+  bool pairs = false;
+  for (int q = 0; q < k; ++q) pairs = pairs || inst_ptr[q + 1] - inst_ptr[q] >= 2;
+  if (pairs && ctx->opts.head_width == 0 &&
+      d - width_candidates(mixed, d).front() > (int64_t)(1u << 20) - 2)
+    return CUAPSS_EINVAL;
   // ---- the folded form, unless a head width or no remap fixes the probing
   const float t_min = *std::min_element(tq, tq + k);
   if (ctx->opts.head_width == 0 && ctx->opts.remap && x.n > 0 && t_min >= kFoldMinT) {

