@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <map>
+#include <set>
 #include <string>
 
 #include "cuapss.h"
@@ -99,8 +100,7 @@ class Workspace {
       want = bytes;
       if (!alloc(&p, want)) {
         // buffers that this call does not use make room
-        if (spare_.empty() || bytes_held(spare_) == 0) return CUAPSS_ENOMEM;
-        release_prefix(spare_);
+        for (const std::string& prefix : spare_) release_prefix(prefix);
         if (!alloc(&p, want)) return CUAPSS_ENOMEM;
       }
     }
@@ -108,12 +108,11 @@ class Workspace {
     *out = p;
     return CUAPSS_OK;
   }
-  // Buffers whose names start with `prefix` may be freed when memory runs out
-  // (empty: none). Returns the prefix set before.
-  std::string set_spare(const std::string& prefix) {
-    std::string before = spare_;
-    spare_ = prefix;
-    return before;
+  // Whether the buffers whose names start with `prefix` may be freed when
+  // memory runs out.
+  void set_spare(const std::string& prefix, bool spare) {
+    if (spare) spare_.insert(prefix);
+    else spare_.erase(prefix);
   }
   template <typename T>
   cuapss_status get(const std::string& name, size_t count, T** out) {
@@ -160,7 +159,7 @@ class Workspace {
     return false;
   }
   std::map<std::string, Buf> bufs_;
-  std::string spare_;
+  std::set<std::string> spare_;
 };
 
 // NVTX ranges of a call's host-side stages (prepare, tiles, finalize), for

@@ -1395,8 +1395,8 @@ bool verifiable(const DevCsr& x) { return x.nnz < (int64_t)UINT32_MAX; }
 // go.
 class FoldMemory {
  public:
-  explicit FoldMemory(Workspace& ws) : ws_(ws) { ws.set_spare(""); }
-  ~FoldMemory() { ws_.set_spare("fold:"); }
+  explicit FoldMemory(Workspace& ws) : ws_(ws) { ws.set_spare("fold:", false); }
+  ~FoldMemory() { ws_.set_spare("fold:", true); }
   cuapss_status or_probe(cuapss_status s, bool* done) {
     if (s != CUAPSS_ENOMEM) return s;
     *done = false;

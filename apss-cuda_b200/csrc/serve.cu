@@ -25,11 +25,13 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <chrono>
 #include <cmath>
 #include <cstring>
 #include <memory>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "ctx.cuh"
@@ -77,10 +79,10 @@ class DevHeap {
     size_t bytes = std::max<size_t>(count * sizeof(T), 256), step = 256;
     while (step * 16 <= bytes) step *= 2;
     bytes = (bytes + step - 1) / step * step;
-    const cudaError_t e = alloc_st_ ? cudaMallocAsync(&p, bytes, alloc_st_) : cudaMalloc(&p, bytes);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      return CUAPSS_ENOMEM;
+    const size_t exact = std::max<size_t>(count * sizeof(T), 256);
+    if (!take(&p, bytes)) {
+      bytes = exact;
+      if (!take(&p, bytes)) return CUAPSS_ENOMEM;
     }
     ptrs_.push_back(p);
     bytes_ += bytes;
@@ -98,15 +100,28 @@ class DevHeap {
   size_t bytes() const { return bytes_; }
 
  private:
+  bool take(void** p, size_t bytes) {
+    if ((alloc_st_ ? cudaMallocAsync(p, bytes, alloc_st_) : cudaMalloc(p, bytes)) == cudaSuccess)
+      return true;
+    cudaGetLastError();
+    return false;
+  }
   std::vector<void*> ptrs_;
   size_t bytes_ = 0;
   cudaStream_t alloc_st_ = nullptr;
   cudaStream_t free_st_ = nullptr;
 };
 
+// A segment's folded rows (fold.cuh), in memory of their own.
+struct FoldRows {
+  DevHeap heap;
+  FoldSide side;
+};
+
 // One immutable run of index rows and its J-side arrays.
 struct Segment {
   int64_t row0 = 0, n = 0, nnz = 0;
+  bool nonneg = false;
   int nb = 0;
   int p = 0;
   double nrm = 1.0;
@@ -125,8 +140,9 @@ struct Segment {
   int64_t* hptr = nullptr;
   uint2* rec = nullptr;
   int64_t ntail = 0;
-  // folded rows (fold.cuh), if the index has them
-  std::unique_ptr<FoldSide> fold;
+  // folded rows, if the index has them: queries hold them while they run, an
+  // index short of memory gives them up (guarded by the index's mu)
+  mutable std::shared_ptr<FoldRows> fold;
 };
 
 using SegList = std::vector<std::shared_ptr<const Segment>>;
@@ -154,7 +170,7 @@ struct cuapss_index {
   cudaStream_t free_st = nullptr;  // stream-ordered frees of dropped segments
   bool mixed = false;
   int p = 0;
-  bool fold = false;      // queries go through the folded rows where those prune
+  bool fold = false;      // queries go through the folded rows where those prune (under mu)
   double tile_ns = 0.0;   // modelled SM-nanoseconds of a probing tile
   int64_t d = 0;
   float norm_tol = 1e-4f;
@@ -175,11 +191,79 @@ namespace {
 constexpr double kPoolSegment = 8e9, kFoldRowBytes = 1400.0;
 constexpr size_t kKeepTemps = (size_t)2 << 30;
 
+// Hands the memory of the device's pool that nobody uses, except for `keep`
+// bytes, back to the device.
+void trim_pool(int device, size_t keep) {
+  cudaMemPool_t pool = nullptr;
+  uint64_t used = 0;
+  if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess)
+    cudaMemPoolTrimTo(pool, (size_t)used + keep);
+  cudaGetLastError();
+}
+
+// Gives up the folded rows of all segments, for good: the index's queries probe
+// from here on. Waits (up to 2 s) for the queries that read them and hands the
+// memory back to the device. False: there are none.
+bool drop_folds(cuapss_index* idx) {
+  std::vector<std::weak_ptr<FoldRows>> left;
+  {
+    std::lock_guard<std::mutex> lk(idx->mu);
+    if (!idx->fold) return false;
+    idx->fold = false;
+    for (const auto& g : idx->segs) {
+      left.push_back(g->fold);
+      g->fold.reset();
+    }
+  }
+  auto in_use = [&] {
+    for (const auto& w : left)
+      if (!w.expired()) return true;
+    return false;
+  };
+  for (int ms = 0; ms < 2000 && in_use(); ++ms)
+    std::this_thread::sleep_for(std::chrono::milliseconds(1));
+  cudaStreamSynchronize(idx->free_st);
+  trim_pool(idx->device, 0);
+  return true;
+}
+
+// Runs f, and once more without the index's folded rows if it ran out of
+// memory: they are 0.6 of the index's memory and not needed for its answers.
+template <typename F>
+cuapss_status or_unfolded(cuapss_ctx* ctx, cuapss_index* idx, F&& f) {
+  cuapss_status s = f();
+  if (s != CUAPSS_ENOMEM) return s;
+  cudaStreamSynchronize(ctx->stream);
+  if (!drop_folds(idx)) return s;
+  ctx->ws.release_prefix("fold:");
+  return f();
+}
+
+// Build temporaries stay in the context for its next build; other calls may
+// free them when memory runs out.
+class BuildTemps {
+ public:
+  explicit BuildTemps(cuapss_ctx* ctx) : ws_(ctx->ws) { spare(false); }
+  ~BuildTemps() { spare(true); }
+
+ private:
+  void spare(bool on) {
+    for (const char* prefix : {"seg:", "IX:", "AP:", "merge:"}) ws_.set_spare(prefix, on);
+  }
+  Workspace& ws_;
+};
+
 // Builds a segment from device CSR x (rows become index rows row0..).
-cuapss_status build_segment(cuapss_ctx* ctx, const cuapss_index* idx, const DevCsr& x,
+cuapss_status build_segment(cuapss_ctx* ctx, cuapss_index* idx, const DevCsr& x,
                             int64_t row0, double nrm, std::shared_ptr<Segment>* out) {
   cudaStream_t st = ctx->stream;
   auto seg = std::make_shared<Segment>();
+  // a build that fails halfway frees its memory after its last kernel
+  struct Finish {
+    cudaStream_t st;
+    ~Finish() { cudaStreamSynchronize(st); }
+  } finish{st};
   // Segments come from the device's pool, which appends and merges return to
   // without waiting for the device; a large one, made once, from cudaMalloc,
   // which maps its memory ten times faster than a growing pool (5M rows, 20
@@ -187,8 +271,10 @@ cuapss_status build_segment(cuapss_ctx* ctx, const cuapss_index* idx, const DevC
   // cudaMalloc, 85 from the pool).
   const double bytes = 16.0 * (double)x.nnz +
                        (double)x.n * ((idx->mixed ? 2.0 : 4.0) * idx->p + kFoldRowBytes);
-  if (bytes <= kPoolSegment) seg->heap.set_streams(st, idx->free_st);
+  const bool pooled = bytes <= kPoolSegment;
+  if (pooled) seg->heap.set_streams(st, idx->free_st);
   seg->row0 = row0;
+  seg->nonneg = x.nonneg;
   seg->n = x.n;
   seg->nnz = x.nnz;
   seg->nrm = nrm;
@@ -226,19 +312,26 @@ cuapss_status build_segment(cuapss_ctx* ctx, const cuapss_index* idx, const DevC
   }
   ST_TRY(H.copy(S.hptr, (size_t)kJSegs * nb + 1, &seg->hptr, st));
   ST_TRY(H.copy(S.bil_rec, (size_t)std::max<int64_t>(S.ntail, 1), &seg->rec, st));
-  if (idx->fold && x.n > 0) {
+  bool fold = false;
+  {
+    std::lock_guard<std::mutex> lk(idx->mu);
+    fold = idx->fold;
+  }
+  if (fold && x.n > 0) {
     DevCsr own = x;
     own.rp = seg->rp;
     own.col = seg->col;
     own.val = seg->val;
-    seg->fold = std::make_unique<FoldSide>();
-    auto alloc = [&H](const std::string&, size_t bytes, void** out) {
+    seg->fold = std::make_shared<FoldRows>();
+    DevHeap& FH = seg->fold->heap;
+    if (pooled) FH.set_streams(st, idx->free_st);
+    auto alloc = [&FH](const std::string&, size_t bytes, void** out) {
       uint8_t* p = nullptr;
-      const cuapss_status r = H.alloc(bytes, &p);
+      const cuapss_status r = FH.alloc(bytes, &p);
       *out = p;
       return r;
     };
-    ST_TRY(fold_index(ctx, idx->mixed, own, idx->perm, alloc, seg->fold.get()));
+    ST_TRY(fold_index(ctx, idx->mixed, own, idx->perm, alloc, &seg->fold->side));
   }
   CU_TRY(cudaStreamSynchronize(st));
   *out = std::move(seg);
@@ -291,20 +384,9 @@ cuapss_status concat_segments(cuapss_ctx* ctx, const Segment& a, const Segment& 
 
 constexpr size_t kMaxSegments = 24;
 
-// The device's pool keeps at most a sixteenth of the device's memory that
-// nobody uses (destroyed indexes return their segments there); the rest goes
-// back to the device.
+// What destroyed indexes leave in the device's pool for the next ones: at most
+// a sixteenth of the device's memory.
 constexpr uint64_t kPoolSlackShare = 16;
-void trim_pool(int device) {
-  cudaMemPool_t pool = nullptr;
-  uint64_t used = 0;
-  size_t free_b = 0, total_b = 0;
-  if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess &&
-      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
-      cudaMemGetInfo(&free_b, &total_b) == cudaSuccess)
-    cudaMemPoolTrimTo(pool, (size_t)used + total_b / kPoolSlackShare);
-  cudaGetLastError();
-}
 
 void query_times(cuapss_ctx* ctx, cuapss_stats* stats) {
   float ms = 0.f;
@@ -328,6 +410,7 @@ extern "C" cuapss_status cuapss_index_create(cuapss_ctx* ctx, const cuapss_csr* 
   if (!ctx || !x || !out) return CUAPSS_EINVAL;
   *out = nullptr;
   CU_TRY(cudaSetDevice(ctx->device));
+  BuildTemps temps(ctx);
   DevCsr a;
   ST_TRY(stage_csr(ctx, x, "IX", &a));
   auto idx = std::make_unique<cuapss_index>();
@@ -371,7 +454,8 @@ extern "C" cuapss_status cuapss_index_create(cuapss_ctx* ctx, const cuapss_csr* 
   if (a.d - p > (int64_t)(1u << 20) - 2) return CUAPSS_EINVAL;  // 20-bit tail features
   idx->p = p;
   std::shared_ptr<Segment> seg;
-  ST_TRY(build_segment(ctx, idx.get(), a, 0, nrm, &seg));
+  ST_TRY(or_unfolded(ctx, idx.get(),
+                     [&] { return build_segment(ctx, idx.get(), a, 0, nrm, &seg); }));
   idx->p = seg->p;
   // the temporaries of a small build stay in the context (its next index
   // needs them again: freeing and allocating them took 20 of 34 ms at 200,000
@@ -395,18 +479,21 @@ cuapss_status index_append_segment(cuapss_ctx* ctx, cuapss_index* idx, const cua
   if (x->n == 0) return CUAPSS_OK;
   CU_TRY(cudaSetDevice(ctx->device));
   std::lock_guard<std::mutex> alk(idx->append_mu);
+  BuildTemps temps(ctx);
   DevCsr a;
-  ST_TRY(stage_csr(ctx, x, "AP", &a));
   double nrm = 1.0;
-  ST_TRY(check_rows(ctx, idx, a, nullptr, &nrm, "AP"));
-  if (nrm >= 1.37) return CUAPSS_EINVAL;
   int64_t rows = 0;
   {
     std::lock_guard<std::mutex> lk(idx->mu);
     rows = idx->rows;
   }
   std::shared_ptr<Segment> seg;
-  ST_TRY(build_segment(ctx, idx, a, rows, nrm, &seg));
+  ST_TRY(or_unfolded(ctx, idx, [&]() -> cuapss_status {
+    ST_TRY(stage_csr(ctx, x, "AP", &a));
+    ST_TRY(check_rows(ctx, idx, a, nullptr, &nrm, "AP"));
+    if (nrm >= 1.37) return CUAPSS_EINVAL;
+    return build_segment(ctx, idx, a, rows, nrm, &seg);
+  }));
   // the build temporaries stay in ctx's grow-only workspace: freeing them
   // here would synchronize the device under running queries
   std::lock_guard<std::mutex> lk(idx->mu);
@@ -432,12 +519,15 @@ cuapss_status index_merge_step(cuapss_ctx* ctx, cuapss_index* idx, bool* merged)
     B = segs[segs.size() - 1];
     if (!(2 * B->n >= A->n || segs.size() > kMaxSegments)) return CUAPSS_OK;
   }
+  BuildTemps temps(ctx);
   DevCsr m;
-  ST_TRY(concat_segments(ctx, *A, *B, &m));
-  m.d = idx->d;
-  m.nonneg = A->fold && A->fold->x.nonneg && B->fold && B->fold->x.nonneg;
   std::shared_ptr<Segment> ab;
-  ST_TRY(build_segment(ctx, idx, m, A->row0, std::max(A->nrm, B->nrm), &ab));
+  ST_TRY(or_unfolded(ctx, idx, [&]() -> cuapss_status {
+    ST_TRY(concat_segments(ctx, *A, *B, &m));
+    m.d = idx->d;
+    m.nonneg = A->nonneg && B->nonneg;
+    return build_segment(ctx, idx, m, A->row0, std::max(A->nrm, B->nrm), &ab);
+  }));
   std::lock_guard<std::mutex> lk(idx->mu);
   // appends may have added segments behind B meanwhile; only merges remove
   // segments, so A and B are still adjacent
@@ -473,7 +563,8 @@ extern "C" cuapss_status cuapss_index_info(const cuapss_index* idx, int64_t* row
   if (head_width) *head_width = idx->p;
   if (device_bytes) {
     int64_t b = (int64_t)idx->heap.bytes();
-    for (auto& s : idx->segs) b += (int64_t)s->heap.bytes();
+    for (auto& s : idx->segs)
+      b += (int64_t)(s->heap.bytes() + (s->fold ? s->fold->heap.bytes() : 0));
     *device_bytes = b;
   }
   return CUAPSS_OK;
@@ -485,7 +576,8 @@ extern "C" cuapss_status cuapss_index_destroy(cuapss_index* idx) {
   cudaSetDevice(device);
   cudaDeviceSynchronize();
   delete idx;
-  trim_pool(device);
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) trim_pool(device, total_b / kPoolSlackShare);
   return CUAPSS_OK;
 }
 
@@ -512,14 +604,21 @@ cuapss_status cuapss::index_query_rows(cuapss_ctx* ctx, const cuapss_index* idx,
   cudaEventRecord(ctx->ev[0], st);
   StageRange nvtx("cuapss_index_query:prepare");
   SegList segs;
+  std::vector<std::shared_ptr<FoldRows>> folds;  // of the segments with rows
   int64_t rows = 0;
   double nrm_idx = 1.0;
+  bool fold = false;
   {
     auto* m = const_cast<cuapss_index*>(idx);
     std::lock_guard<std::mutex> lk(m->mu);
     segs = idx->segs;
     rows = idx->rows;
     nrm_idx = idx->nrm;
+    fold = idx->fold;
+    for (const auto& g : segs) {
+      if (g->n > 0) folds.push_back(g->fold);
+      fold = fold && (g->n == 0 || g->fold);
+    }
   }
   if (rows_seen) *rows_seen = rows;
   DevCsr q;
@@ -534,12 +633,12 @@ cuapss_status cuapss::index_query_rows(cuapss_ctx* ctx, const cuapss_index* idx,
     CU_TRY(cudaMemcpyAsync(t_row, t, sizeof(float) * q.n, cudaMemcpyHostToDevice, st));
   // ---- the folded rows, where they prune
   const float t_min = q.n > 0 ? *std::min_element(t, t + q.n) : 0.0f;
-  if (idx->fold && q.n > 0 && rows > 0 && t_min >= kFoldMinT && nrm_q * nrm_q < 1.9) {
+  if (fold && q.n > 0 && rows > 0 && t_min >= kFoldMinT && nrm_q * nrm_q < 1.9) {
     nvtx.next("cuapss_index_query:tiles");
     cudaEventRecord(ctx->ev[1], st);
     std::vector<FoldSegment> fs;
     for (const auto& g : segs)
-      if (g->fold) fs.push_back({g->fold.get(), g->row0});
+      if (g->n > 0) fs.push_back({&folds[fs.size()]->side, g->row0});
     // a probing tile also streams its J block's head and postings
     const int64_t nbq = ceil_div(q.n, kBlockRows);
     double block_bytes = (double)idx->p * kBlockRows * (idx->mixed ? 2.0 : 4.0);
@@ -575,6 +674,7 @@ cuapss_status cuapss::index_query_rows(cuapss_ctx* ctx, const cuapss_index* idx,
     }
     nvtx.next("cuapss_index_query:prepare");
   }
+  folds.clear();
   // ---- query side (I role)
   PrepOptions po;
   po.p = idx->p;

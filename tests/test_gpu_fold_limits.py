@@ -1,6 +1,10 @@
 """Folded joins at the edges of what they take: such a call gives what the
 probing path gives, whatever the size, the memory at hand and the calls made
 before it."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -149,3 +153,86 @@ def test_batch_feature_limit(precision, head):
                     for q in range(3)]
             assert len(want[0]) > 0
             _check(got, want)
+
+
+_SHORT_INDEX = """
+import sys
+import numpy as np, torch
+import cuapss
+from cuapss import synth
+from oracle import oracle
+
+MB = 1 << 20
+n, m = 300_000, 60_000
+x = synth.generate("serve_5m", n=n, seed=3)
+q = synth.generate("serve_5m", n=40, seed=3, row_offset=n - 20)
+more = synth.generate("serve_5m", n=m, seed=3, row_offset=n)
+t = np.full(q.n, 0.6, np.float32)
+want = oracle.join(q, x, 0.6)
+want2 = oracle.join(q, more, 0.6)
+free = lambda: torch.cuda.mem_get_info()[0]
+
+def check(got, want):
+    assert len(want[0]) >= 20
+    assert np.array_equal(got[0], want[0]) and np.array_equal(got[1], want[1])
+    assert np.max(np.abs(got[2] - want[2])) <= 1e-6
+
+small = x.rows(0, 3000)
+for opts in ({}, {"head_width": 512}):  # module loading
+    with cuapss.Context(precision=PRECISION, **opts) as c, cuapss.Index(c, small) as i:
+        i.query(q, t)
+with cuapss.Context(precision=PRECISION) as c, cuapss.Index(c, x) as i:
+    check(i.query(q, t), want)
+    i.query(q, 1.5 * t)
+    assert c.last_stats["rescored"] == c.last_stats["candidates"] > 0
+    full, p = i.info()["device_bytes"], i.info()["head_width"]
+
+if sys.argv[1] == "create":
+    # room for the probing layout, not for the folded rows beside it. The
+    # device pool's unused memory counts as room: two indexes that stay take
+    # what the first one left there
+    contexts = [cuapss.Context(precision=PRECISION, head_width=p) for _ in range(2)]
+    kept = [cuapss.Index(c, x) for c in contexts]
+    f0 = free()
+    with cuapss.Context(precision=PRECISION, head_width=p) as c, cuapss.Index(c, x) as i:
+        check(i.query(q, t), want)
+        used = f0 - free()
+        bare = i.info()["device_bytes"]
+    assert full > bare + 300 * MB, (full, bare)
+    leave = used - (f0 - free()) + 100 * MB
+    rest = torch.empty(free() - leave, dtype=torch.uint8, device="cuda")
+    with cuapss.Context(precision=PRECISION) as c, cuapss.Index(c, x) as i:
+        assert i.info()["device_bytes"] < bare * 1.02
+        check(i.query(q, t), want)
+else:
+    # an append that needs more than is left takes the folded rows' memory
+    with cuapss.Context(precision=PRECISION) as c, cuapss.Index(c, x) as i:
+        i.query(q, t)
+        got = []
+        before = i.info()["device_bytes"]
+        rest = torch.empty(free() - 30 * MB, dtype=torch.uint8, device="cuda")
+        i.append(more)
+        info = i.info()
+        assert info["rows"] == n + m
+        assert info["device_bytes"] < before
+        gi, gj, gs = i.query(q, t)
+        wi = np.concatenate([want[0], want2[0]])
+        wj = np.concatenate([want[1], want2[1] + n])
+        ws = np.concatenate([want[2], want2[2]])
+        o = np.lexsort((wj, wi))
+        check((gi, gj, gs), (wi[o], wj[o], ws[o]))
+print("fine")
+"""
+
+
+@pytest.mark.parametrize("what", ["create", "append"])
+@pytest.mark.parametrize("precision", [cuapss.PREC_MIXED, cuapss.PREC_FP32], ids=["mixed", "fp32"])
+def test_index_short_of_memory(precision, what):
+    """An index whose probing layout fits is built, and grown, without its
+    folded rows where they do not fit (in a process of its own, whose device
+    memory pool holds nothing yet)."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([root, os.path.join(root, "apss-cuda_b200")]))
+    r = subprocess.run([sys.executable, "-c", f"PRECISION = {precision}\n" + _SHORT_INDEX, what],
+                       env=env, cwd=root, capture_output=True, text=True, timeout=240)
+    assert r.returncode == 0 and "fine" in r.stdout, r.stdout + r.stderr
