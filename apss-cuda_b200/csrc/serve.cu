@@ -28,6 +28,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -52,8 +53,40 @@ inline unsigned grid_for(int64_t work, int threads) {
   return (unsigned)std::min<int64_t>(g, 148 * 16);
 }
 
+// Segment memory comes from a pool of the library's own on each device (the
+// device's default pool has other users): it keeps what dropped segments leave
+// for the next ones. Null if the device has none.
+cudaMemPool_t index_pool(int device) {
+  static std::mutex mu;
+  static std::map<int, cudaMemPool_t> pools;
+  std::lock_guard<std::mutex> lk(mu);
+  auto it = pools.find(device);
+  if (it != pools.end()) return it->second;
+  cudaMemPoolProps props{};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = device;
+  cudaMemPool_t pool = nullptr;
+  uint64_t keep = UINT64_MAX;
+  if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) pool = nullptr;
+  else cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  cudaGetLastError();
+  pools[device] = pool;
+  return pool;
+}
+
+// Hands the pool's memory that nobody uses, except for `keep` bytes, back to
+// the device.
+void trim_pool(int device, size_t keep) {
+  cudaMemPool_t pool = index_pool(device);
+  uint64_t used = 0;
+  if (pool && cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess)
+    cudaMemPoolTrimTo(pool, (size_t)used + keep);
+  cudaGetLastError();
+}
+
 // Exact-size device allocations owned by one object, stream-ordered: taken
-// with cudaMallocAsync on the building stream and returned with
+// from the pool on the building stream and returned with
 // cudaFreeAsync on the index's own stream, so that neither stalls the other
 // streams' work (cudaMalloc / cudaFree can synchronize the whole device).
 class DevHeap {
@@ -67,7 +100,9 @@ class DevHeap {
   }
   DevHeap(const DevHeap&) = delete;
   DevHeap& operator=(const DevHeap&) = delete;
-  void set_streams(cudaStream_t alloc_stream, cudaStream_t free_stream) {
+  void set_pool(cudaMemPool_t pool, cudaStream_t alloc_stream, cudaStream_t free_stream) {
+    if (!pool) return;
+    pool_ = pool;
     alloc_st_ = alloc_stream;
     free_st_ = free_stream;
   }
@@ -101,13 +136,15 @@ class DevHeap {
 
  private:
   bool take(void** p, size_t bytes) {
-    if ((alloc_st_ ? cudaMallocAsync(p, bytes, alloc_st_) : cudaMalloc(p, bytes)) == cudaSuccess)
+    if ((pool_ ? cudaMallocFromPoolAsync(p, bytes, pool_, alloc_st_) : cudaMalloc(p, bytes)) ==
+        cudaSuccess)
       return true;
     cudaGetLastError();
     return false;
   }
   std::vector<void*> ptrs_;
   size_t bytes_ = 0;
+  cudaMemPool_t pool_ = nullptr;
   cudaStream_t alloc_st_ = nullptr;
   cudaStream_t free_st_ = nullptr;
 };
@@ -191,17 +228,6 @@ namespace {
 constexpr double kPoolSegment = 8e9, kFoldRowBytes = 1400.0;
 constexpr size_t kKeepTemps = (size_t)2 << 30;
 
-// Hands the memory of the device's pool that nobody uses, except for `keep`
-// bytes, back to the device.
-void trim_pool(int device, size_t keep) {
-  cudaMemPool_t pool = nullptr;
-  uint64_t used = 0;
-  if (cudaDeviceGetDefaultMemPool(&pool, device) == cudaSuccess &&
-      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess)
-    cudaMemPoolTrimTo(pool, (size_t)used + keep);
-  cudaGetLastError();
-}
-
 // Gives up the folded rows of all segments, for good: the index's queries probe
 // from here on. Waits (up to 2 s) for the queries that read them and hands the
 // memory back to the device. False: there are none.
@@ -272,7 +298,7 @@ cuapss_status build_segment(cuapss_ctx* ctx, cuapss_index* idx, const DevCsr& x,
   const double bytes = 16.0 * (double)x.nnz +
                        (double)x.n * ((idx->mixed ? 2.0 : 4.0) * idx->p + kFoldRowBytes);
   const bool pooled = bytes <= kPoolSegment;
-  if (pooled) seg->heap.set_streams(st, idx->free_st);
+  if (pooled) seg->heap.set_pool(index_pool(idx->device), st, idx->free_st);
   seg->row0 = row0;
   seg->nonneg = x.nonneg;
   seg->n = x.n;
@@ -324,7 +350,7 @@ cuapss_status build_segment(cuapss_ctx* ctx, cuapss_index* idx, const DevCsr& x,
     own.val = seg->val;
     seg->fold = std::make_shared<FoldRows>();
     DevHeap& FH = seg->fold->heap;
-    if (pooled) FH.set_streams(st, idx->free_st);
+    if (pooled) FH.set_pool(index_pool(idx->device), st, idx->free_st);
     auto alloc = [&FH](const std::string&, size_t bytes, void** out) {
       uint8_t* p = nullptr;
       const cuapss_status r = FH.alloc(bytes, &p);
@@ -416,15 +442,6 @@ extern "C" cuapss_status cuapss_index_create(cuapss_ctx* ctx, const cuapss_csr* 
   auto idx = std::make_unique<cuapss_index>();
   idx->device = ctx->device;
   CU_TRY(cudaStreamCreateWithFlags(&idx->free_st, cudaStreamNonBlocking));
-  {
-    // keep freed segment memory in the device's pool for the next segments
-    cudaMemPool_t pool = nullptr;
-    if (cudaDeviceGetDefaultMemPool(&pool, ctx->device) == cudaSuccess) {
-      uint64_t keep = UINT64_MAX;
-      cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    }
-    cudaGetLastError();
-  }
   idx->mixed = ctx->opts.precision == CUAPSS_PREC_MIXED;
   idx->d = a.d;
   idx->norm_tol = ctx->opts.norm_tol;

@@ -155,6 +155,14 @@ def test_batch_feature_limit(precision, head):
             _check(got, want)
 
 
+def _in_process(program, *args):
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([root, os.path.join(root, "apss-cuda_b200")]))
+    r = subprocess.run([sys.executable, "-c", program, *args], env=env, cwd=root,
+                       capture_output=True, text=True, timeout=240)
+    assert r.returncode == 0 and "fine" in r.stdout, r.stdout + r.stderr
+
+
 _SHORT_INDEX = """
 import sys
 import numpy as np, torch
@@ -231,8 +239,38 @@ def test_index_short_of_memory(precision, what):
     """An index whose probing layout fits is built, and grown, without its
     folded rows where they do not fit (in a process of its own, whose device
     memory pool holds nothing yet)."""
-    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-    env = dict(os.environ, PYTHONPATH=os.pathsep.join([root, os.path.join(root, "apss-cuda_b200")]))
-    r = subprocess.run([sys.executable, "-c", f"PRECISION = {precision}\n" + _SHORT_INDEX, what],
-                       env=env, cwd=root, capture_output=True, text=True, timeout=240)
-    assert r.returncode == 0 and "fine" in r.stdout, r.stdout + r.stderr
+    _in_process(f"PRECISION = {precision}\n" + _SHORT_INDEX, what)
+
+
+_DEFAULT_POOL = """
+import ctypes
+import numpy as np, torch
+import cuapss
+from cuapss import synth
+
+torch.cuda.init()
+rt = ctypes.CDLL("libcudart.so.12")
+pool = ctypes.c_void_p()
+assert rt.cudaDeviceGetDefaultMemPool(ctypes.byref(pool), 0) == 0
+
+def attr(which):
+    v = ctypes.c_uint64()
+    assert rt.cudaMemPoolGetAttribute(pool, which, ctypes.byref(v)) == 0
+    return v.value
+
+before = attr(4), attr(5)  # release threshold, reserved bytes
+x = synth.generate("plain_20k", n=3000, seed=1)
+with cuapss.Context() as c:
+    for _ in range(2):
+        with cuapss.Index(c, x) as i:
+            i.append(x.rows(0, 500))
+            assert (attr(4), attr(5)) == before
+    assert (attr(4), attr(5)) == before
+print("fine")
+"""
+
+
+def test_default_pool_is_left_alone():
+    """An index takes nothing from the device's default memory pool and changes
+    none of its settings: the process's other users share it."""
+    _in_process(_DEFAULT_POOL)
