@@ -225,7 +225,7 @@ struct cuapss_index {
 namespace cuapss {
 namespace {
 
-constexpr double kPoolSegment = 8e9, kFoldRowBytes = 1400.0;
+constexpr double kGrowBytes = 8e9, kFoldRowBytes = 1400.0;
 constexpr size_t kKeepTemps = (size_t)2 << 30;
 
 // Gives up the folded rows of all segments, for good: the index's queries probe
@@ -290,15 +290,19 @@ cuapss_status build_segment(cuapss_ctx* ctx, cuapss_index* idx, const DevCsr& x,
     cudaStream_t st;
     ~Finish() { cudaStreamSynchronize(st); }
   } finish{st};
-  // Segments come from the device's pool, which appends and merges return to
-  // without waiting for the device; a large one, made once, from cudaMalloc,
-  // which maps its memory ten times faster than a growing pool (5M rows, 20
-  // GB: 0.3 against 1.8 s; 1M rows, 4 GB, built again and again: 135 ms from
-  // cudaMalloc, 85 from the pool).
-  const double bytes = 16.0 * (double)x.nnz +
+  cudaMemPool_t pool = index_pool(idx->device);
+  seg->heap.set_pool(pool, st, idx->free_st);
+  // A large segment grows the pool by all it takes (about) at once: the first
+  // index of 5M rows, 20 GB, 0.16-0.20 s instead of 0.81 (0.07 from cudaMalloc,
+  // whose cudaFree would wait for the whole device when a merge drops the
+  // segment); 1M rows, 4 GB, are better taken block by block (0.06 against 0.2).
+  const double bytes = 16.0 * (double)x.nnz + 28.0 * (double)x.n +
                        (double)x.n * ((idx->mixed ? 2.0 : 4.0) * idx->p + kFoldRowBytes);
-  const bool pooled = bytes <= kPoolSegment;
-  if (pooled) seg->heap.set_pool(index_pool(idx->device), st, idx->free_st);
+  if (pool && bytes > kGrowBytes) {
+    void* all = nullptr;
+    if (cudaMallocFromPoolAsync(&all, (size_t)bytes, pool, st) == cudaSuccess) cudaFreeAsync(all, st);
+    cudaGetLastError();
+  }
   seg->row0 = row0;
   seg->nonneg = x.nonneg;
   seg->n = x.n;
@@ -350,7 +354,7 @@ cuapss_status build_segment(cuapss_ctx* ctx, cuapss_index* idx, const DevCsr& x,
     own.val = seg->val;
     seg->fold = std::make_shared<FoldRows>();
     DevHeap& FH = seg->fold->heap;
-    if (pooled) FH.set_pool(index_pool(idx->device), st, idx->free_st);
+    FH.set_pool(pool, st, idx->free_st);
     auto alloc = [&FH](const std::string&, size_t bytes, void** out) {
       uint8_t* p = nullptr;
       const cuapss_status r = FH.alloc(bytes, &p);
