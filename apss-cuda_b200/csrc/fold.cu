@@ -22,8 +22,8 @@ constexpr int kClasses = kFoldClasses;
 // long rows, whose folded products spread the most.
 constexpr double kClassEdge[kClasses] = {0.125, 0.25, 0.375, 0.5,  0.625, 0.75,  0.8125, 0.875,
                                          0.92,  0.95, 0.97,  0.98, 0.988, 0.994, 0.998,  1.0};
-// Joins of fewer 128 x 128 tiles keep the caller's order and one width, whose
-// candidates are few or, past kSmallMaxCand, make the join fall back.
+// Joins of fewer 128 x 128 tiles keep the caller's order and one width,
+// unsampled, and take at most kSmallMaxCand candidates (small_limit).
 constexpr double kSampleMinTiles = 2048.0;
 constexpr int kSmallLevel = 3;
 constexpr int64_t kSmallMaxCand = 1 << 21;
@@ -36,6 +36,17 @@ constexpr int64_t kSmallMaxCand = 1 << 21;
 // and verify) + kCandEntryNs per entry of its longer row.
 constexpr double kTileNs = 55.0, kChunkNs = 328.0, kTileMinNs = 610.0, kStreamNs = 415.0;
 constexpr double kCandNs = 45.0, kCandEntryNs = 0.3;
+// An unsampled join gains on the probing path at least kSmallGainNs plus
+// kSmallGainEntryNs per non-zero of preprocessed rows (500 .. 8,000 rows of 20
+// .. 800 entries in both precisions, few candidates: 0.57-0.70 -> 0.20-0.22 ms
+// at 500 rows, 0.92 -> 0.23 at 8,000 of 40, 3.8 -> 0.5 of 400), an index query
+// kSmallGainNs. A candidate costs kSmallCandNs + kSmallCandEntryNs per entry
+// of a row (2,000 rows where all pairs pass: 67 SM-ns at 75 entries, 160 at
+// 200, 325 at 400, 655 at 800); where few pass, theirs are the longer rows
+// (120 entries in the mean: 102 SM-ns where 0.6 of the pairs pass, 222 where
+// 0.02 to 0.08 do).
+constexpr double kSmallGainNs = 350e3, kSmallGainEntryNs = 0.6;
+constexpr double kSmallCandNs = 10.0, kSmallCandEntryNs = 0.8;
 // Folding a row at a width, per entry and per column.
 constexpr double kFoldEntryNs = 0.35, kFoldColumnNs = 0.05;
 // FP32, 128 x 128 tiles.
@@ -584,6 +595,7 @@ struct FoldTask {
   int64_t tiles = 0;
   int4* d_units = nullptr;
   int64_t cap = 0;
+  int64_t limit = 0;  // > 0: with more candidates the probing path is faster
 };
 
 // Whether a level is sampled for a pair of classes: the widest ones only pay
@@ -834,6 +846,36 @@ void one_level(FoldTask& k) {
     for (int& l : row) l = kSmallLevel;  // K = 256 or 64
 }
 
+// The share of the pairs of unrelated rows of mean length len that a fold of K
+// columns lets pass at t: it depends on y = (1 - t) len / K alone, within a
+// factor of about three (rows of 20 .. 800 entries, d = 1,000 and 50,000, Zipf
+// 0.6 .. 1.1, both precisions, t = 0.3 .. 0.9: at y = 0.08 1e-4, 0.12 2e-3,
+// 0.18 0.02, 0.34 0.2, 0.5 0.5).
+double passing_share(double len, int K, double t) {
+  constexpr double y[] = {0.08, 0.12, 0.18, 0.34, 0.5, 0.8};
+  constexpr double s[] = {-4.0, -2.7, -1.7, -0.7, -0.3, 0.0};
+  const double x = (1.0 - t) * len / K;
+  int k = 1;
+  while (k < 5 && x > y[k]) ++k;
+  return std::pow(10.0, std::min(0.0, s[k - 1] + (x - y[k - 1]) * (s[k] - s[k - 1]) / (y[k] - y[k - 1])));
+}
+
+double mean_len(const DevCsr& x) { return (double)x.nnz / (double)std::max<int64_t>(x.n, 1); }
+
+// The candidates, among so many pairs of rows of mean length len, at which an
+// unsampled join stops being faster than the probing path by gain_ns. 0: it is
+// not worth a try, three times as many are expected (2,000 rows of 800 entries
+// at t = 0.5, mixed: 2.0 ms probing, 9.0 folded with every pair a candidate).
+int64_t small_limit(cuapss_ctx* ctx, double len, double pairs, double expected, double gain_ns) {
+  double n = 0.0;
+  for (int it = 0; it < 4; ++it) {
+    const double longer = 2.0 - std::min(1.0, n / std::max(pairs, 1.0));
+    n = std::min((double)kSmallMaxCand,
+                 gain_ns * ctx->sms / (kSmallCandNs + kSmallCandEntryNs * len * longer));
+  }
+  return expected > 3.0 * n ? 0 : (int64_t)n;
+}
+
 // The levels the sides of a task need, per class.
 void needed(const FoldTask& k, uint32_t (&needI)[kClasses], uint32_t (&needJ)[kClasses]) {
   for (int x = 0; x < kClasses; ++x)
@@ -938,7 +980,8 @@ cuapss_status run_tasks(cuapss_ctx* ctx, std::vector<FoldTask>& tasks, double nr
       ta.units = k.d_units;
       ta.nunits = (int)k.units.size();
       ta.cand = cand;
-      ta.cand_cap = k.cap;
+      ta.cand_cap = k.limit > 0 ? k.limit : k.cap;
+      ta.give_up_at = k.limit;
       ta.cand_count = ctl + 1 + 3 * i;
       ta.unit_counter = reinterpret_cast<int*>(ctl + 2 + 3 * i);
       ta.err = reinterpret_cast<int*>(ctl + 3 + 3 * i);
@@ -946,7 +989,7 @@ cuapss_status run_tasks(cuapss_ctx* ctx, std::vector<FoldTask>& tasks, double nr
       VerifyArgs va = common;
       va.cand = cand;
       va.ncand = ctl + 1 + 3 * i;
-      va.cap = k.cap;
+      va.cap = ta.cand_cap;
       va.work = reinterpret_cast<unsigned*>(ctl + 2 + 3 * i) + 1;
       va.permI = k.I->rowmap;
       va.permJ = k.J->rowmap;
@@ -966,7 +1009,7 @@ cuapss_status run_tasks(cuapss_ctx* ctx, std::vector<FoldTask>& tasks, double nr
     }
     CU_TRY(cudaMemcpyAsync(h.data(), ctl, 8 * (1 + 3 * nt), cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaStreamSynchronize(st));
-    bool over = false, past_own = false;
+    bool over = false, past_own = false, given_up = false;
     int64_t want = 0;
     for (size_t i = 0; i < nt; ++i) {
       const int herr = (int)h[3 + 3 * i];
@@ -976,11 +1019,12 @@ cuapss_status run_tasks(cuapss_ctx* ctx, std::vector<FoldTask>& tasks, double nr
       want += c;
       over = over || c > tasks[i].cap;
       past_own = past_own || c > own[i];
+      given_up = given_up || (tasks[i].limit > 0 && c > tasks[i].limit);
       tasks[i].cap = std::max(tasks[i].cap, c);
     }
     r->npairs = (int64_t)h[0];
     r->ncand = want;
-    if (past_own && want > max_cand) return CUAPSS_OK;
+    if (given_up || (past_own && want > max_cand)) return CUAPSS_OK;
     if (!over) {
       *done = true;
       return CUAPSS_OK;
@@ -1056,6 +1100,14 @@ cuapss_status join_fold_as(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, fl
   auto allocJ = [&ws](const std::string& name, size_t bytes, void** out) {
     return ws.get("fold:J:" + name, bytes, out);
   };
+  if (!sampled) {
+    const double n = (double)a.n, pairs = self ? 0.5 * n * (n - 1.0) : n * (double)b->n;
+    const double len = self ? mean_len(a) : 0.5 * (mean_len(a) + mean_len(*b));
+    const double entries = (double)(a.nnz + (self ? 0 : b->nnz));
+    k.limit = small_limit(ctx, len, pairs, pairs * passing_share(len, fold_k(MIXED, kSmallLevel), t),
+                          kSmallGainNs + kSmallGainEntryNs * entries);
+    if (k.limit == 0) return CUAPSS_OK;
+  }
   ST_TRY(order_side(SI, sampled, allocI, ws, "fold:I", st));
   if (!self) ST_TRY(order_side(SJ, sampled, allocJ, ws, "fold:J", st));
   if (sampled) {
@@ -1078,14 +1130,13 @@ cuapss_status join_fold_as(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, fl
   r->rbitsI = std::max(1, bits_for((uint64_t)SI.x.n));
   r->rbitsJ = std::max(1, bits_for((uint64_t)k.J->x.n));
   // twice what the sample promises: a run that does not fit is run again
-  const int64_t expect = std::max<int64_t>(sampled ? (int64_t)(2.0 * k.cands) : 0, 1 << 20);
-  k.cap = expect + SI.x.n + k.J->x.n;
+  const int64_t expect = std::max<int64_t>((int64_t)(2.0 * k.cands), 1 << 20);
+  k.cap = sampled ? expect + SI.x.n + k.J->x.n : k.limit;
   VerifyArgs va;
   va.t = t;
   va.rbits = r->rbitsJ;
-  // an unsampled join that the bound does not prune, or one whose sample
-  // misjudged it, is left to the probing path
-  return run_tasks<MIXED>(ctx, tasks, nrm2, va, sampled ? 4 * expect : kSmallMaxCand, r, done);
+  // a join whose sample misjudged it is left to the probing path
+  return run_tasks<MIXED>(ctx, tasks, nrm2, va, 4 * expect, r, done);
 }
 
 // ---- resident index -------------------------------------------------------
@@ -1134,9 +1185,9 @@ cuapss_status fold_index_as(cuapss_ctx* ctx, const DevCsr& x, const int32_t* per
 
 template <bool MIXED>
 cuapss_status fold_query_as(cuapss_ctx* ctx, const std::vector<FoldSegment>& segs,
-                            const DevCsr& q, const float* t_row, float t_min, const int32_t* perm,
-                            double nrm2, double other_ns, int64_t rows, FoldResult* r,
-                            bool* done) {
+                            const DevCsr& q, const float* t, const float* t_row,
+                            const int32_t* perm, double nrm2, double other_ns, int64_t rows,
+                            FoldResult* r, bool* done) {
   *done = false;
   Workspace& ws = ctx->ws;
   cudaStream_t st = ctx->stream;
@@ -1148,7 +1199,27 @@ cuapss_status fold_query_as(cuapss_ctx* ctx, const std::vector<FoldSegment>& seg
   };
   // several blocks of queries: those with much to compare together
   ST_TRY(order_side(Q, q.n > 2 * kBlockRows, alloc, ws, "fold:Q", st));
+  const float t_min = *std::min_element(t, t + q.n);
   std::vector<FoldTask> tasks(segs.size());
+  // unsampled segments: their candidates together have one limit
+  auto is_sampled = [&](const FoldSide& s) {
+    return s.sample != nullptr && (double)Q.nb * s.nb >= kSampleMinTiles;
+  };
+  double small_rows = 0.0, small_nnz = 0.0;
+  for (const FoldSegment& g : segs)
+    if (!is_sampled(*g.side)) {
+      small_rows += (double)g.side->x.n;
+      small_nnz += (double)g.side->x.nnz;
+    }
+  int64_t limit = 0;
+  if (small_rows > 0) {
+    const double len = 0.5 * (mean_len(q) + small_nnz / small_rows);
+    double expected = 0.0;
+    for (int64_t i = 0; i < q.n; ++i)
+      expected += small_rows * passing_share(len, fold_k(MIXED, kSmallLevel), t[i]);
+    limit = small_limit(ctx, len, small_rows * (double)q.n, expected, kSmallGainNs);
+    if (limit == 0) return CUAPSS_OK;
+  }
   uint32_t needQ[kClasses] = {};
   double cost = 0.0;
   int64_t max_cand = kSmallMaxCand;
@@ -1161,19 +1232,19 @@ cuapss_status fold_query_as(cuapss_ctx* ctx, const std::vector<FoldSegment>& seg
     k.t_min = t_min;
     k.j_offset = segs[i].row0;
     const double tiles128 = (double)Q.nb * k.J->nb;
-    const bool sampled = k.J->sample != nullptr && tiles128 >= kSampleMinTiles;
-    if (sampled) {
+    if (is_sampled(*k.J)) {
       ST_TRY(plan_levels<MIXED>(ctx, k, perm, nrm2));
       cost += k.cost;
     } else {
       one_level(k);
       cost += tiles128 * tile_cost<MIXED>(kSmallLevel) / kPair<MIXED>;
+      k.limit = std::max<int64_t>(1, (int64_t)((double)limit * (double)k.J->x.n / small_rows));
     }
     uint32_t needJ[kClasses] = {};
     needed(k, needQ, needJ);
     make_units<MIXED>(k, ctx->sms);
     r->tiles += k.tiles;
-    k.cap = std::max<int64_t>(sampled ? (int64_t)(2.0 * k.cands) : 0, 1 << 18);
+    k.cap = k.limit > 0 ? k.limit : std::max<int64_t>((int64_t)(2.0 * k.cands), 1 << 18);
     max_cand = std::max(max_cand, 4 * k.cap);
   }
   if (cost >= (double)r->tiles * other_ns) return CUAPSS_OK;
@@ -1444,7 +1515,7 @@ cuapss_status fold_index(cuapss_ctx* ctx, bool mixed, const DevCsr& x, const int
 }
 
 cuapss_status fold_query(cuapss_ctx* ctx, bool mixed, const std::vector<FoldSegment>& segs,
-                         const DevCsr& q, const float* t_row, float t_min, const int32_t* perm,
+                         const DevCsr& q, const float* t, const float* t_row, const int32_t* perm,
                          double nrm2, double other_ns, int64_t rows, FoldResult* r, bool* done) {
   *done = false;
   if (!verifiable(q)) return CUAPSS_OK;
@@ -1452,8 +1523,8 @@ cuapss_status fold_query(cuapss_ctx* ctx, bool mixed, const std::vector<FoldSegm
     if (!verifiable(g.side->x)) return CUAPSS_OK;
   FoldMemory mem(ctx->ws);
   return mem.or_probe(
-      mixed ? fold_query_as<true>(ctx, segs, q, t_row, t_min, perm, nrm2, other_ns, rows, r, done)
-            : fold_query_as<false>(ctx, segs, q, t_row, t_min, perm, nrm2, other_ns, rows, r, done),
+      mixed ? fold_query_as<true>(ctx, segs, q, t, t_row, perm, nrm2, other_ns, rows, r, done)
+            : fold_query_as<false>(ctx, segs, q, t, t_row, perm, nrm2, other_ns, rows, r, done),
       done);
 }
 

@@ -77,6 +77,9 @@ struct FoldTileArgs {
   uint64_t* cand = nullptr;      // {I row << 32 | J row}
   unsigned long long* cand_count = nullptr;
   int64_t cand_cap = 0;
+  // > 0: a join with more candidates than this is given up. Once the list says
+  // so, CTAs take no more units and warps list no more candidates.
+  int64_t give_up_at = 0;
   int* err = nullptr;
   uint32_t* class_count = nullptr;  // sampling: [level][I block][J block] pairs at or above t - eps
 };
@@ -189,11 +192,11 @@ struct FoldSegment {
   int64_t row0 = 0;
 };
 
-// The folded join of query rows (thresholds t_row, device, at least t_min)
+// The folded join of query rows (thresholds t on the host, t_row on the device)
 // with the segments of an index of `rows` rows. *done and other_ns as in
 // join_fold.
 cuapss_status fold_query(cuapss_ctx* ctx, bool mixed, const std::vector<FoldSegment>& segs,
-                         const DevCsr& q, const float* t_row, float t_min, const int32_t* perm,
+                         const DevCsr& q, const float* t, const float* t_row, const int32_t* perm,
                          double nrm2, double other_ns, int64_t rows, FoldResult* r, bool* done);
 
 // The folded form of a batch of self-joins: instance q is the rows

@@ -36,9 +36,18 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volati
   return live && got;
 }
 
+// The next unit of a CTA's producer (the two round trips to L2 overlap: one
+// after the other they took 9 of the 213 us of a one-row index query).
+__device__ __forceinline__ int next_unit(const FoldTileArgs& A) {
+  const int u = atomicAdd(A.unit_counter, 1);
+  if (A.give_up_at <= 0) return u;
+  const unsigned long long found = *const_cast<const volatile unsigned long long*>(A.cand_count);
+  return found > (unsigned long long)A.give_up_at ? A.nunits : u;
+}
+
 // Appends a warp's held candidates to the list: one reservation for up to
-// kHits of them.
-__device__ __forceinline__ void flush_hits(const FoldTileArgs& A, const uint64_t* hits, int n,
+// kHits of them. True: the join is given up.
+__device__ __forceinline__ bool flush_hits(const FoldTileArgs& A, const uint64_t* hits, int n,
                                            int lane) {
   __syncwarp();
   unsigned long long w = 0;
@@ -47,6 +56,7 @@ __device__ __forceinline__ void flush_hits(const FoldTileArgs& A, const uint64_t
   for (int k = lane; k < n; k += 32)
     if ((int64_t)w + k < A.cand_cap) A.cand[w + k] = hits[k];
   __syncwarp();
+  return A.give_up_at > 0 && (int64_t)w + n > A.give_up_at;
 }
 
 }  // namespace cuapss

@@ -667,7 +667,7 @@ cuapss_status cuapss::index_query_rows(cuapss_ctx* ctx, const cuapss_index* idx,
     const double stream_ns = block_bytes * ctx->sms / 6500.0 / (double)nbq;
     FoldResult fr;
     bool done = false;
-    ST_TRY(fold_query(ctx, idx->mixed, fs, q, t_row, t_min, idx->perm, nrm2,
+    ST_TRY(fold_query(ctx, idx->mixed, fs, q, t, t_row, idx->perm, nrm2,
                       std::max(idx->tile_ns, stream_ns), rows, &fr, &done));
     cuapss_status result = CUAPSS_ENOMEM;
     if (done) {

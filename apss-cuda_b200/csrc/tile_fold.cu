@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
           give_up(A.err, abort);
           break;
         }
-        const int u = atomicAdd(A.unit_counter, 1);
+        const int u = next_unit(A);
         uring[slot] = u;
         mbar_arrive(&ufull[slot]);
         if (u >= A.nunits) break;
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
     const int row = 32 * q4 + lane;      // J row within its block
     uint64_t* hits = reinterpret_cast<uint64_t*>(base + kOffHits) + (warp - kFirstEpi) * kHits;
     int held = 0;                        // candidates in hits, the same in every lane
-    bool live = true;
+    bool live = true, given_up = false;
     uint32_t tt = 0;
     for (uint32_t k = 0;; ++k) {
       const uint32_t slot = k % kRing, ur = k / kRing;
@@ -338,7 +338,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
         tc_fence_before();
         __syncwarp();
         if (live && lane == 0) mbar_arrive(&tempty[b]);
-        if (!work) continue;
+        if (!work || given_up) continue;
         // the groups' maxima first, and one vote: nearly all tiles end here
         float m[kEpiCols / 32];
         float top = largest(v[0]);
@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
           uint32_t n_hits = 0;
 #pragma unroll
           for (int g = 0; g < kEpiCols / 32; ++g) {
-            if (!__any_sync(0xffffffffu, m[g] >= thr)) continue;
+            if (given_up || !__any_sync(0xffffffffu, m[g] >= thr)) continue;
             uint32_t pass = passing(v[g], thr, (int)lim - 32 * g);
             if (COUNT) {
               n_hits += (uint32_t)__popc(pass);
@@ -365,8 +365,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_tiles_fold(const __grid_constan
               const unsigned some = __ballot_sync(0xffffffffu, pass != 0u);
               if (!some) break;
               if (held > kHits - 32) {
-                flush_hits(A, hits, held, lane);
+                given_up = flush_hits(A, hits, held, lane);
                 held = 0;
+                if (given_up) break;
               }
               if (pass) {
                 const int j = __ffs(pass) - 1;

@@ -92,7 +92,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_tiles_fold32(const __grid_const
           give_up(A.err, abort);
           break;
         }
-        const int u = atomicAdd(A.unit_counter, 1);
+        const int u = next_unit(A);
         uring[slot] = u;
         mbar_arrive(&ufull[slot]);
         if (u >= A.nunits) break;
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_tiles_fold32(const __grid_const
   const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
   uint64_t* hits = reinterpret_cast<uint64_t*>(smem + kOffHits) + warp * kHits;
   int held = 0;  // candidates in hits, the same in every lane
-  bool live = true;
+  bool live = true, given_up = false;
   uint32_t ii = 0, ij = 0;  // first I slice of the unit or tile, J slices used
   for (uint32_t k = 0;; ++k) {
     const uint32_t slot = k % kRing, ur = k / kRing;
@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_tiles_fold32(const __grid_const
       if (stream || last) ii += (uint32_t)nkc;
       // ---- pairs at or above t - eps
       uint64_t pass = 0ull;  // bit 8 i + j
-      if (live) {
+      if (live && !given_up) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const int c = (j < 4 ? 0 : 64) + 4 * tx + (j & 3);
@@ -229,8 +229,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_tiles_fold32(const __grid_const
             const unsigned some = __ballot_sync(0xffffffffu, pass != 0ull);
             if (!some) break;
             if (held > kHits - 32) {
-              flush_hits(A, hits, held, lane);
+              given_up = flush_hits(A, hits, held, lane);
               held = 0;
+              if (given_up) break;
             }
             if (pass) {
               const int b = __ffsll((long long)pass) - 1;

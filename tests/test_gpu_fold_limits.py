@@ -274,3 +274,57 @@ def test_default_pool_is_left_alone():
     """An index takes nothing from the device's default memory pool and changes
     none of its settings: the process's other users share it."""
     _in_process(_DEFAULT_POOL)
+
+
+def _rows(n, nnz, seed):
+    cfg = synth.CONFIGS["plain_800k"].replace(nnz_mean=nnz, nnz_sigma=0.7, nnz_max=8 * nnz, seed=seed)
+    return synth.generate(cfg, n=n)
+
+
+def _probed(ctx):
+    return ctx.last_stats["rescored"] < ctx.last_stats["candidates"]
+
+
+@pytest.mark.parametrize("precision,n,nnz,t,tried", [
+    (cuapss.PREC_MIXED, 2000, 800, 0.5, False), (cuapss.PREC_MIXED, 2000, 200, 0.3, False),
+    (cuapss.PREC_MIXED, 8000, 75, 0.4, True), (cuapss.PREC_FP32, 2000, 400, 0.6, False),
+    (cuapss.PREC_FP32, 8000, 120, 0.5, False), (cuapss.PREC_FP32, 8000, 75, 0.8, True)])
+def test_small_joins_that_folding_slows_down(precision, n, nnz, t, tried):
+    """Unsampled joins with more candidates than are worth computing probe:
+    expected (not tried) or found while the tiles run (given up)."""
+    x = _rows(n, nnz, 31)
+    rows = np.unique(np.random.default_rng(n).choice(n, size=100)).astype(np.int32)
+    wi, wj, ws = oracle.rows(x, t, rows)
+    with cuapss.Context(precision=precision) as ctx:
+        got = ctx.run(x, t, capacity=1 << 20)
+        assert _probed(ctx)
+        launches = ctx.last_stats["launches"]
+        again = ctx.run(x, t, capacity=1 << 20)
+        p = ctx.last_stats["head_width"]
+    assert all(np.array_equal(a, b) for a, b in zip(got, again))
+    sel = np.isin(got[0], rows) | np.isin(got[1], rows)
+    _check(tuple(g[sel] for g in got), (wi, wj, ws))
+    with cuapss.Context(precision=precision, head_width=p) as ctx:
+        same = ctx.run(x, t, capacity=1 << 20)
+        assert (launches > ctx.last_stats["launches"]) == tried
+    assert all(np.array_equal(a, b) for a, b in zip(got, same))
+
+
+@pytest.mark.parametrize("precision,t", [(cuapss.PREC_MIXED, 0.1), (cuapss.PREC_FP32, 0.3)],
+                         ids=["mixed", "fp32"])
+def test_small_queries_that_folding_slows_down(precision, t):
+    """The same for a query batch over an unsampled number of tiles."""
+    x = synth.generate("serve_5m", n=30_000, seed=32)
+    q = synth.generate("serve_5m", n=100, seed=32, row_offset=29_950)
+    sign = np.random.default_rng(33).choice(np.array([-1, 1], np.float32), size=x.nnz + q.nnz)
+    x = synth.Csr(x.rowptr, x.col, x.val * sign[:x.nnz], x.d)
+    q = synth.Csr(q.rowptr, q.col, q.val * sign[x.nnz:], q.d)
+    with cuapss.Context(precision=precision) as ctx, cuapss.Index(ctx, x) as idx:
+        got = idx.query(q, np.full(q.n, t, np.float32))
+        assert _probed(ctx)
+        again = idx.query(q, np.full(q.n, 0.9, np.float32))
+    want = oracle.join(q, x, t)
+    assert len(want[0]) > 100
+    _check(got, want)
+    keep = want[2] >= np.float64(np.float32(0.9))
+    _check(again, tuple(w[keep] for w in want))
