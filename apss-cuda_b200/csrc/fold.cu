@@ -36,17 +36,23 @@ constexpr int64_t kSmallMaxCand = 1 << 21;
 // and verify) + kCandEntryNs per entry of its longer row.
 constexpr double kTileNs = 55.0, kChunkNs = 328.0, kTileMinNs = 610.0, kStreamNs = 415.0;
 constexpr double kCandNs = 45.0, kCandEntryNs = 0.3;
-// An unsampled join gains on the probing path at least kSmallGainNs plus
-// kSmallGainEntryNs per non-zero of preprocessed rows (500 .. 8,000 rows of 20
-// .. 800 entries in both precisions, few candidates: 0.57-0.70 -> 0.20-0.22 ms
-// at 500 rows, 0.92 -> 0.23 at 8,000 of 40, 3.8 -> 0.5 of 400), an index query
-// kSmallGainNs. A candidate costs kSmallCandNs + kSmallCandEntryNs per entry
-// of a row (2,000 rows where all pairs pass: 67 SM-ns at 75 entries, 160 at
+// The probing path's launches and round trips, and its preprocessing per
+// non-zero, that a folded join does without (500 .. 8,000 rows of 20 .. 800
+// entries in both precisions, few candidates: 0.57-0.70 -> 0.20-0.22 ms at 500
+// rows, 0.92 -> 0.23 at 8,000 of 40, 3.8 -> 0.5 of 400; 76 ms of preprocessing
+// for 120M non-zeros). An index query prepares nothing but its own rows; a
+// batch, whose probing path plans no rare features, about 0.1 ns (400
+// instances, 16M non-zeros: 3.1-3.7 ms in all).
+constexpr double kProbeFixedNs = 350e3, kProbeEntryNs = 0.6, kBatchProbeEntryNs = 0.1;
+// Without length classes a candidate costs kMeanCandNs + kMeanCandEntryNs per
+// entry of a row (2,000 rows where all pairs pass: 67 SM-ns at 75 entries, 160 at
 // 200, 325 at 400, 655 at 800); where few pass, theirs are the longer rows
 // (120 entries in the mean: 102 SM-ns where 0.6 of the pairs pass, 222 where
 // 0.02 to 0.08 do).
-constexpr double kSmallGainNs = 350e3, kSmallGainEntryNs = 0.6;
-constexpr double kSmallCandNs = 10.0, kSmallCandEntryNs = 0.8;
+constexpr double kMeanCandNs = 10.0, kMeanCandEntryNs = 0.8;
+double cand_ns(double len, double share) {
+  return kMeanCandNs + kMeanCandEntryNs * len * (2.0 - std::min(1.0, share));
+}
 // Folding a row at a width, per entry and per column.
 constexpr double kFoldEntryNs = 0.35, kFoldColumnNs = 0.05;
 // FP32, 128 x 128 tiles.
@@ -119,18 +125,6 @@ __global__ void k_batch_places(const int64_t* __restrict__ tab, int k, int32_t* 
       t_place[S + r] = t;
     }
   }
-}
-
-// kBatchSample rows evenly spaced over all n (rows past n: none).
-__global__ void k_spread_rows(const int64_t* __restrict__ rp, int64_t n, int slots,
-                              int32_t* __restrict__ sample, unsigned long long* __restrict__ len_sum) {
-  unsigned long long len = 0;
-  for (int i = threadIdx.x; i < slots; i += blockDim.x) {
-    const int64_t r = n >= slots ? (int64_t)i * n / slots : i;
-    sample[i] = r < n ? (int32_t)r : -1;
-    if (r < n) len += (unsigned long long)(rp[r + 1] - rp[r]);
-  }
-  if (len) atomicAdd(len_sum, len);
 }
 
 // ---- rows too short for one another ---------------------------------------
@@ -606,6 +600,16 @@ bool sampled_level(int l, int a, int b) {
   return l < 7 || (l == 7 && sum >= 10) || (l == 8 && sum >= 16) || (l == 9 && lo >= 9);
 }
 
+// The levels worth sampling when a sampled tile may take at_most_ns (an FP32
+// tile of 1,024 columns takes 190 us beside another).
+template <bool MIXED>
+uint32_t sampled_levels(double at_most_ns) {
+  uint32_t all = (1u << kFoldLevels) - 1u;
+  for (int l = kSmallLevel + 1; l < kFoldLevels; ++l)
+    if ((MIXED ? 1.0 : 2.0) * tile_cost<MIXED>(l) > at_most_ns) all &= ~(1u << l);
+  return all;
+}
+
 // The width of every pair of classes, from the products of sampled rows, the
 // modelled cost of the join and its expected candidates. Levels the J side
 // does not hold (FoldSide::levels) are left out.
@@ -624,11 +628,9 @@ cuapss_status plan_levels(cuapss_ctx* ctx, FoldTask& k, const int32_t* perm, dou
   CU_TRY(cudaMemsetAsync(stats, 0, stat_bytes, st));
   uint32_t all = 0;
   for (uint32_t m : J.levels) all |= m;
-  // a sampled tile of a wide level may not take more than a tenth of a small
-  // join (an FP32 tile of 1,024 columns takes 190 us beside another)
-  const double whole = (k.self ? 0.5 : 1.0) * I.nb * J.nb / kPair<MIXED> * tile_cost<MIXED>(kSmallLevel);
-  for (int l = kSmallLevel + 1; l < kFoldLevels; ++l)
-    if ((MIXED ? 1.0 : 2.0) * tile_cost<MIXED>(l) > 0.1 * whole / ctx->sms) all &= ~(1u << l);
+  // no more than a tenth of a small join
+  all &= sampled_levels<MIXED>(0.1 / ctx->sms * (k.self ? 0.5 : 1.0) * I.nb * J.nb / kPair<MIXED> *
+                               tile_cost<MIXED>(kSmallLevel));
   auto temp = [&](const char* tag) {
     return [&ws, tag](const std::string& name, size_t bytes, void** out) {
       return ws.get(tag + name, bytes, out);
@@ -869,9 +871,8 @@ double mean_len(const DevCsr& x) { return (double)x.nnz / (double)std::max<int64
 int64_t small_limit(cuapss_ctx* ctx, double len, double pairs, double expected, double gain_ns) {
   double n = 0.0;
   for (int it = 0; it < 4; ++it) {
-    const double longer = 2.0 - std::min(1.0, n / std::max(pairs, 1.0));
     n = std::min((double)kSmallMaxCand,
-                 gain_ns * ctx->sms / (kSmallCandNs + kSmallCandEntryNs * len * longer));
+                 gain_ns * ctx->sms / cand_ns(len, n / std::max(pairs, 1.0)));
   }
   return expected > 3.0 * n ? 0 : (int64_t)n;
 }
@@ -981,7 +982,8 @@ cuapss_status run_tasks(cuapss_ctx* ctx, std::vector<FoldTask>& tasks, double nr
       ta.nunits = (int)k.units.size();
       ta.cand = cand;
       ta.cand_cap = k.limit > 0 ? k.limit : k.cap;
-      ta.give_up_at = k.limit;
+      // (what makes a sampled join probe, below)
+      ta.give_up_at = k.limit > 0 ? k.limit : nt == 1 ? std::max(max_cand, own[0]) : 0;
       ta.cand_count = ctl + 1 + 3 * i;
       ta.unit_counter = reinterpret_cast<int*>(ctl + 2 + 3 * i);
       ta.err = reinterpret_cast<int*>(ctl + 3 + 3 * i);
@@ -1100,12 +1102,13 @@ cuapss_status join_fold_as(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, fl
   auto allocJ = [&ws](const std::string& name, size_t bytes, void** out) {
     return ws.get("fold:J:" + name, bytes, out);
   };
+  const double probing_gain =
+      kProbeFixedNs + kProbeEntryNs * (double)(a.nnz + (self ? 0 : b->nnz));
   if (!sampled) {
     const double n = (double)a.n, pairs = self ? 0.5 * n * (n - 1.0) : n * (double)b->n;
     const double len = self ? mean_len(a) : 0.5 * (mean_len(a) + mean_len(*b));
-    const double entries = (double)(a.nnz + (self ? 0 : b->nnz));
     k.limit = small_limit(ctx, len, pairs, pairs * passing_share(len, fold_k(MIXED, kSmallLevel), t),
-                          kSmallGainNs + kSmallGainEntryNs * entries);
+                          probing_gain);
     if (k.limit == 0) return CUAPSS_OK;
   }
   ST_TRY(order_side(SI, sampled, allocI, ws, "fold:I", st));
@@ -1217,7 +1220,7 @@ cuapss_status fold_query_as(cuapss_ctx* ctx, const std::vector<FoldSegment>& seg
     double expected = 0.0;
     for (int64_t i = 0; i < q.n; ++i)
       expected += small_rows * passing_share(len, fold_k(MIXED, kSmallLevel), t[i]);
-    limit = small_limit(ctx, len, small_rows * (double)q.n, expected, kSmallGainNs);
+    limit = small_limit(ctx, len, small_rows * (double)q.n, expected, kProbeFixedNs);
     if (limit == 0) return CUAPSS_OK;
   }
   uint32_t needQ[kClasses] = {};
@@ -1259,10 +1262,14 @@ cuapss_status fold_query_as(cuapss_ctx* ctx, const std::vector<FoldSegment>& seg
 }
 
 // ---- batches ---------------------------------------------------------------
-// Thresholds the sample is compared at: an instance takes the shares of the
-// highest of them that does not exceed its own.
+// The batch's pairs in order of their threshold make kBatchT classes of equal
+// size. Up to kBatchRows rows of the instance in the middle of each class are
+// compared with one another at the class's lowest threshold: rows of different
+// instances never meet, and their products say nothing about those that do
+// (instances of 10 and of 300 entries a row in one batch).
 constexpr int kBatchT = kClasses;
-constexpr int kBatchI = 4;  // sampled I blocks
+constexpr int kBatchRows = 2 * kBlockRows;
+constexpr int kBatchBlocks = kBatchT * kBatchRows / kBlockRows;
 
 template <bool MIXED>
 cuapss_status fold_batch_as(cuapss_ctx* ctx, const DevCsr& x, int k, const int64_t* inst_ptr,
@@ -1284,105 +1291,128 @@ cuapss_status fold_batch_as(cuapss_ctx* ctx, const DevCsr& x, int k, const int64
   width->assign((size_t)k, 0);
   if (inst.empty()) return CUAPSS_OK;
   std::sort(inst.begin(), inst.end(), [&](int a, int b) { return t[a] != t[b] ? t[a] < t[b] : a < b; });
-  float grid[kBatchT];  // thresholds at equal shares of the pairs, the lowest first
+  float grid[kBatchT];  // each class's lowest threshold
+  int mid[kBatchT];     // and its sampled instance
   {
     double seen = 0.0;
-    int g = 0;
+    int g = 0, m = 0;
     for (int q : inst) {
       const double n = (double)(inst_ptr[q + 1] - inst_ptr[q]);
       while (g < kBatchT && seen >= all_pairs * g / kBatchT) grid[g++] = t[q];
       seen += n * n;
+      while (m < kBatchT && seen > all_pairs * (m + 0.5) / kBatchT) mid[m++] = q;
     }
     while (g < kBatchT) grid[g++] = t[inst.back()];
+    while (m < kBatchT) mid[m++] = inst.back();
   }
-  // ---- shares of sampled pairs at or above each of them, per level
-  const int64_t slots = kSampleSlots;
-  const size_t ncnt = (size_t)kFoldLevels * kBatchI * kBatchT;
-  unsigned long long* stats = nullptr;  // length sum, control words, counts
-  ST_TRY(ws.get("fold:stats", 2 + ncnt / 2, &stats));
-  CU_TRY(cudaMemsetAsync(stats, 0, 8 * 2 + 4 * ncnt, st));
+  // ---- shares of their pairs at or above those thresholds, per level
+  double tiles = 0.0;
+  for (int q : inst) {
+    const double nb = (double)ceil_div(inst_ptr[q + 1] - inst_ptr[q], kBlockRows);
+    tiles += 0.5 * nb * (nb + 1.0);
+  }
+  // what probing would take; a sampled tile gets no more than a tenth of it
+  const double probing_ns =
+      tiles * other_ns / ctx->sms + kProbeFixedNs + kBatchProbeEntryNs * (double)x.nnz;
+  const uint32_t all = sampled_levels<MIXED>(0.1 * probing_ns);
+  const int64_t slots = (int64_t)kBatchBlocks * kBlockRows;
+  std::vector<int32_t> rows((size_t)slots, -1);
+  std::vector<float> ht((size_t)slots);
+  for (int g = 0; g < kBatchT; ++g) {
+    const int64_t first = inst_ptr[mid[g]], n = inst_ptr[mid[g] + 1] - first;
+    for (int64_t i = 0; i < kBatchRows; ++i) {
+      // evenly spaced; classes that share an instance take different rows
+      const int64_t r = n >= kBatchRows ? ((i * kBatchT + g) * n) / (kBatchRows * kBatchT) : i;
+      if (r < n) rows[(size_t)(g * kBatchRows + i)] = (int32_t)(first + r);
+      ht[(size_t)(g * kBatchRows + i)] = grid[g];
+    }
+  }
+  const size_t ncnt = (size_t)kFoldLevels * kBatchBlocks * kBatchBlocks;
+  unsigned long long* stats = nullptr;  // control words, counts
+  ST_TRY(ws.get("fold:stats", 1 + ncnt / 2, &stats));
+  CU_TRY(cudaMemsetAsync(stats, 0, 8 + 4 * ncnt, st));
   FoldSide B;
   B.x = x;
   int32_t* sample = nullptr;
   float* sample_t = nullptr;
   ST_TRY(ws.get("fold:sI:sample", (size_t)slots, &sample));
   ST_TRY(ws.get("fold:sI:t", (size_t)slots, &sample_t));
-  k_spread_rows<<<1, 1024, 0, st>>>(x.rp, x.n, (int)slots, sample, stats);
-  LAUNCH_CHECK();
-  std::vector<float> ht((size_t)slots);
-  for (int64_t i = 0; i < slots; ++i) ht[(size_t)i] = grid[i / kBlockRows];
+  CU_TRY(cudaMemcpyAsync(sample, rows.data(), 4 * (size_t)slots, cudaMemcpyHostToDevice, st));
   CU_TRY(cudaMemcpyAsync(sample_t, ht.data(), 4 * (size_t)slots, cudaMemcpyHostToDevice, st));
   FoldOut so;
   uint8_t* samples = nullptr;
-  ST_TRY(ws.get("fold:sI:samples", kClasses * fold_offset_bytes(MIXED, kFoldLevels), &samples));
+  ST_TRY(ws.get("fold:sI:samples", kBatchBlocks * fold_offset_bytes(MIXED, kFoldLevels), &samples));
   for (int l = 0; l < kFoldLevels; ++l)
-    so.base[l] = samples + kClasses * fold_offset_bytes(MIXED, l);
-  const uint32_t every = (1u << kFoldLevels) - 1u;
-  ST_TRY(fold_places<MIXED>(B, sample, slots, {}, every, perm, so, ws, "fold:sI", st));
+    so.base[l] = samples + kBatchBlocks * fold_offset_bytes(MIXED, l);
+  ST_TRY(fold_places<MIXED>(B, sample, slots, {}, all, perm, so, ws, "fold:sI", st));
   FoldTileArgs ta;
   std::vector<int4> units;
   for (int l = kFoldLevels - 1; l >= 0; --l) {
+    if (!((all >> l) & 1u)) continue;
     ta.lev[l].I = ta.lev[l].J = so.base[l];
     ta.lev[l].nkc = fold_k(MIXED, l) / kChunk<MIXED>;
     ta.lev[l].eps = fold_eps(MIXED, l, nrm2, 1.0, x.nonneg, x.nonneg);
-    for (int a = 0; a < kBatchI; a += pair)
-      for (int b = 0; b < kBatchT; ++b) units.push_back(make_int4(a, b, b + 1, l));
+    for (int a = 0; a < kBatchBlocks; a += pair)
+      for (int b = a; b < a / 2 * 2 + 2; ++b) units.push_back(make_int4(a, b, b + 1, l));
   }
   int4* d_units = nullptr;
   ST_TRY(ws.get("fold:sunits", units.size(), &d_units));
   CU_TRY(cudaMemcpyAsync(d_units, units.data(), sizeof(int4) * units.size(),
                          cudaMemcpyHostToDevice, st));
-  ta.nI = kBatchI * kBlockRows;
-  ta.nJ = slots;
-  ta.nbI = kBatchI;
-  ta.nbJ = kBatchT;
+  ta.nI = ta.nJ = slots;
+  ta.nbI = ta.nbJ = kBatchBlocks;
+  ta.self = 1;
   ta.t_row = sample_t;
   ta.units = d_units;
   ta.nunits = (int)units.size();
-  ta.unit_counter = reinterpret_cast<int*>(stats + 1);
+  ta.unit_counter = reinterpret_cast<int*>(stats);
   ta.err = ta.unit_counter + 1;
-  ta.class_count = reinterpret_cast<uint32_t*>(stats + 2);
+  ta.class_count = reinterpret_cast<uint32_t*>(stats + 1);
   ST_TRY(launch_fold<MIXED>(ta, ctx->sms, st, true));
-  std::vector<unsigned long long> h(2 + ncnt / 2);
-  CU_TRY(cudaMemcpyAsync(h.data(), stats, 8 * h.size(), cudaMemcpyDeviceToHost, st));
+  static_assert(8 + 4 * kFoldLevels * kBatchBlocks * kBatchBlocks <= kPinnedBytes, "pinned scratch");
+  const auto* h = static_cast<const unsigned long long*>(ctx->pinned);
+  CU_TRY(cudaMemcpyAsync(ctx->pinned, stats, 8 + 4 * ncnt, cudaMemcpyDeviceToHost, st));
   CU_TRY(cudaStreamSynchronize(st));
-  const int herr = (int)(h[1] >> 32);
+  const int herr = (int)(h[0] >> 32);
   if (herr & kErrTimeout) return CUAPSS_ETIMEOUT;
   if (herr) return CUAPSS_ECUDA;
-  const uint32_t* hc = reinterpret_cast<const uint32_t*>(h.data() + 2);
-  const int64_t have = std::min<int64_t>(slots, x.n);  // sampled rows
-  const double mean_len = have > 0 ? (double)h[0] / (double)have : 0.0;
+  const uint32_t* hc = reinterpret_cast<const uint32_t*>(h + 1);
+  const double mean = mean_len(x);
   double share[kFoldLevels][kBatchT];
   for (int l = 0; l < kFoldLevels; ++l)
-    for (int b = 0; b < kBatchT; ++b) {
-      const double rowsJ = (double)std::max<int64_t>(0, std::min<int64_t>(kBlockRows, have - b * kBlockRows));
-      const double rowsI = (double)std::min<int64_t>(kBatchI * kBlockRows, have);
+    for (int g = 0; g < kBatchT; ++g) {
+      const double m = (double)std::min<int64_t>(kBatchRows, inst_ptr[mid[g] + 1] - inst_ptr[mid[g]]);
       double c = 0.0;
-      for (int a = 0; a < kBatchI; ++a) c += (double)hc[((size_t)l * kBatchI + a) * kBatchT + b];
-      if (b < kBatchI) c -= rowsJ;  // rows with themselves
-      share[l][b] = rowsJ > 0 ? std::max(c, 0.5) / (rowsI * rowsJ) : 1.0;
+      for (int a = 2 * g; a < 2 * g + 2; ++a)
+        for (int b = a; b < 2 * g + 2; ++b)
+          c += (double)hc[((size_t)l * kBatchBlocks + a) * kBatchBlocks + b];
+      share[l][g] = std::max(c, 0.5) / (0.5 * m * (m - 1.0));
     }
-  // a sample short of blocks knows nothing of the last thresholds: take the
-  // lowest one's shares, which are no smaller
-  for (int l = 0; l < kFoldLevels; ++l)
-    for (int b = 1; b < kBatchT; ++b)
-      if (have < (b + 1) * kBlockRows) share[l][b] = share[l][0];
   // ---- a level per instance; instances laid out level by level
   std::vector<int> lev((size_t)k, 0);
-  double cost = 0.0, cands = 0.0, tiles = 0.0;
+  double cost = 0.0, cands = 0.0;
   std::vector<int> by_level[kFoldLevels];
   int g = 0;
   for (int q : inst) {
     while (g + 1 < kBatchT && grid[g + 1] <= t[q]) ++g;
+    // the classes of the instance's threshold and their neighbours: several
+    // instances' shares
+    int g0 = g;
+    while (g0 > 0 && grid[g0 - 1] == grid[g]) --g0;
+    g0 = std::max(0, g0 - 1);
+    const int g1 = std::min(kBatchT - 1, g + 1);
     const int64_t n = inst_ptr[q + 1] - inst_ptr[q];
     const double nb = (double)ceil_div(n, kBlockRows);
     const double pairs = 0.5 * (double)n * (double)(n - 1);
     double best = 1e300, best_cand = 0.0;
     for (int l = 0; l < kFoldLevels; ++l) {
-      const double cand = share[l][g] * pairs;
+      if (!((all >> l) & 1u)) continue;
+      double sum = 0.0;
+      for (int c = g0; c <= g1; ++c) sum += share[l][c];
+      const double passing = sum / (g1 - g0 + 1), cand = passing * pairs;
       const double ns = std::ceil(nb / pair) * (nb + 1.0) * 0.5 * tile_cost<MIXED>(l) +
-                        cand * (kCandNs + kCandEntryNs * mean_len) +
-                        (double)n * (mean_len * kFoldEntryNs + fold_k(MIXED, l) * kFoldColumnNs);
+                        cand * (kCandNs + kCandEntryNs * mean) +
+                        (double)n * (mean * kFoldEntryNs + fold_k(MIXED, l) * kFoldColumnNs);
       if (ns < best) {
         best = ns;
         best_cand = cand;
@@ -1391,7 +1421,6 @@ cuapss_status fold_batch_as(cuapss_ctx* ctx, const DevCsr& x, int k, const int64
     }
     cost += best;
     cands += best_cand;
-    tiles += 0.5 * nb * (nb + 1.0);
     by_level[lev[(size_t)q]].push_back(q);
   }
   if (cost >= tiles * other_ns) return CUAPSS_OK;

@@ -328,3 +328,42 @@ def test_small_queries_that_folding_slows_down(precision, t):
     _check(got, want)
     keep = want[2] >= np.float64(np.float32(0.9))
     _check(again, tuple(w[keep] for w in want))
+
+
+def _batch(sizes, lens, d, seed):
+    """Instances of the given rows, of rows of the given mean length each."""
+    parts = []
+    for k, (n, nnz) in enumerate(zip(sizes, lens)):
+        cfg = synth.CONFIGS["batch_instance"].replace(d=d, nnz_mean=nnz, nnz_sigma=0.7,
+                                                      nnz_max=8 * nnz, seed=seed + k)
+        parts.append(synth.generate(cfg, n=n))
+    off = np.cumsum([0] + [p.nnz for p in parts])
+    rowptr = np.concatenate([[0]] + [p.rowptr[1:] + o for p, o in zip(parts, off)])
+    ptr = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    x = synth.Csr(rowptr.astype(np.int64), np.concatenate([p.col for p in parts]),
+                  np.concatenate([p.val for p in parts]), d)
+    return x, ptr, parts
+
+
+# sampled batches: few and many instances for the sixteen threshold classes,
+# instances of fewer rows than a sample takes, equal and different thresholds
+@pytest.mark.parametrize("precision", [cuapss.PREC_MIXED, cuapss.PREC_FP32], ids=["mixed", "fp32"])
+@pytest.mark.parametrize("sizes,lens,t", [
+    ([4000], [30], [0.6]), ([200, 257], [30, 30], [0.5, 0.9]),
+    ([40] * 30, [30] * 30, [0.4] * 30), ([700] * 20, [30] * 20, np.linspace(0.3, 0.9, 20)),
+    ([4000] * 20 + [4000] * 10, [10] * 20 + [300] * 10, [0.7] * 30),
+    ([4000] * 10 + [4000] * 20, [300] * 10 + [10] * 20, [0.7] * 30)],
+    ids=["one", "two", "tiny", "spread", "short-long", "long-short"])
+def test_sampled_batches(precision, sizes, lens, t):
+    x, ptr, parts = _batch(sizes, lens, 30_000, 41)
+    t = np.asarray(t, np.float32)
+    want = [oracle.apss(p, float(q)) for p, q in zip(parts, t)]
+    want = [np.concatenate([w[k] + (a if k < 2 else 0) for a, w in zip(ptr, want)])
+            for k in range(3)]
+    assert len(want[0]) > 0
+    with cuapss.Context(precision=precision) as ctx:
+        _check(ctx.batch_run(x, ptr, t, capacity=1 << 20), want)
+        # rows of different instances never meet: a sample across instances
+        # promised candidates that a fold of this batch does not have
+        if precision == cuapss.PREC_MIXED:
+            assert ctx.last_stats["rescored"] == ctx.last_stats["candidates"] > 0
