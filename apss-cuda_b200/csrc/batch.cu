@@ -40,8 +40,11 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kNumBuckets = CUAPSS_BATCH_BUCKETS;
 // SM-nanoseconds of a mixed probing tile of the batched workload (512
-// instances of 64 .. 20,000 rows, 30 non-zeros: 21 ms over 0.55M tiles).
-constexpr double kBatchTileNs = 5600.0;
+// instances of 64 .. 20,000 rows, 30 non-zeros: 21 ms over 0.55M tiles), taken
+// for rows of up to kBatchTileLen. Longer ones ask the joins' tile model (a
+// round trip): 400 instances of 64 .. 1,000 rows of 800 at t = 0.9 probed in 26
+// ms where folding takes 2.4.
+constexpr double kBatchTileNs = 5600.0, kBatchTileLen = 60.0;
 constexpr int64_t kTuneRows = 65536;  // rows of a bucket's tuning sample
 
 inline int bucket_of(int64_t n) { return n <= 1024 ? 0 : (n <= 8192 ? 1 : 2); }
@@ -417,8 +420,13 @@ cuapss_status batch_device(cuapss_ctx* ctx, const DevCsr& x, int k, const int64_
   if (ctx->opts.head_width == 0 && ctx->opts.remap && x.n > 0 && t_min >= kFoldMinT) {
     cudaEventRecord(ctx->ev[1], st);
     nvtx.next("cuapss_batch_run:tiles");
-    // a mixed probing tile at p = 512 (its tuned width): 8 head chunks
-    const double other_ns = mixed ? kBatchTileNs : plain_tile_ns(x.nnz, x.n);
+    double other_ns = mixed ? kBatchTileNs : plain_tile_ns(x.nnz, x.n);
+    if (mixed && (double)x.nnz > kBatchTileLen * (double)x.n) {
+      std::vector<int64_t> prefix;
+      ST_TRY(rank_count_prefix(counts, d, ctx->opts.remap, 8192, ws, st, &prefix));
+      const TilePlan plan = plan_tiles(ctx->opts.precision, x.n, d, x.nnz, prefix, {}, 0, 0);
+      other_ns = std::max(other_ns, plan.tile_ns);
+    }
     std::vector<int> width;
     FoldResult fr;
     bool done = false;

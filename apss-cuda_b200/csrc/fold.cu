@@ -982,8 +982,10 @@ cuapss_status run_tasks(cuapss_ctx* ctx, std::vector<FoldTask>& tasks, double nr
       ta.nunits = (int)k.units.size();
       ta.cand = cand;
       ta.cand_cap = k.limit > 0 ? k.limit : k.cap;
-      // (what makes a sampled join probe, below)
-      ta.give_up_at = k.limit > 0 ? k.limit : nt == 1 ? std::max(max_cand, own[0]) : 0;
+      // (what makes a sampled batch probe, below; for the other joins, whose
+      // samples see all their rows, the look at the count costs 8 of the 480 us
+      // of a 256-row index query)
+      ta.give_up_at = k.limit > 0 ? k.limit : k.J->t_place ? std::max(max_cand, own[i]) : 0;
       ta.cand_count = ctl + 1 + 3 * i;
       ta.unit_counter = reinterpret_cast<int*>(ctl + 2 + 3 * i);
       ta.err = reinterpret_cast<int*>(ctl + 3 + 3 * i);
@@ -1117,7 +1119,7 @@ cuapss_status join_fold_as(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, fl
     ST_TRY(plan_levels<MIXED>(ctx, k, perm, nrm2));
     double ns = 0.0;
     ST_TRY(other_ns(&ns));
-    if (k.cost >= tiles128 * ns) return CUAPSS_OK;
+    if (k.cost >= tiles128 * ns + probing_gain * ctx->sms) return CUAPSS_OK;
   } else {
     one_level(k);
   }
@@ -1250,7 +1252,7 @@ cuapss_status fold_query_as(cuapss_ctx* ctx, const std::vector<FoldSegment>& seg
     k.cap = k.limit > 0 ? k.limit : std::max<int64_t>((int64_t)(2.0 * k.cands), 1 << 18);
     max_cand = std::max(max_cand, 4 * k.cap);
   }
-  if (cost >= (double)r->tiles * other_ns) return CUAPSS_OK;
+  if (cost >= (double)r->tiles * other_ns + kProbeFixedNs * ctx->sms) return CUAPSS_OK;
   ST_TRY(build_levels<MIXED>(Q, needQ, perm, alloc, ws, "fold:Q", st));
   ST_TRY(upload_units(tasks, ws, st));
   r->rbitsI = std::max(1, bits_for((uint64_t)q.n));
@@ -1411,7 +1413,7 @@ cuapss_status fold_batch_as(cuapss_ctx* ctx, const DevCsr& x, int k, const int64
       for (int c = g0; c <= g1; ++c) sum += share[l][c];
       const double passing = sum / (g1 - g0 + 1), cand = passing * pairs;
       const double ns = std::ceil(nb / pair) * (nb + 1.0) * 0.5 * tile_cost<MIXED>(l) +
-                        cand * (kCandNs + kCandEntryNs * mean) +
+                        cand * cand_ns(mean, passing) +
                         (double)n * (mean * kFoldEntryNs + fold_k(MIXED, l) * kFoldColumnNs);
       if (ns < best) {
         best = ns;
@@ -1423,7 +1425,7 @@ cuapss_status fold_batch_as(cuapss_ctx* ctx, const DevCsr& x, int k, const int64
     cands += best_cand;
     by_level[lev[(size_t)q]].push_back(q);
   }
-  if (cost >= tiles * other_ns) return CUAPSS_OK;
+  if (cost >= probing_ns * ctx->sms) return CUAPSS_OK;
   std::vector<int64_t> tab;
   std::vector<FoldTask> tasks(1);
   FoldTask& task = tasks[0];

@@ -367,3 +367,19 @@ def test_sampled_batches(precision, sizes, lens, t):
         # promised candidates that a fold of this batch does not have
         if precision == cuapss.PREC_MIXED:
             assert ctx.last_stats["rescored"] == ctx.last_stats["candidates"] > 0
+
+
+@pytest.mark.parametrize("precision,n,nnz,t", [(cuapss.PREC_FP32, 500, 30, 0.6),
+                                               (cuapss.PREC_MIXED, 400, 200, 0.6),
+                                               (cuapss.PREC_MIXED, 400, 800, 0.9)])
+def test_probing_cost_counts_its_preparation(precision, n, nnz, t):
+    """Small batches, whose probing time is launches and preparation, and
+    batches of long rows, whose probing tiles are slow, fold."""
+    x, ptr, parts = _batch([n] * 12, [nnz] * 12, 30_000, 51)
+    t = np.full(12, t, np.float32)
+    want = [oracle.apss(p, float(q)) for p, q in zip(parts, t)]
+    want = [np.concatenate([w[k] + (a if k < 2 else 0) for a, w in zip(ptr, want)])
+            for k in range(3)]
+    with cuapss.Context(precision=precision) as ctx:
+        _check(ctx.batch_run(x, ptr, t, capacity=1 << 20), want)
+        assert ctx.last_stats["rescored"] == ctx.last_stats["candidates"] > 0
