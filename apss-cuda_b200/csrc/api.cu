@@ -339,6 +339,7 @@ cuapss_status emit_pairs(cuapss_ctx* ctx, uint64_t* key, uint32_t* idx, const fl
 cuapss_status join_device(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float t,
                           cuapss_pairs* out, cuapss_stats* stats, int shard, int nshards) {
   if (nshards < 1 || shard < 0 || shard >= nshards) return CUAPSS_EINVAL;
+  note_fold(ctx, false, nullptr);
   const bool self = (b == nullptr);
   const DevCsr& bb = self ? a : *b;
   if (!self && a.d != bb.d) return CUAPSS_EINVAL;
@@ -455,6 +456,7 @@ cuapss_status join_device(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, flo
       if (result == CUAPSS_ENOMEM) ws.release_prefix("out:");  // the probing path's are smaller
     }
     if (result != CUAPSS_ENOMEM) {
+      note_fold(ctx, mixed, &fr);
       if (result != CUAPSS_OK && result != CUAPSS_EOVERFLOW) return result;
       cudaEventRecord(ctx->ev[3], st);
       CU_TRY(cudaStreamSynchronize(st));
@@ -772,6 +774,13 @@ cuapss_status cuapss_create(cuapss_ctx** out, const cuapss_opts* opts) {
   }
   for (auto& e : c->ev) cudaEventCreate(&e);
   *out = c;
+  return CUAPSS_OK;
+}
+
+cuapss_status cuapss_fold_tiles(const cuapss_ctx* c, int32_t* columns, int64_t* tiles) {
+  if (!c || !columns || !tiles) return CUAPSS_EINVAL;
+  std::copy(c->fold_columns, c->fold_columns + CUAPSS_FOLD_WIDTHS, columns);
+  std::copy(c->fold_tiles, c->fold_tiles + CUAPSS_FOLD_WIDTHS, tiles);
   return CUAPSS_OK;
 }
 

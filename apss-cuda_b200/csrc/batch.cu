@@ -389,6 +389,7 @@ cuapss_status batch_device(cuapss_ctx* ctx, const DevCsr& x, int k, const int64_
     if (inst_ptr[q + 1] < inst_ptr[q]) return CUAPSS_EINVAL;
     if (!(tq[q] > 0.0f) || !std::isfinite(tq[q])) return CUAPSS_EINVAL;
   }
+  note_fold(ctx, false, nullptr);
   cudaStream_t st = ctx->stream;
   Workspace& ws = ctx->ws;
   const int64_t d = x.d;
@@ -442,6 +443,7 @@ cuapss_status batch_device(cuapss_ctx* ctx, const DevCsr& x, int k, const int64_
       if (result == CUAPSS_ENOMEM) ws.release_prefix("out:");  // the probing path's are smaller
     }
     if (result != CUAPSS_ENOMEM) {
+      note_fold(ctx, mixed, &fr);
       if (result != CUAPSS_OK && result != CUAPSS_EOVERFLOW) return result;
       cudaEventRecord(ctx->ev[3], st);
       CU_TRY(cudaStreamSynchronize(st));

@@ -22,6 +22,9 @@ struct cuapss_ctx {
   cudaEvent_t ev[6] = {};
   int64_t cand_cap = 0;
   void* pinned = nullptr;  // kPinnedBytes of host memory for small copies back
+  // folded 128 x 128 tiles of the last call by width (columns 0: none)
+  int32_t fold_columns[CUAPSS_FOLD_WIDTHS] = {};
+  int64_t fold_tiles[CUAPSS_FOLD_WIDTHS] = {};
   // batched joins: the captured tile launches (updated in place when the
   // next batch has the same launch topology) and the tuner's choices
   cudaGraph_t batch_graph = nullptr;

@@ -590,6 +590,14 @@ struct FoldTask {
   int4* d_units = nullptr;
   int64_t cap = 0;
   int64_t limit = 0;  // > 0: with more candidates the probing path is faster
+  int64_t level_tiles[kFoldLevels] = {};
+  // Blocks I, I + 1 (one: I alone) x [J0, J1) at a width.
+  void add_unit(int I, bool one, int J0, int J1, int code) {
+    units.push_back(make_int4(I, J0, J1, code));
+    int64_t n = (int64_t)(J1 - J0) * (one ? 1 : 2);
+    if (self && !one && J0 == I) --n;  // block I + 1 starts at itself
+    level_tiles[code & 0x7f] += n;
+  }
 };
 
 // Whether a level is sampled for a pair of classes: the widest ones only pay
@@ -834,7 +842,7 @@ void make_units(FoldTask& k, int sms) {
           const int len = std::min(e1 - f, step);
           // spread the starts of neighbouring units over the range
           const int turn = (int)(((int64_t)(k.units.size() % 16) * len) / 16);
-          k.units.push_back(make_int4(i, f, f + len, lv | turn << 8));
+          k.add_unit(i, pair == 1 || i + 1 >= I.nb, f, f + len, lv | turn << 8);
         }
       }
     }
@@ -1030,6 +1038,8 @@ cuapss_status run_tasks(cuapss_ctx* ctx, std::vector<FoldTask>& tasks, double nr
     r->ncand = want;
     if (given_up || (past_own && want > max_cand)) return CUAPSS_OK;
     if (!over) {
+      for (const FoldTask& k : tasks)
+        for (int l = 0; l < kFoldLevels; ++l) r->level_tiles[l] += k.level_tiles[l];
       *done = true;
       return CUAPSS_OK;
     }
@@ -1429,6 +1439,8 @@ cuapss_status fold_batch_as(cuapss_ctx* ctx, const DevCsr& x, int k, const int64
   std::vector<int64_t> tab;
   std::vector<FoldTask> tasks(1);
   FoldTask& task = tasks[0];
+  task.I = task.J = &B;
+  task.self = true;
   int64_t S = 0;
   size_t size[kFoldLevels] = {}, total = 0;
   std::vector<uint16_t> masks;
@@ -1444,7 +1456,7 @@ cuapss_status fold_batch_as(cuapss_ctx* ctx, const DevCsr& x, int k, const int64
       for (int i = b0; i < b1; i += pair) {
         const int single = MIXED && i + 1 >= b1 ? kFoldSingle : 0;
         for (int f = i; f < b1; f += most)
-          task.units.push_back(make_int4(i, f, std::min(b1, f + most), l | single));
+          task.add_unit(i, pair == 1 || single, f, std::min(b1, f + most), l | single);
       }
       task.tiles += (int64_t)(b1 - b0) * (b1 - b0 + 1) / 2;
       (*width)[(size_t)q] = fold_k(MIXED, l);
@@ -1474,8 +1486,6 @@ cuapss_status fold_batch_as(cuapss_ctx* ctx, const DevCsr& x, int k, const int64
   LAUNCH_CHECK();
   B.t_place = t_place;
   ST_TRY(fold_places<MIXED>(B, B.rowmap, S, masks, 0, perm, B.out, ws, "fold:B", st));
-  task.I = task.J = &B;
-  task.self = true;
   const int64_t expect = std::max<int64_t>((int64_t)(2.0 * cands), 1 << 20);
   task.cap = expect + x.n;
   ST_TRY(upload_units(tasks, ws, st));
@@ -1512,6 +1522,13 @@ class FoldMemory {
 };
 
 }  // namespace
+
+void note_fold(cuapss_ctx* ctx, bool mixed, const FoldResult* r) {
+  for (int l = 0; l < kFoldLevels; ++l) {
+    ctx->fold_columns[l] = r ? fold_k(mixed, l) : 0;
+    ctx->fold_tiles[l] = r ? r->level_tiles[l] : 0;
+  }
+}
 
 cuapss_status join_fold(cuapss_ctx* ctx, const DevCsr& a, const DevCsr* b, float t,
                         const int32_t* perm, double nrm2, const CostFn& other_ns, FoldResult* r,

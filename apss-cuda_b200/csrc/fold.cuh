@@ -38,7 +38,7 @@ constexpr float kFoldMinT = 0.05f;
 // 64-column chunks. FP32: FP32 folds multiplied on the CUDA cores, whose time
 // is proportional to K (65 ns per column and 128 x 128 tile), so the widths
 // are narrower and more candidates are computed.
-constexpr int kFoldLevels = 10;
+constexpr int kFoldLevels = CUAPSS_FOLD_WIDTHS;
 __host__ __device__ constexpr int fold_k(bool mixed, int level) {
   constexpr int k16[kFoldLevels] = {64, 128, 192, 256, 320, 384, 512, 768, 1024, 2048};
   constexpr int k32[kFoldLevels] = {16, 32, 48, 64, 96, 128, 192, 256, 512, 1024};
@@ -169,7 +169,11 @@ struct FoldResult {
   float* osim = nullptr;
   int rbitsI = 1, rbitsJ = 1;
   double max_band = 0.0;  // widest margin of the widths used
+  int64_t level_tiles[kFoldLevels] = {};  // 128 x 128 tiles multiplied at each width
 };
+
+// Records what the context's call did (null: it probed), for cuapss_fold_tiles.
+void note_fold(cuapss_ctx* ctx, bool mixed, const FoldResult* r);
 
 // Modelled cost, asked for only when it is needed.
 using CostFn = std::function<cuapss_status(double* ns)>;

@@ -618,6 +618,7 @@ cuapss_status cuapss::index_query_rows(cuapss_ctx* ctx, const cuapss_index* idx,
   if (qx->n > 0 && !t) return CUAPSS_EINVAL;
   for (int64_t i = 0; i < qx->n; ++i)
     if (!(t[i] > 0.0f) || !std::isfinite(t[i])) return CUAPSS_EINVAL;
+  note_fold(ctx, false, nullptr);
   CU_TRY(cudaSetDevice(ctx->device));
   cudaStream_t st = ctx->stream;
   Workspace& ws = ctx->ws;
@@ -678,6 +679,7 @@ cuapss_status cuapss::index_query_rows(cuapss_ctx* ctx, const cuapss_index* idx,
       if (result == CUAPSS_ENOMEM) ws.release_prefix("out:");  // the probing path's are smaller
     }
     if (result != CUAPSS_ENOMEM) {
+      note_fold(ctx, idx->mixed, &fr);
       if (result != CUAPSS_OK && result != CUAPSS_EOVERFLOW) return result;
       cudaEventRecord(ctx->ev[3], st);
       CU_TRY(cudaStreamSynchronize(st));

@@ -117,7 +117,7 @@ class RequestInfo(ctypes.Structure):
 EXPORTED = [
     "cuapss_default_opts", "cuapss_status_string", "cuapss_abi_version", "cuapss_create",
     "cuapss_destroy", "cuapss_run", "cuapss_join", "cuapss_build_index", "cuapss_feature_remap",
-    "cuapss_batch_run", "cuapss_selftest_bounded_wait", "cuapss_run_shard", "cuapss_shard_blocks", "cuapss_index_create", "cuapss_index_append", "cuapss_index_query",
+    "cuapss_batch_run", "cuapss_fold_tiles", "cuapss_selftest_bounded_wait", "cuapss_run_shard", "cuapss_shard_blocks", "cuapss_index_create", "cuapss_index_append", "cuapss_index_query",
     "cuapss_index_info", "cuapss_index_destroy", "cuapss_server_default_opts",
     "cuapss_server_create", "cuapss_server_submit_query", "cuapss_server_submit_append",
     "cuapss_server_wait", "cuapss_server_destroy",
@@ -155,6 +155,8 @@ def lib():
         L.cuapss_batch_run.argtypes = [_P, ctypes.POINTER(CsrDesc), ctypes.c_int32, _P, _P,
                                        ctypes.POINTER(PairsDesc), ctypes.POINTER(Stats), _P]
         L.cuapss_batch_run.restype = ctypes.c_int
+        L.cuapss_fold_tiles.argtypes = [_P, _P, _P]
+        L.cuapss_fold_tiles.restype = ctypes.c_int
         L.cuapss_selftest_bounded_wait.argtypes = [_P, ctypes.c_int32,
                                                    ctypes.POINTER(ctypes.c_int64)]
         L.cuapss_selftest_bounded_wait.restype = ctypes.c_int
@@ -288,6 +290,14 @@ class Context:
         """Self-join: (i, j, sim) numpy arrays, i < j, sorted by (i, j)."""
         d, keep = _desc(x)
         return self._pairs_call(lib().cuapss_run, (ctypes.byref(d), ctypes.c_float(t)), capacity)
+
+    def fold_tiles(self) -> dict:
+        """128 x 128 tiles of the last call by folded width (columns: tiles);
+        empty if the call probed."""
+        columns, tiles = np.zeros(10, np.int32), np.zeros(10, np.int64)
+        _check(lib().cuapss_fold_tiles(self._h, columns.ctypes.data, tiles.ctypes.data),
+               "cuapss_fold_tiles")
+        return {int(c): int(n) for c, n in zip(columns, tiles) if n}
 
     def selftest_bounded_wait(self, limit_us: int = 1000):
         """(status, device ns waited) of the bounded-wait self-check with a

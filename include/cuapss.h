@@ -309,6 +309,13 @@ cuapss_status cuapss_batch_run(cuapss_ctx* ctx, const cuapss_csr* x, int32_t k,
                                cuapss_pairs* out, cuapss_stats* stats,
                                int32_t* bucket_p);
 
+/* The folded tiles of the context's last join, batch or index query: tiles[k]
+ * 128 x 128 pair tiles were multiplied as rows folded into columns[k] columns
+ * (CUAPSS_FOLD_WIDTHS entries each; tiles that the call skipped are not
+ * counted). All zero: the call probed. No reference counterpart. */
+#define CUAPSS_FOLD_WIDTHS 10
+cuapss_status cuapss_fold_tiles(const cuapss_ctx* ctx, int32_t* columns, int64_t* tiles);
+
 /* Inverted index of the tail features, reference semantics: for every
  * feature f with f >= p (on the caller's ids, no remap), the rows that
  * contain f and their values, lists sorted by row. dim_ptr has d+1 entries

@@ -383,3 +383,37 @@ def test_probing_cost_counts_its_preparation(precision, n, nnz, t):
     with cuapss.Context(precision=precision) as ctx:
         _check(ctx.batch_run(x, ptr, t, capacity=1 << 20), want)
         assert ctx.last_stats["rescored"] == ctx.last_stats["candidates"] > 0
+
+
+# The routes themselves. cuapss_fold_tiles says which one a call took and what
+# it multiplied.
+@pytest.mark.parametrize("precision", [cuapss.PREC_MIXED, cuapss.PREC_FP32], ids=["mixed", "fp32"])
+def test_fold_tiles_reports_the_route(precision):
+    x = synth.generate("plain_800k", n=9000, seed=61)
+    widths = {64, 128, 192, 256, 320, 384, 512, 768, 1024, 2048}
+    if precision == cuapss.PREC_FP32:
+        widths = {16, 32, 48, 64, 96, 128, 192, 256, 512, 1024}
+    with cuapss.Context(precision=precision) as ctx:
+        assert ctx.fold_tiles() == {}
+        t = 0.95
+        ctx.run(x.rows(0, 1000), t)  # 8 blocks, one width
+        assert list(ctx.fold_tiles().values()) == [36]
+        ctx.join(x.rows(0, 130), x.rows(0, 1000), t)
+        assert list(ctx.fold_tiles().values()) == [16]
+        ctx.run(x, t)  # sampled widths; 71 blocks, none skipped in so small a join
+        tiles = ctx.fold_tiles()
+        assert set(tiles) <= widths and sum(tiles.values()) == 71 * 72 // 2
+        ctx.batch_run(x.rows(0, 1000), np.array([0, 300, 1000], np.int64),
+                      np.array([t, t], np.float32))
+        tiles = ctx.fold_tiles()
+        assert set(tiles) <= widths and sum(tiles.values()) == 6 + 21
+        with cuapss.Index(ctx, x.rows(0, 1000)) as idx:
+            idx.query(x.rows(0, 130), np.full(130, t, np.float32))
+            assert list(ctx.fold_tiles().values()) == [16]
+            idx.query(x.rows(0, 130), np.full(130, 0.04, np.float32))
+            assert ctx.fold_tiles() == {}
+        ctx.run(x.rows(0, 1000), 0.04)
+        assert ctx.fold_tiles() == {}
+    with cuapss.Context(precision=precision, head_width=64) as ctx:
+        ctx.run(x, t)
+        assert ctx.fold_tiles() == {}
