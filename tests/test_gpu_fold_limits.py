@@ -417,3 +417,62 @@ def test_fold_tiles_reports_the_route(precision):
     with cuapss.Context(precision=precision, head_width=64) as ctx:
         ctx.run(x, t)
         assert ctx.fold_tiles() == {}
+
+
+@pytest.mark.parametrize("precision", [cuapss.PREC_MIXED, cuapss.PREC_FP32], ids=["mixed", "fp32"])
+@pytest.mark.parametrize("opts,low", [({"head_width": 128}, 0.3), ({}, 0.03)],
+                         ids=["head_width", "low threshold"])
+def test_probing_index_query(precision, opts, low):
+    """The probing form of an index query, over appends and merges."""
+    x = synth.generate("plain_20k", n=5000, seed=62)
+    q = synth.generate("plain_20k", n=129, seed=62, row_offset=4950)
+    t = np.random.default_rng(63).uniform(0.4, 0.9, size=q.n).astype(np.float32)
+    t[77] = low
+    with cuapss.Context(precision=precision, **opts) as ctx:
+        with cuapss.Index(ctx, x.rows(0, 3000)) as idx:
+            idx.append(x.rows(3000, 3100))
+            idx.append(x.rows(3100, 5000))
+            got = idx.query(q, t, capacity=1 << 20)
+            assert ctx.fold_tiles() == {}
+    wi, wj, ws = oracle.join(q, x, low)
+    keep = ws >= t[wi].astype(np.float64)
+    assert keep.sum() > 100
+    _check(got, (wi[keep], wj[keep], ws[keep]))
+
+
+@pytest.mark.parametrize("precision", [cuapss.PREC_MIXED, cuapss.PREC_FP32], ids=["mixed", "fp32"])
+@pytest.mark.parametrize("opts,low", [({}, 0.04), ({"head_width": 64}, 0.3)],
+                         ids=["low threshold", "head_width"])
+def test_probing_batch(precision, opts, low):
+    """The probing form of a batch, all three size buckets."""
+    sizes = [1, 129, 1100, 0, 8300, 500]
+    x, ptr, parts = _batch([s for s in sizes if s], [30] * 5, 30_000, 64)
+    ptr = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    t = np.array([0.5, low, 0.6, 0.7, 0.8, 0.4], np.float32)
+    want = [oracle.apss(x.rows(a, b), float(q)) if b > a else [np.empty(0)] * 3
+            for a, b, q in zip(ptr, ptr[1:], t)]
+    want = [np.concatenate([w[k] + (a if k < 2 else 0) for a, w in zip(ptr, want)])
+            for k in range(3)]
+    with cuapss.Context(precision=precision, **opts) as ctx:
+        got = ctx.batch_run(x, ptr, t, capacity=1 << 20)
+        assert ctx.fold_tiles() == {} and (ctx.last_bucket_p > 0).all()
+    _check(got, want)
+
+
+@pytest.mark.parametrize("precision", [cuapss.PREC_MIXED, cuapss.PREC_FP32], ids=["mixed", "fp32"])
+def test_probing_join_with_the_modelled_explicit_pairs(precision):
+    """The plan of a default self-join, run by the probing path: the explicit
+    pairs are built and added."""
+    x = synth.generate("mixed_1m", n=40_000, seed=65)
+    plan = cuapss.plan_self_join(x, precision)
+    assert plan["explicit_pairs"] > 0
+    rows = np.unique(np.random.default_rng(66).choice(x.n, size=120)).astype(np.int32)
+    with cuapss.Context(precision=precision, rare_max_count=plan["rare_max_count"]) as ctx:
+        got = ctx.run(x, 0.6, capacity=1 << 20)
+        assert ctx.fold_tiles() == {}
+        assert ctx.last_stats["explicit_pairs"] > 0
+        assert ctx.last_stats["tail_products"] > 0
+    wi, wj, ws = oracle.rows(x, 0.6, rows)
+    sel = np.isin(got[0], rows) | np.isin(got[1], rows)
+    assert len(wi) > 0
+    _check(tuple(g[sel] for g in got), (wi, wj, ws))
