@@ -278,6 +278,11 @@ class Runner:
         self.out = None
 
 
+def call_stats(ctx):
+    """A call's statistics, with the tiles that it folded by width."""
+    return {**ctx.last_stats, "fold_tiles": ctx.fold_tiles()}
+
+
 def timed(runner, torch, stream, t, steps, warmup, clocks=None, shard=0, nshards=1):
     """warmup untimed steps, then `steps` steps between CUDA events on the
     library's stream; returns (ms per step, per-step stats)."""
@@ -292,7 +297,7 @@ def timed(runner, torch, stream, t, steps, warmup, clocks=None, shard=0, nshards
     e0.record(stream)
     for _ in range(steps):
         runner.step(t, shard, nshards)
-        stats.append(dict(runner.ctx.last_stats))
+        stats.append(call_stats(runner.ctx))
     e1.record(stream)
     torch.cuda.synchronize()
     if clocks:
@@ -306,23 +311,25 @@ def mean_stage(stats):
 
 
 def folded(s):
-    """Whether a call's join was folded: every candidate is then computed in
-    FP64 (the probing path rescores only its error band)."""
-    return s["candidates"] > 0 and s["rescored"] == s["candidates"]
+    """Whether a call's join was folded."""
+    return bool(s["fold_tiles"])
 
 
 def folded_roofline(tile_ms, s, prec_mixed, bf16_sus, src):
     """The folded join multiplies rows of 64 .. 2,048 (FP32: 16 .. 1,024)
     columns, chosen per pair of length classes from sampled rows, and skips
-    tiles whose rows are too short for one another; the call does not report
-    that mix, so no rate is claimed for it here."""
-    return {"bound": "tensor" if prec_mixed else "fp32 fma", "achieved": None,
-            "peak": bf16_sus if prec_mixed else None, "unit": "TFLOP/s", "frac": None,
+    tiles whose rows are too short for one another."""
+    flops = sum(2.0 * 128 * 128 * columns * tiles for columns, tiles in s["fold_tiles"].items())
+    achieved = flops / (tile_ms / 1e3) / 1e12
+    return {"bound": "tensor" if prec_mixed else "fp32 fma", "achieved": achieved,
+            "peak": bf16_sus if prec_mixed else None, "unit": "TFLOP/s",
+            "frac": achieved / bf16_sus if prec_mixed else None,
             "traffic": None, "peak_source": src,
             "kernel": "k_tiles_fold" if prec_mixed else "k_tiles_fold32",
             "kernel_ms": tile_ms, "tiles": s["tiles"], "candidates": s["candidates"],
-            "note": "kernel_ms covers folding, tiles and verification; the tile kernel's "
-                    "tensor-pipe share is in profiles/k_tiles_fold.md"}
+            "tiles_by_columns": s["fold_tiles"], "algorithmic_flops": flops,
+            "note": "products of the folded tiles actually multiplied over the whole of "
+                    "kernel_ms, which also covers sampling, folding and verification"}
 
 
 def tile_roofline(stats, p, pairs, n, world, prec_mixed, x, peaks_):
@@ -343,8 +350,7 @@ def tile_roofline(stats, p, pairs, n, world, prec_mixed, x, peaks_):
                 "frac": achieved / bf16_sus,
                 "traffic": traffic,
                 "traffic_source": "one-pass ncu capture of the full-size n = d = 1M launch, "
-                                  "scaled by tiles x p / 64 "
-                                  "(profiles/k_tiles_mma_mixed1m_n1m_dram.md)",
+                                  "scaled by tiles x p / 64",
                 "peak_source": f"{src} (sustained BF16: the kernel runs for about a second "
                                f"inside a multi-second step)",
                 "frac_of_burst": achieved / bf16,
@@ -667,7 +673,7 @@ def run_batch(args, rank, world, local):
         e0.record(stream)
         for _ in range(args.steps):
             npairs = step()
-            stats.append(dict(ctx.last_stats))
+            stats.append(call_stats(ctx))
         e1.record(stream)
         torch.cuda.synchronize()
     if dist:
