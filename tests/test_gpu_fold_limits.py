@@ -476,3 +476,44 @@ def test_probing_join_with_the_modelled_explicit_pairs(precision):
     sel = np.isin(got[0], rows) | np.isin(got[1], rows)
     assert len(wi) > 0
     _check(tuple(g[sel] for g in got), (wi, wj, ws))
+
+
+def _clusters(n, size, count, within, seed):
+    """n rows of 20 entries: `count` runs of `size` rows among the first
+    `within` that share their features (every pair of a run is at 0.9 or more),
+    the others unrelated."""
+    rng = np.random.default_rng(seed)
+    d = 200_000
+    col = np.sort(rng.integers(0, d // 20, size=(n, 20)) + np.arange(20) * (d // 20), axis=1)
+    for k in range(count):
+        a = k * (within // count)
+        col[a:a + size] = col[a]
+    val = 1.0 + 0.1 * rng.standard_normal((n, 20))
+    val = (val / np.linalg.norm(val, axis=1, keepdims=True)).astype(np.float32)
+    return synth.Csr(np.arange(n + 1, dtype=np.int64) * 20, col.astype(np.int32).ravel(),
+                     val.ravel(), d)
+
+
+# rows of one length keep their order, and a sample takes every 195th of the
+# first 125,000 of a join of 200,000 (every 234th of one instance of 60,000):
+# runs shorter than that hide their pairs from it
+@pytest.mark.parametrize("precision", [cuapss.PREC_MIXED, cuapss.PREC_FP32], ids=["mixed", "fp32"])
+@pytest.mark.parametrize("n,size,count,batch,folds", [
+    (200_000, 190, 170, False, True),   # 3.1M candidates: past the list, run again
+    (200_000, 190, 640, False, False),  # 11.5M: past four times the list, probes
+    (60_000, 230, 260, True, False)],   # 6.8M: the batch's tile kernel gives up
+    ids=["retry", "fallback", "batch"])
+def test_candidates_hidden_from_the_sample(precision, n, size, count, batch, folds):
+    x = _clusters(n, size, count, n if batch else n * 5 // 8, 71)
+    rows = np.unique(np.random.default_rng(72).choice(n, size=60)).astype(np.int32)
+    wi, wj, ws = oracle.rows(x, 0.9, rows)
+    with cuapss.Context(precision=precision) as ctx:
+        if batch:
+            got = ctx.batch_run(x, np.array([0, n], np.int64), np.array([0.9], np.float32),
+                                capacity=1 << 24)
+        else:
+            got = ctx.run(x, 0.9, capacity=1 << 25)
+        assert (ctx.fold_tiles() != {}) == folds
+    assert len(got[0]) > 0.9 * count * size * (size - 1) / 2
+    sel = np.isin(got[0], rows) | np.isin(got[1], rows)
+    _check(tuple(g[sel] for g in got), (wi, wj, ws))
