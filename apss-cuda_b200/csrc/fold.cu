@@ -619,6 +619,43 @@ uint32_t sampled_levels(double at_most_ns) {
   return all;
 }
 
+// The share of the pairs of unrelated rows of mean length len that a fold of K
+// columns lets pass at t: it depends on y = (1 - t) len / K alone, within a
+// factor of about three (rows of 20 .. 800 entries, d = 1,000 and 50,000, Zipf
+// 0.6 .. 1.1, both precisions, t = 0.3 .. 0.9: at y = 0.08 1e-4, 0.12 2e-3,
+// 0.18 0.02, 0.34 0.2, 0.5 0.5).
+double passing_share(double len, int K, double t) {
+  constexpr double y[] = {0.08, 0.12, 0.18, 0.34, 0.5, 0.8};
+  constexpr double s[] = {-4.0, -2.7, -1.7, -0.7, -0.3, 0.0};
+  const double x = (1.0 - t) * len / K;
+  int k = 1;
+  while (k < 5 && x > y[k]) ++k;
+  return std::pow(10.0, std::min(0.0, s[k - 1] + (x - y[k - 1]) * (s[k] - s[k - 1]) / (y[k] - y[k - 1])));
+}
+
+double mean_len(const DevCsr& x) { return (double)x.nnz / (double)std::max<int64_t>(x.n, 1); }
+
+// The wider levels whose sampled tiles take at most a tenth of the probing
+// path's fixed cost, where rows of kLongRows times the mean length have
+// candidates at the next narrower width that cost more than a tenth of its
+// tile. (Mixed joins of few thousand rows; 8,320 rows of 75 entries at t = 0.5
+// with nothing wider than 256 sampled: 1.47 ms, now 0.44; of 30 entries at
+// t = 0.7, where no wider one is useful: 0.35 with all sampled, 0.32. FP32
+// samples and small tiles cost more than the model says: 8,320 rows of 120 at t
+// = 0.8 2.05 -> 2.49 ms.)
+constexpr double kLongRows = 3.0;
+template <bool MIXED>
+uint32_t useful_levels(double len, double t) {
+  uint32_t use = sampled_levels<MIXED>(0.1 * kProbeFixedNs);
+  for (int l = kSmallLevel + 1; l < kFoldLevels; ++l) {
+    const double share = passing_share(kLongRows * len, fold_k(MIXED, l - 1), t);
+    if (share * kPair<MIXED> * kBlockRows * kBlockRows * cand_ns(len, share) <
+        0.1 * tile_cost<MIXED>(l - 1))
+      use &= ~(1u << l);
+  }
+  return use;
+}
+
 // The width of every pair of classes, from the products of sampled rows, the
 // modelled cost of the join and its expected candidates. Levels the J side
 // does not hold (FoldSide::levels) are left out.
@@ -638,8 +675,10 @@ cuapss_status plan_levels(cuapss_ctx* ctx, FoldTask& k, const int32_t* perm, dou
   uint32_t all = 0;
   for (uint32_t m : J.levels) all |= m;
   // no more than a tenth of a small join
-  all &= sampled_levels<MIXED>(0.1 / ctx->sms * (k.self ? 0.5 : 1.0) * I.nb * J.nb / kPair<MIXED> *
-                               tile_cost<MIXED>(kSmallLevel));
+  const double tiles_ns = (k.self ? 0.5 : 1.0) * I.nb * J.nb / kPair<MIXED> / ctx->sms *
+                          tile_cost<MIXED>(kSmallLevel);
+  all &= sampled_levels<MIXED>(0.1 * tiles_ns) |
+         (MIXED ? useful_levels<MIXED>(std::max(mean_len(I.x), mean_len(J.x)), k.t * k.t_min) : 0u);
   auto temp = [&](const char* tag) {
     return [&ws, tag](const std::string& name, size_t bytes, void** out) {
       return ws.get(tag + name, bytes, out);
@@ -862,22 +901,6 @@ void one_level(FoldTask& k) {
   for (auto& row : k.level)
     for (int& l : row) l = kSmallLevel;  // K = 256 or 64
 }
-
-// The share of the pairs of unrelated rows of mean length len that a fold of K
-// columns lets pass at t: it depends on y = (1 - t) len / K alone, within a
-// factor of about three (rows of 20 .. 800 entries, d = 1,000 and 50,000, Zipf
-// 0.6 .. 1.1, both precisions, t = 0.3 .. 0.9: at y = 0.08 1e-4, 0.12 2e-3,
-// 0.18 0.02, 0.34 0.2, 0.5 0.5).
-double passing_share(double len, int K, double t) {
-  constexpr double y[] = {0.08, 0.12, 0.18, 0.34, 0.5, 0.8};
-  constexpr double s[] = {-4.0, -2.7, -1.7, -0.7, -0.3, 0.0};
-  const double x = (1.0 - t) * len / K;
-  int k = 1;
-  while (k < 5 && x > y[k]) ++k;
-  return std::pow(10.0, std::min(0.0, s[k - 1] + (x - y[k - 1]) * (s[k] - s[k - 1]) / (y[k] - y[k - 1])));
-}
-
-double mean_len(const DevCsr& x) { return (double)x.nnz / (double)std::max<int64_t>(x.n, 1); }
 
 // The candidates, among so many pairs of rows of mean length len, at which an
 // unsampled join stops being faster than the probing path by gain_ns. 0: it is

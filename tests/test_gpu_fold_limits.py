@@ -517,3 +517,14 @@ def test_candidates_hidden_from_the_sample(precision, n, size, count, batch, fol
     assert len(got[0]) > 0.9 * count * size * (size - 1) / 2
     sel = np.isin(got[0], rows) | np.isin(got[1], rows)
     _check(tuple(g[sel] for g in got), (wi, wj, ws))
+
+
+@pytest.mark.parametrize("cfg,n,t", [("plain_800k", 8320, 0.5), ("plain_800k", 8320, 0.6)])
+def test_small_sampled_joins_take_wide_rows(cfg, n, t):
+    """Just past the unsampled joins, long rows still get the widths that they
+    need (mixed precision: at 256 columns half of the time went to candidates)."""
+    x = synth.generate(cfg, n=n, seed=71)
+    with cuapss.Context(precision=cuapss.PREC_MIXED) as ctx:
+        got = ctx.run(x, t, capacity=1 << 16)
+        assert max(ctx.fold_tiles()) > 256
+    _check(got, oracle.apss(x, t))
