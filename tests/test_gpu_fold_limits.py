@@ -528,3 +528,59 @@ def test_small_sampled_joins_take_wide_rows(cfg, n, t):
         got = ctx.run(x, t, capacity=1 << 16)
         assert max(ctx.fold_tiles()) > 256
     _check(got, oracle.apss(x, t))
+
+
+# Forms of folded calls whose inputs elsewhere may probe: the route is checked.
+def _signed(x, seed):
+    sign = np.random.default_rng(seed).choice(np.array([-1, 1], np.float32), size=x.nnz)
+    return synth.Csr(x.rowptr, x.col, x.val * sign, x.d)
+
+
+@pytest.mark.parametrize("precision", [cuapss.PREC_MIXED, cuapss.PREC_FP32], ids=["mixed", "fp32"])
+@pytest.mark.parametrize("cfg,n,t,sign", [
+    ("batch_instance", 18_815, 0.7, False), ("batch_instance", 18_817, 0.7, False),
+    ("batch_instance", 37_760, 0.8, False), ("batch_instance", 37_761, 0.8, False),
+    ("plain_20k", 9000, 0.6, True)])
+def test_folded_self_joins(precision, cfg, n, t, sign):
+    """Folded rows by 32, 16 and 8 threads each, and signed ones, against the
+    probing path (a fixed head width)."""
+    x = synth.generate(cfg, n=n, seed=n)
+    if sign:
+        x = _signed(x, 5)
+    with cuapss.Context(precision=precision, head_width=64) as ctx:
+        want = ctx.run(x, t, capacity=1 << 16)
+        assert ctx.fold_tiles() == {} and len(want[0]) > 0
+    with cuapss.Context(precision=precision) as ctx:
+        got = ctx.run(x, t, capacity=1 << 16)
+        assert ctx.fold_tiles() != {}
+    assert all(np.array_equal(a, b) for a, b in zip(got[:2], want[:2]))
+    # both are within SIM_TOL of the oracle
+    assert np.max(np.abs(got[2] - want[2])) <= 2 * SIM_TOL
+
+
+@pytest.mark.parametrize("precision", [cuapss.PREC_MIXED, cuapss.PREC_FP32], ids=["mixed", "fp32"])
+@pytest.mark.parametrize("sign", [False, True], ids=["unsigned", "signed"])
+def test_folded_sampled_query(precision, sign):
+    """Widths from samples, thresholds of their own, both sides signed or not."""
+    x = synth.generate("batch_instance", n=20_000, seed=8)
+    q = synth.generate("batch_instance", n=2000, seed=8, row_offset=19_000)
+    if sign:
+        x, q = _signed(x, 9), _signed(q, 10)
+    t = np.random.default_rng(12).uniform(0.5, 0.9, size=q.n).astype(np.float32)
+    with cuapss.Context(precision=precision) as ctx, cuapss.Index(ctx, x) as idx:
+        got = idx.query(q, t)
+        assert len(ctx.fold_tiles()) > 1
+    wi, wj, ws = oracle.join(q, x, 0.5)
+    keep = ws >= t[wi].astype(np.float64)
+    assert keep.sum() > 100
+    _check(got, (wi[keep], wj[keep], ws[keep]))
+
+
+@pytest.mark.parametrize("precision", [cuapss.PREC_MIXED, cuapss.PREC_FP32], ids=["mixed", "fp32"])
+def test_folded_unsampled_cross_join(precision):
+    x = synth.generate("batch_instance", n=9098, seed=3)
+    a, b = x.rows(0, 5001), x.rows(5001, 9098)
+    with cuapss.Context(precision=precision) as ctx:
+        got = ctx.join(a, b, 0.6, capacity=1 << 16)
+        assert sum(ctx.fold_tiles().values()) == 40 * 33
+    _check(got, oracle.join(a, b, 0.6))
