@@ -636,22 +636,20 @@ double passing_share(double len, int K, double t) {
 double mean_len(const DevCsr& x) { return (double)x.nnz / (double)std::max<int64_t>(x.n, 1); }
 
 // The wider levels whose sampled tiles take at most a tenth of the probing
-// path's fixed cost, where rows of kLongRows times the mean length have
-// candidates at the next narrower width that cost more than a tenth of its
-// tile. (Mixed joins of few thousand rows; 8,320 rows of 75 entries at t = 0.5
-// with nothing wider than 256 sampled: 1.47 ms, now 0.44; of 30 entries at
-// t = 0.7, where no wider one is useful: 0.35 with all sampled, 0.32. FP32
-// samples and small tiles cost more than the model says: 8,320 rows of 120 at t
-// = 0.8 2.05 -> 2.49 ms.)
-constexpr double kLongRows = 3.0;
+// path's fixed cost, where the long rows (kLongRows times the mean, kLongShare
+// of the pairs) have candidates at the next narrower width that cost more than
+// sampling another does. (Mixed joins of few thousand rows; 8,320 rows of 75
+// entries at t = 0.5 with nothing wider than 256 sampled: 1.47 ms, now 0.44; of
+// 30 entries at t = 0.7, where no wider one is useful: 0.35 with all sampled,
+// 0.32. FP32 samples and small tiles cost more than the model says: 8,320 rows
+// of 120 at t = 0.8 2.05 -> 2.49 ms.)
+constexpr double kLongRows = 3.0, kLongShare = 0.06, kWideSampleNs = 20e3;
 template <bool MIXED>
-uint32_t useful_levels(double len, double t) {
+uint32_t useful_levels(double len, double t, double pairs, int sms) {
   uint32_t use = sampled_levels<MIXED>(0.1 * kProbeFixedNs);
   for (int l = kSmallLevel + 1; l < kFoldLevels; ++l) {
     const double share = passing_share(kLongRows * len, fold_k(MIXED, l - 1), t);
-    if (share * kPair<MIXED> * kBlockRows * kBlockRows * cand_ns(len, share) <
-        0.1 * tile_cost<MIXED>(l - 1))
-      use &= ~(1u << l);
+    if (share * kLongShare * pairs * cand_ns(len, share) < kWideSampleNs * sms) use &= ~(1u << l);
   }
   return use;
 }
@@ -675,10 +673,12 @@ cuapss_status plan_levels(cuapss_ctx* ctx, FoldTask& k, const int32_t* perm, dou
   uint32_t all = 0;
   for (uint32_t m : J.levels) all |= m;
   // no more than a tenth of a small join
-  const double tiles_ns = (k.self ? 0.5 : 1.0) * I.nb * J.nb / kPair<MIXED> / ctx->sms *
-                          tile_cost<MIXED>(kSmallLevel);
-  all &= sampled_levels<MIXED>(0.1 * tiles_ns) |
-         (MIXED ? useful_levels<MIXED>(std::max(mean_len(I.x), mean_len(J.x)), k.t * k.t_min) : 0u);
+  const double tiles128 = (k.self ? 0.5 : 1.0) * I.nb * J.nb;
+  all &= sampled_levels<MIXED>(0.1 * tiles128 / kPair<MIXED> / ctx->sms *
+                               tile_cost<MIXED>(kSmallLevel)) |
+         (MIXED ? useful_levels<MIXED>(std::max(mean_len(I.x), mean_len(J.x)), k.t * k.t_min,
+                                       tiles128 * kBlockRows * kBlockRows, ctx->sms)
+                : 0u);
   auto temp = [&](const char* tag) {
     return [&ws, tag](const std::string& name, size_t bytes, void** out) {
       return ws.get(tag + name, bytes, out);
