@@ -584,3 +584,19 @@ def test_folded_unsampled_cross_join(precision):
         got = ctx.join(a, b, 0.6, capacity=1 << 16)
         assert sum(ctx.fold_tiles().values()) == 40 * 33
     _check(got, oracle.join(a, b, 0.6))
+
+
+@pytest.mark.parametrize("cfg,t", [("plain_800k", 0.5), ("batch_instance", 0.7)])
+def test_small_batch_widths(cfg, t):
+    """Small mixed batches sample wide rows only where the mean length calls for
+    them: rows of 75 entries and of 30."""
+    x = synth.generate(cfg, n=3000, seed=72)
+    ptr = np.array([0, 300, 1500, 3000], np.int64)
+    parts = [oracle.apss(x.rows(a, b), t) for a, b in zip(ptr, ptr[1:])]
+    want = [np.concatenate([p[k] + (a if k < 2 else 0) for a, p in zip(ptr, parts)])
+            for k in range(3)]
+    with cuapss.Context(precision=cuapss.PREC_MIXED) as ctx:
+        got = ctx.batch_run(x, ptr, np.full(3, t, np.float32), capacity=1 << 16)
+        if cfg == "batch_instance":
+            assert 0 < max(ctx.fold_tiles()) <= 256
+    _check(got, want)
